@@ -155,6 +155,14 @@ struct Handle {
     int live_tz = 0, live_ry = 0;
     bool live_valid = false;
 
+    // units of the resident-anatomy population kernel (rd_lanes.cu): which
+    // hold a live cell, the list of those with its length behind it, the
+    // length on the host, and the kernel's barrier words
+    unsigned char *unit_live = nullptr;
+    int *unit_list = nullptr;
+    int units = 0;
+    unsigned *lane_sync = nullptr;
+
     // events bracketing the latest population-kernel launch
     cudaEvent_t ev_pop[2] = {nullptr, nullptr};
     bool ev_pop_recorded = false;
@@ -273,6 +281,13 @@ int population_variant_name(int n, int vi, char *buf, int len);
 int check_device_status(Handle &h);
 int batch_solve_device(Handle &h, const gbg_sample *samples_device, int S,
                        const gbg_batch_opts &o, gbg_lik_result *loglik_device, long *nsteps_host);
+
+// ---- rd_lanes.cu ----
+// the live units of the anatomy; enqueues, h.units is valid once the stream is idle
+int lanes_set_anatomy(Handle &h);
+bool lanes_fit(const Handle &h, int S);
+// as population_steps with boxes, on records sorted by step count
+int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0);
 
 // ---- propagation.cu ----
 // batched solve of S samples, then per-cell mean and variance of their final

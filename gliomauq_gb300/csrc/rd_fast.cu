@@ -1103,6 +1103,7 @@ struct PopVariant {
     size_t smem;
     bool tb = false;  // two steps per round (start buffer per sample, see k_gaussian_ic)
     bool skip = false;  // visits only tiles that can be nonzero (needs the batched solver's set-up)
+    bool resident = false;  // the resident-anatomy kernel of rd_lanes.cu (ry, g, threads, tz for information)
     bool counts = false;  // counts the tiles it computes (gbg_last_population_cells)
     char name[64] = {0};  // kernel and template arguments, plus the tile depth
 };
@@ -1133,6 +1134,21 @@ PopVariant make_skip_variant(int tz) {
     v.skip = true;
     v.counts = true;
     std::snprintf(v.name, sizeof(v.name), "k_population10<%d,%d> TZ %d", LR, MINB, tz);
+    return v;
+}
+
+PopVariant make_resident_variant(int n) {
+    PopVariant v;
+    v.fn = nullptr;
+    v.ry = 2 * (128 / n);
+    v.g = 8;
+    v.threads = 512;
+    v.tz = 8;  // the tile depth of the slot kernel and of the fallback
+    v.smem = 0;
+    v.skip = true;
+    v.resident = true;
+    v.counts = true;
+    std::snprintf(v.name, sizeof(v.name), "k_population10<%d,4> resident", n / 4);
     return v;
 }
 
@@ -1183,6 +1199,7 @@ int variants_for(int n, PopVariant *out) {
     int k = 0;
     switch (n) {
         case 128:
+            out[k++] = make_resident_variant(128);
             out[k++] = make_skip_variant<32, 4>(8);
             out[k++] = make_skip_variant<32, 4>(16);
             out[k++] = make_signmask_variant<32, 4>(16);
@@ -1194,11 +1211,13 @@ int variants_for(int n, PopVariant *out) {
             out[k++] = make_ws_variant<32, 8, 3, 3>(32);
             break;
         case 64:
+            out[k++] = make_resident_variant(64);
             out[k++] = make_skip_variant<16, 4>(8);
             out[k++] = make_signmask_variant<16, 4>(16);
             out[k++] = make_signmask_variant<16, 5>(16);
             break;
         case 32:
+            out[k++] = make_resident_variant(32);
             out[k++] = make_skip_variant<8, 4>(8);
             out[k++] = make_signmask_variant<8, 4>(8);
             break;
@@ -1324,6 +1343,12 @@ int launch_population(Handle &h, float *buf0, float *buf1, const SampleRec *rec_
     // skipping shape's tile depth (the default one's otherwise)
     const int slot_tz = (h.pop_variant >= 0 && h.pop_variant < nv && vs[h.pop_variant].skip) ? vs[h.pop_variant].tz
                                                                                             : vs[0].tz;
+    if (!slot && vs[vi].resident) {
+        // an anatomy whose units do not fit the CTAs' shared memory (fewer SMs
+        // than a GB300 has) runs the tile march, the next variant
+        if (lanes_fit(h, S)) return lanes_launch(h, buf0, buf1, rec_sorted, S, box ? box : batch_boxes(h), grow0);
+        ++vi;
+    }
     const PopVariant v = slot ? slot_variant(h.n, box != nullptr, slot_tz) : vs[vi];
     PopArgs a;
     a.n = h.n;
@@ -1534,8 +1559,8 @@ int batch_prepare(Handle &h, int S, const gbg_batch_opts &o) {
     if (variant_is_skip(h)) {
         PopVariant vs[32];
         variants_for(h.n, vs);
-        const PopVariant &v = vs[h.pop_variant];
-        if (h.n % v.tz == 0 && h.n % v.ry == 0)
+        const PopVariant &v = vs[h.pop_variant + (vs[h.pop_variant].resident && !lanes_fit(h, S) ? 1 : 0)];
+        if (!v.resident && h.n % v.tz == 0 && h.n % v.ry == 0)
             if (int rc = ensure_live_tiles(h, v.ry, v.tz)) return rc;
     }
     if (o.with_loglik)

@@ -1,0 +1,455 @@
+// The skipping population kernel with resident anatomy (the batched solver's
+// default). A step of the tumour model needs 4 bytes of density and 16 bytes
+// of face coefficients per cell from the neighbourhood of that cell; the
+// tile-march kernel of rd_fast.cu advances every sample of a population once
+// per round and so streams both through L2 for each step (at 128^3 with 512
+// samples it ran at 0.67 of the HBM copy rate, and neither deeper staging nor
+// wider tiles moved it). Here nothing but the density moves:
+//   * The grid's live units (a unit: 2 rows per lane segment of one z-plane,
+//     full x-rows, holding at least one cell with the mask) are dealt once to
+//     the CTAs of a team, one CTA per SM. A CTA keeps the face coefficients of
+//     its units in shared memory for the whole launch (3.5 KB per unit: 93 KB
+//     at 128^3 on an ellipsoidal brain, 194 KB if every unit is live).
+//   * A team advances up to 8 samples side by side, one per "lane" of warps.
+//     A lane takes its sample through all its steps before the next one, so
+//     only the samples in flight are hot: 8 x 2 buffers of the live units fit
+//     in L2, and HBM sees a sample's first and last state only.
+//   * The lanes of a CTA are independent: each has its own barrier among the
+//     team's CTAs, and while one lane waits for its barrier (2.5 us from the
+//     last store to the release) the others have the SM.
+//   * A warp marches its share of units up z, two rows in registers, with the
+//     loads of the next planes in flight.
+// What bounds it: shared-memory and L1 bandwidth (28 of the 58 wavefronts a
+// unit costs are coefficients) and, for one sample, the barrier.
+// Per-cell operations and their order are those of march_tile_s (a difference
+// taken the other way round is its exact negative), so every population
+// kernel gives the same bits. Measured on a GB300, before (tile march) and
+// now: 512 prior draws at 128^3 243 -> 164 ms; 64 draws near the mode, stable
+// grid, 14.0 -> 10.0 ms; one of them 1.01 -> 0.61 ms; 512 at 64^3 53 -> 26 ms.
+#include <algorithm>
+
+#include "gbg_internal.cuh"
+
+namespace gbg {
+namespace {
+
+constexpr int kWps = 4;                    // warps per scheduler: 16 warps of up to 128 registers
+constexpr int kThreads = 128 * kWps;
+// Samples a team has in flight. More lanes hide more of the barrier (4: 205
+// ms, 8: 164 ms on the 512-sample population); beyond 8 the states of a 128^3
+// population outgrow L2.
+constexpr int kMaxLanes = 8;
+// a unit's table, one float4 per lane and slot: cxs (2 rows), cy (rows y-1,
+// y, y+1), cz (2 rows)
+constexpr int kSlots = 7;
+constexpr size_t kUnitBytes = (size_t)kSlots * 32 * sizeof(float4);
+constexpr int kMaxUnits = 64;              // units a CTA can own
+// Planes loaded ahead: one plane's arithmetic does not cover an L2 load (170
+// ms), a third plane spills registers (207 ms).
+constexpr int kAhead = 2;
+constexpr int kSyncStride = 32;            // words per lane of the barrier array
+
+__device__ __forceinline__ int wrapm(int i, int n) { return i == 0 ? n - 1 : i - 1; }
+__device__ __forceinline__ int wrapp(int i, int n) { return i == n - 1 ? 0 : i + 1; }
+
+struct LaneArgs {
+    int S, T, teams, lanes, warps;
+    int nlive, units, grow0;
+    size_t stride;
+    float *buf0, *buf1;
+    const float *cxs, *cy, *cz;
+    const SampleRec *rec;
+    const int *list;
+    const unsigned char *live;
+    const int *box;
+    unsigned *sync;   // queue counter, then per lane: arrivals, next sample (two slots)
+    int *status;
+    unsigned long long *visited;
+};
+
+// what a lane's warps share of the sample they are on
+struct Sample {
+    SampleRec rec;
+    int ylo, yhi, zlo, zhi;
+    int next, ok;
+    unsigned target, slot;
+};
+
+__device__ __forceinline__ bool span_hits(int lo, int hi, int grow, int a, int b, int n) {
+    lo -= grow;
+    hi += grow;
+    if (lo < 0 || hi > n - 1) return true;
+    return lo <= b && a <= hi;
+}
+
+__device__ __forceinline__ void group_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release(unsigned *p) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(p) : "memory");
+}
+
+struct V4 {
+    float v[4];
+};
+__device__ __forceinline__ V4 v4(const float4 &a) { return V4{{a.x, a.y, a.z, a.w}}; }
+__device__ __forceinline__ V4 ldp(const float *p) { return v4(*reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ V4 ldg4(const float *p) { return v4(__ldg(reinterpret_cast<const float4 *>(p))); }
+__device__ __forceinline__ V4 lds(const float4 *p) { return v4(*p); }
+__device__ __forceinline__ V4 sub(const V4 &a, const V4 &b) {
+    return V4{{a.v[0] - b.v[0], a.v[1] - b.v[1], a.v[2] - b.v[2], a.v[3] - b.v[3]}};
+}
+
+// One row of four cells. DS = sS * (row(y-1) - P), DT = row(y+1) - P,
+// DB = P - plane(z-1), DF = plane(z+1) - P.
+template <int LR>
+__device__ __forceinline__ float4 row_step(const V4 &P, const V4 &DS, float sS, const V4 &DT, const V4 &DB, const V4 &DF, const V4 &CX,
+                                           const V4 &CYm, const V4 &CY, const V4 &CZp, const V4 &CZ, int li, float a, float b) {
+    const float right = __shfl_sync(0xffffffffu, P.v[0], (li + 1) % LR, LR);
+    const float d[4] = {P.v[1] - P.v[0], P.v[2] - P.v[1], P.v[3] - P.v[2], right - P.v[3]};
+    // the left face of cell 0 is the right face of the lane before: the same
+    // two cells' difference times the same coefficient
+    const float flux = __shfl_sync(0xffffffffu, fabsf(CX.v[3]) * d[3], (li + LR - 1) % LR, LR);
+    float o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float f0 = P.v[i];
+        float lap = i ? -fabsf(CX.v[i - 1]) * d[i - 1] : -flux;
+        lap = fmaf(fabsf(CX.v[i]), d[i], lap);
+        lap = fmaf(sS * CYm.v[i], DS.v[i], lap);
+        lap = fmaf(CY.v[i], DT.v[i], lap);
+        lap = fmaf(-CZp.v[i], DB.v[i], lap);
+        lap = fmaf(CZ.v[i], DF.v[i], lap);
+        const float v = fmaf(a, lap, f0);
+        o[i] = __saturatef(fmaf(b * f0, 1.0f - f0, v));
+        o[i] = signbit(CX.v[i]) ? 0.0f : o[i];
+    }
+    return make_float4(o[0], o[1], o[2], o[3]);
+}
+
+// Planes z .. z + len - 1 of the row pair y, y + 1. tab: the first unit's
+// table at this lane.
+template <int LR>
+__device__ __forceinline__ void march(const float4 *__restrict__ tab, int y, int z, int len, const float *__restrict__ in,
+                                      float *__restrict__ out, const float *__restrict__ cz, float a, float b) {
+    constexpr int n = 4 * LR, plane = n * n;
+    const int li = (threadIdx.x & 31) % LR;
+    const int o0 = 4 * li + n * y + plane * z, below = z == 0 ? plane * (n - 1) : -plane;
+    const float *pN = in + o0;  // the plane last loaded as "next"
+    int dS = y == 0 ? n * (n - 1) : -n, dT = y + 2 == n ? -n * (n - 2) : 2 * n;
+    out += o0;
+    struct Slot {
+        V4 n0, n1, s, t;
+    } sl[kAhead];
+    int zn = z;
+    // loads of plane zn's y neighbours and of the rows above it
+    auto load = [&](Slot &q) {
+        q.s = ldp(pN + dS);
+        q.t = ldp(pN + dT);
+        pN += ++zn == n ? -plane * (n - 1) : plane;
+        q.n0 = ldp(pN);
+        q.n1 = ldp(pN + n);
+    };
+    V4 P0 = ldp(pN), P1 = ldp(pN + n), B0 = ldp(pN + below), B1 = ldp(pN + below + n);
+    B0 = sub(P0, B0);
+    B1 = sub(P1, B1);
+    V4 C0 = ldg4(cz + o0 + below), C1 = ldg4(cz + o0 + below + n);
+#pragma unroll
+    for (int d = 0; d < kAhead; ++d)
+        if (d < len) load(sl[d]);
+    for (int j = 0; j < len; j += kAhead) {
+#pragma unroll
+        for (int d = 0; d < kAhead; ++d) {
+            if (j + d >= len) break;
+            const V4 Z0 = lds(tab + 5 * 32), Y1 = lds(tab + 3 * 32);
+            const V4 DY = sub(P1, P0), F0 = sub(sl[d].n0, P0), F1 = sub(sl[d].n1, P1);
+            *reinterpret_cast<float4 *>(out) = row_step<LR>(P0, sub(sl[d].s, P0), 1.f, DY, B0, F0, lds(tab), lds(tab + 2 * 32), Y1, C0,
+                                                            Z0, li, a, b);
+            __syncwarp();
+            const V4 Z1 = lds(tab + 6 * 32);
+            *reinterpret_cast<float4 *>(out + n) = row_step<LR>(P1, DY, -1.f, sub(sl[d].t, P1), B1, F1, lds(tab + 32), Y1,
+                                                                lds(tab + 4 * 32), C1, Z1, li, a, b);
+            __syncwarp();
+            B0 = F0;
+            B1 = F1;
+            P0 = sl[d].n0;
+            P1 = sl[d].n1;
+            C0 = Z0;
+            C1 = Z1;
+            out += plane;
+            tab += kSlots * 32;
+            if (j + d + kAhead < len) load(sl[d]);
+        }
+    }
+}
+
+template <int LR, int WPS>
+__global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
+    constexpr int n = 4 * LR, SUB = 32 / LR, ROWS = 2 * SUB;
+    extern __shared__ __align__(16) float4 tab[];
+    __shared__ int s_unit[kMaxUnits];  // y0 | z << 10 | length of the run of planes from here on << 20
+    __shared__ Sample s_smp[kMaxLanes];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, li = lane % LR, sub_r = lane / LR;
+    const int team = blockIdx.x / p.T, rank = blockIdx.x % p.T;
+    // this CTA's units: two stretches of the list, half the list apart
+    const int q0 = (int)((long)p.nlive * rank / (2 * p.T)), c0 = (int)((long)p.nlive * (rank + 1) / (2 * p.T)) - q0;
+    const int q1 = (int)((long)p.nlive * (rank + p.T) / (2 * p.T)), c1 = (int)((long)p.nlive * (rank + p.T + 1) / (2 * p.T)) - q1;
+    const int nu = c0 + c1;
+    auto unit_at = [&](int i) { return p.list[i < c0 ? q0 + i : q1 + i - c0]; };  // yu * n + z
+    for (int i = threadIdx.x; i < nu; i += 128 * WPS) {
+        const int u = unit_at(i), end = i < c0 ? c0 : nu;
+        int run = 1;
+        while (i + run < end && unit_at(i + run) == u + run && (u + run) % n != 0) ++run;
+        s_unit[i] = (u / n) * ROWS | (u % n) << 10 | run << 20;  // all below 1024
+    }
+    // the units' face coefficients, one float4 per lane and slot
+    for (int q = warp; q < nu * kSlots; q += 4 * WPS) {
+        const int u = unit_at(q / kSlots), c = q % kSlots, z = u % n;
+        int y = (u / n) * ROWS + 2 * sub_r + (c < 2 ? c : (c < 5 ? c - 3 : c - 5));
+        y = y < 0 ? n - 1 : y;
+        const float *src = c < 2 ? p.cxs : (c < 5 ? p.cy : p.cz);
+        tab[q * 32 + lane] = *reinterpret_cast<const float4 *>(src + 4 * li + (size_t)n * (y + (size_t)n * z));
+    }
+    __syncthreads();
+    const int g = warp / p.warps, w = warp % p.warps;
+    if (g >= p.lanes) return;  // named barriers only from here on
+    Sample &sm = s_smp[g];
+    const int tl = g * p.teams + team;
+    if (w == 0 && lane == 0) {
+        sm.next = tl;
+        sm.target = 0;
+        sm.ok = 1;
+        sm.slot = 0;
+    }
+    unsigned visited = 0;
+    for (;;) {
+        group_sync(1 + g, 32 * p.warps);
+        const int r = sm.next;
+        if (r >= p.S || !sm.ok) break;
+        if (w == 0 && lane == 0) {
+            sm.rec = p.rec[r];
+            const int4 bx = reinterpret_cast<const int4 *>(p.box)[sm.rec.order];
+            sm.ylo = n - bx.x;
+            sm.yhi = bx.y - 1;
+            sm.zlo = n - bx.z;
+            sm.zhi = bx.w - 1;
+            if (bx.y == 0) sm.rec.a = -1.f;  // no nonzero initial cell: the sample stays 0
+        }
+        group_sync(1 + g, 32 * p.warps);
+        const int nsteps = sm.rec.nsteps;
+        if (nsteps <= 0) break;  // sorted: so are all that follow
+        for (int k = 0; k < nsteps; ++k) {
+            {
+                const size_t off = (size_t)sm.rec.order * p.stride;
+                const float *in = ((k & 1) ? p.buf1 : p.buf0) + off;
+                float *out = ((k & 1) ? p.buf0 : p.buf1) + off;
+                const bool lastk = k == nsteps - 1;
+                const float a = lastk ? sm.rec.a2 : sm.rec.a, b = lastk ? sm.rec.b2 : sm.rec.b;
+                const bool any = sm.rec.a >= 0.f;
+                const int grow = p.grow0 + k + 1, u1 = nu * (w + 1) / p.warps;
+                for (int i = nu * w / p.warps; any && i < u1;) {
+                    const int un = s_unit[i], y0 = un & 1023, z = un >> 10 & 1023, len = min(un >> 20, u1 - i);
+                    int za = z, zb = z + len;
+                    if (sm.zlo >= grow && sm.zhi + grow < n) {
+                        za = max(za, sm.zlo - grow);
+                        zb = min(zb, sm.zhi + grow + 1);
+                    }
+                    if (za < zb && span_hits(sm.ylo, sm.yhi, grow, y0, y0 + ROWS - 1, n)) {
+                        march<LR>(tab + (i + za - z) * kSlots * 32 + lane, y0 + 2 * sub_r, za, zb - za, in, out, p.cz, a, b);
+                        visited += zb - za;
+                    }
+                    i += len;
+                }
+                if (k == 1 && any) {
+                    // units without a live cell that the initial state may have
+                    // left values in: zeros, as their step gives
+                    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int u = rank + p.T * w; u < p.units; u += p.T * p.warps) {
+                        const int y0 = (u / n) * ROWS, z = u % n;
+                        if (p.live[u] || !span_hits(sm.ylo, sm.yhi, p.grow0, y0, y0 + ROWS - 1, n) ||
+                            !span_hits(sm.zlo, sm.zhi, p.grow0, z, z, n))
+                            continue;
+                        float *o = out + 4 * li + (size_t)n * (y0 + 2 * sub_r + (size_t)n * z);
+                        *reinterpret_cast<float4 *>(o) = z4;
+                        *reinterpret_cast<float4 *>(o + n) = z4;
+                    }
+                }
+            }
+            // barrier of the team's CTAs on this lane
+            group_sync(1 + g, 32 * p.warps);
+            if (w == 0 && lane == 0) {
+                unsigned *sync = p.sync + (size_t)(tl + 1) * kSyncStride;
+                const bool lastk = k == nsteps - 1;
+                const unsigned target = sm.target + p.T;
+                if (lastk && rank == 0) {
+                    const unsigned nx = atomicAdd(p.sync, 1u) + (unsigned)(p.teams * p.lanes);
+                    *(volatile unsigned *)(sync + 1 + sm.slot) = nx;
+                }
+                red_release(sync);
+                long long spins = 0;
+                while (ld_acquire(sync) < target) {
+                    if (++spins > (1ll << 24)) {  // seconds
+                        atomicExch(p.status, (int)DEV_BARRIER_TIMEOUT);
+                        sm.ok = 0;
+                        break;
+                    }
+                    if ((spins & 1023) == 0 && *(volatile int *)p.status != DEV_OK) {
+                        sm.ok = 0;
+                        break;
+                    }
+                }
+                sm.target = target;
+                if (lastk) {
+                    sm.next = (int)*(volatile unsigned *)(sync + 1 + sm.slot);
+                    sm.slot ^= 1u;
+                }
+            }
+            if (k == nsteps - 1) break;
+            group_sync(1 + g, 32 * p.warps);
+            if (!sm.ok) break;
+        }
+    }
+    if (lane == 0 && visited) atomicAdd(p.visited, (unsigned long long)visited);
+}
+
+// live[u] = unit u (2 rows per lane segment, one plane, full x-rows; u = row
+// group * n + plane) has a cell that is tissue with six tissue neighbours (the
+// fast tables' mask)
+__global__ void k_unit_live(int n, int rows, const double *__restrict__ pw, const double *__restrict__ pg,
+                            unsigned char *__restrict__ live) {
+    const int y0 = (blockIdx.x / n) * rows, z = blockIdx.x % n;
+    int any = 0;
+    for (int i = threadIdx.x; i < n * rows; i += blockDim.x) {
+        const int x = i % n, y = y0 + i / n;
+        auto t = [&](int xx, int yy, int zz) {
+            const size_t c = xx + (size_t)n * (yy + (size_t)n * zz);
+            return pw[c] + pg[c] > 0.0;
+        };
+        any |= t(x, y, z) && t(wrapm(x, n), y, z) && t(wrapp(x, n), y, z) && t(x, wrapm(y, n), z) && t(x, wrapp(y, n), z) &&
+               t(x, y, wrapm(z, n)) && t(x, y, wrapp(z, n));
+    }
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) live[blockIdx.x] = (unsigned char)(any != 0);
+}
+
+// indices of the live units in increasing order, and their count (one CTA)
+__global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned char *__restrict__ live, int *__restrict__ list,
+                                                     int *__restrict__ count) {
+    __shared__ int sums[32];
+    __shared__ int total;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    for (int base = 0; base < units; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int f = i < units && live[i];
+        const unsigned m = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) sums[warp] = __popc(m);
+        __syncthreads();
+        int before = total;
+        for (int k = 0; k < warp; ++k) before += sums[k];
+        if (f) list[before + __popc(m & ((1u << lane) - 1u))] = i;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 32; ++k) total += sums[k];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *count = total;
+}
+
+int unit_rows(int n) { return 2 * (32 / (n / 4)); }
+int units_of(int n) { return (n / unit_rows(n)) * n; }
+}  // namespace
+
+int lanes_set_anatomy(Handle &h) {
+    if (!population_supported(h.n)) return GBG_OK;
+    const int nu = units_of(h.n);
+    if (!h.unit_live) {
+        GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_live, nu));
+        GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_list, (nu + 1) * sizeof(int)));
+        GBG_CUDA_TRY(cudaMalloc((void **)&h.lane_sync, (size_t)(h.num_sms * kMaxLanes + 1) * kSyncStride * sizeof(unsigned)));
+    }
+    k_unit_live<<<nu, 128, 0, h.stream>>>(h.n, unit_rows(h.n), h.pw, h.pg, h.unit_live);
+    k_unit_list<<<1, 1024, 0, h.stream>>>(nu, h.unit_live, h.unit_list, h.unit_list + nu);
+    h.launches += 2;
+    GBG_CUDA_TRY(cudaGetLastError());
+    GBG_CUDA_TRY(cudaMemcpyAsync(&h.units, h.unit_list + nu, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+    return GBG_OK;
+}
+
+// Teams and lanes for S samples. A CTA holds at most 28 units where the chip
+// allows it (more: 30.1 against 26.3 ms at 52 units for 512 samples at 64^3,
+// fewer: 32.2 ms at 14, the lanes then idle at their barriers). Where samples
+// are few the teams grow until 8 lanes each cover them, down to 4 units per
+// CTA, below which a step is all barrier (6 samples at 32^3: 1.71 ms at 28
+// units, 1.42 ms at 4; 32 at 64^3: 4.9 ms at 28, 4.0 ms at 14).
+static void lane_shape(const Handle &h, int S, LaneArgs &a, int &units) {
+    const int nl = std::max(1, h.units), sms = h.num_sms;
+    const int wide = sms / ((S + kMaxLanes - 1) / kMaxLanes), least = (nl + 27) / 28, most = (nl + 3) / 4;
+    a.T = std::min(sms, std::max(least, std::min(wide, most)));
+    a.teams = sms / a.T;
+    a.T = sms / a.teams;
+    a.teams = std::min(a.teams, S);
+    a.lanes = std::min(kMaxLanes, (S + a.teams - 1) / a.teams);
+    a.warps = 4 * kWps / a.lanes;
+    units = 2 * ((nl + 2 * a.T - 1) / (2 * a.T));
+}
+
+bool lanes_fit(const Handle &h, int S) {
+    LaneArgs a;
+    int units;
+    if (!h.unit_list) return false;
+    lane_shape(h, S, a, units);
+    // the rest of the 227 KB is the kernel's static shared memory
+    return units <= kMaxUnits && units * kUnitBytes <= 224 * 1024;
+}
+
+int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0) {
+    const int n = h.n;
+    LaneArgs a;
+    int units;
+    lane_shape(h, S, a, units);
+    a.S = S;
+    a.nlive = h.units;
+    a.units = units_of(n);
+    a.grow0 = grow0;
+    a.stride = h.N;
+    a.buf0 = buf0;
+    a.buf1 = buf1;
+    a.cxs = h.cxs;
+    a.cy = h.cy;
+    a.cz = h.cz;
+    a.rec = sorted;
+    a.list = h.unit_list;
+    a.live = h.unit_live;
+    a.box = box;
+    a.sync = h.lane_sync;
+    a.status = h.dev_status;
+    a.visited = reinterpret_cast<unsigned long long *>(h.barrier + 2);
+    const size_t smem = units * kUnitBytes;
+    const void *fn = n == 128  ? (const void *)k_population10<32, kWps>
+                     : n == 64 ? (const void *)k_population10<16, kWps>
+                               : (const void *)k_population10<8, kWps>;
+    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBG_CUDA_TRY(cudaMemsetAsync(h.barrier, 0, 4 * sizeof(unsigned), h.stream));
+    GBG_CUDA_TRY(
+        cudaMemsetAsync(h.lane_sync, 0, (size_t)(a.teams * a.lanes + 1) * kSyncStride * sizeof(unsigned), h.stream));
+    h.pop_tile_cells = (long long)unit_rows(n) * n;
+    void *args[] = {&a};
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GBG_CUDA_TRY(cudaStreamIsCapturing(h.stream, &cap));
+    const unsigned evf = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
+    GBG_CUDA_TRY(cudaEventRecordWithFlags(h.ev_pop[0], h.stream, evf));
+    GBG_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3((unsigned)(a.teams * a.T)), dim3(kThreads), args, smem, h.stream));
+    GBG_CUDA_TRY(cudaEventRecordWithFlags(h.ev_pop[1], h.stream, evf));
+    h.ev_pop_recorded = true;
+    h.launches++;
+    return GBG_OK;
+}
+
+}  // namespace gbg

@@ -1,0 +1,53 @@
+"""GPU: the resident-anatomy population kernel (the batched solver's default)
+against the dense register kernel, bit for bit, at the edges of its division
+of work: sample counts around a team's lanes, anatomies with no live cell, one
+live plane, every cell live (the most units a CTA can own; stencils across
+every periodic face) and scattered tissue (short runs of planes)."""
+import numpy as np
+import pytest
+
+from gliomauq_gb300 import _lib, synthetic as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _tissue(kind, n, rng):
+    if kind == "ellipsoid":
+        an = S.make_anatomy(n, seed=2)
+        return an.p_w, an.p_g
+    t = np.zeros((n, n, n))
+    if kind == "full":
+        t[:] = 1.0
+    elif kind == "one plane":
+        t[5:8] = 1.0  # live: plane 6, in every row
+    elif kind == "scattered":
+        t[rng.random((n, n, n)) < 0.93] = 1.0
+        t[:, ::7] = 0.0
+    w = rng.random((n, n, n))
+    return t * w, t * (1.0 - w)
+
+
+@pytest.mark.parametrize("n", [32, 64, 128])
+@pytest.mark.parametrize("kind,count", [("ellipsoid", 1), ("ellipsoid", 9), ("ellipsoid", 75), ("full", 3), ("full", 17),
+                                        ("one plane", 5), ("scattered", 10), ("none", 2)])
+def test_resident_kernel_equals_dense(gbg, n, kind, count):
+    rng = np.random.default_rng(n + count)
+    pw, pg = _tissue(kind, n, rng)
+    dt = S.reference_dt(n, 0.0013, n * 0.1)[0]
+    smp = [(0.0013 * rng.uniform(0.3, 1.5), rng.uniform(0.01, 0.2), *rng.uniform(0, n - 1, 3), dt * rng.uniform(-1, 30))
+           for _ in range(count)]
+    with _lib.Handle(n, "f32", max_samples=count) as h:
+        h.set_anatomy(pw, pg)
+        names = [h.population_variant_name(i) for i in range(len(h.population_variants()))]
+        dense = [i for i, nm in enumerate(names) if nm.startswith("k_population8<")][0]
+        assert names[0].endswith("resident")
+        for sigma, dt0 in ((1.0, 0.0), (0.3 * n, -0.75)):
+            out = []
+            for v in (dense, 0):
+                h.set_population_variant(v)
+                out.append(h.batch_solve(smp, n * 0.1, ic_sigma=sigma, with_loglik=False, want_phi=True, dt0=dt0))
+                cells = h.last_population_cells()
+                assert 0 <= cells <= int(np.sum(out[-1]["nsteps"])) * n ** 3
+            assert np.array_equal(out[0]["nsteps"], out[1]["nsteps"])
+            for j in range(count):
+                assert np.array_equal(out[0]["phi"][j], out[1]["phi"][j]), (sigma, j)
