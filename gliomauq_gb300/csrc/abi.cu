@@ -1172,7 +1172,7 @@ int gbg_surrogate_loglik(gbg_surrogate *s, const gbg_sample *samples, int B, gbg
         return GBG_ERR_ARG;
     }
     GBG_CUDA_TRY(cudaMemcpyAsync(d, samples, B * sizeof(gbg_sample), cudaMemcpyHostToDevice, h.stream));
-    if (int rc = gbg::surrogate_predict(*s->s, d, B, (gbg_lik_result *)h.lik_out)) return rc;
+    if (int rc = gbg::surrogate_predict(*s->s, d, B, (gbg_lik_result *)h.lik_out, phi != nullptr)) return rc;
     GBG_CUDA_TRY(cudaMemcpyAsync(out, h.lik_out, B * sizeof(gbg_lik_result), cudaMemcpyDeviceToHost, h.stream));
     if (phi)
         GBG_CUDA_TRY(cudaMemcpyAsync(phi, gbg::surrogate_prediction(*s->s), (size_t)B * h.N * sizeof(float), cudaMemcpyDeviceToHost,

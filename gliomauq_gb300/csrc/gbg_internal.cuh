@@ -335,7 +335,7 @@ int surrogate_loss_grad(Surrogate &s, const gbg_sample *samples, int B, const fl
 int surrogate_features(Surrogate &s, const gbg_sample *samples, int B, float *out);
 int surrogate_train(Surrogate &s, const gbg_sample *samples, int S, int epochs, int batch, double lr,
                     unsigned long long seed, double *loss_out);
-int surrogate_predict(Surrogate &s, const gbg_sample *samples_device, int B, gbg_lik_result *lik_device);
+int surrogate_predict(Surrogate &s, const gbg_sample *samples_device, int B, gbg_lik_result *lik_device, bool want_field);
 
 // ---- likelihood.cu ----
 int lik_set_observations(Handle &h, const double *pet, const double *t1, const double *t2,
@@ -343,6 +343,9 @@ int lik_set_observations(Handle &h, const double *pet, const double *t1, const d
 // phi_f32 or phi_f64 (one non-null): S fields of N cells at stride N.
 int lik_evaluate(Handle &h, const float *phi_f32, const double *phi_f64, int S,
                  gbg_lik_result *out_device);
+// of B fields on a grid of half the handle's n: cell (x, y, z) reads
+// (x/2, y/2, z/2), 0 where mask (n^3) is 0
+int lik_evaluate_coarse(Handle &h, const float *fields, const float *mask, int B, gbg_lik_result *out_device);
 // population: sample s's final field is in buf[recs[s].nsteps & 1] + s*N.
 // log L of B affine models evaluated at the observation cells only
 // (delta_device: B x P; cols: likelihood.cu's AffineSource layout)

@@ -82,6 +82,19 @@ struct AffineSource {
     }
 };
 
+// phi of field s on a grid of half the resolution: cell (x, y, z) of the n^3
+// grid reads (x/2, y/2, z/2), 0 outside the mask.
+struct CoarseSource {
+    const float *f, *mask;
+    int n;
+    __device__ __forceinline__ double at(int s, int c) const {
+        const int m = n / 2, x = c % n, y = c / n % n, z = c / (n * n);
+        return mask[c] != 0.f ? (double)f[((size_t)s * m * m * m) + ((z / 2) * m + y / 2) * m + x / 2] : 0.0;
+    }
+    __device__ __forceinline__ double pet(const LikArgs &a, int s, int i) const { return at(s, a.pet_idx[i]); }
+    __device__ __forceinline__ double ti(const LikArgs &a, int s, int i) const { return at(s, a.ti_idx[i]); }
+};
+
 template <class Src>
 __global__ void __launch_bounds__(kLikThreads) k_lik_partial(LikArgs a, Src src) {
     const int s = blockIdx.y;
@@ -275,6 +288,11 @@ int lik_evaluate(Handle &h, const float *phi_f32, const double *phi_f64, int S,
 int lik_evaluate_affine(Handle &h, const float *cols, int P, const double *delta_device, int B,
                         gbg_lik_result *out_device) {
     AffineSource src{cols, cols + (size_t)(P + 2) * h.obs.n_pet, delta_device, P};
+    return run_lik(h, src, B, out_device);
+}
+
+int lik_evaluate_coarse(Handle &h, const float *fields, const float *mask, int B, gbg_lik_result *out_device) {
+    CoarseSource src{fields, mask, h.n};
     return run_lik(h, src, B, out_device);
 }
 

@@ -1,9 +1,10 @@
 // Learned surrogate of the forward solve: a small 3D convolutional U-Net,
 // trained and evaluated with the kernels in this file. Forward and
-// data-gradient convolutions run on tcgen05 (k_conv_fwd_tc) by default, or
-// on mma.sync tiles (k_conv_fwd); the weight gradient on mma.sync over
-// staged tiles (k_conv_wgrad_tiled: its GEMM has M, N = channels <= 64 and
-// K = voxels, below tcgen05's smallest M of 64).
+// data-gradient convolutions run on tcgen05 by default (k_conv_march; grids
+// not divisible into its tiles gather per tap, k_conv_fwd_tc), or on mma.sync
+// tiles (k_conv_fwd); the weight gradient on mma.sync over staged planes
+// (k_conv_wgrad_tiled: its GEMM has M, N = channels <= 64 and K = voxels, below
+// tcgen05's smallest M of 64).
 //
 // Tensors are channels-last, [batch][z][y][x][channel], bf16 activations and
 // weights with fp32 accumulation; a layer reads or writes a channel slice
@@ -346,46 +347,81 @@ __global__ void __launch_bounds__(128) k_conv_fwd_tc(Geom g, Slice in, int Cin, 
                      : "memory");
 }
 
-// Halo-tile variant (grids with W % 8 == 0 and H % 16 == 0): an output tile
-// is 8 (x) x 16 (y) voxels of one z-plane of one sample, M = 128 rows ordered
-// x-fastest. Its input halo, 10 (x) x 18 (y) x 3 (z) voxels, is loaded into
-// shared memory once, one array per 8-channel chunk, voxels x-fastest at 16
-// bytes each: 8 consecutive x-voxels of a chunk are one 128-byte core matrix.
-// The A operand of tap (dx, dy, dz) is then a descriptor into the halo tile
-// (start = the tap's offset, stride byte offset = one halo row = 160 B,
-// leading byte offset = one chunk array), so all 27 Cin / 16 MMAs of a tile
-// are issued back to back without gathering.
+// Marching variant (grids with W % 8 == 0 and H % 16 == 0). A CTA takes a
+// column of output tiles, 8 (x) x 16 (y) voxels = 128 MMA rows ordered x-fastest,
+// through zc planes. An input plane (10 x 18 voxels with its halo,
+// one array per 8-channel chunk, voxels x-fastest at 16 bytes: 8 consecutive
+// x-voxels of a chunk are one 128-byte core matrix) comes into a ring of stages
+// by cp.async, zero-filled off the grid, and serves all three output planes it
+// touches at once: tap (dx, dy) is a descriptor into the plane, and the
+// weights of dz = +1, 0, -1 are the N = 3 Cout columns of one operand, so that
+// an A tile is read from shared memory once for 3 Cout columns. The
+// accumulators of the output planes are a ring of 4 blocks of Cout tensor
+// memory columns. An output's terms arrive in the order (dz, dy, dx,
+// channels).
+// What bounds it: the A operand's shared-memory reads (4 KB per 128 x 16
+// chunk; the MMA itself is shorter below 64 columns) and the activations'
+// HBM traffic. Staging the 3-plane halo anew for every tile, one tap of one
+// dz per MMA and all index arithmetic per element, took 2.3 ms for the 16 ->
+// 16 layer on 64 samples of 64^3 (1.07 GB in and out); this takes 0.39 ms (six
+// CTAs per SM; with one it takes 2.0 ms, and 0.49 ms when the thread that issues
+// the MMAs also moves data).
 namespace tc {
-constexpr int HX = 10, HY = 18, HZ = 3;
-constexpr int HALO_CHUNK = HX * HY * HZ * 16;  // bytes per 8-channel chunk array (8640)
-inline size_t halo_smem_bytes(int Cin, int N) {  // weights, two halo buffers, barrier, tmem slot
-    return (size_t)(27 * Cin / 16) * N * 32 + 2 * (size_t)(Cin / 8) * HALO_CHUNK + 8 * 2 + 16;
+constexpr int HX = 10, HY = 18, HV = HX * HY;
+constexpr int PLANE_CHUNK = HV * 16;  // bytes per 8-channel chunk of a plane (2880)
+constexpr int kRing = 4;              // accumulator blocks
+__host__ __device__ constexpr int stages(int C8) { return C8 > 4 ? 2 : 4; }
+__host__ __device__ constexpr size_t march_smem(int C8, int N) {  // weights, stages, barriers, tmem slot
+    return (size_t)(27 * C8 / 2) * N * 32 + (size_t)stages(C8) * C8 * PLANE_CHUNK + 8 * 2 + 16;
+}
+// CTAs per SM: by shared memory (228 KB, 1 KB of it reserved per CTA) and tensor
+// memory columns
+__host__ __device__ constexpr int march_ctas(int C8, int N) {
+    const int a = (int)(228 * 1024 / (march_smem(C8, N) + 1024)), b = 512 / (kRing * N);
+    return a < b ? a : b;
+}
+__device__ __forceinline__ void cp16(unsigned dst, const void *src, unsigned bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 }  // namespace tc
 
-template <int N>
-__global__ void __launch_bounds__(128) k_conv_fwd_tc_halo(Geom g, Slice in, int Cin, const __nv_bfloat16 *__restrict__ w,
-                                                          const float *__restrict__ bias, Slice out,
-                                                          float *__restrict__ out_f32, int relu, int *status) {
+struct ConvOut {
+    Slice out;          // bf16 channels (p null: none)
+    float *first;       // channel 0 of each voxel in fp32 (null: none)
+    const float *bias;  // null: none
+    int relu;
+    Slice gate;         // p non-null: zero where this slice is not positive (ReLU backward)
+};
+
+// Warps 0-3 load and store (a row of the tile per thread), warp 4 issues the MMAs.
+template <int C8, int N>
+__global__ void __launch_bounds__(160, tc::march_ctas(C8, N)) k_conv_march(Geom g, int zc, Slice in, const __nv_bfloat16 *__restrict__ w, ConvOut o,
+                                                    int *status) {
+    constexpr int CIN = 8 * C8, CC = C8 / 2, K = 27 * CIN, S = tc::stages(C8), BLK = (N / 8) * 256;
+    constexpr int ENT = (C8 * tc::HV + 127) / 128;  // 16-byte pieces of a plane per thread
+    constexpr unsigned STAGE = C8 * tc::PLANE_CHUNK;
     extern __shared__ __align__(1024) unsigned char sm[];
-    const int K = 27 * Cin, KC = K / 16, CC = Cin / 16, C8 = Cin / 8;
-    unsigned char *Bs = sm;                                   // KC chunks of N x 16 bf16
-    unsigned char *Hs = sm + (size_t)KC * N * 32;             // two halo tiles of C8 chunk arrays
-    unsigned long long *bars = reinterpret_cast<unsigned long long *>(Hs + 2 * (size_t)C8 * tc::HALO_CHUNK);
+    unsigned char *Bs = sm;
+    unsigned char *As = sm + (size_t)(27 * C8 / 2) * N * 32;
+    unsigned long long *bars = reinterpret_cast<unsigned long long *>(As + (size_t)S * STAGE);
     unsigned *tslot = reinterpret_cast<unsigned *>(bars + 2);
     const int tid = threadIdx.x, warp = tid >> 5;
-    for (int pc = tid; pc < N * (K / 8); pc += 128) {
-        const int n = pc / (K / 8), k8 = pc % (K / 8);
-        unsigned char *dst = Bs + (size_t)(k8 >> 1) * N * 32 + (n >> 3) * 256 + (k8 & 1) * 128 + (n & 7) * 16;
+    const bool issuer = tid == 128, mover = tid < 128;
+    // weights: K-chunk (dy, dx, cc) of 3 N rows, row block b = dz + ... 0: dz = +1, 1: dz = 0, 2: dz = -1
+    for (int pc = tid; pc < N * (K / 8); pc += 160) {
+        const int n = pc / (K / 8), k8 = pc % (K / 8), tap = k8 / C8, c8 = k8 % C8;
+        const int row = (2 - tap / 9) * N + n;
+        unsigned char *dst = Bs + (size_t)((tap % 9) * CC + (c8 >> 1)) * 3 * N * 32 + (row >> 3) * 256 + (c8 & 1) * 128 + (row & 7) * 16;
         *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(w + (size_t)n * K + (size_t)k8 * 8);
     }
     if (tid == 0) {
         tc::bar_init(bars);
+        tc::bar_init(bars + 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc::saddr(tslot)),
-                     "r"(tc::ncols(N))
+                     "r"(tc::kRing * N)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
@@ -394,125 +430,132 @@ __global__ void __launch_bounds__(128) k_conv_fwd_tc_halo(Geom g, Slice in, int 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const unsigned tmem = *tslot;
-    constexpr unsigned IDESC = tc::idesc_bf16(128, N);
-    const int tx = g.W / 8, ty = g.H / 16;
-    const long tiles = (long)g.B * g.D * ty * tx;
-    const size_t halo_bytes = (size_t)C8 * tc::HALO_CHUNK;
-    // halo tile of `tile` into buffer `buf` (each thread fences its own stores)
-    auto load_tile = [&](long tile, int buf) {
-        const int x0 = (int)(tile % tx) * 8;
-        long t = tile / tx;
+    const int tx = g.W / 8, ty = g.H / 16, tz = (g.D + zc - 1) / zc;
+    const long items = (long)g.B * tz * ty * tx;
+    const long plane = (long)g.H * g.W * in.stride;  // elements between planes
+    unsigned q = 0;  // planes issued by this CTA: barrier q & 1, parity (q >> 1) & 1
+    bool ok = true;
+    for (long it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        const int x0 = (int)(it % tx) * 8;
+        long t = it / tx;
         const int y0 = (int)(t % ty) * 16;
         t /= ty;
-        const int z = (int)(t % g.D);
-        const int bb = (int)(t / g.D);
-        unsigned char *H = Hs + (size_t)buf * halo_bytes;
-        const int entries = C8 * tc::HX * tc::HY * tc::HZ;
-        for (int e = tid; e < entries; e += 128) {
-            const int hx = e % tc::HX;
-            int r = e / tc::HX;
-            const int hy = r % tc::HY;
-            r /= tc::HY;
-            const int hz = r % tc::HZ, k8 = r / tc::HZ;
-            const int xx = x0 + hx - 1, yy = y0 + hy - 1, zz = z + hz - 1;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (xx >= 0 && xx < g.W && yy >= 0 && yy < g.H && zz >= 0 && zz < g.D)
-                v = *reinterpret_cast<const uint4 *>(
-                    in.p + ((((long)bb * g.D + zz) * g.H + yy) * g.W + xx) * in.stride + in.off + k8 * 8);
-            *reinterpret_cast<uint4 *>(H + (size_t)k8 * tc::HALO_CHUNK + ((hz * tc::HY + hy) * tc::HX + hx) * 16) = v;
+        const int z0 = (int)(t % tz) * zc, bb = (int)(t / tz);
+        const int z1 = min(z0 + zc, g.D), P = z1 - z0 + 2;
+        // this thread's pieces of a plane: consecutive threads read consecutive
+        // 16-byte pieces of a voxel, then the next voxel in x
+        int goff[ENT];       // element offset in a plane, -1: off the grid
+        unsigned soff[ENT];  // byte offset in a stage
+#pragma unroll
+        for (int e = 0; e < ENT; ++e) {
+            const int id = tid + 128 * e, c8 = id % C8, v = id / C8, hx = v % tc::HX, hy = v / tc::HX;
+            const int x = x0 + hx - 1, y = y0 + hy - 1;
+            goff[e] = x >= 0 && x < g.W && y >= 0 && y < g.H ? (y * g.W + x) * in.stride + c8 * 8 : -1;
+            soff[e] = id < C8 * tc::HV ? c8 * tc::PLANE_CHUNK + v * 16 : 0xffffffffu;
         }
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    };
-    unsigned done_phase = 0;
-    bool ok = true;
-    int buf = 0;
-    if (blockIdx.x < tiles) load_tile(blockIdx.x, 0);
-    __syncthreads();
-    for (long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, buf ^= 1) {
-        if (tid == 0) {
+        const __nv_bfloat16 *src = in.p + (long)bb * g.D * plane + in.off;
+        auto load = [&](int p) {  // input plane z0 - 1 + p into stage p % S
+            const int zi = z0 - 1 + p;
+            if (p < P && zi >= 0 && zi < g.D) {
+                const unsigned dst = tc::saddr(As) + (unsigned)(p % S) * STAGE;
+                const __nv_bfloat16 *pl = src + (long)zi * plane;
+#pragma unroll
+                for (int e = 0; e < ENT; ++e)
+                    if (soff[e] != 0xffffffffu)
+                        tc::cp16(dst + soff[e], goff[e] >= 0 ? pl + goff[e] : src, goff[e] >= 0 ? 16u : 0u);
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        auto finish = [&](int zo) {  // accumulator of output plane zo to memory
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const unsigned char *H = Hs + (size_t)buf * halo_bytes;
-            for (int tap = 0; tap < 27; ++tap) {
-                const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;  // halo offsets of the tap
-                const unsigned toff = ((dz * tc::HY + dy) * tc::HX + dx) * 16;
-                for (int cc = 0; cc < CC; ++cc) {
-                    const int c = tap * CC + cc;
-                    // K-chunk cc = channel chunks 2cc and 2cc+1: leading byte offset = one chunk array
-                    const unsigned long long ad =
-                        tc::sdesc(tc::saddr(H + (size_t)(2 * cc) * tc::HALO_CHUNK + toff), tc::HALO_CHUNK, tc::HX * 16);
-                    const unsigned long long bd = tc::sdesc(tc::saddr(Bs + (size_t)c * N * 32), 128, 256);
-                    tc::mma(tmem, ad, bd, IDESC, c > 0 ? 1 : 0);
+            unsigned r[N];
+#pragma unroll
+            for (int k = 0; k < N / 16; ++k) {
+                unsigned part[16];
+                tc::ld16(tmem + ((unsigned)(32 * warp) << 16) + (unsigned)((zo - z0) % tc::kRing) * N + 16 * k, part);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) r[16 * k + e] = part[e];
+            }
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            // row m = tid: x = x0 + m % 8, y = y0 + m / 8
+            const long v = (((long)bb * g.D + zo) * g.H + (y0 + tid / 8)) * g.W + (x0 + tid % 8);
+            if (o.first) o.first[v] = __uint_as_float(r[0]) + (o.bias ? o.bias[0] : 0.f);
+            if (o.out.p) {
+#pragma unroll
+                for (int k = 0; k < N / 8; ++k) {
+                    __nv_bfloat16 h[8];
+                    uint4 gt = make_uint4(0, 0, 0, 0);
+                    if (o.gate.p) gt = *reinterpret_cast<const uint4 *>(o.gate.p + v * o.gate.stride + o.gate.off + 8 * k);
+                    const __nv_bfloat16 *gp = reinterpret_cast<const __nv_bfloat16 *>(&gt);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        float val = __uint_as_float(r[8 * k + e]) + (o.bias ? o.bias[8 * k + e] : 0.f);
+                        if (o.relu) val = fmaxf(val, 0.f);
+                        if (o.gate.p && !(__bfloat162float(gp[e]) > 0.f)) val = 0.f;
+                        h[e] = __float2bfloat16(val);
+                    }
+                    *reinterpret_cast<uint4 *>(o.out.p + v * o.out.stride + o.out.off + 8 * k) =
+                        make_uint4(pack2(h[0], h[1]), pack2(h[2], h[3]), pack2(h[4], h[5]), pack2(h[6], h[7]));
                 }
             }
-            tc::commit(bars);
-        }
-        // the next tile's halo goes to the other buffer while the MMAs run
-        // (that buffer's previous MMAs completed before the last epilogue)
-        if (tile + gridDim.x < tiles) load_tile(tile + gridDim.x, buf ^ 1);
-        const bool okd = tc::bar_wait(bars, done_phase);
-        done_phase ^= 1u;
-        if (__syncthreads_or(!okd)) {
-            ok = false;
-            break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        unsigned r[N];
-#pragma unroll
-        for (int q = 0; q < N / 16; ++q) {
-            unsigned part[16];
-            tc::ld16(tmem + ((unsigned)(32 * warp) << 16) + 16 * q, part);
-#pragma unroll
-            for (int e = 0; e < 16; ++e) r[16 * q + e] = part[e];
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        // row m = tid: x = x0 + m % 8, y = y0 + m / 8
-        {
-            const int x0 = (int)(tile % tx) * 8;
-            long t = tile / tx;
-            const int y0 = (int)(t % ty) * 16;
-            t /= ty;
-            const int z = (int)(t % g.D);
-            const int bb = (int)(t / g.D);
-            const long v = (((long)bb * g.D + z) * g.H + (y0 + tid / 8)) * g.W + (x0 + tid % 8);
-            float val[N];
-#pragma unroll
-            for (int co = 0; co < N; ++co) {
-                val[co] = __uint_as_float(r[co]) + (bias ? bias[co] : 0.f);
-                if (relu) val[co] = fmaxf(val[co], 0.f);
+        };
+        if (mover)
+            for (int p = 0; p < S - 1; ++p) load(p);
+        for (int p = 0; p < P; ++p, ++q) {
+            const int zi = z0 - 1 + p;
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(S - 2) : "memory");
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            // plane p is staged; the accumulator block it opens has been read
+            if (__syncthreads_or(!ok)) {
+                ok = false;
+                break;
             }
-            if (out_f32) {
+            if (issuer) {
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                if (zi >= 0 && zi < g.D) {
+                    // output planes this one feeds: blocks lo .. hi, in the ring up to two runs
+                    const int lo = max(zi - 1, z0), hi = min(zi + 1, z1 - 1), b0 = (lo - z0) % tc::kRing;
+                    const int n0 = min(hi - lo + 1, tc::kRing - b0), n1 = hi - lo + 1 - n0;
+                    // start addresses are the descriptors' low bits, in 16-byte units
+                    const unsigned long long ad = tc::sdesc(tc::saddr(As) + (unsigned)(p % S) * STAGE, tc::PLANE_CHUNK, tc::HX * 16);
+                    const unsigned long long bd0 = tc::sdesc(tc::saddr(Bs) + (unsigned)(lo - zi + 1) * BLK, 128, 256);
+                    const unsigned long long bd1 = bd0 + (unsigned)(n0 * BLK / 16);
+                    const unsigned d0 = tmem + b0 * N, i0 = tc::idesc_bf16(128, n0 * N), i1 = tc::idesc_bf16(128, n1 * N);
+                    // the first chunk block by block, as a block it opens must not accumulate
+                    for (int zo = lo; zo <= hi; ++zo)
+                        tc::mma(tmem + (zo - z0) % tc::kRing * N, ad, bd0 + (unsigned)((zo - lo) * BLK / 16), tc::idesc_bf16(128, N),
+                                zi == zo - 1 || (zo == 0 && zi == 0) ? 0 : 1);
 #pragma unroll
-                for (int q = 0; q < N / 4; ++q)
-                    *reinterpret_cast<float4 *>(out_f32 + v * N + 4 * q) =
-                        make_float4(val[4 * q], val[4 * q + 1], val[4 * q + 2], val[4 * q + 3]);
-            }
-            if (out.p) {
-                // 8 channels per 16-byte store (the slice offset and stride are multiples of 8)
-#pragma unroll
-                for (int q = 0; q < N / 8; ++q) {
-                    uint4 pk;
-                    pk.x = pack2(__float2bfloat16(val[8 * q]), __float2bfloat16(val[8 * q + 1]));
-                    pk.y = pack2(__float2bfloat16(val[8 * q + 2]), __float2bfloat16(val[8 * q + 3]));
-                    pk.z = pack2(__float2bfloat16(val[8 * q + 4]), __float2bfloat16(val[8 * q + 5]));
-                    pk.w = pack2(__float2bfloat16(val[8 * q + 6]), __float2bfloat16(val[8 * q + 7]));
-                    *reinterpret_cast<uint4 *>(out.p + v * out.stride + out.off + 8 * q) = pk;
+                    for (int c = 1; c < 9 * CC; ++c) {
+                        // K-chunk c = (tap, cc), channel chunks 2cc and 2cc+1: leading byte offset = one chunk array
+                        const int tap = c / CC, cc = c % CC;
+                        const unsigned ao = (2 * cc * tc::PLANE_CHUNK + ((tap / 3) * tc::HX + tap % 3) * 16) / 16, bo = c * 3 * N * 32 / 16;
+                        tc::mma(d0, ad + ao, bd0 + bo, i0, 1);
+                        if (n1 > 0) tc::mma(tmem, ad + ao, bd1 + bo, i1, 1);
+                    }
                 }
+                tc::commit(bars + (q & 1u));
+            }
+            // plane p - 1's MMAs: they complete output plane zi - 2 and free its stage
+            if (mover) {
+                if (p > 0) ok = tc::bar_wait(bars + ((q - 1) & 1u), ((q - 1) >> 1) & 1u);
+                if (ok && p >= 3) finish(zi - 2);
+                if (ok) load(p + S - 1);
             }
         }
-        // the accumulator is read, and the next halo stored, before the next tile's MMAs
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
+        if (ok && mover) ok = tc::bar_wait(bars + ((q - 1) & 1u), ((q - 1) >> 1) & 1u);
+        if (ok && mover) finish(z1 - 1);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (__syncthreads_or(!ok)) ok = false;
     }
-    if (!ok) {
-        if (tid == 0) atomicExch(status, (int)DEV_MMA_TIMEOUT);
-        tc::bar_wait(bars, done_phase);
-    }
+    if (!ok && tid == 0) atomicExch(status, (int)DEV_MMA_TIMEOUT);
+    if (!ok && q) tc::bar_wait(bars + ((q - 1) & 1u), ((q - 1) >> 1) & 1u);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tc::ncols(N))
-                     : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(tc::kRing * N) : "memory");
 }
 
 // Weight gradient for one tap: dw[co][tap][ci] += sum_v dout[v][co] * in[v+tap][ci].
@@ -571,17 +614,22 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(Geom g, Slice in, int Cin, S
         }
 }
 
-// Weight gradient on staged tiles. A persistent CTA (8 warps) walks voxel
-// tiles of 8 (x) x 8 (y) of one z-plane; per tile it stages the input's
-// 10 x 10 x 3 halo and the tile's output gradient in shared memory (16-byte
-// loads, rows padded by 8 channels so that ldmatrix rows fall in distinct
-// banks) and accumulates, for every (tap, 16 output channels, 8 input
-// channels) block it owns, dw += dout^T(16 x 16 voxels) in_tap(16 voxels x 8)
-// with mma.sync m16n8k16. Fragments come from ldmatrix.trans (both operands
-// are stored voxel-major, channels contiguous); the tap's shift is the row
-// addresses of the B fragment. Accumulators stay in registers over all of a
-// CTA's tiles and are added to dw (fp32 atomics) once at the end.
-// Needs W % 8 == 0, H % 8 == 0, slice strides and offsets multiples of 8.
+// Weight gradient on staged planes. A CTA takes a column of voxel tiles, 8 (x) x
+// 8 (y), through zc planes; the input planes (10 x 10 voxels with their halo)
+// and the output gradient's tiles come into rings of stages by cp.async, the
+// next plane while the present one is used (rows padded by 8 channels so that
+// ldmatrix rows fall in distinct banks). For every (tap, 16 output channels, 8
+// input channels) block it owns, a warp accumulates dw += dout^T(16 x 16 voxels)
+// in_tap(16 voxels x 8) with mma.sync m16n8k16. Fragments come from
+// ldmatrix.trans (both operands are stored voxel-major, channels contiguous);
+// the tap's shift is the row addresses of the B fragment. Accumulators stay in
+// registers over all of a CTA's columns and are added to dw (fp32 atomics)
+// once at the end. Needs W % 8 == 0, H % 8 == 0, slice strides and offsets
+// multiples of 8.
+// NW warps share the blocks so that a thread needs at most 7 x 4 or 4 x 8
+// accumulators and 32 warps fit an SM. With 8 warps for every layer, and a
+// 3-plane halo loaded and waited for per tile, 16 -> 16 took 306 us and 32 ->
+// 16 435 us on 8 samples of 64^3; now 120 and 215 us.
 __device__ __forceinline__ void ldsm_x4_trans(unsigned r[4], const void *p) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(p);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -596,17 +644,23 @@ __device__ __forceinline__ void ldsm_x2_trans(unsigned r[2], const void *p) {
                  : "r"(a));
 }
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_conv_wgrad_tiled(Geom g, Slice in, Slice dout, float *__restrict__ dw) {
-    constexpr int TX = 8, TY = 8, TV = TX * TY;
-    constexpr int HX = TX + 2, HY = TY + 2, HV = 3 * HY * HX;
+namespace wg {
+constexpr int TX = 8, TY = 8, TV = TX * TY, HX = TX + 2, HY = TY + 2, HV = HY * HX;
+constexpr int kIn = 4, kOut = 2;  // stages
+constexpr size_t smem(int cin, int cout) { return 2 * ((size_t)kIn * HV * (cin + 8) + (size_t)kOut * TV * (cout + 8)); }
+}  // namespace wg
+
+template <int CIN, int COUT, int NW>
+__global__ void __launch_bounds__(32 * NW, 32 / NW) k_conv_wgrad_tiled(Geom g, int zc, Slice in, Slice dout, float *__restrict__ dw) {
+    using namespace wg;
     constexpr int CP = CIN + 8, OP = COUT + 8;  // padded voxel strides (elements)
-    // a warp owns the (tap, 8 input channels) blocks warp, warp + 8, ... for
+    // a warp owns the (tap, 8 input channels) blocks warp, warp + NW, ... for
     // every group of 16 output channels (the B fragment serves them all)
-    constexpr int CT = COUT / 16, NT = CIN / 8, TN = 27 * NT, NW = 8;
+    constexpr int CT = COUT / 16, NT = CIN / 8, TN = 27 * NT;
     constexpr int TPW = (TN + NW - 1) / NW;
-    __shared__ __align__(16) __nv_bfloat16 sh_in[HV * CP];
-    __shared__ __align__(16) __nv_bfloat16 sh_out[TV * OP];
+    static_assert(HV * NT <= 32 * NW && TV * (COUT / 8) <= 32 * NW, "one 16-byte piece of a plane per thread");
+    extern __shared__ __align__(16) unsigned char wsm[];
+    __nv_bfloat16 *sh_in = reinterpret_cast<__nv_bfloat16 *>(wsm), *sh_out = sh_in + kIn * HV * CP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = lane >> 3, i8 = lane & 7;
     float acc[CT][TPW][4];
@@ -614,54 +668,64 @@ __global__ void __launch_bounds__(256) k_conv_wgrad_tiled(Geom g, Slice in, Slic
     for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
         for (int j = 0; j < TPW; ++j) acc[ct][j][0] = acc[ct][j][1] = acc[ct][j][2] = acc[ct][j][3] = 0.f;
-    const int tx_n = g.W / TX, ty_n = g.H / TY;
-    const long ntiles = (long)g.B * g.D * ty_n * tx_n;
-    for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int xt = (int)(t % tx_n);
+    const int tx_n = g.W / TX, ty_n = g.H / TY, tz_n = (g.D + zc - 1) / zc;
+    const long items = (long)g.B * tz_n * ty_n * tx_n;
+    // this thread's piece of an input plane and of an output-gradient tile
+    const int ic = threadIdx.x % NT * 8, iv = threadIdx.x / NT, ix = iv % HX - 1, iy = iv / HX - 1;
+    const int oc = threadIdx.x % (COUT / 8) * 8, ov = threadIdx.x / (COUT / 8);
+    for (long t = blockIdx.x; t < items; t += gridDim.x) {
+        const int x0 = (int)(t % tx_n) * TX;
         long r = t / tx_n;
-        const int yt = (int)(r % ty_n);
+        const int y0 = (int)(r % ty_n) * TY;
         r /= ty_n;
-        const int z = (int)(r % g.D), b = (int)(r / g.D);
-        const int x0 = xt * TX, y0 = yt * TY;
-        __syncthreads();  // the previous tile's fragments are read
-        for (int k = threadIdx.x; k < HV * (CIN / 8); k += blockDim.x) {
-            const int c8 = k % (CIN / 8), hv = k / (CIN / 8);
-            const int hx = hv % HX, hy = (hv / HX) % HY, hz = hv / (HX * HY);
-            const int X = x0 + hx - 1, Y = y0 + hy - 1, Z = z + hz - 1;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (X >= 0 && X < g.W && Y >= 0 && Y < g.H && Z >= 0 && Z < g.D)
-                v = *reinterpret_cast<const uint4 *>(in.p + ((((long)b * g.D + Z) * g.H + Y) * g.W + X) * in.stride +
-                                                     in.off + c8 * 8);
-            *reinterpret_cast<uint4 *>(sh_in + hv * CP + c8 * 8) = v;
-        }
-        for (int k = threadIdx.x; k < TV * (COUT / 8); k += blockDim.x) {
-            const int c8 = k % (COUT / 8), vv = k / (COUT / 8);
-            const int X = x0 + vv % TX, Y = y0 + vv / TX;
-            *reinterpret_cast<uint4 *>(sh_out + vv * OP + c8 * 8) = *reinterpret_cast<const uint4 *>(
-                dout.p + ((((long)b * g.D + z) * g.H + Y) * g.W + X) * dout.stride + dout.off + c8 * 8);
-        }
-        __syncthreads();
+        const int z0 = (int)(r % tz_n) * zc, b = (int)(r / tz_n), z1 = min(z0 + zc, g.D);
+        const bool inside = x0 + ix >= 0 && x0 + ix < g.W && y0 + iy >= 0 && y0 + iy < g.H;
+        const long plane = (long)g.H * g.W;
+        const __nv_bfloat16 *isrc = in.p + ((long)b * g.D * plane + (long)(y0 + iy) * g.W + x0 + ix) * in.stride + in.off + ic;
+        const __nv_bfloat16 *osrc = dout.p + ((long)b * g.D * plane + (long)(y0 + ov / TX) * g.W + x0 + ov % TX) * dout.stride + dout.off + oc;
+        auto load_in = [&](int z) {
+            if (iv < HV) {
+                const bool ok = inside && z >= 0 && z < g.D;
+                tc::cp16(tc::saddr(sh_in + ((z + kIn) % kIn) * HV * CP + iv * CP + ic), ok ? isrc + z * plane * in.stride : in.p, ok ? 16u : 0u);
+            }
+        };
+        auto load_out = [&](int z) {
+            if (ov < TV) tc::cp16(tc::saddr(sh_out + (z % kOut) * TV * OP + ov * OP + oc), osrc + z * plane * dout.stride, 16u);
+        };
+        __syncthreads();  // the previous item's fragments are read
+        load_in(z0 - 1);
+        load_in(z0);
+        load_in(z0 + 1);
+        load_out(z0);
+        for (int z = z0; z < z1; ++z) {
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            __syncthreads();  // planes z - 1 .. z + 1 are staged, plane z - 2 is no longer read
+            if (z + 1 < z1) {
+                load_in(z + 2);
+                load_out(z + 1);
+            }
+            const __nv_bfloat16 *so = sh_out + (z % kOut) * TV * OP;
 #pragma unroll
-        for (int ks = 0; ks < TV / 16; ++ks) {
-            // A = dout^T for 16 voxels (rows 2ks, 2ks+1 of the tile): matrix q
-            // covers channels (q & 1) * 8 .. +7 and voxels (q >> 1) * 8 .. +7
-            unsigned a[CT][4];
+            for (int ks = 0; ks < TV / 16; ++ks) {
+                // A = dout^T for 16 voxels (rows 2ks, 2ks+1 of the tile): matrix q
+                // covers channels (q & 1) * 8 .. +7 and voxels (q >> 1) * 8 .. +7
+                unsigned a[CT][4];
 #pragma unroll
-            for (int ct = 0; ct < CT; ++ct)
-                ldsm_x4_trans(a[ct], sh_out + (ks * 16 + (q >> 1) * 8 + i8) * OP + ct * 16 + (q & 1) * 8);
-            // B rows: voxel (x = i8, y = 2ks + (q & 1)) shifted by the tap
-            const int vy = 2 * ks + (q & 1);
+                for (int ct = 0; ct < CT; ++ct)
+                    ldsm_x4_trans(a[ct], so + (ks * 16 + (q >> 1) * 8 + i8) * OP + ct * 16 + (q & 1) * 8);
+                // B rows: voxel (x = i8, y = 2ks + (q & 1)) shifted by the tap
+                const int vy = 2 * ks + (q & 1);
 #pragma unroll
-            for (int j = 0; j < TPW; ++j) {
-                const int tl = warp + j * NW;
-                if (tl < TN) {
-                    const int tap = tl / NT, nt = tl % NT;
-                    const int dx = tap % 3 - 1, dy = (tap / 3) % 3 - 1, dz = tap / 9 - 1;
-                    const int hidx = ((dz + 1) * HY + (vy + dy + 1)) * HX + (i8 + dx + 1);
-                    unsigned bf[2];
-                    ldsm_x2_trans(bf, sh_in + hidx * CP + nt * 8);
+                for (int j = 0; j < TPW; ++j) {
+                    const int tl = warp + j * NW;
+                    if (tl < TN) {
+                        const int tap = tl / NT, nt = tl % NT;
+                        const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9 - 1;
+                        unsigned bf[2];
+                        ldsm_x2_trans(bf, sh_in + ((z + dz + kIn) % kIn) * HV * CP + ((vy + dy) * HX + i8 + dx) * CP + nt * 8);
 #pragma unroll
-                    for (int ct = 0; ct < CT; ++ct) mma16816(acc[ct][j], a[ct], bf);
+                        for (int ct = 0; ct < CT; ++ct) mma16816(acc[ct][j], a[ct], bf);
+                    }
                 }
             }
         }
@@ -703,89 +767,141 @@ __global__ void k_relu_bwd(long nv, int C, Slice y, Slice dy) {
     }
 }
 
-__global__ void k_bias_grad(long nv, int C, Slice dy, float *__restrict__ db) {
-    __shared__ float red[256];
-    const int c = blockIdx.y;
-    float s = 0.f;
-    for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += (long)gridDim.x * blockDim.x)
-        s += __bfloat162float(dy.p[v * dy.stride + dy.off + c]);
-    red[threadIdx.x] = s;
+// eight channels (16 bytes) of a slice; the slices' strides and offsets are
+// multiples of 8
+struct B8 {
+    __nv_bfloat16 h[8];
+    __device__ __forceinline__ void load(const Slice &s, long v, int c) {
+        *reinterpret_cast<uint4 *>(h) = *reinterpret_cast<const uint4 *>(s.p + v * s.stride + s.off + c);
+    }
+    __device__ __forceinline__ void store(const Slice &s, long v, int c) const {
+        *reinterpret_cast<uint4 *>(s.p + v * s.stride + s.off + c) = *reinterpret_cast<const uint4 *>(h);
+    }
+    __device__ __forceinline__ float operator[](int e) const { return __bfloat162float(h[e]); }
+};
+
+// The elementwise passes below take a sample per blockIdx.y and (voxel, eight
+// channels) items of it per thread, 32-bit index arithmetic inside a sample.
+// Per-element 64-bit divisions and 2-byte accesses bound their first form: at
+// 64^3 with 8 samples the pooling backward, its addition and the ReLU backward
+// took 184 + 96 + 94 us, the fused pass takes 49 us.
+__device__ __forceinline__ long voxel_of(const Geom &g, int v, int &z, int &y, int &x) {
+    x = v % g.W;
+    y = v / g.W % g.H;
+    z = v / (g.W * g.H);
+    return (long)blockIdx.y * g.D * g.H * g.W;
+}
+
+// db[c] += sum_v dy[v][c]
+__global__ void __launch_bounds__(256) k_bias_grad(long nv, int C, Slice dy, float *__restrict__ db) {
+    __shared__ float red[256][9];
+    const int G = C / 8, c = threadIdx.x % G * 8;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const int per = 256 / G;
+    for (long v = blockIdx.x * (long)per + threadIdx.x / G; v < nv; v += (long)gridDim.x * per) {
+        B8 d;
+        d.load(dy, v, c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += d[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) red[threadIdx.x][e] = s[e];
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+    for (int o = per / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o * G)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) red[threadIdx.x][e] += red[threadIdx.x + o * G][e];
         __syncthreads();
     }
-    if (threadIdx.x == 0) atomicAdd(db + c, red[0]);
+    if ((int)threadIdx.x < C) atomicAdd(db + threadIdx.x, red[threadIdx.x / 8][threadIdx.x % 8]);
 }
 
-// 2x average pooling: out (D/2, H/2, W/2) <- in; and its transpose
+// 2x average pooling: out (D/2, H/2, W/2) <- in
 __global__ void k_pool2(Geom go, int C, Slice in, Slice out) {
-    const long n = go.voxels() * C;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long v = i / C;
-        const int c = (int)(i % C);
-        int b, z, y, x;
-        unflat(go, v, b, z, y, x);
-        const int Hi = go.H * 2, Wi = go.W * 2, Di = go.D * 2;
-        float s = 0.f;
+    const int G = C / 8, n = go.D * go.H * go.W * G;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int z, y, x;
+        const int c = i % G * 8;
+        const long base = voxel_of(go, i / G, z, y, x);
+        const int Hi = go.H * 2, Wi = go.W * 2;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const long vi = (((long)b * Di + 2 * z + (q >> 2)) * Hi + 2 * y + ((q >> 1) & 1)) * Wi + 2 * x + (q & 1);
-            s += __bfloat162float(in.p[vi * in.stride + in.off + c]);
+            B8 a;
+            a.load(in, base * 8 + ((long)(2 * z + (q >> 2)) * Hi + 2 * y + ((q >> 1) & 1)) * Wi + 2 * x + (q & 1), c);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e] += a[e];
         }
-        out.p[v * out.stride + out.off + c] = __float2bfloat16(0.125f * s);
+        B8 r;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r.h[e] = __float2bfloat16(0.125f * s[e]);
+        r.store(out, base + i / G, c);
     }
 }
 
-__global__ void k_pool2_bwd(Geom gi, int C, Slice dout, Slice din) {
-    const long n = gi.voxels() * C;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long v = i / C;
-        const int c = (int)(i % C);
-        int b, z, y, x;
-        unflat(gi, v, b, z, y, x);
-        const long vo = (((long)b * (gi.D / 2) + z / 2) * (gi.H / 2) + y / 2) * (gi.W / 2) + x / 2;
-        din.p[v * din.stride + din.off + c] = __float2bfloat16(0.125f * __bfloat162float(dout.p[vo * dout.stride + dout.off + c]));
+// Pooling backward onto a fine slice that already holds a gradient, and the
+// ReLU backward of the layer y that was pooled: d = (y > 0) (d + dp / 8)
+__global__ void k_pool2_bwd(Geom gf, int C, Slice dp, Slice y, Slice d) {
+    const int G = C / 8, n = gf.D * gf.H * gf.W * G;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int z, yy, x;
+        const int c = i % G * 8;
+        const long base = voxel_of(gf, i / G, z, yy, x), v = base + i / G;
+        B8 p, a, r;
+        p.load(dp, base / 8 + ((long)(z / 2) * (gf.H / 2) + yy / 2) * (gf.W / 2) + x / 2, c);
+        a.load(y, v, c);
+        r.load(d, v, c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const __nv_bfloat16 sum = __float2bfloat16(r[e] + __bfloat162float(__float2bfloat16(0.125f * p[e])));
+            r.h[e] = a[e] > 0.f ? sum : __float2bfloat16(0.f);
+        }
+        r.store(d, v, c);
     }
 }
 
-// 2x nearest upsampling: out (fine) <- in (coarse); and its transpose (sum of 8)
+// 2x nearest upsampling: out (fine) <- in (coarse)
 __global__ void k_up2(Geom gf, int C, Slice in, Slice out) {
-    // 8 channels (16 bytes) per item: C, the strides and offsets are multiples of 8
-    const int C8 = C / 8;
-    const long n = gf.voxels() * C8;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long v = i / C8;
-        const int c = (int)(i % C8) * 8;
-        int b, z, y, x;
-        unflat(gf, v, b, z, y, x);
-        const long vc = (((long)b * (gf.D / 2) + z / 2) * (gf.H / 2) + y / 2) * (gf.W / 2) + x / 2;
-        *reinterpret_cast<uint4 *>(out.p + v * out.stride + out.off + c) =
-            *reinterpret_cast<const uint4 *>(in.p + vc * in.stride + in.off + c);
+    const int G = C / 8, n = gf.D * gf.H * gf.W * G;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int z, y, x;
+        const int c = i % G * 8;
+        const long base = voxel_of(gf, i / G, z, y, x);
+        B8 a;
+        a.load(in, base / 8 + ((long)(z / 2) * (gf.H / 2) + y / 2) * (gf.W / 2) + x / 2, c);
+        a.store(out, base + i / G, c);
     }
 }
 
-__global__ void k_up2_bwd(Geom gc, int C, Slice dout, Slice din) {
-    const long n = gc.voxels() * C;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const long v = i / C;
-        const int c = (int)(i % C);
-        int b, z, y, x;
-        unflat(gc, v, b, z, y, x);
-        const int Hf = gc.H * 2, Wf = gc.W * 2, Df = gc.D * 2;
-        float s = 0.f;
+// its transpose (sum of 8) and the ReLU backward of the layer y that was upsampled
+__global__ void k_up2_bwd(Geom gc, int C, Slice dout, Slice y, Slice din) {
+    const int G = C / 8, n = gc.D * gc.H * gc.W * G;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int z, yy, x;
+        const int c = i % G * 8;
+        const long base = voxel_of(gc, i / G, z, yy, x);
+        const int Hf = gc.H * 2, Wf = gc.W * 2;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const long vf = (((long)b * Df + 2 * z + (q >> 2)) * Hf + 2 * y + ((q >> 1) & 1)) * Wf + 2 * x + (q & 1);
-            s += __bfloat162float(dout.p[vf * dout.stride + dout.off + c]);
+            B8 a;
+            a.load(dout, base * 8 + ((long)(2 * z + (q >> 2)) * Hf + 2 * yy + ((q >> 1) & 1)) * Wf + 2 * x + (q & 1), c);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) s[e] += a[e];
         }
-        din.p[v * din.stride + din.off + c] = __float2bfloat16(s);
+        B8 a, r;
+        a.load(y, base + i / G, c);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r.h[e] = a[e] > 0.f ? __float2bfloat16(s[e]) : __float2bfloat16(0.f);
+        r.store(din, base + i / G, c);
     }
 }
 
 // sigmoid output and squared-error loss against targets: loss += sum (s - t)^2 / nv,
-// dlogit = 2 (s - t) s (1 - s) / nv (scaled by loss_scale for bf16 range)
+// dlogit = 2 (s - t) s (1 - s) / nv in channel 0 of 16, the others zero
 // pred may be logit itself (in-place sigmoid): neither is declared restrict
 __global__ void k_loss(long nv, const float *logit, const float *__restrict__ target, float *pred,
-                       __nv_bfloat16 *__restrict__ dlogit, float loss_scale, double *__restrict__ loss) {
+                       __nv_bfloat16 *__restrict__ dlogit, double *__restrict__ loss) {
     __shared__ double red[256];
     double s_acc = 0.0;
     for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < nv; v += (long)gridDim.x * blockDim.x) {
@@ -794,7 +910,12 @@ __global__ void k_loss(long nv, const float *logit, const float *__restrict__ ta
         if (target) {
             const float d = s - target[v];
             s_acc += (double)d * d;
-            if (dlogit) dlogit[v] = __float2bfloat16(loss_scale * 2.f * d * s * (1.f - s) / (float)nv);
+            if (dlogit) {
+                const __nv_bfloat16 z = __float2bfloat16(0.f);
+                uint4 *o = reinterpret_cast<uint4 *>(dlogit + v * 16);
+                o[0] = make_uint4(pack2(__float2bfloat16(2.f * d * s * (1.f - s) / (float)nv), z), 0u, 0u, 0u);
+                o[1] = make_uint4(0u, 0u, 0u, 0u);
+            }
         }
     }
     red[threadIdx.x] = s_acc;
@@ -833,35 +954,44 @@ struct FeatParams {
     double dw_lo, dw_hi, rho_lo, rho_hi, t_lo, t_hi, L, n_solver, blob_sigma;
 };
 
-__global__ void k_features(int S, int n, int factor, const gbg_sample *__restrict__ smp,
-                           const float *__restrict__ pw, const float *__restrict__ pg, FeatParams fp,
-                           __nv_bfloat16 *__restrict__ x) {
-    const long N = (long)n * n * n;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N * S; i += (long)gridDim.x * blockDim.x) {
-        const long s = i / N, c = i % N;
-        const int xx = (int)(c % n), yy = (int)((c / n) % n), zz = (int)(c / ((long)n * n));
-        const gbg_sample q = smp[s];
-        // per-sample scalars in double; per-cell geometry in float (the
-        // features are rounded to bf16)
+// One sample per blockIdx.y. What depends on the sample or on one coordinate
+// alone is formed in double once per CTA (per cell it kept the FP64 pipe, 1/64
+// of the FP32 rate here, busy for 2.1 ms on 64 samples of 64^3; now 0.11 ms).
+__global__ void __launch_bounds__(256) k_features(int n, int factor, const gbg_sample *__restrict__ smp,
+                                                  const float *__restrict__ pw, const float *__restrict__ pg, FeatParams fp,
+                                                  __nv_bfloat16 *__restrict__ x) {
+    extern __shared__ float s_d[];  // distances to the seed per coordinate, x then y then z
+    __shared__ float s_front, s_f[3];
+    const gbg_sample q = smp[blockIdx.y];
+    for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+        const int a = i / n;
+        // cell centre in solver voxel units
+        s_d[i] = (float)((i % n + 0.5) * factor - 0.5 - (a == 0 ? q.x0 : (a == 1 ? q.y0 : q.z0)));
+    }
+    if (threadIdx.x == 0) {
         // front speed 2 sqrt(D rho) in voxels/day: D in voxel^2/day = Dw / L^2 * n_solver^2
         const double dvox = q.Dw / (fp.L * fp.L) * fp.n_solver * fp.n_solver;
-        const float front = (float)(2.0 * sqrt(dvox * q.rho) * q.tend);
-        const float inv2s2 = (float)(1.0 / (2.0 * fp.blob_sigma * fp.blob_sigma));
-        // cell centre in solver voxel units
-        const float dx = (float)((xx + 0.5) * factor - 0.5 - q.x0), dy = (float)((yy + 0.5) * factor - 0.5 - q.y0),
-                    dz = (float)((zz + 0.5) * factor - 0.5 - q.z0);
+        s_front = (float)(2.0 * sqrt(dvox * q.rho) * q.tend);
+        s_f[0] = (float)((q.Dw - fp.dw_lo) / (fp.dw_hi - fp.dw_lo));
+        s_f[1] = (float)((q.rho - fp.rho_lo) / (fp.rho_hi - fp.rho_lo));
+        s_f[2] = (float)((q.tend - fp.t_lo) / (fp.t_hi - fp.t_lo));
+    }
+    __syncthreads();
+    const float front = s_front, inv2s2 = (float)(1.0 / (2.0 * fp.blob_sigma * fp.blob_sigma));
+    const unsigned f34 = pack2(__float2bfloat16(s_f[1]), __float2bfloat16(s_f[2]));
+    const __nv_bfloat16 f3 = __float2bfloat16(s_f[0]);
+    const int N = n * n * n;
+    uint4 *out = reinterpret_cast<uint4 *>(x) + (size_t)blockIdx.y * N * 2;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+        const float dx = s_d[c % n], dy = s_d[n + c / n % n], dz = s_d[2 * n + c / (n * n)];
         const float d2 = dx * dx + dy * dy + dz * dz;
-        const float f[7] = {pw[c], pg[c], expf(-d2 * inv2s2), (float)((q.Dw - fp.dw_lo) / (fp.dw_hi - fp.dw_lo)),
-                            (float)((q.rho - fp.rho_lo) / (fp.rho_hi - fp.rho_lo)),
-                            (float)((q.tend - fp.t_lo) / (fp.t_hi - fp.t_lo)), (sqrtf(d2) - front) * (1.0f / 16.0f)};
-        uint4 lo, hi = make_uint4(0, 0, 0, 0);
-        lo.x = pack2(__float2bfloat16(f[0]), __float2bfloat16(f[1]));
-        lo.y = pack2(__float2bfloat16(f[2]), __float2bfloat16(f[3]));
-        lo.z = pack2(__float2bfloat16(f[4]), __float2bfloat16(f[5]));
-        lo.w = pack2(__float2bfloat16(f[6]), __float2bfloat16(0.f));
-        uint4 *o = reinterpret_cast<uint4 *>(x + i * 16);
-        o[0] = lo;
-        o[1] = hi;
+        uint4 lo;
+        lo.x = pack2(__float2bfloat16(pw[c]), __float2bfloat16(pg[c]));
+        lo.y = pack2(__float2bfloat16(expf(-d2 * inv2s2)), f3);
+        lo.z = f34;
+        lo.w = pack2(__float2bfloat16((sqrtf(d2) - front) * (1.0f / 16.0f)), __float2bfloat16(0.f));
+        out[2 * (size_t)c] = lo;
+        out[2 * (size_t)c + 1] = make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -879,16 +1009,14 @@ __global__ void k_down2_f32(int S, int n, const float *__restrict__ in, float *_
     }
 }
 
-// nearest 2x upsampling of S float fields m^3 -> (2m)^3, zero outside tissue
-__global__ void k_up2_f32(int S, int m, const float *__restrict__ in, const float *__restrict__ mask,
-                          float *__restrict__ out) {
-    const int n = 2 * m;
-    const long N = (long)n * n * n;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < N * S; i += (long)gridDim.x * blockDim.x) {
-        const long s = i / N, c = i % N;
-        const int x = (int)(c % n), y = (int)((c / n) % n), z = (int)(c / ((long)n * n));
-        const float v = in[s * (long)m * m * m + ((long)(z / 2) * m + y / 2) * m + x / 2];
-        out[i] = mask[c] != 0.f ? v : 0.f;
+// nearest 2x upsampling of float fields m^3 -> (2m)^3, zero outside tissue
+__global__ void k_up2_f32(int m, const float *__restrict__ in, const float *__restrict__ mask, float *__restrict__ out) {
+    const int n = 2 * m, N = n * n * n;
+    in += (size_t)blockIdx.y * m * m * m;
+    out += (size_t)blockIdx.y * N;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+        const int x = c % n, y = c / n % n, z = c / (n * n);
+        out[c] = mask[c] != 0.f ? in[((z / 2) * m + y / 2) * m + x / 2] : 0.f;
     }
 }
 
@@ -949,24 +1077,57 @@ inline int grid_n(long work, int cap = 4096) {
     return (int)(g < cap ? g : cap);
 }
 
+// Planes per item of a marching kernel over `cols` columns of D planes with
+// `slots` CTAs resident: the fewest input planes (2 more than output planes per
+// item) in the longest CTA's share, items dealt round by round. 8 samples of
+// 64^3 at 6 CTAs per SM: 1024 items of 16 planes would be 2 rounds x 18, 768
+// of 22 are 1 x 24.
+int planes_per_item(long cols, int D, long slots) {
+    int zc = D;
+    long best = -1;
+    for (int tz = 1; tz <= (D + 1) / 2; ++tz) {
+        const int z = (D + tz - 1) / tz;
+        const long cost = ((cols * tz + slots - 1) / slots) * (z + 2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            zc = z;
+        }
+    }
+    return zc;
+}
+
+template <int C8, int N>
+void conv_march(cudaStream_t st, Geom g, Slice in, const __nv_bfloat16 *w, const ConvOut &o, int num_sms, int *status) {
+    constexpr size_t sm = tc::march_smem(C8, N);
+    cudaFuncSetAttribute(k_conv_march<C8, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    constexpr int bps = tc::march_ctas(C8, N);
+    const long cols = (long)g.B * (g.H / 16) * (g.W / 8), slots = (long)num_sms * bps;
+    const int zc = planes_per_item(cols, g.D, slots);
+    const long items = cols * ((g.D + zc - 1) / zc);
+    k_conv_march<C8, N><<<(int)std::min(items, slots), 160, sm, st>>>(g, zc, in, w, o, status);
+}
+
+// the U-Net's layers and their data gradients on the marching kernel; false:
+// another kernel has to run (a grid not divisible into its tiles, or other
+// widths). Slice strides and offsets are multiples of 8.
+bool conv_march_any(cudaStream_t st, Geom g, Slice in, int cin, const __nv_bfloat16 *w, const ConvOut &o, int cout, int num_sms,
+                    int *status) {
+    if (g.W % 8 || g.H % 16) return false;
+#define GBG_MARCH(ci, co) \
+    if (cin == ci && cout == co) return conv_march<ci / 8, co>(st, g, in, w, o, num_sms, status), true
+    GBG_MARCH(16, 16);
+    GBG_MARCH(16, 32);
+    GBG_MARCH(16, 64);
+    GBG_MARCH(32, 16);
+    GBG_MARCH(32, 32);
+    GBG_MARCH(64, 16);
+#undef GBG_MARCH
+    return false;
+}
+
 // engine 1: tcgen05 kernel (Cout 16, 32 or 64); engine 0: mma.sync kernel
 void conv_fwd(cudaStream_t st, Geom g, Slice in, int cin, const __nv_bfloat16 *w, const float *b, Slice out,
               float *out32, int cout, bool relu, int engine = 0, int num_sms = 0, int *status = nullptr) {
-    if (engine == 1 && (cout == 16 || cout == 32 || cout == 64) && status && g.W % 8 == 0 && g.H % 16 == 0) {
-        const size_t sm = tc::halo_smem_bytes(cin, cout);
-        const long tiles = (long)g.B * g.D * (g.H / 16) * (g.W / 8);
-        const int grid = (int)std::min<long>(tiles, (long)num_sms * 8);
-        const void *fn = cout == 16 ? (const void *)k_conv_fwd_tc_halo<16>
-                                    : (cout == 32 ? (const void *)k_conv_fwd_tc_halo<32>
-                                                  : (const void *)k_conv_fwd_tc_halo<64>);
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        switch (cout) {
-            case 16: k_conv_fwd_tc_halo<16><<<grid, 128, sm, st>>>(g, in, cin, w, b, out, out32, relu, status); break;
-            case 32: k_conv_fwd_tc_halo<32><<<grid, 128, sm, st>>>(g, in, cin, w, b, out, out32, relu, status); break;
-            case 64: k_conv_fwd_tc_halo<64><<<grid, 128, sm, st>>>(g, in, cin, w, b, out, out32, relu, status); break;
-        }
-        return;
-    }
     if (engine == 1 && (cout == 16 || cout == 32 || cout == 64) && status) {
         const size_t sm = tc::smem_bytes(cin, cout);
         const long tiles = (g.voxels() + 127) / 128;
@@ -991,25 +1152,25 @@ void conv_fwd(cudaStream_t st, Geom g, Slice in, int cin, const __nv_bfloat16 *w
     }
 }
 
-template <int CIN, int COUT>
+template <int CIN, int COUT, int NW>
 void wgrad_tiled(cudaStream_t st, Geom g, Slice in, Slice dout, float *dw, int num_sms) {
-    const long ntiles = (long)g.B * g.D * (g.H / 8) * (g.W / 8);
-    int bps = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_conv_wgrad_tiled<CIN, COUT>, 256, 0);
-    long grid = (long)(bps > 0 ? bps : 1) * num_sms;
-    if (grid > ntiles) grid = ntiles;
-    k_conv_wgrad_tiled<CIN, COUT><<<(unsigned)grid, 256, 0, st>>>(g, in, dout, dw);
+    constexpr size_t sm = wg::smem(CIN, COUT);
+    cudaFuncSetAttribute(k_conv_wgrad_tiled<CIN, COUT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const long cols = (long)g.B * (g.H / 8) * (g.W / 8), slots = (long)(32 / NW) * num_sms;
+    const int zc = planes_per_item(cols, g.D, slots);
+    const long items = cols * ((g.D + zc - 1) / zc);
+    k_conv_wgrad_tiled<CIN, COUT, NW><<<(unsigned)std::min(items, slots), 32 * NW, sm, st>>>(g, zc, in, dout, dw);
 }
 
 void conv_wgrad(cudaStream_t st, Geom g, Slice in, int cin, Slice dout, int cout, float *dw, int num_sms) {
     const bool tiled = g.W % 8 == 0 && g.H % 8 == 0 && in.stride % 8 == 0 && in.off % 8 == 0 &&
                        dout.stride % 8 == 0 && dout.off % 8 == 0;
     if (tiled) {
-        if (cin == 16 && cout == 16) return wgrad_tiled<16, 16>(st, g, in, dout, dw, num_sms);
-        if (cin == 16 && cout == 32) return wgrad_tiled<16, 32>(st, g, in, dout, dw, num_sms);
-        if (cin == 32 && cout == 16) return wgrad_tiled<32, 16>(st, g, in, dout, dw, num_sms);
-        if (cin == 32 && cout == 32) return wgrad_tiled<32, 32>(st, g, in, dout, dw, num_sms);
-        if (cin == 64 && cout == 16) return wgrad_tiled<64, 16>(st, g, in, dout, dw, num_sms);
+        if (cin == 16 && cout == 16) return wgrad_tiled<16, 16, 8>(st, g, in, dout, dw, num_sms);
+        if (cin == 16 && cout == 32) return wgrad_tiled<16, 32, 16>(st, g, in, dout, dw, num_sms);
+        if (cin == 32 && cout == 16) return wgrad_tiled<32, 16, 16>(st, g, in, dout, dw, num_sms);
+        if (cin == 32 && cout == 32) return wgrad_tiled<32, 32, 32>(st, g, in, dout, dw, num_sms);
+        if (cin == 64 && cout == 16) return wgrad_tiled<64, 16, 32>(st, g, in, dout, dw, num_sms);
     }
     const long chunk = 2048;
     const int tiles = 27 * (cout / 16) * (cin / 8);
@@ -1055,45 +1216,53 @@ T *salloc(Surrogate &s, size_t count) {
     return (T *)p;
 }
 
-// forward for B samples already featurised in s.x0; logits in s.logits
+// channel 0 of the 16-channel logits (the kernels that store all channels)
+__global__ void k_channel0(long nv, const float *__restrict__ l16, float *__restrict__ l1) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nv; i += (long)gridDim.x * blockDim.x) l1[i] = l16[i * 16];
+}
+
+// grid of the elementwise passes: sample per y, up to 16 CTAs per SM in all
+dim3 grid_bv(const Surrogate &s, int B, long per_sample) {
+    const long want = (per_sample + 255) / 256, cap = std::max<long>(1, (long)s.h->num_sms * 16 / B);
+    return dim3((unsigned)std::min(want, cap), (unsigned)B);
+}
+
+// Layer i: out = conv(in) + bias, ReLU except for the last layer, whose
+// channel 0 goes to s.pred in fp32.
+void layer(Surrogate &s, Geom g, int i, Slice in, Slice out) {
+    const auto &l = s.net.L[i];
+    const __nv_bfloat16 *w = s.wb + l.w_off;
+    const float *b = s.w32 + l.b_off;
+    cudaStream_t st = s.h->stream;
+    const sg::ConvOut o{out, out.p ? nullptr : s.pred, b, l.relu ? 1 : 0, Slice{nullptr, 0, 0}};
+    s.h->launches++;
+    if (s.engine == 1 && sg::conv_march_any(st, g, in, l.cin, w, o, l.cout, s.h->num_sms, s.h->dev_status)) return;
+    sg::conv_fwd(st, g, in, l.cin, w, b, out, out.p ? nullptr : s.logits, l.cout, l.relu, s.engine, s.h->num_sms, s.h->dev_status);
+    if (!out.p) {
+        k_channel0<<<sg::grid_n(g.voxels()), 256, 0, st>>>(g.voxels(), s.logits, s.pred);
+        s.h->launches++;
+    }
+}
+
+// forward for B samples already featurised in s.x0; logits of channel 0 in s.pred
 void forward(Surrogate &s, int B) {
     cudaStream_t st = s.h->stream;
     const int m = s.m;
     Geom g0{B, m, m, m}, g1{B, m / 2, m / 2, m / 2}, g2{B, m / 4, m / 4, m / 4};
-    const auto &Ly = s.net.L;
-    auto W = [&](int i) { return s.wb + Ly[i].w_off; };
-    auto Bi = [&](int i) { return s.w32 + Ly[i].b_off; };
-    sg::conv_fwd(st, g0, Slice{s.x0, 16, 0}, 16, W(0), Bi(0), Slice{s.t0, 16, 0}, nullptr, 16, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::conv_fwd(st, g0, Slice{s.t0, 16, 0}, 16, W(1), Bi(1), Slice{s.c0, 32, 16}, nullptr, 16, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::k_pool2<<<sg::grid_n(g1.voxels() * 16), 256, 0, st>>>(g1, 16, Slice{s.c0, 32, 16}, Slice{s.p1, 16, 0});
-    sg::conv_fwd(st, g1, Slice{s.p1, 16, 0}, 16, W(2), Bi(2), Slice{s.t1, 32, 0}, nullptr, 32, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::conv_fwd(st, g1, Slice{s.t1, 32, 0}, 32, W(3), Bi(3), Slice{s.c1, 64, 32}, nullptr, 32, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::k_pool2<<<sg::grid_n(g2.voxels() * 32), 256, 0, st>>>(g2, 32, Slice{s.c1, 64, 32}, Slice{s.p2, 32, 0});
-    sg::conv_fwd(st, g2, Slice{s.p2, 32, 0}, 32, W(4), Bi(4), Slice{s.q2, 32, 0}, nullptr, 32, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::k_up2<<<sg::grid_n(g1.voxels() * 32), 256, 0, st>>>(g1, 32, Slice{s.q2, 32, 0}, Slice{s.c1, 64, 0});
-    sg::conv_fwd(st, g1, Slice{s.c1, 64, 0}, 64, W(5), Bi(5), Slice{s.u1, 16, 0}, nullptr, 16, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::k_up2<<<sg::grid_n(g0.voxels() * 16), 256, 0, st>>>(g0, 16, Slice{s.u1, 16, 0}, Slice{s.c0, 32, 0});
-    sg::conv_fwd(st, g0, Slice{s.c0, 32, 0}, 32, W(6), Bi(6), Slice{s.u0, 16, 0}, nullptr, 16, true, s.engine, s.h->num_sms, s.h->dev_status);
-    sg::conv_fwd(st, g0, Slice{s.u0, 16, 0}, 16, W(7), Bi(7), Slice{nullptr, 0, 0}, s.logits, 16, false, s.engine, s.h->num_sms, s.h->dev_status);
-    s.h->launches += 12;
-}
-
-// data gradient of layer i: din (cin channels) from dout (cout channels)
-void data_grad(Surrogate &s, Geom g, int i, Slice dout, Slice din) {
-    const auto &l = s.net.L[i];
-    const long n = (long)l.cout * 27 * l.cin;
-    sg::k_flip_weights<<<sg::grid_n(n), 256, 0, s.h->stream>>>(s.wb + l.w_off, l.cout, l.cin, s.wflip);
-    sg::conv_fwd(s.h->stream, g, dout, l.cout, s.wflip, nullptr, din, nullptr, l.cin, false, s.engine, s.h->num_sms,
-                 s.h->dev_status);
-    s.h->launches += 2;
-}
-
-void param_grad(Surrogate &s, Geom g, int i, Slice in, Slice dout) {
-    const auto &l = s.net.L[i];
-    sg::conv_wgrad(s.h->stream, g, in, l.cin, dout, l.cout, s.g32 + l.w_off, s.h->num_sms);
-    dim3 gb(64, l.cout);
-    sg::k_bias_grad<<<gb, 256, 0, s.h->stream>>>(g.voxels(), l.cout, dout, s.g32 + l.b_off);
-    s.h->launches += 2;
+    const long n0 = (long)m * m * m, n1 = n0 / 8, n2 = n0 / 64;
+    layer(s, g0, 0, Slice{s.x0, 16, 0}, Slice{s.t0, 16, 0});
+    layer(s, g0, 1, Slice{s.t0, 16, 0}, Slice{s.c0, 32, 16});
+    sg::k_pool2<<<grid_bv(s, B, n1 * 2), 256, 0, st>>>(g1, 16, Slice{s.c0, 32, 16}, Slice{s.p1, 16, 0});
+    layer(s, g1, 2, Slice{s.p1, 16, 0}, Slice{s.t1, 32, 0});
+    layer(s, g1, 3, Slice{s.t1, 32, 0}, Slice{s.c1, 64, 32});
+    sg::k_pool2<<<grid_bv(s, B, n2 * 4), 256, 0, st>>>(g2, 32, Slice{s.c1, 64, 32}, Slice{s.p2, 32, 0});
+    layer(s, g2, 4, Slice{s.p2, 32, 0}, Slice{s.q2, 32, 0});
+    sg::k_up2<<<grid_bv(s, B, n1 * 4), 256, 0, st>>>(g1, 32, Slice{s.q2, 32, 0}, Slice{s.c1, 64, 0});
+    layer(s, g1, 5, Slice{s.c1, 64, 0}, Slice{s.u1, 16, 0});
+    sg::k_up2<<<grid_bv(s, B, n0 * 2), 256, 0, st>>>(g0, 16, Slice{s.u1, 16, 0}, Slice{s.c0, 32, 0});
+    layer(s, g0, 6, Slice{s.c0, 32, 0}, Slice{s.u0, 16, 0});
+    layer(s, g0, 7, Slice{s.u0, 16, 0}, Slice{nullptr, 0, 0});
+    s.h->launches += 4;
 }
 
 void relu_bwd(Surrogate &s, Geom g, int C, Slice y, Slice dy) {
@@ -1101,14 +1270,28 @@ void relu_bwd(Surrogate &s, Geom g, int C, Slice y, Slice dy) {
     s.h->launches++;
 }
 
-// accumulate src slice into dst slice (bf16, fp32 add)
-__global__ void k_add_slice(long nv, int C, Slice src, Slice dst) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nv * C; i += (long)gridDim.x * blockDim.x) {
-        const long v = i / C;
-        const int c = (int)(i % C);
-        __nv_bfloat16 &d = dst.p[v * dst.stride + dst.off + c];
-        d = __float2bfloat16(__bfloat162float(d) + __bfloat162float(src.p[v * src.stride + src.off + c]));
-    }
+// data gradient of layer i: din (cin channels) from dout (cout channels); gate
+// non-null: times (gate > 0), the ReLU backward of the layer whose output is
+// layer i's whole input
+void data_grad(Surrogate &s, Geom g, int i, Slice dout, Slice din, Slice gate = Slice{nullptr, 0, 0}) {
+    const auto &l = s.net.L[i];
+    const long n = (long)l.cout * 27 * l.cin;
+    sg::k_flip_weights<<<sg::grid_n(n), 256, 0, s.h->stream>>>(s.wb + l.w_off, l.cout, l.cin, s.wflip);
+    s.h->launches += 2;
+    const sg::ConvOut o{din, nullptr, nullptr, 0, gate};
+    if (s.engine == 1 && sg::conv_march_any(s.h->stream, g, dout, l.cout, s.wflip, o, l.cin, s.h->num_sms, s.h->dev_status)) return;
+    sg::conv_fwd(s.h->stream, g, dout, l.cout, s.wflip, nullptr, din, nullptr, l.cin, false, s.engine, s.h->num_sms,
+                 s.h->dev_status);
+    if (gate.p) relu_bwd(s, g, l.cin, gate, din);
+}
+
+void param_grad(Surrogate &s, Geom g, int i, Slice in, Slice dout) {
+    const auto &l = s.net.L[i];
+    sg::conv_wgrad(s.h->stream, g, in, l.cin, dout, l.cout, s.g32 + l.w_off, s.h->num_sms);
+    const long per = 256 / (l.cout / 8);
+    sg::k_bias_grad<<<(unsigned)std::min<long>((g.voxels() + per - 1) / per, s.h->num_sms * 4), 256, 0, s.h->stream>>>(
+        g.voxels(), l.cout, dout, s.g32 + l.b_off);
+    s.h->launches += 2;
 }
 
 // backward from s.dlog (bf16 [voxels][16], channel 0 nonzero); gradients into s.g32
@@ -1116,62 +1299,44 @@ void backward(Surrogate &s, int B) {
     cudaStream_t st = s.h->stream;
     const int m = s.m;
     Geom g0{B, m, m, m}, g1{B, m / 2, m / 2, m / 2}, g2{B, m / 4, m / 4, m / 4};
+    const long n0 = (long)m * m * m, n1 = n0 / 8, n2 = n0 / 64;
     // out
     param_grad(s, g0, 7, Slice{s.u0, 16, 0}, Slice{s.dlog, 16, 0});
-    data_grad(s, g0, 7, Slice{s.dlog, 16, 0}, Slice{s.du0, 16, 0});
+    data_grad(s, g0, 7, Slice{s.dlog, 16, 0}, Slice{s.du0, 16, 0}, Slice{s.u0, 16, 0});
     // d0
-    relu_bwd(s, g0, 16, Slice{s.u0, 16, 0}, Slice{s.du0, 16, 0});
     param_grad(s, g0, 6, Slice{s.c0, 32, 0}, Slice{s.du0, 16, 0});
     data_grad(s, g0, 6, Slice{s.du0, 16, 0}, Slice{s.dc0, 32, 0});
     // up -> u1
-    sg::k_up2_bwd<<<sg::grid_n(g1.voxels() * 16), 256, 0, st>>>(g1, 16, Slice{s.dc0, 32, 0}, Slice{s.du1, 16, 0});
+    sg::k_up2_bwd<<<grid_bv(s, B, n1 * 2), 256, 0, st>>>(g1, 16, Slice{s.dc0, 32, 0}, Slice{s.u1, 16, 0}, Slice{s.du1, 16, 0});
     // d1
-    relu_bwd(s, g1, 16, Slice{s.u1, 16, 0}, Slice{s.du1, 16, 0});
     param_grad(s, g1, 5, Slice{s.c1, 64, 0}, Slice{s.du1, 16, 0});
     data_grad(s, g1, 5, Slice{s.du1, 16, 0}, Slice{s.dc1, 64, 0});
     // up -> q2
-    sg::k_up2_bwd<<<sg::grid_n(g2.voxels() * 32), 256, 0, st>>>(g2, 32, Slice{s.dc1, 64, 0}, Slice{s.dq2, 32, 0});
+    sg::k_up2_bwd<<<grid_bv(s, B, n2 * 4), 256, 0, st>>>(g2, 32, Slice{s.dc1, 64, 0}, Slice{s.q2, 32, 0}, Slice{s.dq2, 32, 0});
     // mid
-    relu_bwd(s, g2, 32, Slice{s.q2, 32, 0}, Slice{s.dq2, 32, 0});
     param_grad(s, g2, 4, Slice{s.p2, 32, 0}, Slice{s.dq2, 32, 0});
     data_grad(s, g2, 4, Slice{s.dq2, 32, 0}, Slice{s.dp2, 32, 0});
     // pool -> c1[32:64], added to d1's gradient there
-    sg::k_pool2_bwd<<<sg::grid_n(g1.voxels() * 32), 256, 0, st>>>(g1, 32, Slice{s.dp2, 32, 0}, Slice{s.tmp, 32, 0});
-    k_add_slice<<<sg::grid_n(g1.voxels() * 32), 256, 0, st>>>(g1.voxels(), 32, Slice{s.tmp, 32, 0}, Slice{s.dc1, 64, 32});
+    sg::k_pool2_bwd<<<grid_bv(s, B, n1 * 4), 256, 0, st>>>(g1, 32, Slice{s.dp2, 32, 0}, Slice{s.c1, 64, 32}, Slice{s.dc1, 64, 32});
     // e1b
-    relu_bwd(s, g1, 32, Slice{s.c1, 64, 32}, Slice{s.dc1, 64, 32});
     param_grad(s, g1, 3, Slice{s.t1, 32, 0}, Slice{s.dc1, 64, 32});
-    data_grad(s, g1, 3, Slice{s.dc1, 64, 32}, Slice{s.dt1, 32, 0});
+    data_grad(s, g1, 3, Slice{s.dc1, 64, 32}, Slice{s.dt1, 32, 0}, Slice{s.t1, 32, 0});
     // e1a
-    relu_bwd(s, g1, 32, Slice{s.t1, 32, 0}, Slice{s.dt1, 32, 0});
     param_grad(s, g1, 2, Slice{s.p1, 16, 0}, Slice{s.dt1, 32, 0});
     data_grad(s, g1, 2, Slice{s.dt1, 32, 0}, Slice{s.dp1, 16, 0});
     // pool -> c0[16:32], added to d0's gradient there
-    sg::k_pool2_bwd<<<sg::grid_n(g0.voxels() * 16), 256, 0, st>>>(g0, 16, Slice{s.dp1, 16, 0}, Slice{s.tmp, 16, 0});
-    k_add_slice<<<sg::grid_n(g0.voxels() * 16), 256, 0, st>>>(g0.voxels(), 16, Slice{s.tmp, 16, 0}, Slice{s.dc0, 32, 16});
+    sg::k_pool2_bwd<<<grid_bv(s, B, n0 * 2), 256, 0, st>>>(g0, 16, Slice{s.dp1, 16, 0}, Slice{s.c0, 32, 16}, Slice{s.dc0, 32, 16});
     // e0b
-    relu_bwd(s, g0, 16, Slice{s.c0, 32, 16}, Slice{s.dc0, 32, 16});
     param_grad(s, g0, 1, Slice{s.t0, 16, 0}, Slice{s.dc0, 32, 16});
-    data_grad(s, g0, 1, Slice{s.dc0, 32, 16}, Slice{s.dt0, 16, 0});
+    data_grad(s, g0, 1, Slice{s.dc0, 32, 16}, Slice{s.dt0, 16, 0}, Slice{s.t0, 16, 0});
     // e0a
-    relu_bwd(s, g0, 16, Slice{s.t0, 16, 0}, Slice{s.dt0, 16, 0});
     param_grad(s, g0, 0, Slice{s.x0, 16, 0}, Slice{s.dt0, 16, 0});
-    s.h->launches += 6;
-}
-
-// dlogit buffer: channel 0 from the loss, the other 15 channels zero
-__global__ void k_scatter_dlogit(long nv, const __nv_bfloat16 *__restrict__ d0, __nv_bfloat16 *__restrict__ d16) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nv * 16; i += (long)gridDim.x * blockDim.x)
-        d16[i] = (i % 16 == 0) ? d0[i / 16] : __float2bfloat16(0.f);
-}
-
-__global__ void k_channel0(long nv, const float *__restrict__ l16, float *__restrict__ l1) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nv; i += (long)gridDim.x * blockDim.x) l1[i] = l16[i * 16];
+    s.h->launches += 4;
 }
 
 void featurise(Surrogate &s, const gbg_sample *dsamples, int B) {
-    sg::k_features<<<sg::grid_n((long)B * s.m * s.m * s.m), 256, 0, s.h->stream>>>(B, s.m, s.factor, dsamples, s.pw_s,
-                                                                                   s.pg_s, s.fp, s.x0);
+    sg::k_features<<<grid_bv(s, B, (long)s.m * s.m * s.m), 256, 3 * s.m * sizeof(float), s.h->stream>>>(
+        s.m, s.factor, dsamples, s.pw_s, s.pg_s, s.fp, s.x0);
     s.h->launches++;
 }
 
@@ -1179,16 +1344,12 @@ void featurise(Surrogate &s, const gbg_sample *dsamples, int B) {
 int loss_and_backward(Surrogate &s, int B, const float *targets, bool grad, double *loss) {
     cudaStream_t st = s.h->stream;
     const long nv = (long)B * s.m * s.m * s.m;
-    float *l1 = s.pred;  // reuse: channel-0 logits, then predictions
-    k_channel0<<<sg::grid_n(nv), 256, 0, st>>>(nv, s.logits, l1);
     GBG_CUDA_TRY(cudaMemsetAsync(s.dloss, 0, sizeof(double), st));
-    sg::k_loss<<<sg::grid_n(nv, 1024), 256, 0, st>>>(nv, l1, targets, s.pred, grad ? s.tmp : nullptr, 1.f, s.dloss);
-    s.h->launches += 2;
+    sg::k_loss<<<sg::grid_n(nv, 1024), 256, 0, st>>>(nv, s.pred, targets, s.pred, grad ? s.dlog : nullptr, s.dloss);
+    s.h->launches++;
     if (grad) {
-        k_scatter_dlogit<<<sg::grid_n(nv * 16), 256, 0, st>>>(nv, s.tmp, s.dlog);
         GBG_CUDA_TRY(cudaMemsetAsync(s.g32, 0, s.net.nparams * sizeof(float), st));
         backward(s, B);
-        s.h->launches++;
     }
     if (loss) {
         GBG_CUDA_TRY(cudaMemcpyAsync(loss, s.dloss, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1442,20 +1603,23 @@ int surrogate_train(Surrogate &s, const gbg_sample *samples, int S, int epochs, 
     return GBG_OK;
 }
 
-// predicted final densities of B samples on the solver grid (nearest 2x
-// upsampling of the surrogate field, zero off tissue) into s.up_pred, and
-// optionally their log-likelihoods (device results)
-int surrogate_predict(Surrogate &s, const gbg_sample *samples_device, int B, gbg_lik_result *lik_device) {
+// Predicted final densities of B samples on the solver grid (nearest 2x
+// upsampling of the surrogate field, zero off tissue) into s.up_pred when
+// want_field, and optionally their log-likelihoods (device results), which
+// read the surrogate field at the observations' cells.
+int surrogate_predict(Surrogate &s, const gbg_sample *samples_device, int B, gbg_lik_result *lik_device, bool want_field) {
     cudaStream_t st = s.h->stream;
     const long nv = (long)B * s.m * s.m * s.m;
     featurise(s, samples_device, B);
     forward(s, B);
-    k_channel0<<<sg::grid_n(nv), 256, 0, st>>>(nv, s.logits, s.pred);
-    sg::k_loss<<<sg::grid_n(nv, 1024), 256, 0, st>>>(nv, s.pred, nullptr, s.pred, nullptr, 1.f, nullptr);
-    sg::k_up2_f32<<<sg::grid_n((long)B * s.h->N), 256, 0, st>>>(B, s.m, s.pred, s.mask_solver, s.up_pred);
-    s.h->launches += 3;
+    sg::k_loss<<<sg::grid_n(nv, 1024), 256, 0, st>>>(nv, s.pred, nullptr, s.pred, nullptr, nullptr);
+    s.h->launches++;
+    if (want_field) {
+        sg::k_up2_f32<<<grid_bv(s, B, (long)s.h->N), 256, 0, st>>>(s.m, s.pred, s.mask_solver, s.up_pred);
+        s.h->launches++;
+    }
     GBG_CUDA_TRY(cudaGetLastError());
-    if (lik_device) return lik_evaluate(*s.h, s.up_pred, nullptr, B, lik_device);
+    if (lik_device) return lik_evaluate_coarse(*s.h, s.pred, s.mask_solver, B, lik_device);
     return GBG_OK;
 }
 
