@@ -89,3 +89,16 @@ def test_statistics_argument_errors(gbg):
             h.batch_statistics([(0.0013, 0.025, 15.2, 16.1, 15.7, 60.0)] * 3, an.L)
         with pytest.raises(_lib.GbgError):
             h.batch_statistics([(-1.0, 0.025, 15.2, 16.1, 15.7, 60.0)], an.L)
+
+
+@pytest.mark.parametrize("n,count", [(20, 1), (21, 2), (33, 72), (16, 73), (35, 144), (12, 145), (16, 288), (9, 289), (12, 576),
+                                     (9, 577), (16, 600)])
+def test_field_statistics_at_the_edges_of_the_cell_groups(gbg, oracle_lib, n, count):
+    """72, 144, 288 and 576 samples are the most a CTA holds of 256, 128, 64 and
+    32 cells; more read the fields twice. Odd n takes single-value copies."""
+    fields = propagation_fields(n, count, n + count)
+    for rules in (True, False):
+        mean, var = _device_stats(gbg, fields, rules)
+        om, ov = oracle_lib.propagation_stats(fields, reference_rules=rules)
+        assert np.array_equal(mean, om)
+        assert np.array_equal(var, ov)
