@@ -492,24 +492,59 @@ __global__ void k_adj_seed_ti(int S, size_t N, int nti, const int *__restrict__ 
     }
 }
 
+// lambda_0 off the live units, which adj_lanes_segment leaves out: from mu_0
+struct RimLambda {
+    const unsigned char *live;  // null: lambda_0 is stored everywhere
+    int rows;                   // rows of a unit
+    const float *mu, *cxs, *cy, *cz;
+    const SampleRec *rec;
+};
+__device__ __forceinline__ float rim_lambda(const RimLambda &r, int n, int s, size_t i, float p, int c, int x, int y, int z) {
+    const int pl = n * n;
+    const size_t o = i - c;
+    const float u0 = r.mu[i];
+    const float *u = r.mu + o;
+    const bool last = r.rec[s].nsteps == 1;
+    const float a = last ? r.rec[s].a2 : r.rec[s].a, b = last ? r.rec[s].b2 : r.rec[s].b;
+    const int cW = c - x + wm(x, n), cE = c - x + wp(x, n), cS = c + (wm(y, n) - y) * n, cN = c + (wp(y, n) - y) * n;
+    const int cB = c + (wm(z, n) - z) * pl, cF = c + (wp(z, n) - z) * pl;
+    float lu = fabsf(r.cxs[cW]) * (u[cW] - u0);
+    lu = fmaf(fabsf(r.cxs[c]), u[cE] - u0, lu);
+    lu = fmaf(r.cy[cS], u[cS] - u0, lu);
+    lu = fmaf(r.cy[c], u[cN] - u0, lu);
+    lu = fmaf(r.cz[cB], u[cB] - u0, lu);
+    lu = fmaf(r.cz[c], u[cF] - u0, lu);
+    return fmaf(a, lu, u0 * (1.0f + b * (1.0f - 2.0f * p)));
+}
+
 // dlogL/dx0 = sum_c lambda0_c * phi0_c * (x_c - x0) / sigma^2 (same for y0, z0)
 template <typename Real>
 // lam1 non-null: lambda_0 of sample s is in lam1 when ns[s] is odd (the fused
 // backward kernel's ping-pong), else in lam
 __global__ void k_adj_ic_grad(int n, const gbg_sample *__restrict__ smp, double sigma, const Real *__restrict__ lam_,
                               const Real *__restrict__ lam1, const int *__restrict__ ns, const Real *__restrict__ phi0,
-                              double *__restrict__ gx) {
+                              double *__restrict__ gx, RimLambda rim, const int *__restrict__ box) {
     const size_t N = (size_t)n * n * n;
     const int s = blockIdx.y;
     const Real *lam = (lam1 && (ns[s] & 1)) ? lam1 : lam_;
     double acc[3] = {0, 0, 0};
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < (int)N; c += gridDim.x * blockDim.x) {
+    // the rows of the initial support's box where one is given
+    int y0 = 0, ny = n, z0 = 0, nz = n;
+    if (box) {
+        y0 = n - box[4 * s];
+        ny = box[4 * s + 1] ? box[4 * s + 1] - y0 : 0;
+        z0 = n - box[4 * s + 2];
+        nz = box[4 * s + 3] ? box[4 * s + 3] - z0 : 0;
+    }
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n * ny * nz; q += gridDim.x * blockDim.x) {
+        const int c = q % n + n * (y0 + q / n % ny + n * (z0 + q / (n * ny)));
         const size_t i = (size_t)s * N + c;
         // a cell outside the initial support adds exactly zero: skip its FP64 work
         if (phi0[i] == (Real)0) continue;
-        const double w = (double)lam[i] * (double)phi0[i] / (sigma * sigma);
         int x, y, z;
         decomp(c, n, x, y, z);
+        const Real l0 = rim.live && rim.live[y / rim.rows * n + z] != 1 ? (Real)rim_lambda(rim, n, s, i, (float)phi0[i], c, x, y, z) : lam[i];
+        const double w = (double)l0 * (double)phi0[i] / (sigma * sigma);
         acc[0] += w * (x - smp[s].x0);
         acc[1] += w * (y - smp[s].y0);
         acc[2] += w * (z - smp[s].z0);
@@ -818,7 +853,15 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
     // sample: before step k sample s has taken ns[s] - 1 - k backward steps, so
     // its lambda is in mu when that count is odd.
     const unsigned gcx = (unsigned)std::min<size_t>((N + 255) / 256, (size_t)h.num_sms * 4);
-    const bool fused = f32 && n == fb::NN;
+    // Where the anatomy's units fit the CTAs' shared memory (any on a GB300)
+    // the lanes kernel takes its place: lambda in lam, mu in mu and fin, whose
+    // final states the seed has read.
+    const bool lanes = f32 && pop_fwd && adj_lanes_fit(h);
+    const bool fused = f32 && n == fb::NN && !lanes;
+    if (lanes) {
+        ADJ_TRY(cudaMemsetAsync(mu, 0, SN * sizeof(Real), st));
+        ADJ_TRY(cudaMemsetAsync(fin, 0, SN * sizeof(Real), st));
+    }
     std::vector<SampleRec> rrec(pop_fwd ? S : 0);
     if (fused) {
         constexpr int tiles = (fb::NN / fb::RY) * (fb::NN / fb::TZ);
@@ -852,7 +895,7 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
             if (most > 0) {
                 ADJ_TRY(cudaMemcpyAsync(drec, rrec.data(), (size_t)act * sizeof(SampleRec), cudaMemcpyHostToDevice,
                                         st));
-                rc = population_steps(h, (float *)seg, (float *)seg, drec, dsorted, drank, act, SN, dbox, k0);
+                rc = population_steps(h, (float *)seg, (float *)seg, drec, dsorted, drank, act, SN, dbox, k0, !lanes);
                 if (rc) {
                     release();
                     return rc;
@@ -866,7 +909,15 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
                 h.launches++;
             }
         }
-        for (int k = k1 - 1; k >= k0; --k) {
+        if (lanes) {
+            rc = adj_lanes_segment(h, A[k0], k0, k1, recs.data(), drec, (const float *)seg, SN, (float *)lam, (float *)mu, (float *)fin,
+                                   S, gA, gB);
+            if (rc) {
+                release();
+                return rc;
+            }
+        }
+        for (int k = k1 - 1; k >= k0 && !lanes; --k) {
             const Real *phik = seg + (size_t)(k - k0) * S * N;
             if (fused) {
                 constexpr int tiles = (fb::NN / fb::RY) * (fb::NN / fb::TZ);
@@ -887,8 +938,9 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
             }
         }
     }
+    const RimLambda rim{lanes ? h.unit_live : nullptr, 2, (const float *)mu, h.cxs, h.cy, h.cz, drec};
     k_adj_ic_grad<Real><<<dim3(gcx, (unsigned)S), 256, 0, st>>>(n, dsm, o.ic_sigma, lam, fused ? mu : nullptr, dns,
-                                                                ck, gX);
+                                                                ck, gX, rim, f32 ? dbox : nullptr);
     h.launches++;
     ADJ_TRY(cudaGetLastError());
     std::vector<double> hA((size_t)nmax * S), hB((size_t)nmax * S), hX(3 * S);

@@ -155,12 +155,16 @@ struct Handle {
     int live_tz = 0, live_ry = 0;
     bool live_valid = false;
 
-    // units of the resident-anatomy population kernel (rd_lanes.cu): which
-    // hold a live cell, the list of those with its length behind it, the
-    // length on the host, and the kernel's barrier words
+    // units of the resident-anatomy kernels (rd_lanes.cu): which hold a live
+    // cell (1) or border one that does (2), the lists of the first, the second
+    // and of all but the first with their lengths, and the kernels' barrier
+    // words; for n = 128 the adjoint's blocks of 16 units with a live one
+    // (adj_lanes.cu) and their number
     unsigned char *unit_live = nullptr;
     int *unit_list = nullptr;
-    int units = 0;
+    int units[3] = {0, 0, 0};
+    int *block_list = nullptr;
+    int blocks = 0;
     unsigned *lane_sync = nullptr;
 
     // events bracketing the latest population-kernel launch
@@ -256,9 +260,11 @@ int launch_schedule_smooth(Handle &h, const gbg_sample *samples_device, int S, d
 // as launch_gaussian_ic records them (indexed by record order) of an initial
 // state whose support lies within them grown by grow0 cells; with slot 0 it
 // also needs that state zero on every cell without the mask unless
-// grow0 = 0, and a zero-filled buf1 (in slot mode it writes every tile).
+// grow0 = 0, and a zero-filled buf1. In slot mode it writes every cell of a
+// state, or with fill_all = false at least those that a cell with the mask or
+// its stencil reads.
 int population_steps(Handle &h, float *buf0, float *buf1, const SampleRec *recs, SampleRec *sorted, int *rank,
-                     int S, size_t slot = 0, const int *box = nullptr, int grow0 = 0);
+                     int S, size_t slot = 0, const int *box = nullptr, int grow0 = 0, bool fill_all = true);
 bool population_supported(int n);
 // Builds and allocates what batch_solve_device would build or allocate on
 // first use (fast tables, the skipping kernel's tile list, likelihood
@@ -287,7 +293,17 @@ int batch_solve_device(Handle &h, const gbg_sample *samples_device, int S,
 int lanes_set_anatomy(Handle &h);
 bool lanes_fit(const Handle &h, int S);
 // as population_steps with boxes, on records sorted by step count
-int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0);
+int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0, size_t slot = 0,
+                 bool fill_all = true);
+// ---- adj_lanes.cu ----
+int adj_lanes_set_anatomy(Handle &h);
+bool adj_lanes_fit(const Handle &h);
+// backward steps of the segment [k0, k1) at n = 128 (float states): lam is
+// lambda at the segment's end and becomes lambda at its start on the live
+// units; mu0, mu1 hold zeros off them. recs: host records of the S samples
+// running at k0, longest first (nsteps of the whole solve)
+int adj_lanes_segment(Handle &h, int S, int k0, int k1, const SampleRec *recs, SampleRec *drec, const float *seg, size_t slot,
+                      float *lam, float *mu0, float *mu1, int strideS, double *gA, double *gB);
 
 // ---- propagation.cu ----
 // batched solve of S samples, then per-cell mean and variance of their final

@@ -1,0 +1,95 @@
+// What the kernels with resident anatomy (rd_lanes.cu, adj_lanes.cu) share: the
+// division of an SM into lanes, their barrier and the row arithmetic.
+#pragma once
+#include "gbg_internal.cuh"
+
+namespace gbg {
+namespace lanes {
+
+constexpr int kWps = 4;                    // warps per scheduler: 16 warps of up to 128 registers
+constexpr int kThreads = 128 * kWps;
+// Samples a team has in flight. More lanes hide more of the barrier (4: 205
+// ms, 8: 164 ms on the 512-sample population); beyond 8 the states of a 128^3
+// population outgrow L2.
+constexpr int kMaxLanes = 8;
+// a unit's table, one float4 per lane and slot: cxs (2 rows), cy (rows y-1,
+// y, y+1), cz (2 rows)
+constexpr int kSlots = 7;
+constexpr size_t kUnitBytes = (size_t)kSlots * 32 * sizeof(float4);
+constexpr int kMaxUnits = 64;              // units a CTA can own
+// Planes loaded ahead: one plane's arithmetic does not cover an L2 load (170
+// ms), a third plane spills registers (207 ms).
+constexpr int kAhead = 2;
+constexpr int kSyncStride = 32;            // words per lane of the barrier array
+
+__device__ __forceinline__ int wrapm(int i, int n) { return i == 0 ? n - 1 : i - 1; }
+__device__ __forceinline__ int wrapp(int i, int n) { return i == n - 1 ? 0 : i + 1; }
+
+// what a lane's warps share of its samples and its barrier
+struct Lane {
+    int next, ok;            // sample to take next (sorted order), no timeout so far
+    unsigned target, slot;   // arrivals the next barrier waits for, slot of the next sample number
+};
+
+__device__ __forceinline__ bool span_hits(int lo, int hi, int grow, int a, int b, int n) {
+    lo -= grow;
+    hi += grow;
+    if (lo < 0 || hi > n - 1) return true;
+    return lo <= b && a <= hi;
+}
+
+__device__ __forceinline__ void group_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release(unsigned *p) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(p) : "memory");
+}
+
+struct V4 {
+    float v[4];
+};
+__device__ __forceinline__ V4 v4(const float4 &a) { return V4{{a.x, a.y, a.z, a.w}}; }
+__device__ __forceinline__ V4 ldp(const float *p) { return v4(*reinterpret_cast<const float4 *>(p)); }
+__device__ __forceinline__ V4 ldg4(const float *p) { return v4(__ldg(reinterpret_cast<const float4 *>(p))); }
+__device__ __forceinline__ V4 lds(const float4 *p) { return v4(*p); }
+__device__ __forceinline__ V4 sub(const V4 &a, const V4 &b) {
+    return V4{{a.v[0] - b.v[0], a.v[1] - b.v[1], a.v[2] - b.v[2], a.v[3] - b.v[3]}};
+}
+
+// Barrier of a team's T CTAs on one lane, by one thread of the lane after its
+// warps have met: sync[0] counts arrivals. With `last` (the sample's last
+// step) rank 0 draws the lane's next sample from `queue` before it arrives, and
+// everyone reads it after: two slots in turn, as a CTA may still have to read
+// one when the next is written. Bounded (seconds); on a timeout the status word
+// is set and every lane leaves at its next barrier.
+__device__ __forceinline__ void lane_barrier(Lane &ln, unsigned *sync, unsigned *queue, int T, int rank, int lanes, bool last,
+                                             int *status) {
+    const unsigned target = ln.target + T;
+    if (last && rank == 0) *(volatile unsigned *)(sync + 1 + ln.slot) = atomicAdd(queue, 1u) + (unsigned)lanes;
+    red_release(sync);
+    long long spins = 0;
+    while (ld_acquire(sync) < target) {
+        if (++spins > (1ll << 24)) {
+            atomicExch(status, (int)DEV_BARRIER_TIMEOUT);
+            ln.ok = 0;
+            break;
+        }
+        if ((spins & 1023) == 0 && *(volatile int *)status != DEV_OK) {
+            ln.ok = 0;
+            break;
+        }
+    }
+    ln.target = target;
+    if (last) {
+        ln.next = (int)*(volatile unsigned *)(sync + 1 + ln.slot);
+        ln.slot ^= 1u;
+    }
+}
+
+}  // namespace lanes
+}  // namespace gbg

@@ -226,64 +226,68 @@ __device__ __forceinline__ float gaussian_ic_value(int x, int y, int z, double x
     return v;
 }
 
-// Grid: y over samples, x over groups of four consecutive cells of one
-// sample (float4 stores when n is a multiple of 4, cell by cell otherwise).
+// The nonzero cells of the initial densities, over zero-filled fields. Grid: y
+// over samples, x over the cells of the box around the seed outside which the
+// screen above gives 0 (the whole grid where it does not apply). Looking at
+// every cell of every field instead took 1.0 ms for 64 samples of 128^3 and 53
+// us for one; filling the fields with zeros and this kernel take MEASURED.
 // 32-bit index arithmetic inside a sample (n <= 1024, n^3 < 2^32).
-// box non-null (the skipping population kernel): the y and z extent of the
+// box non-null (the skipping population kernels): the y and z extent of the
 // cells given a nonzero value is recorded per sample as four ints
 // {n - ymin, ymax + 1, n - zmin, zmax + 1} (all 0: no nonzero cell) with
 // atomicMax, from zero-filled entries.
-__device__ __forceinline__ void record_support(int *box, int n, int y, int z) {
-    atomicMax(box + 0, n - y);
-    atomicMax(box + 1, y + 1);
-    atomicMax(box + 2, n - z);
-    atomicMax(box + 3, z + 1);
-}
-
-__global__ void k_gaussian_ic(int n, const gbg_sample *__restrict__ smp, int S, double peak,
+__global__ void __launch_bounds__(256) k_gaussian_ic(int n, const gbg_sample *__restrict__ smp, int S, double peak,
                               double sigma, const double *__restrict__ pw, const double *__restrict__ pg,
                               float *__restrict__ phi, float *__restrict__ phi1 = nullptr,
                               const SampleRec *__restrict__ recs = nullptr, int *__restrict__ box = nullptr) {
-    const unsigned un = (unsigned)n, N = un * un * un, groups = (N + 3) / 4;
+    const unsigned un = (unsigned)n, N = un * un * un;
     const double two_s2 = __dmul_rn(__dmul_rn(2.0, sigma), sigma);
     const float screen = (float)(two_s2 * 120.0) + 1.0f;
+    const float reach = peak > 1.0 ? 4.0f * n : sqrtf(screen) + 2.0f;  // 2: float rounding of the distances
     for (unsigned s = blockIdx.y; s < (unsigned)S; s += gridDim.y) {
-        const double x0 = smp[s].x0, y0 = smp[s].y0, z0 = smp[s].z0;
+        const double p0[3] = {smp[s].x0, smp[s].y0, smp[s].z0};
+        int lo[3], len[3];
+        for (int d = 0; d < 3; ++d) {
+            // the screen compares float distances, so a seed far outside the
+            // grid has an empty box in either form
+            const float c = (float)p0[d];
+            lo[d] = c - reach > 0.0f ? (c - reach < (float)n ? (int)(c - reach) : n) : 0;
+            const int hi = c + reach < (float)(n - 1) ? (c + reach >= 0.0f ? (int)(c + reach) : -1) : n - 1;
+            len[d] = hi >= lo[d] ? hi - lo[d] + 1 : 0;
+        }
+        if (peak > 1.0)
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = 0;
+                len[d] = n;
+            }
         float *dst = ((phi1 && recs && ((recs[s].nsteps / 2) & 1)) ? phi1 : phi) + (size_t)s * N;
-        for (unsigned g = blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += gridDim.x * blockDim.x) {
-            const unsigned c = 4 * g;
-            if ((un & 3u) == 0) {
-                const unsigned row = c / un;
-                const int x = (int)(c - row * un), y = (int)(row % un), z = (int)(row / un);
-                float v[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    v[j] = gaussian_ic_value(x + j, y, z, x0, y0, z0, peak, two_s2, screen, pw, pg, c + j);
-                *reinterpret_cast<float4 *>(dst + c) = make_float4(v[0], v[1], v[2], v[3]);
-                if (box && (v[0] != 0.0f || v[1] != 0.0f || v[2] != 0.0f || v[3] != 0.0f))
-                    record_support(box + 4 * s, n, y, z);
-            } else {
-                for (unsigned cj = c; cj < c + 4 && cj < N; ++cj) {
-                    const unsigned row = cj / un;
-                    const float v = gaussian_ic_value((int)(cj - row * un), (int)(row % un), (int)(row / un), x0,
-                                                      y0, z0, peak, two_s2, screen, pw, pg, cj);
-                    dst[cj] = v;
-                    if (box && v != 0.0f) record_support(box + 4 * s, n, (int)(row % un), (int)(row / un));
-                }
+        const unsigned cells = (unsigned)len[0] * (unsigned)len[1] * (unsigned)len[2];
+        int ext[4] = {0, 0, 0, 0};
+        for (unsigned g = blockIdx.x * blockDim.x + threadIdx.x; g < cells; g += gridDim.x * blockDim.x) {
+            const unsigned r = g / (unsigned)len[0];
+            const int x = lo[0] + (int)(g % (unsigned)len[0]), y = lo[1] + (int)(r % (unsigned)len[1]), z = lo[2] + (int)(r / (unsigned)len[1]);
+            const unsigned c = (unsigned)x + un * ((unsigned)y + un * (unsigned)z);
+            const float v = gaussian_ic_value(x, y, z, p0[0], p0[1], p0[2], peak, two_s2, screen, pw, pg, c);
+            if (v != 0.0f) {
+                dst[c] = v;
+                ext[0] = max(ext[0], n - y);
+                ext[1] = max(ext[1], y + 1);
+                ext[2] = max(ext[2], n - z);
+                ext[3] = max(ext[3], z + 1);
             }
         }
+        if (box)
+            for (int k = 0; k < 4; ++k) {
+                const int m = __reduce_max_sync(0xffffffffu, ext[k]);
+                if ((threadIdx.x & 31) == 0 && m) atomicMax(box + 4 * s + k, m);
+            }
     }
 }
 
 dim3 ic_grid(const Handle &h, int S) {
-    const unsigned groups = (unsigned)((h.N + 3) / 4);
-    unsigned gx = (groups + 255) / 256;
-    if (gx > 128) gx = 128;
-    unsigned gy = (unsigned)h.num_sms * 16 / gx;
-    if (gy < 1) gy = 1;
-    if (gy > (unsigned)S) gy = (unsigned)S;
-    if (gy > 65535) gy = 65535;
-    return dim3(gx, gy);
+    const unsigned per = (unsigned)((h.N + 255) / 256);
+    const unsigned gx = per < 32 ? per : 32;
+    return dim3(gx, (unsigned)(S < 65535 ? S : 65535));
 }
 
 // Bounded grid barrier for the cooperative persistent kernel. Returns false
@@ -1328,7 +1332,7 @@ int ensure_live_tiles(Handle &h, int rows, int tz) {
 // kernel
 int launch_population(Handle &h, float *buf0, float *buf1, const SampleRec *rec_sorted, int S,
                       bool allow_tb = true, bool allow_skip = false, size_t slot = 0,
-                      const int *box = nullptr, int grow0 = 0) {
+                      const int *box = nullptr, int grow0 = 0, bool fill_all = true) {
     const int LR = lanes_per_row(h.n);
     if (!LR) {
         set_error("fast path supports n = 32, 64 or 128");
@@ -1343,10 +1347,11 @@ int launch_population(Handle &h, float *buf0, float *buf1, const SampleRec *rec_
     // skipping shape's tile depth (the default one's otherwise)
     const int slot_tz = (h.pop_variant >= 0 && h.pop_variant < nv && vs[h.pop_variant].skip) ? vs[h.pop_variant].tz
                                                                                             : vs[0].tz;
-    if (!slot && vs[vi].resident) {
+    if (vs[vi].resident) {
         // an anatomy whose units do not fit the CTAs' shared memory (fewer SMs
         // than a GB300 has) runs the tile march, the next variant
-        if (lanes_fit(h, S)) return lanes_launch(h, buf0, buf1, rec_sorted, S, box ? box : batch_boxes(h), grow0);
+        if (lanes_fit(h, S))
+            return lanes_launch(h, buf0, buf1, rec_sorted, S, box ? box : batch_boxes(h), grow0, slot, fill_all);
         ++vi;
     }
     const PopVariant v = slot ? slot_variant(h.n, box != nullptr, slot_tz) : vs[vi];
@@ -1391,7 +1396,7 @@ int launch_population(Handle &h, float *buf0, float *buf1, const SampleRec *rec_
 }  // namespace
 
 int population_steps(Handle &h, float *buf0, float *buf1, const SampleRec *recs, SampleRec *sorted, int *rank,
-                     int S, size_t slot, const int *box, int grow0) {
+                     int S, size_t slot, const int *box, int grow0, bool fill_all) {
     if (!lanes_per_row(h.n)) {
         set_error("fast path supports n = 32, 64 or 128");
         return GBG_ERR_UNSUPPORTED;
@@ -1400,7 +1405,7 @@ int population_steps(Handle &h, float *buf0, float *buf1, const SampleRec *recs,
     k_sort_schedule<<<(S + 127) / 128, 128, 0, h.stream>>>(recs, S, sorted, rank);
     h.launches++;
     GBG_CUDA_TRY(cudaGetLastError());
-    return launch_population(h, buf0, buf1, sorted, S, false, box != nullptr, slot, box, grow0);
+    return launch_population(h, buf0, buf1, sorted, S, false, box != nullptr, slot, box, grow0, fill_all);
 }
 
 bool population_supported(int n) { return lanes_per_row(n) != 0; }
@@ -1455,6 +1460,7 @@ int launch_schedule_smooth(Handle &h, const gbg_sample *samples_device, int S, d
 
 int launch_gaussian_ic(Handle &h, const gbg_sample *samples_device, int S, double peak, double sigma,
                        float *phi, int *box) {
+    GBG_CUDA_TRY(cudaMemsetAsync(phi, 0, (size_t)S * h.N * sizeof(float), h.stream));
     k_gaussian_ic<<<ic_grid(h, S), 256, 0, h.stream>>>(h.n, samples_device, S, peak, sigma, h.pw, h.pg, phi,
                                                         nullptr, nullptr, box);
     h.launches++;
@@ -1506,33 +1512,31 @@ int batch_solve_device(Handle &h, const gbg_sample *samples_device, int S,
         set_error("S out of range (1..max_samples)");
         return GBG_ERR_ARG;
     }
-    const bool f32ref = h.prec == GBG_PREC_F32REF;
+    if (h.prec != GBG_PREC_F32) {  // no population buffers
+        set_error("the batched solver runs on the fast path (GBG_PREC_F32) only");
+        return GBG_ERR_UNSUPPORTED;
+    }
     SampleRec *unsorted = batch_unsorted(h);
     SampleRec *sorted = batch_sorted(h);
     int *rank_of = batch_rank_of(h);
     if (o.dt0 != 0)
         k_schedule_smooth<<<(S + 127) / 128, 128, 0, h.stream>>>(samples_device, S, h.n, o.L, o.dt0, unsorted);
     else
-        k_schedule<<<(S + 127) / 128, 128, 0, h.stream>>>(samples_device, S, h.n, o.L, f32ref ? 1 : 0,
+        k_schedule<<<(S + 127) / 128, 128, 0, h.stream>>>(samples_device, S, h.n, o.L, 0,
                                                           unsorted);
     k_sort_schedule<<<(S + 127) / 128, 128, 0, h.stream>>>(unsorted, S, sorted, rank_of);
     const bool tb = variant_is_tb(h);
     // the skipping kernel: initial-support boxes recorded by the IC kernel and
     // a zero-filled second buffer (it holds zeros wherever a round skips)
-    const bool skip = !f32ref && variant_is_skip(h);
-    if (skip) {
-        GBG_CUDA_TRY(cudaMemsetAsync(batch_boxes(h), 0, (size_t)S * 4 * sizeof(int), h.stream));
-        GBG_CUDA_TRY(cudaMemsetAsync(h.bphi[1], 0, (size_t)S * h.N * sizeof(float), h.stream));
-    }
+    const bool skip = variant_is_skip(h);
+    if (skip) GBG_CUDA_TRY(cudaMemsetAsync(batch_boxes(h), 0, (size_t)S * 4 * sizeof(int), h.stream));
+    GBG_CUDA_TRY(cudaMemsetAsync(h.bphi[0], 0, (size_t)S * h.N * sizeof(float), h.stream));
+    if (skip || tb) GBG_CUDA_TRY(cudaMemsetAsync(h.bphi[1], 0, (size_t)S * h.N * sizeof(float), h.stream));
     k_gaussian_ic<<<ic_grid(h, S), 256, 0, h.stream>>>(h.n, samples_device, S, o.ic_peak, o.ic_sigma, h.pw,
                                                         h.pg, h.bphi[0], tb ? h.bphi[1] : nullptr,
                                                         tb ? unsorted : nullptr, skip ? batch_boxes(h) : nullptr);
     h.launches += 3;
     GBG_CUDA_TRY(cudaGetLastError());
-    if (f32ref) {
-        set_error("the batched solver runs on the fast path (GBG_PREC_F32) only");
-        return GBG_ERR_UNSUPPORTED;
-    }
     int rc = fast_build_tables(h, (double)0.1f);
     if (rc) return rc;
     rc = launch_population(h, h.bphi[0], h.bphi[1], sorted, S, true, skip);

@@ -27,39 +27,23 @@
 // now: 512 prior draws at 128^3 243 -> 164 ms; 64 draws near the mode, stable
 // grid, 14.0 -> 10.0 ms; one of them 1.01 -> 0.61 ms; 512 at 64^3 53 -> 26 ms.
 #include <algorithm>
+#include <type_traits>
 
-#include "gbg_internal.cuh"
+#include "lanes.cuh"
 
 namespace gbg {
 namespace {
-
-constexpr int kWps = 4;                    // warps per scheduler: 16 warps of up to 128 registers
-constexpr int kThreads = 128 * kWps;
-// Samples a team has in flight. More lanes hide more of the barrier (4: 205
-// ms, 8: 164 ms on the 512-sample population); beyond 8 the states of a 128^3
-// population outgrow L2.
-constexpr int kMaxLanes = 8;
-// a unit's table, one float4 per lane and slot: cxs (2 rows), cy (rows y-1,
-// y, y+1), cz (2 rows)
-constexpr int kSlots = 7;
-constexpr size_t kUnitBytes = (size_t)kSlots * 32 * sizeof(float4);
-constexpr int kMaxUnits = 64;              // units a CTA can own
-// Planes loaded ahead: one plane's arithmetic does not cover an L2 load (170
-// ms), a third plane spills registers (207 ms).
-constexpr int kAhead = 2;
-constexpr int kSyncStride = 32;            // words per lane of the barrier array
-
-__device__ __forceinline__ int wrapm(int i, int n) { return i == 0 ? n - 1 : i - 1; }
-__device__ __forceinline__ int wrapp(int i, int n) { return i == n - 1 ? 0 : i + 1; }
+using namespace lanes;
 
 struct LaneArgs {
     int S, T, teams, lanes, warps;
     int nlive, units, grow0;
-    size_t stride;
+    size_t stride, slot;  // slot: floats between kept states (kernels with KEEP)
     float *buf0, *buf1;
     const float *cxs, *cy, *cz;
     const SampleRec *rec;
-    const int *list;
+    const int *list, *fill;  // live units; units KEEP writes zeros in (nfill of them)
+    int nfill;
     const unsigned char *live;
     const int *box;
     unsigned *sync;   // queue counter, then per lane: arrivals, next sample (two slots)
@@ -71,39 +55,8 @@ struct LaneArgs {
 struct Sample {
     SampleRec rec;
     int ylo, yhi, zlo, zhi;
-    int next, ok;
-    unsigned target, slot;
+    Lane lane;
 };
-
-__device__ __forceinline__ bool span_hits(int lo, int hi, int grow, int a, int b, int n) {
-    lo -= grow;
-    hi += grow;
-    if (lo < 0 || hi > n - 1) return true;
-    return lo <= b && a <= hi;
-}
-
-__device__ __forceinline__ void group_sync(int id, int threads) {
-    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
-}
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_release(unsigned *p) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(p) : "memory");
-}
-
-struct V4 {
-    float v[4];
-};
-__device__ __forceinline__ V4 v4(const float4 &a) { return V4{{a.x, a.y, a.z, a.w}}; }
-__device__ __forceinline__ V4 ldp(const float *p) { return v4(*reinterpret_cast<const float4 *>(p)); }
-__device__ __forceinline__ V4 ldg4(const float *p) { return v4(__ldg(reinterpret_cast<const float4 *>(p))); }
-__device__ __forceinline__ V4 lds(const float4 *p) { return v4(*p); }
-__device__ __forceinline__ V4 sub(const V4 &a, const V4 &b) {
-    return V4{{a.v[0] - b.v[0], a.v[1] - b.v[1], a.v[2] - b.v[2], a.v[3] - b.v[3]}};
-}
 
 // One row of four cells. DS = sS * (row(y-1) - P), DT = row(y+1) - P,
 // DB = P - plane(z-1), DF = plane(z+1) - P.
@@ -188,7 +141,10 @@ __device__ __forceinline__ void march(const float4 *__restrict__ tab, int y, int
     }
 }
 
-template <int LR, int WPS>
+// KEEP: every state is kept (step k reads buf0 + k * slot, writes buf0 + (k + 1)
+// * slot) over arbitrary older contents, so the live units outside the grown
+// support and the units of the fill list are written with zeros.
+template <int LR, int WPS, bool KEEP>
 __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
     constexpr int n = 4 * LR, SUB = 32 / LR, ROWS = 2 * SUB;
     extern __shared__ __align__(16) float4 tab[];
@@ -221,16 +177,13 @@ __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
     Sample &sm = s_smp[g];
     const int tl = g * p.teams + team;
     if (w == 0 && lane == 0) {
-        sm.next = tl;
-        sm.target = 0;
-        sm.ok = 1;
-        sm.slot = 0;
+        sm.lane = Lane{tl, 1, 0u, 0u};
     }
     unsigned visited = 0;
     for (;;) {
         group_sync(1 + g, 32 * p.warps);
-        const int r = sm.next;
-        if (r >= p.S || !sm.ok) break;
+        const int r = sm.lane.next;
+        if (r >= p.S || !sm.lane.ok) break;
         if (w == 0 && lane == 0) {
             sm.rec = p.rec[r];
             const int4 bx = reinterpret_cast<const int4 *>(p.box)[sm.rec.order];
@@ -246,72 +199,56 @@ __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
         for (int k = 0; k < nsteps; ++k) {
             {
                 const size_t off = (size_t)sm.rec.order * p.stride;
-                const float *in = ((k & 1) ? p.buf1 : p.buf0) + off;
-                float *out = ((k & 1) ? p.buf0 : p.buf1) + off;
+                const float *in = (KEEP ? p.buf0 + (size_t)k * p.slot : ((k & 1) ? p.buf1 : p.buf0)) + off;
+                float *out = (KEEP ? p.buf0 + (size_t)(k + 1) * p.slot : ((k & 1) ? p.buf0 : p.buf1)) + off;
+                auto zero = [&](int y0, int z) {  // unit (row group y0, plane z) of the output
+                    float *o = out + 4 * li + (size_t)n * (y0 + 2 * sub_r + (size_t)n * z);
+                    *reinterpret_cast<float4 *>(o) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4 *>(o + n) = make_float4(0.f, 0.f, 0.f, 0.f);
+                };
                 const bool lastk = k == nsteps - 1;
                 const float a = lastk ? sm.rec.a2 : sm.rec.a, b = lastk ? sm.rec.b2 : sm.rec.b;
                 const bool any = sm.rec.a >= 0.f;
                 const int grow = p.grow0 + k + 1, u1 = nu * (w + 1) / p.warps;
-                for (int i = nu * w / p.warps; any && i < u1;) {
+                for (int i = nu * w / p.warps; (KEEP || any) && i < u1;) {
                     const int un = s_unit[i], y0 = un & 1023, z = un >> 10 & 1023, len = min(un >> 20, u1 - i);
                     int za = z, zb = z + len;
                     if (sm.zlo >= grow && sm.zhi + grow < n) {
                         za = max(za, sm.zlo - grow);
                         zb = min(zb, sm.zhi + grow + 1);
                     }
-                    if (za < zb && span_hits(sm.ylo, sm.yhi, grow, y0, y0 + ROWS - 1, n)) {
+                    if (!any || !span_hits(sm.ylo, sm.yhi, grow, y0, y0 + ROWS - 1, n)) zb = za;
+                    if (za < zb) {
                         march<LR>(tab + (i + za - z) * kSlots * 32 + lane, y0 + 2 * sub_r, za, zb - za, in, out, p.cz, a, b);
                         visited += zb - za;
                     }
+                    if (KEEP)
+                        for (int q = z; q < z + len; ++q)
+                            if (q < za || q >= zb) zero(y0, q);
                     i += len;
                 }
-                if (k == 1 && any) {
+                if (KEEP) {
+                    for (int i = rank + p.T * w; i < p.nfill; i += p.T * p.warps) zero(p.fill[i] / n * ROWS, p.fill[i] % n);
+                } else if (k == 1 && any) {
                     // units without a live cell that the initial state may have
                     // left values in: zeros, as their step gives
-                    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
                     for (int u = rank + p.T * w; u < p.units; u += p.T * p.warps) {
                         const int y0 = (u / n) * ROWS, z = u % n;
-                        if (p.live[u] || !span_hits(sm.ylo, sm.yhi, p.grow0, y0, y0 + ROWS - 1, n) ||
-                            !span_hits(sm.zlo, sm.zhi, p.grow0, z, z, n))
-                            continue;
-                        float *o = out + 4 * li + (size_t)n * (y0 + 2 * sub_r + (size_t)n * z);
-                        *reinterpret_cast<float4 *>(o) = z4;
-                        *reinterpret_cast<float4 *>(o + n) = z4;
+                        if (p.live[u] != 1 && span_hits(sm.ylo, sm.yhi, p.grow0, y0, y0 + ROWS - 1, n) &&
+                            span_hits(sm.zlo, sm.zhi, p.grow0, z, z, n))
+                            zero(y0, z);
                     }
                 }
             }
             // barrier of the team's CTAs on this lane
             group_sync(1 + g, 32 * p.warps);
             if (w == 0 && lane == 0) {
-                unsigned *sync = p.sync + (size_t)(tl + 1) * kSyncStride;
-                const bool lastk = k == nsteps - 1;
-                const unsigned target = sm.target + p.T;
-                if (lastk && rank == 0) {
-                    const unsigned nx = atomicAdd(p.sync, 1u) + (unsigned)(p.teams * p.lanes);
-                    *(volatile unsigned *)(sync + 1 + sm.slot) = nx;
-                }
-                red_release(sync);
-                long long spins = 0;
-                while (ld_acquire(sync) < target) {
-                    if (++spins > (1ll << 24)) {  // seconds
-                        atomicExch(p.status, (int)DEV_BARRIER_TIMEOUT);
-                        sm.ok = 0;
-                        break;
-                    }
-                    if ((spins & 1023) == 0 && *(volatile int *)p.status != DEV_OK) {
-                        sm.ok = 0;
-                        break;
-                    }
-                }
-                sm.target = target;
-                if (lastk) {
-                    sm.next = (int)*(volatile unsigned *)(sync + 1 + sm.slot);
-                    sm.slot ^= 1u;
-                }
+                lane_barrier(sm.lane, p.sync + (size_t)(tl + 1) * kSyncStride, p.sync, p.T, rank, p.teams * p.lanes, k == nsteps - 1,
+                             p.status);
             }
             if (k == nsteps - 1) break;
             group_sync(1 + g, 32 * p.warps);
-            if (!sm.ok) break;
+            if (!sm.lane.ok) break;
         }
     }
     if (lane == 0 && visited) atomicAdd(p.visited, (unsigned long long)visited);
@@ -337,8 +274,19 @@ __global__ void k_unit_live(int n, int rows, const double *__restrict__ pw, cons
     if (threadIdx.x == 0) live[blockIdx.x] = (unsigned char)(any != 0);
 }
 
-// indices of the live units in increasing order, and their count (one CTA)
-__global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned char *__restrict__ live, int *__restrict__ list,
+// live[u] = 2 for units without a live cell next to a live one (rows or planes)
+__global__ void k_unit_rim(int n, int units, unsigned char *__restrict__ live) {
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= units || live[u] == 1) return;
+    const int z = u % n, y = u / n, ny = units / n;
+    if (live[y * n + wrapm(z, n)] == 1 || live[y * n + wrapp(z, n)] == 1 || live[wrapm(y, ny) * n + z] == 1 ||
+        live[wrapp(y, ny) * n + z] == 1)
+        live[u] = 2;
+}
+
+// indices of the units with live == want (want < 0: with live != 1) in increasing
+// order, and their count (one CTA)
+__global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned char *__restrict__ live, int want, int *__restrict__ list,
                                                      int *__restrict__ count) {
     __shared__ int sums[32];
     __shared__ int total;
@@ -347,7 +295,7 @@ __global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned ch
     __syncthreads();
     for (int base = 0; base < units; base += 1024) {
         const int i = base + threadIdx.x;
-        const int f = i < units && live[i];
+        const int f = i < units && (want < 0 ? live[i] != 1 : live[i] == want);
         const unsigned m = __ballot_sync(0xffffffffu, f);
         if (lane == 0) sums[warp] = __popc(m);
         __syncthreads();
@@ -371,15 +319,21 @@ int lanes_set_anatomy(Handle &h) {
     const int nu = units_of(h.n);
     if (!h.unit_live) {
         GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_live, nu));
-        GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_list, (nu + 1) * sizeof(int)));
+        GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_list, 3 * (nu + 1) * sizeof(int)));
         GBG_CUDA_TRY(cudaMalloc((void **)&h.lane_sync, (size_t)(h.num_sms * kMaxLanes + 1) * kSyncStride * sizeof(unsigned)));
     }
     k_unit_live<<<nu, 128, 0, h.stream>>>(h.n, unit_rows(h.n), h.pw, h.pg, h.unit_live);
-    k_unit_list<<<1, 1024, 0, h.stream>>>(nu, h.unit_live, h.unit_list, h.unit_list + nu);
-    h.launches += 2;
+    k_unit_rim<<<(nu + 127) / 128, 128, 0, h.stream>>>(h.n, nu, h.unit_live);
+    // live units | units without a live cell that a live unit's stencil reads |
+    // all units without a live cell, each list with its length behind it
+    for (int l = 0; l < 3; ++l)
+        k_unit_list<<<1, 1024, 0, h.stream>>>(nu, h.unit_live, l == 0 ? 1 : (l == 1 ? 2 : -1), h.unit_list + l * (nu + 1),
+                                              h.unit_list + l * (nu + 1) + nu);
+    h.launches += 5;
     GBG_CUDA_TRY(cudaGetLastError());
-    GBG_CUDA_TRY(cudaMemcpyAsync(&h.units, h.unit_list + nu, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
-    return GBG_OK;
+    for (int l = 0; l < 3; ++l)
+        GBG_CUDA_TRY(cudaMemcpyAsync(&h.units[l], h.unit_list + l * (nu + 1) + nu, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+    return adj_lanes_set_anatomy(h);
 }
 
 // Teams and lanes for S samples. A CTA holds at most 28 units where the chip
@@ -389,7 +343,7 @@ int lanes_set_anatomy(Handle &h) {
 // CTA, below which a step is all barrier (6 samples at 32^3: 1.71 ms at 28
 // units, 1.42 ms at 4; 32 at 64^3: 4.9 ms at 28, 4.0 ms at 14).
 static void lane_shape(const Handle &h, int S, LaneArgs &a, int &units) {
-    const int nl = std::max(1, h.units), sms = h.num_sms;
+    const int nl = std::max(1, h.units[0]), sms = h.num_sms;
     const int wide = sms / ((S + kMaxLanes - 1) / kMaxLanes), least = (nl + 27) / 28, most = (nl + 3) / 4;
     a.T = std::min(sms, std::max(least, std::min(wide, most)));
     a.teams = sms / a.T;
@@ -409,13 +363,14 @@ bool lanes_fit(const Handle &h, int S) {
     return units <= kMaxUnits && units * kUnitBytes <= 224 * 1024;
 }
 
-int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0) {
+int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0, size_t slot,
+                 bool fill_all) {
     const int n = h.n;
     LaneArgs a;
     int units;
     lane_shape(h, S, a, units);
     a.S = S;
-    a.nlive = h.units;
+    a.nlive = h.units[0];
     a.units = units_of(n);
     a.grow0 = grow0;
     a.stride = h.N;
@@ -426,15 +381,22 @@ int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, i
     a.cz = h.cz;
     a.rec = sorted;
     a.list = h.unit_list;
+    a.fill = h.unit_list + (fill_all ? 2 : 1) * (a.units + 1);
+    a.nfill = h.units[fill_all ? 2 : 1];
+    a.slot = slot;
     a.live = h.unit_live;
     a.box = box;
     a.sync = h.lane_sync;
     a.status = h.dev_status;
     a.visited = reinterpret_cast<unsigned long long *>(h.barrier + 2);
     const size_t smem = units * kUnitBytes;
-    const void *fn = n == 128  ? (const void *)k_population10<32, kWps>
-                     : n == 64 ? (const void *)k_population10<16, kWps>
-                               : (const void *)k_population10<8, kWps>;
+    auto kernel = [&](auto keep) {
+        constexpr bool K = decltype(keep)::value;
+        return n == 128  ? (const void *)k_population10<32, kWps, K>
+               : n == 64 ? (const void *)k_population10<16, kWps, K>
+                         : (const void *)k_population10<8, kWps, K>;
+    };
+    const void *fn = slot ? kernel(std::true_type{}) : kernel(std::false_type{});
     GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     GBG_CUDA_TRY(cudaMemsetAsync(h.barrier, 0, 4 * sizeof(unsigned), h.stream));
     GBG_CUDA_TRY(
