@@ -629,7 +629,10 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(Geom g, Slice in, int Cin, S
 // NW warps share the blocks so that a thread needs at most 7 x 4 or 4 x 8
 // accumulators and 32 warps fit an SM. With 8 warps for every layer, and a
 // 3-plane halo loaded and waited for per tile, 16 -> 16 took 306 us and 32 ->
-// 16 435 us on 8 samples of 64^3; now 120 and 215 us.
+// 16 435 us on 8 samples of 64^3; now 125 and 215 us. (16 -> 16 with four CTAs
+// of 8 warps takes 120 us, but twice the CTAs halve the length of the tensor
+// cores' fp32 sums, whose truncation then differs by 1e-5 from that of other
+// launches.)
 __device__ __forceinline__ void ldsm_x4_trans(unsigned r[4], const void *p) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(p);
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -1166,7 +1169,7 @@ void conv_wgrad(cudaStream_t st, Geom g, Slice in, int cin, Slice dout, int cout
     const bool tiled = g.W % 8 == 0 && g.H % 8 == 0 && in.stride % 8 == 0 && in.off % 8 == 0 &&
                        dout.stride % 8 == 0 && dout.off % 8 == 0;
     if (tiled) {
-        if (cin == 16 && cout == 16) return wgrad_tiled<16, 16, 8>(st, g, in, dout, dw, num_sms);
+        if (cin == 16 && cout == 16) return wgrad_tiled<16, 16, 16>(st, g, in, dout, dw, num_sms);
         if (cin == 16 && cout == 32) return wgrad_tiled<16, 32, 16>(st, g, in, dout, dw, num_sms);
         if (cin == 32 && cout == 16) return wgrad_tiled<32, 16, 16>(st, g, in, dout, dw, num_sms);
         if (cin == 32 && cout == 32) return wgrad_tiled<32, 32, 32>(st, g, in, dout, dw, num_sms);
