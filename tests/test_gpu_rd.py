@@ -116,3 +116,40 @@ def test_errors_are_reported(gbg):
     with pytest.raises(_lib.GbgError) as e:
         _lib.Handle(2, "f64")
     assert e.value.status == -1
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32ref"])
+@pytest.mark.parametrize("kind,n", [("ellipsoid", 37), ("scattered", 20), ("full", 24), ("grey", 21), ("none", 16), ("one", 17)])
+def test_exact_steps_over_the_live_cells_equal_oracle(gbg, oracle_lib, prec, kind, n):
+    """From the third step on the exact modes compute the cells of a list only:
+    dead cells (a NaN face) leave it, cells with a zero face (p_g only and Dg =
+    0) stay on it with the doubling. Split over calls, after a new density and
+    with new diffusivities; bit for bit the oracle's steps over every cell."""
+    rng = np.random.default_rng(n)
+    if kind == "ellipsoid":
+        an = S.make_anatomy(n, seed=2)
+        pw, pg = an.p_w, an.p_g
+    else:
+        t = {"scattered": (rng.random((n, n, n)) < 0.9), "full": np.ones((n, n, n)), "grey": rng.random((n, n, n)) < 0.97,
+             "none": np.zeros((n, n, n)), "one": np.zeros((n, n, n))}[kind].astype(float)
+        if kind == "one":
+            t[5:8, 5:8, 5:8] = 1
+        w = (rng.random((n, n, n)) < 0.5) * 1.0 if kind == "grey" else rng.random((n, n, n))
+        pw, pg = t * w, t * (1.0 - w)
+    f32 = prec == "f32ref"
+    with _lib.Handle(n, prec) as h:
+        h.set_anatomy(pw, pg)
+        for Dw_file, ratio in ((0.0013, 0.1), (0.0009, 0.0 if kind == "grey" else 0.1)):
+            dt, dw, dg = S.reference_dt(n, Dw_file, n * 0.1, f32=f32)
+            dg = dg if ratio else 0.0
+            phi = np.where(pw + pg > 0, rng.random((n, n, n)) ** 8, 0.0)
+            phi[0, 0, 0] = 0.5  # tissue or not
+            if f32:
+                phi = phi.astype(np.float32).astype(np.float64)
+            h.set_phi(phi)
+            done = 0
+            for steps in (1, 1, 1, 4, 9):
+                h.rd_step(dw, dg, 0.025, dt, steps)
+                done += steps
+                ref = oracle_lib.rd_solve(pw, pg, phi, dw, dg, 0.025, dt, done, "f32ref" if f32 else "f64")
+                assert np.array_equal(h.get_phi(), ref.astype(np.float64)), (Dw_file, done)
