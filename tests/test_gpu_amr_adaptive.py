@@ -123,3 +123,54 @@ def test_adaptive_run_argument_errors(gbg):
             h.run(0.0013, 0.1, 30.0, 6.4, bpd=4)  # no grid set
         with pytest.raises(_lib.GbgError):
             h.set_grid(amr.uniform_blocks(2), pw, pg, phi)  # 64 blocks > max_blocks 8
+
+
+def _tree(kind):
+    """Blocks of a tree: one block, a path to level 8 (beyond the device's
+    lookup), or random splits that leave jumps of several levels."""
+    if kind == "root":
+        return np.array([[0, 0, 0, 0]], dtype=np.int32)
+    rng = np.random.default_rng(kind if isinstance(kind, int) else 0)
+    leaves, done = [(0, 0, 0, 0)], []
+    while leaves:
+        lv, x, y, z = leaves.pop()
+        split = (x == y == z and x % 2 == 0 and lv < 8) if kind == "path" else (lv < 2 or (lv < 4 and rng.random() < 0.15))
+        if split:
+            leaves += [(lv + 1, 2 * x + (c & 1), 2 * y + (c >> 1 & 1), 2 * z + (c >> 2)) for c in range(8)]
+        else:
+            done.append((lv, x, y, z))
+    return np.array(done, dtype=np.int32)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32ref", "f32"])
+@pytest.mark.parametrize("kind", ["root", "path", 1, 2, 3])
+def test_device_ghost_tables_equal_host_tables(gbg, prec, kind):
+    """The tables gbg_amr_build_ghosts compiles on the device give the details
+    and steps of the host's tables (gbg_amr_ghost_tables) bit for bit, or both
+    refuse the tree; the room for them grows and is kept over grids."""
+    blocks = _tree(kind)
+    small = amr.uniform_blocks(1)
+    outs = []
+    for host in (True, False):
+        rng = np.random.default_rng(5)
+        pw, pg, phi = rng.uniform(0.05, 1.0, (3, len(blocks) * 4096))
+        with _lib.AmrHandle(max(len(blocks), 8), prec) as h:
+            h.set_grid(small, *rng.uniform(0.05, 1.0, (3, 8 * 4096)))
+            h.build_ghosts()
+            h.step(2e-6, 2e-7, 0.1, 0.5, 2)
+            h.set_grid(blocks, pw, pg, phi)
+            try:
+                if host:
+                    h.set_ghosts(*_lib.amr_ghost_tables(blocks))
+                else:
+                    h.build_ghosts()
+            except _lib.GbgError as e:
+                outs.append(str(e))
+                continue
+            detail = h.fwt_detail()
+            h.step(2e-6, 2e-7, 0.1, 0.5, 4)
+            outs.append(np.concatenate([detail.ravel(), h.get_phi().ravel()]))
+    if isinstance(outs[0], str):
+        assert isinstance(outs[1], str)
+    else:
+        assert np.array_equal(outs[0], outs[1])
