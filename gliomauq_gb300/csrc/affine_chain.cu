@@ -3,8 +3,8 @@
 //   log pi*(v) = log L(phi(v)) + log prior(v),
 //   phi(v) = m * clamp(phi0 + sum_p c_p(v - u_ref) J_p, 0, 1)
 // (the affine model of affine.cu, evaluated at the observation lists' cells
-// from the same gathered columns) for B chains at once, one CTA per chain, so
-// that a whole inner chain is one launch instead of one host round trip per
+// from the same gathered columns) for B chains at once, a cluster of CTAs per
+// chain, so that a whole inner chain is one launch instead of one host round trip per
 // step. The moves are those of the host sampler's inner chain
 // (gliomauq_gb300/mcmc.py, da): with probability axis_prob a redraw of the
 // symmetry coordinate from its prior conditional, accepted with the ratio of
@@ -72,26 +72,44 @@ __device__ __forceinline__ double uniform01(unsigned long long seed, int chain, 
     return (double)((x >> 11) + 1) * (1.0 / 9007199254740992.0);
 }
 
-__device__ double prior_logp(const ChainArgs &a, const double *v) {
-    double u[6], th[6], jac = 0.0;
-    for (int i = 0; i < 6; ++i) {
-        double s = 0.0;
-        for (int j = 0; j < 6; ++j) s += a.Ai[i * 6 + j] * v[j];
-        u[i] = s;
+// One proposal (or the start): the state it moves from, the proposed state, their
+// log priors, the move and what its acceptance needs besides the likelihood.
+struct Proposal {
+    double v[6], y[6], lpv, lpy, lqd, logu;
+    float c[12];   // the affine model's coefficients at y
+    int eval, kind;  // inside the prior; 0 random walk, 2 axis redraw, 4 independence
+};
+
+struct Matrices {
+    double chol[36], Ai[36], ind_chol[36], ind_inv[36];
+};
+
+// The functions below are a warp's: lane i < 6 holds coordinate i (the other
+// lanes hold copies of coordinate 0 that nobody reads), and every sum runs in
+// the order of the coordinates.
+__device__ __forceinline__ double coord(double x, int i) { return __shfl_sync(0xffffffffu, x, i); }
+
+__device__ __forceinline__ double row_times(const double *m, double x) {
+    const int i = (threadIdx.x & 31) < 6 ? threadIdx.x & 31 : 0;
+    double s = 0.0;
+    for (int j = 0; j < 6; ++j) s += m[i * 6 + j] * coord(x, j);
+    return s;
+}
+
+__device__ double prior_logp(const ChainArgs &a, const Matrices &m, double v) {
+    const int lane = threadIdx.x & 31, i = lane < 6 ? lane : 0;
+    const double u = row_times(m.Ai, v);
+    const bool lg = (a.log_mask >> i) & 1;
+    double th = u, jac = 0.0;
+    if (lg) th = exp(u);
+    for (int k = 0; k < 6; ++k) {
+        const double uk = coord(u, k);
+        if ((a.log_mask >> k) & 1) jac += uk;
     }
-    for (int i = 0; i < 6; ++i) {
-        if ((a.log_mask >> i) & 1) {
-            th[i] = exp(u[i]);
-            jac += u[i];
-        } else {
-            th[i] = u[i];
-        }
-    }
-    for (int i = 0; i < 6; ++i)
-        if (!(th[i] >= a.lo[i] && th[i] <= a.hi[i])) return -CUDART_INF;
+    if (!__all_sync(0xffffffffu, th >= a.lo[i] && th <= a.hi[i])) return -CUDART_INF;
     int c[3];
     for (int k = 0; k < 3; ++k) {
-        const double r = rint(th[2 + k]);
+        const double r = rint(coord(th, 2 + k));
         if (!(r >= 0.0 && r < (double)a.n)) return -CUDART_INF;
         c[k] = (int)r;
     }
@@ -102,44 +120,103 @@ __device__ double prior_logp(const ChainArgs &a, const double *v) {
 // coordinate `axis` of v redrawn from the prior conditional given the others:
 // on the line v + t e_axis the prior density is exp(alpha t) on the interval
 // the box allows; v is left unchanged when the line misses the box
-__device__ void redraw_axis(const ChainArgs &a, double *v, double q) {
-    const int ax = a.axis;
-    double u[6];
-    for (int i = 0; i < 6; ++i) {
-        double s = 0.0;
-        for (int j = 0; j < 6; ++j) s += a.Ai[i * 6 + j] * v[j];
-        u[i] = s;
+__device__ double redraw_axis(const ChainArgs &a, const Matrices &m, double v, double q) {
+    const int lane = threadIdx.x & 31, i = lane < 6 ? lane : 0, ax = a.axis;
+    const double u = row_times(m.Ai, v), col = m.Ai[i * 6 + ax];
+    const bool lg = (a.log_mask >> i) & 1;
+    double b1 = 0.0, b2 = 0.0;
+    if (lg && col != 0.0) {
+        b1 = (a.ulo[i] - u) / col;
+        b2 = (a.uhi[i] - u) / col;
     }
     double t_lo = -CUDART_INF, t_hi = CUDART_INF, alpha = 0.0;
-    for (int i = 0; i < 6; ++i) {
-        if (!((a.log_mask >> i) & 1)) continue;
-        const double col = a.Ai[i * 6 + ax];
-        alpha += col;
-        if (col == 0.0) continue;
-        const double b1 = (a.ulo[i] - u[i]) / col, b2 = (a.uhi[i] - u[i]) / col;
-        t_lo = fmax(t_lo, fmin(b1, b2));
-        t_hi = fmin(t_hi, fmax(b1, b2));
+    for (int k = 0; k < 6; ++k) {
+        const double ck = coord(col, k), k1 = coord(b1, k), k2 = coord(b2, k);
+        if (!((a.log_mask >> k) & 1)) continue;
+        alpha += ck;
+        if (ck == 0.0) continue;
+        t_lo = fmax(t_lo, fmin(k1, k2));
+        t_hi = fmin(t_hi, fmax(k1, k2));
     }
-    if (!(isfinite(t_lo) && isfinite(t_hi) && t_hi > t_lo)) return;
+    if (!(isfinite(t_lo) && isfinite(t_hi) && t_hi > t_lo)) return v;
     double t;
     if (fabs(alpha) < 1e-12)
         t = t_lo + q * (t_hi - t_lo);
     else
         t = t_lo + log1p(q * expm1(alpha * (t_hi - t_lo))) / alpha;
-    v[ax] += t;
+    return lane == ax ? v + t : v;
 }
 
-__device__ void coefficients(const ChainArgs &a, const double *v, double *c) {
-    double d[6];
-    for (int i = 0; i < 6; ++i) d[i] = v[i] - a.u_ref[i];
-    for (int i = 0; i < 6; ++i) c[i] = d[i];
+// six normals from the step's draws 2 to 7, in float: their precision does not
+// matter, the state they move stays double
+__device__ double normals(const ChainArgs &a, int chain, int s) {
+    const int lane = threadIdx.x & 31, i = lane < 6 ? lane : 0, k = i / 2;
+    const float r = sqrtf(-2.0f * logf((float)uniform01(a.seed, chain, s, 2 + 2 * k)));
+    float sn, cs;
+    sincospif(2.0f * (float)uniform01(a.seed, chain, s, 3 + 2 * k), &sn, &cs);
+    return (double)(i & 1 ? r * sn : r * cs);
+}
+
+// fills in what follows from y: the prior and the coefficients
+__device__ void finish(const ChainArgs &a, const Matrices &m, double v, double y, double lpv, double lqd, int kind, double logu,
+                       Proposal *o) {
+    const int lane = threadIdx.x & 31;
+    const double lpy = prior_logp(a, m, y);
+    const double d = lane < 6 ? y - a.u_ref[lane] : 0.0;
+    if (lane < 6) {
+        o->v[lane] = v;
+        o->y[lane] = y;
+        o->c[lane] = (float)d;
+    }
     if (a.quad_axis >= 0) {
         const int ax = a.quad_axis;
-        c[6] = 0.5 * (d[ax] * d[ax]);
-        int k = 7;
-        for (int i = 0; i < 6; ++i)
-            if (i != ax) c[k++] = d[ax] * d[i];
+        const double da = coord(d, ax);
+        if (lane < 6) {
+            if (lane == ax)
+                o->c[6] = (float)(0.5 * (da * da));
+            else
+                o->c[lane < ax ? 7 + lane : 6 + lane] = (float)(da * d);
+        }
     }
+    if (lane == 0) {
+        o->lpv = lpv;
+        o->lpy = lpy;
+        o->lqd = lqd;
+        o->logu = logu;
+        o->eval = isfinite(lpy) ? 1 : 0;
+        o->kind = kind;
+    }
+}
+
+// the proposal of step s from v
+__device__ void propose(const ChainArgs &a, const Matrices &m, int chain, int s, double v, double lpv, Proposal *o) {
+    const int lane = threadIdx.x & 31, i = lane < 6 ? lane : 0;
+    const double um = uniform01(a.seed, chain, s, 0);
+    const bool jump = a.axis >= 0 && um <= a.axis_prob;
+    const bool indep = !jump && um <= (a.axis >= 0 ? a.axis_prob : 0.0) + a.ind_prob;
+    double y = v, lqd = 0.0;  // log proposal-density ratio of an independence move
+    if (jump) {
+        y = redraw_axis(a, m, v, uniform01(a.seed, chain, s, 1));
+    } else if (indep) {
+        // y = m + G xi on the coordinates other than the axis; the density
+        // ratio q(v) / q(y) with z = G^-1 (x - m)
+        double xi = normals(a, chain, s);
+        if (i == a.axis) xi = 0.0;
+        const double d = row_times(m.ind_chol, xi), z = row_times(m.ind_inv, v - a.ind_mean[i]);
+        if (i != a.axis) y = a.ind_mean[i] + d;
+        double qy = 0.0, qv = 0.0;
+        for (int k = 0; k < 6; ++k) {
+            const double xk = coord(xi, k), zk = coord(z, k);
+            if (k == a.axis) continue;
+            qy += xk * xk;
+            qv += zk * zk;
+        }
+        lqd = 0.5 * (qy - qv);  // log q(v) - log q(y)
+    } else {
+        const double d = row_times(m.chol, normals(a, chain, s));
+        if (i != a.axis) y = v + a.step * d;
+    }
+    finish(a, m, v, y, lpv, lqd, jump ? 2 : (indep ? 4 : 0), log(uniform01(a.seed, chain, s, 8)), o);
 }
 
 // log Bernoulli(alpha(u)) of observation y in float, without cancellation
@@ -161,168 +238,222 @@ __device__ __forceinline__ float log_bernoulli_f(float u, float y, float uc, flo
     return y == 1.f ? la : lna;
 }
 
-// log L of the model with coefficients s_c (block-wide; the total on thread 0).
-// Point i (PET list first, then the T1/T2 list) is one 16-float record:
-// phi0, J_0 .. J_{P-1}, mask, then PET or T1, T2.
-template <int P>
-__device__ double eval_lik(const ChainArgs &a, const double *s_c, double (*s_red)[kChainWarps]) {
-    float cf[P];
+__device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// *p of CTA `rank` of the cluster = v, p in shared memory
+__device__ __forceinline__ void store_to_rank(double *p, int rank, double v) {
+    unsigned at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+
+__device__ __forceinline__ void load_record(const ChainArgs &a, int i, float4 (&r)[4]) {
+    if (i < a.n_pet + a.n_ti) {
 #pragma unroll
-    for (int p = 0; p < P; ++p) cf[p] = (float)s_c[p];
+        for (int q = 0; q < 4; ++q) r[q] = __ldg(a.rec + (size_t)i * 4 + q);
+    }
+}
+
+// The chains are short of parallelism: 64 of them on one CTA each used 64 of
+// the 152 SMs, and half of a step went by while one thread formed the proposal
+// in double precision (44 us a step at 20632 points). So
+//   * a cluster of K CTAs runs a chain, K the largest of 1, 2, 4, 8 for which
+//     every CTA gets an SM of its own. The likelihood is the sum of 512 partial
+//     sums, over every 512th point each, then by warps of partial sums, then
+//     over these; it stays the same sum in the same order for every K: a CTA
+//     has 512 / K partial sums, K neighbouring lanes form K consecutive terms
+//     of one of them and all add them in order, and each warp's double goes to
+//     the shared memory of every CTA of the cluster, which all take the same
+//     decision: one cluster barrier a step.
+//   * two more warps form the next step's proposals, one for each outcome of
+//     the present step, while the others evaluate it.
+//   * a warp whose points are all far from the tumour (u too small to change
+//     u - uc) takes the Bernoulli terms formed once.
+// 64 chains of 64 steps: 2.85 ms before, MEASURED now.
+constexpr int kBlock = kChainThreads + 64;
+
+template <int P, int K>
+__global__ void __launch_bounds__(kBlock, 1) k_affine_chain(ChainArgs a) {
+    constexpr int kSums = kChainThreads / K, kSumWarps = kChainWarps / K;
+    const int chain = blockIdx.x / K, rank = blockIdx.x % K;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    __shared__ Matrices m;
+    __shared__ Proposal prop[2][2];  // by step, by the outcome of the step before
+    __shared__ float s_f[3][kSums];
+    __shared__ double s_red[2][3][kChainWarps];
+    __shared__ int s_acc;
+    if (t < 36) {
+        m.chol[t] = a.chol[t];
+        m.Ai[t] = a.Ai[t];
+        m.ind_chol[t] = a.ind_chol[t];
+        m.ind_inv[t] = a.ind_inv[t];
+    }
+    __syncthreads();
+    if (warp == kChainWarps) {
+        const double v = a.v[(size_t)chain * 6 + (lane < 6 ? lane : 0)];
+        finish(a, m, v, v, 0.0, 0.0, 0, 0.0, &prop[0][0]);
+    }
+    if (K > 1)
+        cluster_sync();  // every CTA of the cluster runs before its shared memory is written
+    else
+        __syncthreads();
+
     const float scale = (float)a.pet_scale, uc1 = (float)a.t1_uc, uc2 = (float)a.t2_uc, is2 = (float)a.is2;
-    float fp = 0.f, f1 = 0.f, f2 = 0.f;
-    const int items = a.n_pet + a.n_ti;
-#pragma unroll 2
-    for (int i = threadIdx.x; i < items; i += kChainThreads) {
-        float x[16];
+    const float zero1 = 0.f - uc1, zero2 = 0.f - uc2;
+    const float far1[2] = {log_bernoulli_f(0.f, 0.f, uc1, is2), log_bernoulli_f(0.f, 1.f, uc1, is2)};
+    const float far2[2] = {log_bernoulli_f(0.f, 0.f, uc2, is2), log_bernoulli_f(0.f, 1.f, uc2, is2)};
+    const int items = a.n_pet + a.n_ti, rounds = ((items + kChainThreads - 1) / kChainThreads + K - 1) / K;
+    const int first = rank * kSums + t / K + kChainThreads * (t % K);
+    double ly = 0.0, p1 = 0.0, ip = 0.0;  // warp 0
+    int cnt[6] = {0, 0, 0, 0, 0, 0};
+    if (warp == 0) {
+        p1 = -0.5 * a.n_pet * log(2. * 3.14159265358979323846 * a.pet_sigma2);
+        ip = -0.5 * (1. / a.pet_sigma2);
+    }
+    int branch = 0, buf = 0;
+    for (int s = -1; s < a.steps; ++s) {  // -1: the start
+        const Proposal &now = prop[(s + 1) & 1][branch];
+        const bool eval = now.eval;
+        if (warp >= kChainWarps) {
+            if (s + 1 < a.steps) {
+                const int accepted = warp - kChainWarps, l = lane < 6 ? lane : 0;
+                propose(a, m, chain, s + 1, accepted || s < 0 ? now.y[l] : now.v[l], accepted || s < 0 ? now.lpy : now.lpv,
+                        &prop[s & 1][accepted]);
+            }
+        } else if (eval) {
+            float cf[P], fp = 0.f, f1 = 0.f, f2 = 0.f;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float4 v = __ldg(a.rec + (size_t)i * 4 + q);
-            x[4 * q] = v.x;
-            x[4 * q + 1] = v.y;
-            x[4 * q + 2] = v.z;
-            x[4 * q + 3] = v.w;
-        }
-        float u = x[0];
+            for (int p = 0; p < P; ++p) cf[p] = now.c[p];
+            float4 next[4] = {};
+            load_record(a, first, next);
+            for (int q = 0; q < rounds; ++q) {
+                const int i = first + q * kChainThreads * K;
+                float x[16];
 #pragma unroll
-        for (int p = 0; p < P; ++p) u = fmaf(cf[p], x[1 + p], u);
-        u = fminf(fmaxf(u, 0.f), 1.f);
-        if (x[P + 1] == 0.f) u = 0.f;
-        if (i < a.n_pet) {
-            const float r = u - scale * x[P + 2];
-            fp += r * r;
-        } else {
-            f1 += log_bernoulli_f(u, x[P + 2], uc1, is2);
-            f2 += log_bernoulli_f(u, x[P + 3], uc2, is2);
+                for (int k = 0; k < 4; ++k) {
+                    x[4 * k] = next[k].x;
+                    x[4 * k + 1] = next[k].y;
+                    x[4 * k + 2] = next[k].z;
+                    x[4 * k + 3] = next[k].w;
+                }
+                if (q + 1 < rounds) load_record(a, i + kChainThreads * K, next);
+                float u = x[0];
+#pragma unroll
+                for (int p = 0; p < P; ++p) u = fmaf(cf[p], x[1 + p], u);
+                u = fminf(fmaxf(u, 0.f), 1.f);
+                if (x[P + 1] == 0.f) u = 0.f;
+                const bool pet = i < a.n_pet, ti = !pet && i < items;
+                // a sum without a term here adds +0, which changes no bit of it
+                const bool any_pet = __any_sync(0xffffffffu, pet), any_ti = __any_sync(0xffffffffu, ti);
+                if (any_pet) {
+                    const float r = u - scale * x[P + 2];
+                    const float term = pet ? r * r : 0.f;
+#pragma unroll
+                    for (int e = 0; e < K; ++e) fp += K > 1 ? __shfl_sync(0xffffffffu, term, e, K) : term;
+                }
+                if (any_ti) {
+                    float t1, t2;
+                    if (__all_sync(0xffffffffu, !ti || (u - uc1 == zero1 && u - uc2 == zero2))) {
+                        t1 = x[P + 2] == 1.f ? far1[1] : far1[0];
+                        t2 = x[P + 3] == 1.f ? far2[1] : far2[0];
+                    } else {
+                        t1 = log_bernoulli_f(u, x[P + 2], uc1, is2);
+                        t2 = log_bernoulli_f(u, x[P + 3], uc2, is2);
+                    }
+                    if (!ti) t1 = t2 = 0.f;
+#pragma unroll
+                    for (int e = 0; e < K; ++e) {
+                        f1 += K > 1 ? __shfl_sync(0xffffffffu, t1, e, K) : t1;
+                        f2 += K > 1 ? __shfl_sync(0xffffffffu, t2, e, K) : t2;
+                    }
+                }
+            }
+            if (t % K == 0) {
+                s_f[0][t / K] = fp;
+                s_f[1][t / K] = f1;
+                s_f[2][t / K] = f2;
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kChainThreads) : "memory");
+            for (int k = warp; k < 3 * kSumWarps; k += kChainWarps) {
+                const double sum = warp_sum((double)s_f[k / kSumWarps][k % kSumWarps * 32 + lane]);
+                double *dst = &s_red[buf][k / kSumWarps][rank * kSumWarps + k % kSumWarps];
+                if (K == 1) {
+                    if (lane == 0) *dst = sum;
+                } else {
+                    const double v = __shfl_sync(0xffffffffu, sum, 0);
+                    if (lane < K) store_to_rank(dst, lane, v);
+                }
+            }
         }
+        if (K > 1 && eval)
+            cluster_sync();
+        else
+            __syncthreads();
+        if (warp == 0) {
+            double L = 0.0;
+            if (eval) {
+                double part = 0.0;
+                if (lane < 3)
+                    for (int j = 0; j < kChainWarps; ++j) part += s_red[buf][lane][j];
+                const double p2 = ip * coord(part, 0);
+                L = (p1 + p2) + coord(part, 1) + coord(part, 2);
+            }
+            const double lq = eval ? L + now.lpy : -CUDART_INF;
+            bool acc = false;
+            if (s < 0) {
+                ly = lq;
+                if (t == 0 && rank == 0) a.lp_start[chain] = lq;
+            } else {
+                // a prior-conditional redraw: its proposal density cancels the
+                // prior; an independence move: the proposal density ratio
+                const double corr = now.kind == 2 ? now.lpv - now.lpy : (now.kind == 4 ? now.lqd : 0.0);
+                acc = isfinite(lq) && (now.logu < lq - ly + corr);
+                if (acc) ly = lq;
+#pragma unroll
+                for (int k = 0; k < 6; k += 2) {
+                    cnt[k] += now.kind == k && acc ? 1 : 0;
+                    cnt[k + 1] += now.kind == k ? 1 : 0;
+                }
+                if (s == a.steps - 1 && rank == 0 && lane < 6) a.v[(size_t)chain * 6 + lane] = acc ? now.y[lane] : now.v[lane];
+            }
+            if (t == 0) s_acc = acc;
+        }
+        buf ^= eval ? 1 : 0;
+        __syncthreads();
+        branch = s_acc;
     }
-    double sp = warp_sum((double)fp), s1 = warp_sum((double)f1), s2 = warp_sum((double)f2);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        s_red[0][w] = sp;
-        s_red[1][w] = s1;
-        s_red[2][w] = s2;
+    if (t == 0 && rank == 0) {
+        a.lp_end[chain] = ly;
+        for (int k = 0; k < 6; ++k) a.counts[(size_t)chain * 6 + k] = cnt[k];
     }
-    __syncthreads();
-    double total = 0.0;
-    if (threadIdx.x == 0) {
-        double t[3] = {0.0, 0.0, 0.0};
-        for (int k = 0; k < 3; ++k)
-            for (int j = 0; j < kChainWarps; ++j) t[k] += s_red[k][j];
-        const double p1 = -0.5 * a.n_pet * log(2. * 3.14159265358979323846 * a.pet_sigma2);
-        const double p2 = -0.5 * (1. / a.pet_sigma2) * t[0];
-        total = (p1 + p2) + t[1] + t[2];
-    }
-    __syncthreads();
-    return total;
+}
+
+template <int P, int K>
+cudaError_t launch_chain(int B, cudaStream_t stream, const ChainArgs &a) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)B * K);
+    c.blockDim = dim3(kBlock);
+    c.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = K;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = K > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&c, k_affine_chain<P, K>, a);
 }
 
 template <int P>
-__global__ void __launch_bounds__(kChainThreads) k_affine_chain(ChainArgs a) {
-    const int b = blockIdx.x;
-    __shared__ double s_c[16];
-    __shared__ double s_red[3][kChainWarps];
-    __shared__ int s_eval;
-    double v[6], y[6], lpv = 0.0, lpy = 0.0, ly = 0.0;
-    int cnt[6] = {0, 0, 0, 0, 0, 0};
-    bool jump = false, indep = false;
-    double lqd = 0.0;  // log proposal-density ratio of an independence move
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 6; ++i) v[i] = a.v[(size_t)b * 6 + i];
-        lpv = prior_logp(a, v);
-        coefficients(a, v, s_c);
-        s_eval = isfinite(lpv) ? 1 : 0;
-    }
-    __syncthreads();
-    {
-        const double L = s_eval ? eval_lik<P>(a, s_c, s_red) : 0.0;
-        if (threadIdx.x == 0) {
-            ly = s_eval ? L + lpv : -CUDART_INF;
-            a.lp_start[b] = ly;
-        }
-    }
-    __syncthreads();  // every thread has read s_eval before thread 0 rewrites it
-    for (int s = 0; s < a.steps; ++s) {
-        if (threadIdx.x == 0) {
-            const double um = uniform01(a.seed, b, s, 0);
-            jump = a.axis >= 0 && um <= a.axis_prob;
-            indep = !jump && um <= (a.axis >= 0 ? a.axis_prob : 0.0) + a.ind_prob;
-            for (int i = 0; i < 6; ++i) y[i] = v[i];
-            if (jump) {
-                redraw_axis(a, y, uniform01(a.seed, b, s, 1));
-            } else if (indep) {
-                // y = m + G xi on the coordinates other than the axis; the
-                // density ratio q(v) / q(y) with z = G^-1 (x - m)
-                double xi[6], zv[6];
-                for (int k = 0; k < 3; ++k) {
-                    const float r = sqrtf(-2.0f * logf((float)uniform01(a.seed, b, s, 2 + 2 * k)));
-                    float sn, cs;
-                    sincospif(2.0f * (float)uniform01(a.seed, b, s, 3 + 2 * k), &sn, &cs);
-                    xi[2 * k] = (double)(r * cs);
-                    xi[2 * k + 1] = (double)(r * sn);
-                }
-                if (a.axis >= 0) xi[a.axis] = 0.0;
-                double qy = 0.0, qv = 0.0;
-                for (int i = 0; i < 6; ++i) {
-                    if (i == a.axis) continue;
-                    double d = 0.0, z = 0.0;
-                    for (int j = 0; j < 6; ++j) {
-                        d += a.ind_chol[i * 6 + j] * xi[j];
-                        z += a.ind_inv[i * 6 + j] * (v[j] - a.ind_mean[j]);
-                    }
-                    y[i] = a.ind_mean[i] + d;
-                    zv[i] = z;
-                    qy += xi[i] * xi[i];
-                    qv += zv[i] * zv[i];
-                }
-                lqd = 0.5 * (qy - qv);  // log q(v) - log q(y)
-            } else {
-                // normals in float: their precision does not matter, the
-                // state they move stays double
-                double xi[6];
-                for (int k = 0; k < 3; ++k) {
-                    const float r = sqrtf(-2.0f * logf((float)uniform01(a.seed, b, s, 2 + 2 * k)));
-                    float sn, cs;
-                    sincospif(2.0f * (float)uniform01(a.seed, b, s, 3 + 2 * k), &sn, &cs);
-                    xi[2 * k] = (double)(r * cs);
-                    xi[2 * k + 1] = (double)(r * sn);
-                }
-                for (int i = 0; i < 6; ++i) {
-                    double d = 0.0;
-                    for (int j = 0; j < 6; ++j) d += a.chol[i * 6 + j] * xi[j];
-                    y[i] = v[i] + a.step * d;
-                }
-                if (a.axis >= 0) y[a.axis] = v[a.axis];
-            }
-            lpy = prior_logp(a, y);
-            coefficients(a, y, s_c);
-            s_eval = isfinite(lpy) ? 1 : 0;
-        }
-        __syncthreads();
-        const double L = s_eval ? eval_lik<P>(a, s_c, s_red) : 0.0;
-        if (threadIdx.x == 0) {
-            const double lq = s_eval ? L + lpy : -CUDART_INF;
-            // a prior-conditional redraw: its proposal density cancels the
-            // prior; an independence move: the proposal density ratio
-            const double corr = jump ? lpv - lpy : (indep ? lqd : 0.0);
-            const double logu = log(uniform01(a.seed, b, s, 8));
-            const bool acc = isfinite(lq) && (logu < lq - ly + corr);
-            if (acc) {
-                for (int i = 0; i < 6; ++i) v[i] = y[i];
-                ly = lq;
-                lpv = lpy;
-            }
-            const int kind = jump ? 2 : (indep ? 4 : 0);
-            cnt[kind] += acc ? 1 : 0;
-            cnt[kind + 1] += 1;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 6; ++i) a.v[(size_t)b * 6 + i] = v[i];
-        a.lp_end[b] = ly;
-        for (int k = 0; k < 6; ++k) a.counts[(size_t)b * 6 + k] = cnt[k];
-    }
+cudaError_t launch_chains(int B, int sms, cudaStream_t stream, const ChainArgs &a) {
+    const int per = sms / B;
+    if (per >= 8) return launch_chain<P, 8>(B, stream, a);
+    if (per >= 4) return launch_chain<P, 4>(B, stream, a);
+    if (per >= 2) return launch_chain<P, 2>(B, stream, a);
+    return launch_chain<P, 1>(B, stream, a);
 }
 
 }  // namespace
@@ -404,12 +535,8 @@ int affine_chain(Handle &h, const gbg_affine_chain_opts &o, int B, int steps, un
     a.lp_end = d_l1;
     a.counts = d_cnt;
     GBG_CUDA_TRY(cudaMemcpyAsync(d_v, v, (size_t)B * 6 * sizeof(double), cudaMemcpyHostToDevice, h.stream));
-    if (P == 12)
-        k_affine_chain<12><<<B, kChainThreads, 0, h.stream>>>(a);
-    else
-        k_affine_chain<6><<<B, kChainThreads, 0, h.stream>>>(a);
+    GBG_CUDA_TRY(P == 12 ? launch_chains<12>(B, h.num_sms, h.stream, a) : launch_chains<6>(B, h.num_sms, h.stream, a));
     h.launches++;
-    GBG_CUDA_TRY(cudaGetLastError());
     GBG_CUDA_TRY(cudaMemcpyAsync(v, d_v, (size_t)B * 6 * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
     GBG_CUDA_TRY(cudaMemcpyAsync(lp_start, d_l0, (size_t)B * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
     GBG_CUDA_TRY(cudaMemcpyAsync(lp_end, d_l1, (size_t)B * sizeof(double), cudaMemcpyDeviceToHost, h.stream));

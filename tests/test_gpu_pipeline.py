@@ -155,3 +155,30 @@ def test_gpu_screening_chain_moves_like_the_host_chain(gbg, with_ind):
     assert abs(ag - ah) < 0.03
     assert np.all(np.abs(yg.mean(axis=0) - yh.mean(axis=0)) < 5 * se)
     assert np.all(np.abs(yg.std(axis=0) / yh.std(axis=0) - 1) < 0.1)
+
+
+@pytest.mark.parametrize("quad_axis", [0, None])
+def test_gpu_screening_chain_is_the_same_alone_and_among_others(gbg, quad_axis):
+    """A chain depends on its index and start alone: run in populations whose
+    chains get eight CTAs, four, two or one each, the first chains come out bit
+    for bit the same, with every kind of move, and a start outside the prior."""
+    an = S.make_anatomy(N, seed=4)
+    with _lib.Handle(N, "f32", max_samples=64) as h:
+        h.set_anatomy(an.p_w, an.p_g)
+        truth = _problem(h, an)
+        prior = mcmc.Prior.from_anatomy(an)
+        lc = mcmc.LogCoords(mcmc.Posterior(h, an.L, -1.0, prior), A=mcmc.INVARIANT_MAP)
+        v_ref = lc.to_u(np.array([truth.as_tuple()]))[0]
+        d = 0.01 * lc.prior.width
+        sur = mcmc.AffineSurrogate(lc, v_ref, d, quad_axis=quad_axis)
+        rng = np.random.default_rng(6)
+        v = v_ref + 0.3 * d * rng.standard_normal((300, 6))
+        v[1, 1] += 50.0
+        runs = []
+        for B in (300, 80, 40, 20, 2):
+            out = sur.chain(v[:B], 40, 0.5, np.diag(d), 0, 0.3, 13, ind=(0.3, v_ref, np.diag(d)))
+            runs.append([x[:2] for x in out[:3]])
+        assert not np.array_equal(runs[0][0], v[:2])  # it moved
+    for r in runs[1:]:
+        for x, y in zip(runs[0], r):
+            assert np.array_equal(x, y)
