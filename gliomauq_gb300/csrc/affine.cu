@@ -33,8 +33,9 @@ __global__ void k_affine_gather(int len, const int *__restrict__ idx, size_t N, 
 
 // one 16-float record per observation point for the screening chain: phi0,
 // the P basis fields, the mask, then the observation values (PET; or T1, T2),
-// zero padding
-__global__ void k_affine_records(int len, int P, const float *__restrict__ cols, const double *__restrict__ v1,
+// zero padding; rec points at the list's first point in the first of four
+// arrays of one float4 per point of both lists (npts)
+__global__ void k_affine_records(int len, size_t npts, int P, const float *__restrict__ cols, const double *__restrict__ v1,
                                  const double *__restrict__ v2, float4 *__restrict__ rec) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
         float r[16];
@@ -42,7 +43,7 @@ __global__ void k_affine_records(int len, int P, const float *__restrict__ cols,
         for (int k = 0; k < P + 2; ++k) r[k] = cols[(size_t)k * len + i];
         r[P + 2] = (float)v1[i];
         if (v2) r[P + 3] = (float)v2[i];
-        for (int q = 0; q < 4; ++q) rec[(size_t)i * 4 + q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+        for (int q = 0; q < 4; ++q) rec[q * npts + i] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
     }
 }
 
@@ -82,11 +83,11 @@ int affine_gather_columns(Handle &h) {
         }
         if (h.obs.n_pet > 0)
             k_affine_records<<<std::min((h.obs.n_pet + 255) / 256, h.num_sms * 8), 256, 0, h.stream>>>(
-                h.obs.n_pet, P, h.aff_cols, h.obs.pet_val, nullptr, h.aff_rec);
+                h.obs.n_pet, npts, P, h.aff_cols, h.obs.pet_val, nullptr, h.aff_rec);
         if (h.obs.n_ti > 0)
             k_affine_records<<<std::min((h.obs.n_ti + 255) / 256, h.num_sms * 8), 256, 0, h.stream>>>(
-                h.obs.n_ti, P, h.aff_cols + (size_t)(P + 2) * h.obs.n_pet, h.obs.t1_val, h.obs.t2_val,
-                h.aff_rec + (size_t)h.obs.n_pet * 4);
+                h.obs.n_ti, npts, P, h.aff_cols + (size_t)(P + 2) * h.obs.n_pet, h.obs.t1_val, h.obs.t2_val,
+                h.aff_rec + h.obs.n_pet);
         h.launches += 2;
     }
     GBG_CUDA_TRY(cudaGetLastError());

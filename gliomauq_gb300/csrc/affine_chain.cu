@@ -4,8 +4,8 @@
 //   phi(v) = m * clamp(phi0 + sum_p c_p(v - u_ref) J_p, 0, 1)
 // (the affine model of affine.cu, evaluated at the observation lists' cells
 // from the same gathered columns) for B chains at once, a cluster of CTAs per
-// chain, so that a whole inner chain is one launch instead of one host round trip per
-// step. The moves are those of the host sampler's inner chain
+// chain, so that a whole inner chain is one launch instead of one host round
+// trip per step. The moves are those of the host sampler's inner chain
 // (gliomauq_gb300/mcmc.py, da): with probability axis_prob a redraw of the
 // symmetry coordinate from its prior conditional, accepted with the ratio of
 // pi*'s likelihood factors; with probability ind_prob an independence
@@ -23,11 +23,11 @@
 //
 // Each observation point's model (phi0, the basis fields, the mask) and its
 // observed values are one 16-float record (affine.cu builds them), read with
-// four vector loads. The per-point likelihood terms are evaluated in float (this GPU's FP64 rate
-// is a small fraction of its FP32 rate, and the screen only has to be one
-// fixed function: the chain returns its own log pi* at the start and end
-// points, which is what the second stage's ratio uses), summed in float per
-// thread and in double across the block. The Bernoulli terms of
+// four vector loads. The per-point likelihood terms are evaluated in float
+// (this GPU's FP64 rate is a small fraction of its FP32 rate, and the screen
+// only has to be one fixed function: the chain returns its own log pi* at the
+// start and end points, which is what the second stage's ratio uses), summed
+// in float per partial sum and in double over these. The Bernoulli terms of
 // HGG_Likelihood (:136-153) in a form without cancellation: with
 // q = (u - uc)^2 / slope, alpha = 1 - e^-q / 2 above uc and e^-q / 2 below,
 // so log alpha and log(1 - alpha) are log1p(-e^-q / 2) and log(1/2) - q.
@@ -51,7 +51,7 @@ struct ChainArgs {
     double ind_mean[6], ind_chol[36], ind_inv[36];
     const unsigned char *mask;
     unsigned long long seed;
-    const float4 *rec;  // per observation point, PET list then T1/T2 list: 16 floats
+    const float4 *rec;  // 16 floats per observation point, PET list then T1/T2 list: four arrays of float4
     int n_pet, n_ti;
     double pet_scale, t1_uc, t2_uc, is2, pet_sigma2;
     double *v, *lp_start, *lp_end;
@@ -251,10 +251,65 @@ __device__ __forceinline__ void store_to_rank(double *p, int rank, double v) {
 }
 
 __device__ __forceinline__ void load_record(const ChainArgs &a, int i, float4 (&r)[4]) {
-    if (i < a.n_pet + a.n_ti) {
+    const int items = a.n_pet + a.n_ti;
+    if (i < items) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) r[q] = __ldg(a.rec + (size_t)i * 4 + q);
+        for (int q = 0; q < 4; ++q) r[q] = __ldg(a.rec + (size_t)q * items + i);
     }
+}
+
+// rounds [q0, q1) of a lane's points first + q * kChainThreads * K, all PET
+// points (kPet), all T1/T2 points (kTi) or some of both or of neither; next
+// holds the record of round q0, and of round q1 afterwards
+enum { kPet = 1, kTi = 2 };
+template <int P, int K, int KIND>
+__device__ __forceinline__ void rounds_of(const ChainArgs &a, int q0, int q1, int first, const float (&cf)[P], float4 (&next)[4],
+                                          float &fp, float &f1, float &f2) {
+    const float scale = (float)a.pet_scale, uc1 = (float)a.t1_uc, uc2 = (float)a.t2_uc, is2 = (float)a.is2;
+#pragma unroll 2
+    for (int q = q0; q < q1; ++q) {
+        const int i = first + q * kChainThreads * K;
+        float x[16];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            x[4 * k] = next[k].x;
+            x[4 * k + 1] = next[k].y;
+            x[4 * k + 2] = next[k].z;
+            x[4 * k + 3] = next[k].w;
+        }
+        load_record(a, i + kChainThreads * K, next);
+        float u = x[0];
+#pragma unroll
+        for (int p = 0; p < P; ++p) u = fmaf(cf[p], x[1 + p], u);
+        u = fminf(fmaxf(u, 0.f), 1.f);
+        if (x[P + 1] == 0.f) u = 0.f;
+        // a sum without a term here adds +0, which changes no bit of it
+        if (KIND & kPet) {
+            const float r = u - scale * x[P + 2];
+            const float term = KIND == kPet || i < a.n_pet ? r * r : 0.f;
+#pragma unroll
+            for (int e = 0; e < K; ++e) fp += K > 1 ? __shfl_sync(0xffffffffu, term, e, K) : term;
+        }
+        if (KIND & kTi) {
+            float t1 = log_bernoulli_f(u, x[P + 2], uc1, is2), t2 = log_bernoulli_f(u, x[P + 3], uc2, is2);
+            if (KIND != kTi && !(i >= a.n_pet && i < a.n_pet + a.n_ti)) t1 = t2 = 0.f;
+#pragma unroll
+            for (int e = 0; e < K; ++e) {
+                f1 += K > 1 ? __shfl_sync(0xffffffffu, t1, e, K) : t1;
+                f2 += K > 1 ? __shfl_sync(0xffffffffu, t2, e, K) : t2;
+            }
+        }
+    }
+}
+
+// the sum of 32 floats f[0..31] in double, formed by 8 neighbouring lanes (l of
+// them is this one) in the order of warp_sum; valid on their first
+__device__ __forceinline__ double sum32(const float *f, int l) {
+    const double a = (double)f[l] + (double)f[l + 16], b = (double)f[l + 8] + (double)f[l + 24];
+    double v = a + b;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // The chains are short of parallelism: 64 of them on one CTA each used 64 of
@@ -270,9 +325,10 @@ __device__ __forceinline__ void load_record(const ChainArgs &a, int i, float4 (&
 //     decision: one cluster barrier a step.
 //   * two more warps form the next step's proposals, one for each outcome of
 //     the present step, while the others evaluate it.
-//   * a warp whose points are all far from the tumour (u too small to change
-//     u - uc) takes the Bernoulli terms formed once.
-// 64 chains of 64 steps: 2.85 ms before, MEASURED now.
+//   * a point's record lies in four arrays of 16 bytes a point: as 64 bytes in
+//     a row, its four loads took four times the passes through L1, which was
+//     then 64 % busy.
+// 64 chains of 64 steps: 2.81 ms before, 0.86 now.
 constexpr int kBlock = kChainThreads + 64;
 
 template <int P, int K>
@@ -301,11 +357,10 @@ __global__ void __launch_bounds__(kBlock, 1) k_affine_chain(ChainArgs a) {
     else
         __syncthreads();
 
-    const float scale = (float)a.pet_scale, uc1 = (float)a.t1_uc, uc2 = (float)a.t2_uc, is2 = (float)a.is2;
-    const float zero1 = 0.f - uc1, zero2 = 0.f - uc2;
-    const float far1[2] = {log_bernoulli_f(0.f, 0.f, uc1, is2), log_bernoulli_f(0.f, 1.f, uc1, is2)};
-    const float far2[2] = {log_bernoulli_f(0.f, 0.f, uc2, is2), log_bernoulli_f(0.f, 1.f, uc2, is2)};
-    const int items = a.n_pet + a.n_ti, rounds = ((items + kChainThreads - 1) / kChainThreads + K - 1) / K;
+    // rounds of PET points only, from there on of both, of T1/T2 points only, of
+    // both or of the last few points
+    const int per = kChainThreads * K, items = a.n_pet + a.n_ti, rounds = (items + per - 1) / per;
+    const int pet_end = a.n_pet / per, ti_end = items / per, ti_begin = min((a.n_pet + per - 1) / per, ti_end);
     const int first = rank * kSums + t / K + kChainThreads * (t % K);
     double ly = 0.0, p1 = 0.0, ip = 0.0;  // warp 0
     int cnt[6] = {0, 0, 0, 0, 0, 0};
@@ -329,62 +384,26 @@ __global__ void __launch_bounds__(kBlock, 1) k_affine_chain(ChainArgs a) {
             for (int p = 0; p < P; ++p) cf[p] = now.c[p];
             float4 next[4] = {};
             load_record(a, first, next);
-            for (int q = 0; q < rounds; ++q) {
-                const int i = first + q * kChainThreads * K;
-                float x[16];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    x[4 * k] = next[k].x;
-                    x[4 * k + 1] = next[k].y;
-                    x[4 * k + 2] = next[k].z;
-                    x[4 * k + 3] = next[k].w;
-                }
-                if (q + 1 < rounds) load_record(a, i + kChainThreads * K, next);
-                float u = x[0];
-#pragma unroll
-                for (int p = 0; p < P; ++p) u = fmaf(cf[p], x[1 + p], u);
-                u = fminf(fmaxf(u, 0.f), 1.f);
-                if (x[P + 1] == 0.f) u = 0.f;
-                const bool pet = i < a.n_pet, ti = !pet && i < items;
-                // a sum without a term here adds +0, which changes no bit of it
-                const bool any_pet = __any_sync(0xffffffffu, pet), any_ti = __any_sync(0xffffffffu, ti);
-                if (any_pet) {
-                    const float r = u - scale * x[P + 2];
-                    const float term = pet ? r * r : 0.f;
-#pragma unroll
-                    for (int e = 0; e < K; ++e) fp += K > 1 ? __shfl_sync(0xffffffffu, term, e, K) : term;
-                }
-                if (any_ti) {
-                    float t1, t2;
-                    if (__all_sync(0xffffffffu, !ti || (u - uc1 == zero1 && u - uc2 == zero2))) {
-                        t1 = x[P + 2] == 1.f ? far1[1] : far1[0];
-                        t2 = x[P + 3] == 1.f ? far2[1] : far2[0];
-                    } else {
-                        t1 = log_bernoulli_f(u, x[P + 2], uc1, is2);
-                        t2 = log_bernoulli_f(u, x[P + 3], uc2, is2);
-                    }
-                    if (!ti) t1 = t2 = 0.f;
-#pragma unroll
-                    for (int e = 0; e < K; ++e) {
-                        f1 += K > 1 ? __shfl_sync(0xffffffffu, t1, e, K) : t1;
-                        f2 += K > 1 ? __shfl_sync(0xffffffffu, t2, e, K) : t2;
-                    }
-                }
-            }
+            rounds_of<P, K, kPet>(a, 0, pet_end, first, cf, next, fp, f1, f2);
+            rounds_of<P, K, kPet | kTi>(a, pet_end, max(pet_end, ti_begin), first, cf, next, fp, f1, f2);
+            rounds_of<P, K, kTi>(a, max(pet_end, ti_begin), ti_end, first, cf, next, fp, f1, f2);
+            rounds_of<P, K, kPet | kTi>(a, max(max(pet_end, ti_begin), ti_end), rounds, first, cf, next, fp, f1, f2);
             if (t % K == 0) {
                 s_f[0][t / K] = fp;
                 s_f[1][t / K] = f1;
                 s_f[2][t / K] = f2;
             }
             asm volatile("bar.sync 1, %0;" ::"n"(kChainThreads) : "memory");
-            for (int k = warp; k < 3 * kSumWarps; k += kChainWarps) {
-                const double sum = warp_sum((double)s_f[k / kSumWarps][k % kSumWarps * 32 + lane]);
-                double *dst = &s_red[buf][k / kSumWarps][rank * kSumWarps + k % kSumWarps];
+            // four sums of 32 partial sums to a warp
+            for (int w = warp; 4 * w < 3 * kSumWarps; w += kChainWarps) {
+                const int k = min(4 * w + lane / 8, 3 * kSumWarps - 1), kind = k / kSumWarps, part = k % kSumWarps;
+                double sum = sum32(&s_f[kind][part * 32], lane & 7);
+                double *dst = &s_red[buf][kind][rank * kSumWarps + part];
                 if (K == 1) {
-                    if (lane == 0) *dst = sum;
+                    if ((lane & 7) == 0) *dst = sum;
                 } else {
-                    const double v = __shfl_sync(0xffffffffu, sum, 0);
-                    if (lane < K) store_to_rank(dst, lane, v);
+                    sum = __shfl_sync(0xffffffffu, sum, lane & ~7);
+                    if ((lane & 7) < K) store_to_rank(dst, lane & 7, sum);
                 }
             }
         }
