@@ -19,13 +19,15 @@
 //     last store to the release) the others have the SM.
 //   * A warp marches its share of units up z, two rows in registers, with the
 //     loads of the next planes in flight.
-// What bounds it: shared-memory and L1 bandwidth (28 of the 58 wavefronts a
-// unit costs are coefficients) and, for one sample, the barrier.
+// What bounds it: a warp's latencies (16 warps an SM, of which a fifth waits at
+// a barrier; L1's data path is 62 % busy, 28 of the 58 passes a unit takes
+// through it are coefficients, and instructions issue in 44 % of the cycles),
+// and, for one sample, the barrier.
 // Per-cell operations and their order are those of march_tile_s (a difference
 // taken the other way round is its exact negative), so every population
 // kernel gives the same bits. Measured on a GB300, before (tile march) and
-// now: 512 prior draws at 128^3 243 -> 164 ms; 64 draws near the mode, stable
-// grid, 14.0 -> 10.0 ms; one of them 1.01 -> 0.61 ms; 512 at 64^3 53 -> 26 ms.
+// now: 512 prior draws at 128^3 243 -> 150 ms; 64 draws near the mode, stable
+// grid, 14.7 -> 9.5 ms; one of them 1.04 -> 0.62 ms; 512 at 64^3 51 -> 24.5 ms.
 #include <algorithm>
 #include <type_traits>
 
@@ -73,7 +75,7 @@ __device__ __forceinline__ float4 row_step(const V4 &P, const V4 &DS, float sS, 
     for (int i = 0; i < 4; ++i) {
         const float f0 = P.v[i];
         float lap = i ? -fabsf(CX.v[i - 1]) * d[i - 1] : -flux;
-        lap = fmaf(fabsf(CX.v[i]), d[i], lap);
+        lap = fmaf(CX.v[i], d[i], lap);  // of either sign where the cell's result is dropped
         lap = fmaf(sS * CYm.v[i], DS.v[i], lap);
         lap = fmaf(CY.v[i], DT.v[i], lap);
         lap = fmaf(-CZp.v[i], DB.v[i], lap);
@@ -93,50 +95,65 @@ __device__ __forceinline__ void march(const float4 *__restrict__ tab, int y, int
     constexpr int n = 4 * LR, plane = n * n;
     const int li = (threadIdx.x & 31) % LR;
     const int o0 = 4 * li + n * y + plane * z, below = z == 0 ? plane * (n - 1) : -plane;
-    const float *pN = in + o0;  // the plane last loaded as "next"
+    const float *pN = in + o0;  // the plane last loaded
     int dS = y == 0 ? n * (n - 1) : -n, dT = y + 2 == n ? -n * (n - 2) : 2 * n;
     out += o0;
-    struct Slot {
-        V4 n0, n1, s, t;
-    } sl[kAhead];
+    // Registers in rings, so that no plane's values are moved: the rows of
+    // planes j .. j + 2, the rows below and above them of planes j and j + 1,
+    // the difference and the face to the plane before. Unrolled by the rings'
+    // common period. (Moving them plane by plane, and taking the coefficients'
+    // magnitude in masked cells too: 232 instructions a unit instead of 204,
+    // 164 ms instead of 150 on the population above.)
+    V4 X0[kAhead + 1], X1[kAhead + 1], S[kAhead], T[kAhead], B0[2], B1[2], C0[2], C1[2];
     int zn = z;
-    // loads of plane zn's y neighbours and of the rows above it
-    auto load = [&](Slot &q) {
-        q.s = ldp(pN + dS);
-        q.t = ldp(pN + dT);
+    auto load_st = [&](int d) {  // of the plane pN is on; then to the next plane
+        S[d] = ldp(pN + dS);
+        T[d] = ldp(pN + dT);
         pN += ++zn == n ? -plane * (n - 1) : plane;
-        q.n0 = ldp(pN);
-        q.n1 = ldp(pN + n);
     };
-    V4 P0 = ldp(pN), P1 = ldp(pN + n), B0 = ldp(pN + below), B1 = ldp(pN + below + n);
-    B0 = sub(P0, B0);
-    B1 = sub(P1, B1);
-    V4 C0 = ldg4(cz + o0 + below), C1 = ldg4(cz + o0 + below + n);
+    X0[0] = ldp(pN);
+    X1[0] = ldp(pN + n);
+    B0[0] = ldp(pN + below);
+    B1[0] = ldp(pN + below + n);
+    C0[0] = ldg4(cz + o0 + below);
+    C1[0] = ldg4(cz + o0 + below + n);
 #pragma unroll
     for (int d = 0; d < kAhead; ++d)
-        if (d < len) load(sl[d]);
-    for (int j = 0; j < len; j += kAhead) {
+        if (d < len) {
+            load_st(d);
+            X0[d + 1] = ldp(pN);
+            X1[d + 1] = ldp(pN + n);
+        }
+    B0[0] = sub(X0[0], B0[0]);
+    B1[0] = sub(X1[0], B1[0]);
+    constexpr int kPeriod = 2 * (kAhead + 1);
+    static_assert(kAhead == 2, "the rings' common period");
+    for (int j = 0; j < len; j += kPeriod) {
 #pragma unroll
-        for (int d = 0; d < kAhead; ++d) {
+        for (int d = 0; d < kPeriod; ++d) {
             if (j + d >= len) break;
-            const V4 Z0 = lds(tab + 5 * 32), Y1 = lds(tab + 3 * 32);
-            const V4 DY = sub(P1, P0), F0 = sub(sl[d].n0, P0), F1 = sub(sl[d].n1, P1);
-            *reinterpret_cast<float4 *>(out) = row_step<LR>(P0, sub(sl[d].s, P0), 1.f, DY, B0, F0, lds(tab), lds(tab + 2 * 32), Y1, C0,
-                                                            Z0, li, a, b);
+            constexpr int R = kAhead + 1;
+            const V4 &P0 = X0[d % R], &P1 = X1[d % R], &N0 = X0[(d + 1) % R], &N1 = X1[(d + 1) % R];
+            const int h = d & 1, q = d % kAhead;
+            C0[h ^ 1] = lds(tab + 5 * 32);
+            const V4 Y1 = lds(tab + 3 * 32);
+            const V4 DY = sub(P1, P0);
+            B0[h ^ 1] = sub(N0, P0);
+            B1[h ^ 1] = sub(N1, P1);
+            *reinterpret_cast<float4 *>(out) = row_step<LR>(P0, sub(S[q], P0), 1.f, DY, B0[h], B0[h ^ 1], lds(tab), lds(tab + 2 * 32), Y1,
+                                                            C0[h], C0[h ^ 1], li, a, b);
             __syncwarp();
-            const V4 Z1 = lds(tab + 6 * 32);
-            *reinterpret_cast<float4 *>(out + n) = row_step<LR>(P1, DY, -1.f, sub(sl[d].t, P1), B1, F1, lds(tab + 32), Y1,
-                                                                lds(tab + 4 * 32), C1, Z1, li, a, b);
+            C1[h ^ 1] = lds(tab + 6 * 32);
+            *reinterpret_cast<float4 *>(out + n) = row_step<LR>(P1, DY, -1.f, sub(T[q], P1), B1[h], B1[h ^ 1], lds(tab + 32), Y1,
+                                                                lds(tab + 4 * 32), C1[h], C1[h ^ 1], li, a, b);
             __syncwarp();
-            B0 = F0;
-            B1 = F1;
-            P0 = sl[d].n0;
-            P1 = sl[d].n1;
-            C0 = Z0;
-            C1 = Z1;
             out += plane;
             tab += kSlots * 32;
-            if (j + d + kAhead < len) load(sl[d]);
+            if (j + d + kAhead < len) {
+                load_st(q);
+                X0[d % R] = ldp(pN);
+                X1[d % R] = ldp(pN + n);
+            }
         }
     }
 }
