@@ -268,11 +268,11 @@ int gbg_get_phi(gbg_handle *hh, double *phi) {
     GBG_CUDA_TRY(cudaSetDevice(h.device));
     if (h.prec == GBG_PREC_F64) {
         GBG_CUDA_TRY(cudaMemcpyAsync(phi, h.phi[h.cur], h.N * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
-        GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+        if (int rc = gbg::finish_steps(h)) return rc;
     } else {
         std::vector<float> tmp(h.N);
         GBG_CUDA_TRY(cudaMemcpyAsync(tmp.data(), h.phi[h.cur], h.N * sizeof(float), cudaMemcpyDeviceToHost, h.stream));
-        GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+        if (int rc = gbg::finish_steps(h)) return rc;
         for (size_t i = 0; i < h.N; ++i) phi[i] = (double)tmp[i];
     }
     return GBG_OK;
@@ -445,7 +445,7 @@ int gbg_run(gbg_handle *hh, double Dw_file, double rho, double tend, double L, l
     if (dt_out) *dt_out = dt;
     int rc = gbg_rd_step(hh, Dw, Dg, r, dt, ns);
     if (rc) return rc;
-    GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    if (int rc = gbg::finish_steps(h)) return rc;
     return GBG_OK;
 }
 
@@ -481,7 +481,7 @@ int gbg_loglik(gbg_handle *hh, gbg_lik_result *out) {
         rc = gbg::lik_evaluate(h, (const float *)h.phi[h.cur], nullptr, 1, (gbg_lik_result *)h.lik_out);
     if (rc) return rc;
     GBG_CUDA_TRY(cudaMemcpyAsync(out, h.lik_out, sizeof(gbg_lik_result), cudaMemcpyDeviceToHost, h.stream));
-    GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    if (int rc = gbg::finish_steps(h)) return rc;
     return GBG_OK;
 }
 
@@ -1402,8 +1402,7 @@ int gbg_autotune(gbg_handle *hh, int probe_samples, const char *cache_path, int 
 int gbg_sync(gbg_handle *hh) {
     if (int rc = check_handle(hh)) return rc;
     GBG_CUDA_TRY(cudaSetDevice(hh->h.device));
-    GBG_CUDA_TRY(cudaStreamSynchronize(hh->h.stream));
-    return GBG_OK;
+    return gbg::finish_steps(hh->h);
 }
 
 }  // extern "C"

@@ -124,6 +124,7 @@ struct Handle {
     int *exact_list = nullptr;
     double *exact_dsum = nullptr;
     bool exact_listed = false;
+    bool exact_waited = false;  // a launch whose CTAs wait for one another is not yet checked (finish_steps)
     int exact_full = 0;
 
     // MALA variant (exact modes): slopes sRho, sD ping-pong in the storage
@@ -305,6 +306,8 @@ int population_variant_shape(int n, int vi, int *ry, int *g, int *threads);
 int population_variant_name(int n, int vi, char *buf, int len);
 // reads and clears the device status word (synchronises the stream)
 int check_device_status(Handle &h);
+// the stream's work is done; an error if steps among it gave up waiting
+int finish_steps(Handle &h);
 int batch_solve_device(Handle &h, const gbg_sample *samples_device, int S,
                        const gbg_batch_opts &o, gbg_lik_result *loglik_device, long *nsteps_host);
 

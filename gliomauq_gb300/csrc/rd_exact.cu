@@ -119,7 +119,8 @@ __global__ void k_exact_step(int n, const Real *__restrict__ phi, Real *__restri
 // (densities are finite and in [0, 1] from the first step on). k_exact_list
 // runs over the list of plain and special cells; two steps over every cell
 // leave the dead ones' zeros in both buffers. Measured on 64^3 (32 % plain),
-// 237 steps with upload and download: 7.0 ms on every cell, 2.3 ms on the list.
+// 237 steps with upload and download: 7.0 ms on every cell, 2.3 ms on the list
+// with a launch per step, 1.6 in one launch (k_exact_resident).
 struct Cell {
     size_t W, E, S, N, B, F;
 };
@@ -171,6 +172,178 @@ __global__ void __launch_bounds__(256) k_exact_collect(int n, const Real *__rest
     dsum[at] = d[0] + d[1] + d[2] + d[3] + d[4] + d[5];
 }
 
+// a value clamped to [0, 1], NaN to 0, in double on its bits: comparisons would
+// go to the FP64 pipe
+__device__ __forceinline__ float clamp01(float v) {
+    v = 0.f < v ? v : 0.f;
+    return v < 1.f ? v : 1.f;
+}
+__device__ __forceinline__ double clamp01(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v);
+    if (hi < 0x3ff00000u) return v;
+    const bool nan = (hi & 0x7fffffffu) > 0x7ff00000u || ((hi & 0x7fffffffu) == 0x7ff00000u && __double2loint(v) != 0);
+    return (int)hi < 0 || nan ? 0.0 : 1.0;
+}
+
+// the step of listed cell e: d, the faces W E S N B F, and their sum; p, the
+// densities of the cell and its neighbours in the same order
+template <typename Real>
+__device__ __forceinline__ Real listed_step(int e, const double (&t)[6], double sum, const Real (&p)[7], const Real *b0, Real rho, double dt,
+                                            double ih2) {
+    double d[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) d[f] = t[f];
+    if (e < 0) {
+        const Real tissue = b0[~e] + p[0];
+        if (!(tissue > 0.)) d[0] = d[1] = d[2] = d[3] = d[4] = d[5] = 0.0;
+#pragma unroll
+        for (int f = 0; f < 6; f += 2) {
+            if (d[f] == 0 && p[1 + f] > 0.) d[f + 1] *= 2.0;
+            if (d[f + 1] == 0 && p[2 + f] > 0.) d[f] *= 2.0;
+        }
+        sum = d[0] + d[1] + d[2] + d[3] + d[4] + d[5];
+    }
+    const double fin = ih2 * (d[0] * widen(p[1]) + d[1] * widen(p[2]) + d[2] * widen(p[3]) + d[3] * widen(p[4]) + d[4] * widen(p[5]) +
+                              d[5] * widen(p[6]));
+    const double fout = -(sum * widen(p[0]) * ih2);
+    const double react = reaction(rho, p[0]);
+    const Real dphidt = (Real)(fout + fin + react);
+    return clamp01((Real)(widen(p[0]) + dt * (double)dphidt));
+}
+
+template <typename Real>
+struct ExactArgs {
+    int n, nsteps, cap;  // cap: cells with their faces in shared memory
+    const int *count, *list;
+    const double *dsum, *dfx, *dfy, *dfz;
+    const Real *b0;
+    Real *phi, *other;  // the density, and the buffer the first step writes
+    Real rho;
+    double dt, ih2;
+    unsigned *flag;  // per CTA, kFlagStride apart: steps done
+    int *status;
+};
+constexpr int kFlagStride = 32;
+constexpr int kResidentSteps = 4;  // fewer do not repay the fill of shared memory (the faces, once: about a step)
+constexpr int kResidentThreads = 1024;
+constexpr size_t kCellBytes = 7 * sizeof(double) + sizeof(int);
+
+// All steps in one launch: a CTA keeps a stretch of the list, with the faces and
+// their sums, in shared memory (what does not fit it reads again each step),
+// and waits after each step for the CTAs that own cells within a plane of its
+// own. The FP64 pipe's share of a step is 21 operations a cell at 16 cycles per
+// warp and SM: 3.1 us on 64^3, 24 on 128^3. The rest of the 8.2 and 28.8 us that
+// a launch per step took were the launch, the loads of the list and the faces
+// and the last CTAs' tail; this takes 5.7 and 26.0 us.
+template <typename Real>
+__global__ void __launch_bounds__(kResidentThreads, 1) k_exact_resident(ExactArgs<Real> a) {
+    extern __shared__ double s_d[];  // faces and sum, [7][cap]; then the cells
+    __shared__ int s_own[2];         // first and last CTA to wait for
+    int *s_cell = (int *)(s_d + 7 * (size_t)a.cap);
+    const int T = gridDim.x, rank = blockIdx.x, tid = threadIdx.x, m = *a.count, n2 = a.n * a.n;
+    auto begin_of = [&](int r) { return (int)((long)m * r / T); };
+    const int q0 = begin_of(rank), own = begin_of(rank + 1) - q0;
+    unsigned *flag = a.flag + (size_t)rank * kFlagStride;
+    if (own == 0) {  // nobody waits for this CTA's cells
+        if (tid == 0) *(volatile unsigned *)flag = 0x7fffffffu;
+        return;
+    }
+    auto faces = [&](int c, const Cell &q, double (&d)[6]) {
+        d[0] = a.dfx[q.W];
+        d[1] = a.dfx[c];
+        d[2] = a.dfy[q.S];
+        d[3] = a.dfy[c];
+        d[4] = a.dfz[q.B];
+        d[5] = a.dfz[c];
+    };
+    for (int i = tid; i < min(own, a.cap); i += kResidentThreads) {
+        const int e = a.list[q0 + i], c = e < 0 ? ~e : e;
+        double d[6];
+        faces(c, neighbours_of((size_t)c, a.n), d);
+#pragma unroll
+        for (int f = 0; f < 6; ++f) s_d[(size_t)f * a.cap + i] = d[f];
+        s_d[(size_t)6 * a.cap + i] = a.dsum[q0 + i];
+        s_cell[i] = e;
+    }
+    if (tid < 2) {
+        // the owner of the first listed cell from this stretch's first cell less a
+        // plane on, and of the last one up to its last cell and a plane; a
+        // stretch that wraps around in z waits for all
+        auto cell_at = [&](int i) {
+            const int e = a.list[i];
+            return (long)(e < 0 ? ~e : e);
+        };
+        const long first = cell_at(q0) - n2, last = cell_at(q0 + own - 1) + n2, N = (long)n2 * a.n;
+        int r = tid ? T - 1 : 0;
+        if (first >= 0 && last < N) {
+            const long want = tid ? last + 1 : first;
+            int lo = 0, hi = m;
+            while (lo < hi) {
+                const int mid = (lo + hi) / 2;
+                if (cell_at(mid) < want)
+                    lo = mid + 1;
+                else
+                    hi = mid;
+            }
+            const int at = tid ? lo - 1 : lo;
+            r = (int)((long)at * T / m);
+            while (begin_of(r + 1) <= at) ++r;
+            while (begin_of(r) > at) --r;
+        }
+        s_own[tid] = r;
+    }
+    __syncthreads();
+    const int wait = s_own[0] + tid;
+    const bool waits = wait <= s_own[1] && wait != rank;
+    Real *in = a.phi, *out = a.other;
+    for (int s = 0; s < a.nsteps; ++s) {
+        for (int i = tid; i < own; i += kResidentThreads) {
+            const bool here = i < a.cap;
+            const int e = here ? s_cell[i] : a.list[q0 + i], c = e < 0 ? ~e : e;
+            const Cell q = neighbours_of((size_t)c, a.n);
+            const Real p[7] = {in[c], in[q.W], in[q.E], in[q.S], in[q.N], in[q.B], in[q.F]};
+            double d[6], sum;
+            if (here) {
+#pragma unroll
+                for (int f = 0; f < 6; ++f) d[f] = s_d[(size_t)f * a.cap + i];
+                sum = s_d[(size_t)6 * a.cap + i];
+            } else {
+                faces(c, q, d);
+                sum = a.dsum[q0 + i];
+            }
+            out[c] = listed_step<Real>(e, d, sum, p, a.b0, a.rho, a.dt, a.ih2);
+        }
+        if (s == a.nsteps - 1) break;
+        // no cell of the next step's input is written again before its readers
+        // are done: they are the CTAs waited for here
+        __syncthreads();
+        if (tid == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(flag), "r"(s + 1) : "memory");
+        int ok = 1;
+        if (waits) {
+            const unsigned *f = a.flag + (size_t)wait * kFlagStride;
+            long long spins = 0;
+            for (;;) {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(f) : "memory");
+                if (v >= (unsigned)(s + 1)) break;
+                if (++spins > (1ll << 24)) {
+                    atomicExch(a.status, (int)DEV_BARRIER_TIMEOUT);
+                    ok = 0;
+                    break;
+                }
+                if ((spins & 1023) == 0 && *(volatile int *)a.status != DEV_OK) {
+                    ok = 0;
+                    break;
+                }
+            }
+        }
+        if (!__syncthreads_and(ok)) break;
+        Real *const t = in;
+        in = out;
+        out = t;
+    }
+}
+
 template <typename Real>
 __global__ void __launch_bounds__(64) k_exact_list(int n, const int *__restrict__ count, const int *__restrict__ list,
                                                    const double *__restrict__ dsum, const Real *__restrict__ phi,
@@ -182,29 +355,9 @@ __global__ void __launch_bounds__(64) k_exact_list(int n, const int *__restrict_
         const int e = list[i];
         const size_t c = (size_t)(e < 0 ? ~e : e);
         const Cell q = neighbours_of(c, n);
-        const Real p0 = phi[c], pW = phi[q.W], pE = phi[q.E], pS = phi[q.S], pN = phi[q.N], pB = phi[q.B], pF = phi[q.F];
-        double df0 = dfx[q.W], df1 = dfx[c], df2 = dfy[q.S], df3 = dfy[c], df4 = dfz[q.B], df5 = dfz[c];
-        double sum = dsum[i];
-        if (e < 0) {
-            const Real tissue = b0[c] + p0;
-            if (!(tissue > 0.)) df0 = df1 = df2 = df3 = df4 = df5 = 0.0;
-            if (df0 == 0 && pW > 0.) df1 *= 2.0;
-            if (df1 == 0 && pE > 0.) df0 *= 2.0;
-            if (df2 == 0 && pS > 0.) df3 *= 2.0;
-            if (df3 == 0 && pN > 0.) df2 *= 2.0;
-            if (df4 == 0 && pB > 0.) df5 *= 2.0;
-            if (df5 == 0 && pF > 0.) df4 *= 2.0;
-            sum = df0 + df1 + df2 + df3 + df4 + df5;
-        }
-        const double fin = ih2 * (df0 * widen(pW) + df1 * widen(pE) + df2 * widen(pS) + df3 * widen(pN) + df4 * widen(pB) +
-                                  df5 * widen(pF));
-        const double fout = -(sum * widen(p0) * ih2);
-        const double react = reaction(rho, p0);
-        const Real dphidt = (Real)(fout + fin + react);
-        Real v = (Real)(widen(p0) + dt * (double)dphidt);
-        v = ((Real)0 < v) ? v : (Real)0;
-        v = (v < (Real)1) ? v : (Real)1;
-        out[c] = v;
+        const Real p[7] = {phi[c], phi[q.W], phi[q.E], phi[q.S], phi[q.N], phi[q.B], phi[q.F]};
+        const double d[6] = {dfx[q.W], dfx[c], dfy[q.S], dfy[c], dfz[q.B], dfz[c]};
+        out[c] = listed_step<Real>(e, d, dsum[i], p, b0, rho, dt, ih2);
     }
 }
 
@@ -323,12 +476,50 @@ int exact_build_tables(Handle &h, double Dw, double Dg) {
 
 void exact_alloc_list(Handle &h) {
     const size_t chunks = (h.N + 255) / 256;
-    if (cudaMalloc((void **)&h.exact_list, (h.N + chunks + 1) * sizeof(int)) != cudaSuccess ||
+    if (cudaMalloc((void **)&h.exact_list, (h.N + chunks + 1 + (size_t)h.num_sms * kFlagStride) * sizeof(int)) != cudaSuccess ||
         cudaMalloc((void **)&h.exact_dsum, h.N * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         if (h.exact_list) cudaFree(h.exact_list);
         h.exact_list = nullptr;
     }
+}
+
+// nsteps steps over the list in one launch; GBG_ERR_UNSUPPORTED: not here
+template <typename Real>
+int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps) {
+    const int T = h.num_sms, chunks = (int)((h.N + 255) / 256);
+    ExactArgs<Real> a;
+    a.n = h.n;
+    a.nsteps = (int)nsteps;
+    a.cap = (int)std::min<size_t>((h.N + T - 1) / T, (224 * 1024) / kCellBytes);
+    a.cap += a.cap & 1;
+    const size_t smem = a.cap * kCellBytes;
+    a.count = h.exact_list + h.N + chunks;
+    a.list = h.exact_list;
+    a.dsum = h.exact_dsum;
+    a.dfx = h.dfx;
+    a.dfy = h.dfy;
+    a.dfz = h.dfz;
+    a.b0 = (const Real *)h.b0;
+    a.phi = (Real *)h.phi[h.cur];
+    a.other = (Real *)h.phi[h.cur ^ 1];
+    a.rho = (Real)rho;
+    a.dt = dt;
+    a.ih2 = ih2;
+    a.flag = (unsigned *)(h.exact_list + h.N + chunks + 1);
+    a.status = h.dev_status;
+    const void *fn = (const void *)k_exact_resident<Real>;
+    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBG_CUDA_TRY(cudaMemsetAsync(a.flag, 0, (size_t)T * kFlagStride * sizeof(unsigned), h.stream));
+    void *args[] = {&a};
+    if (cudaLaunchCooperativeKernel(fn, dim3((unsigned)T), dim3(kResidentThreads), args, smem, h.stream) != cudaSuccess) {
+        cudaGetLastError();
+        return GBG_ERR_UNSUPPORTED;
+    }
+    h.exact_waited = true;
+    h.launches++;
+    if (nsteps & 1) h.cur ^= 1;
+    return GBG_OK;
 }
 
 int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nsteps) {
@@ -338,19 +529,19 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
     const double ih2 = 1. / (hh * hh);
     const int g = grid_for(h), chunks = (int)((h.N + 255) / 256);
     const int gl = (int)std::min<size_t>((h.N + 63) / 64, (size_t)h.num_sms * 16);
+    auto collect = [&](auto real) {
+        using Real = decltype(real);
+        int *offset = h.exact_list + h.N;
+        const Real *b0 = (const Real *)h.b0;
+        k_exact_collect<Real, false><<<chunks, 256, 0, h.stream>>>(h.n, b0, h.dfx, h.dfy, h.dfz, offset, nullptr, nullptr);
+        k_exact_offsets<<<1, 1024, 0, h.stream>>>(chunks, offset);
+        k_exact_collect<Real, true><<<chunks, 256, 0, h.stream>>>(h.n, b0, h.dfx, h.dfy, h.dfz, offset, h.exact_list, h.exact_dsum);
+        h.launches += 3;
+        h.exact_listed = true;
+    };
     auto step = [&](auto real, const void *in, void *out) {
         using Real = decltype(real);
         if (h.exact_full >= 2 && h.exact_list) {
-            if (!h.exact_listed) {
-                int *offset = h.exact_list + h.N;
-                const Real *b0 = (const Real *)h.b0;
-                k_exact_collect<Real, false><<<chunks, 256, 0, h.stream>>>(h.n, b0, h.dfx, h.dfy, h.dfz, offset, nullptr, nullptr);
-                k_exact_offsets<<<1, 1024, 0, h.stream>>>(chunks, offset);
-                k_exact_collect<Real, true><<<chunks, 256, 0, h.stream>>>(h.n, b0, h.dfx, h.dfy, h.dfz, offset, h.exact_list,
-                                                                          h.exact_dsum);
-                h.launches += 3;
-                h.exact_listed = true;
-            }
             k_exact_list<Real><<<gl, 64, 0, h.stream>>>(h.n, h.exact_list + h.N + chunks, h.exact_list, h.exact_dsum, (const Real *)in,
                                                         (Real *)out, (const Real *)h.b0, h.dfx, h.dfy, h.dfz, (Real)rho, dt, ih2);
         } else {
@@ -360,6 +551,15 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
         }
     };
     for (long s = 0; s < nsteps; ++s) {
+        if (h.exact_full >= 2 && h.exact_list) {
+            if (!h.exact_listed) h.prec == GBG_PREC_F64 ? collect(double{}) : collect(float{});
+            if (nsteps - s >= kResidentSteps && nsteps - s < 0x7fffffffL) {
+                const int rc = h.prec == GBG_PREC_F64 ? resident_steps<double>(h, rho, dt, ih2, nsteps - s)
+                                                      : resident_steps<float>(h, rho, dt, ih2, nsteps - s);
+                if (rc == GBG_OK) break;
+                if (rc != GBG_ERR_UNSUPPORTED) return rc;
+            }
+        }
         if (h.prec == GBG_PREC_F64)
             step(double{}, h.phi[h.cur], h.phi[h.cur ^ 1]);
         else

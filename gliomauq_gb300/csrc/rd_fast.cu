@@ -1450,6 +1450,15 @@ int check_device_status(Handle &h) {
     return GBG_OK;
 }
 
+int finish_steps(Handle &h) {
+    if (h.exact_waited) {
+        h.exact_waited = false;
+        return check_device_status(h);
+    }
+    GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    return GBG_OK;
+}
+
 int launch_schedule_smooth(Handle &h, const gbg_sample *samples_device, int S, double L, double dt0,
                            SampleRec *dev_out) {
     k_schedule_smooth<<<(S + 127) / 128, 128, 0, h.stream>>>(samples_device, S, h.n, L, dt0, dev_out);

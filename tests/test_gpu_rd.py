@@ -153,3 +153,31 @@ def test_exact_steps_over_the_live_cells_equal_oracle(gbg, oracle_lib, prec, kin
                 done += steps
                 ref = oracle_lib.rd_solve(pw, pg, phi, dw, dg, 0.025, dt, done, "f32ref" if f32 else "f64")
                 assert np.array_equal(h.get_phi(), ref.astype(np.float64)), (Dw_file, done)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32ref"])
+@pytest.mark.parametrize("n,dense", [(5, True), (16, False), (40, True), (64, False), (100, True)])
+def test_exact_steps_in_one_call_equal_single_steps(gbg, precision, n, dense):
+    """Many exact steps in one call run in one launch whose CTAs wait for their
+    neighbours: the bits of the same steps in calls of their own, with fewer
+    cells than CTAs, tissue up to the periodic faces (dense), more cells than
+    the CTAs' shared memory holds, and an even and an odd number of steps."""
+    rng = np.random.default_rng(n)
+    if dense:
+        pw, pg = rng.uniform(0.05, 1.0, (2, n, n, n))
+    else:
+        an = S.make_anatomy(n, seed=3)
+        pw, pg = an.p_w, an.p_g
+    phi = rng.uniform(0.0, 1.0, (n, n, n)) * (pw + pg > 0)
+    D = 0.1 / n ** 2
+    with _lib.Handle(n, precision) as h:
+        h.set_anatomy(pw, pg)
+        outs = []
+        for calls in ((1,) * 13, (13,), (2, 4, 7), (6, 1, 6)):
+            h.set_phi(phi)
+            for k in calls:
+                h.rd_step(D, 0.1 * D, 0.05, 0.6, k)
+            outs.append(h.get_phi())
+    assert outs[0].max() > 0
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0])
