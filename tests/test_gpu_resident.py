@@ -51,3 +51,24 @@ def test_resident_kernel_equals_dense(gbg, n, kind, count):
             assert np.array_equal(out[0]["nsteps"], out[1]["nsteps"])
             for j in range(count):
                 assert np.array_equal(out[0]["phi"][j], out[1]["phi"][j]), (sigma, j)
+
+
+@pytest.mark.parametrize("n", [32, 64, 128])
+@pytest.mark.parametrize("steps", [(4,), (5,), (3, 4, 6), (25,)])
+def test_single_solve_equals_the_dense_kernel(gbg, n, steps):
+    """gbg_rd_step on the resident kernel takes any state (values outside the
+    tissue and beyond [0, 1] too) to the dense kernel's bits."""
+    an = S.make_anatomy(n, seed=6)
+    phi = np.random.default_rng(n).uniform(-0.2, 1.2, (n, n, n))
+    D = 0.1 / n ** 2
+    outs = []
+    for variant in (0, 1):
+        with _lib.Handle(n, "f32", max_samples=1) as h:
+            h.set_anatomy(an.p_w, an.p_g)
+            h.set_population_variant(variant)
+            h.set_phi(phi)
+            for k in steps:
+                h.rd_step(D, 0.1 * D, 0.05, 0.6, k)
+            outs.append(h.get_phi())
+    assert np.array_equal(outs[0], outs[1])
+    assert outs[0].max() > 0
