@@ -220,34 +220,28 @@ struct ExactArgs {
     Real *phi, *other;  // the density, and the buffer the first step writes
     Real rho;
     double dt, ih2;
-    unsigned *flag;  // per CTA, kFlagStride apart: steps done
+    unsigned *arrived;  // arrivals at the barrier between steps
     int *status;
 };
-constexpr int kFlagStride = 32;
 constexpr int kResidentSteps = 4;  // fewer do not repay the fill of shared memory (the faces, once: about a step)
 constexpr int kResidentThreads = 1024;
 constexpr size_t kCellBytes = 7 * sizeof(double) + sizeof(int);
 
 // All steps in one launch: a CTA keeps a stretch of the list, with the faces and
-// their sums, in shared memory (what does not fit it reads again each step),
-// and waits after each step for the CTAs that own cells within a plane of its
-// own. The FP64 pipe's share of a step is 21 operations a cell at 16 cycles per
-// warp and SM: 3.1 us on 64^3, 24 on 128^3. The rest of the 8.2 and 28.8 us that
-// a launch per step took were the launch, the loads of the list and the faces
-// and the last CTAs' tail; this takes 5.7 and 26.0 us.
+// their sums, in shared memory (what does not fit it reads again each step). The
+// FP64 pipe's share of a step is 21 operations a cell at 16 cycles per warp and
+// SM: 3.1 us on 64^3, 24 on 128^3. The rest of the 8.2 and 28.8 us that a launch
+// per step took were the launch, the loads of the list and the faces and the
+// last CTAs' tail; this takes 5.6 and 26.0 us. (Waiting for the CTAs that own
+// cells within a plane, by flags of their own, instead of counting all: 5.7, and
+// 2.8 against 2.7 us at 33^3.)
 template <typename Real>
 __global__ void __launch_bounds__(kResidentThreads, 1) k_exact_resident(ExactArgs<Real> a) {
     extern __shared__ double s_d[];  // faces and sum, [7][cap]; then the cells
-    __shared__ int s_own[2];         // first and last CTA to wait for
     int *s_cell = (int *)(s_d + 7 * (size_t)a.cap);
-    const int T = gridDim.x, rank = blockIdx.x, tid = threadIdx.x, m = *a.count, n2 = a.n * a.n;
+    const int T = gridDim.x, rank = blockIdx.x, tid = threadIdx.x, m = *a.count;
     auto begin_of = [&](int r) { return (int)((long)m * r / T); };
     const int q0 = begin_of(rank), own = begin_of(rank + 1) - q0;
-    unsigned *flag = a.flag + (size_t)rank * kFlagStride;
-    if (own == 0) {  // nobody waits for this CTA's cells
-        if (tid == 0) *(volatile unsigned *)flag = 0x7fffffffu;
-        return;
-    }
     auto faces = [&](int c, const Cell &q, double (&d)[6]) {
         d[0] = a.dfx[q.W];
         d[1] = a.dfx[c];
@@ -265,36 +259,6 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_exact_resident(ExactArg
         s_d[(size_t)6 * a.cap + i] = a.dsum[q0 + i];
         s_cell[i] = e;
     }
-    if (tid < 2) {
-        // the owner of the first listed cell from this stretch's first cell less a
-        // plane on, and of the last one up to its last cell and a plane; a
-        // stretch that wraps around in z waits for all
-        auto cell_at = [&](int i) {
-            const int e = a.list[i];
-            return (long)(e < 0 ? ~e : e);
-        };
-        const long first = cell_at(q0) - n2, last = cell_at(q0 + own - 1) + n2, N = (long)n2 * a.n;
-        int r = tid ? T - 1 : 0;
-        if (first >= 0 && last < N) {
-            const long want = tid ? last + 1 : first;
-            int lo = 0, hi = m;
-            while (lo < hi) {
-                const int mid = (lo + hi) / 2;
-                if (cell_at(mid) < want)
-                    lo = mid + 1;
-                else
-                    hi = mid;
-            }
-            const int at = tid ? lo - 1 : lo;
-            r = (int)((long)at * T / m);
-            while (begin_of(r + 1) <= at) ++r;
-            while (begin_of(r) > at) --r;
-        }
-        s_own[tid] = r;
-    }
-    __syncthreads();
-    const int wait = s_own[0] + tid;
-    const bool waits = wait <= s_own[1] && wait != rank;
     Real *in = a.phi, *out = a.other;
     for (int s = 0; s < a.nsteps; ++s) {
         for (int i = tid; i < own; i += kResidentThreads) {
@@ -314,18 +278,16 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_exact_resident(ExactArg
             out[c] = listed_step<Real>(e, d, sum, p, a.b0, a.rho, a.dt, a.ih2);
         }
         if (s == a.nsteps - 1) break;
-        // no cell of the next step's input is written again before its readers
-        // are done: they are the CTAs waited for here
         __syncthreads();
-        if (tid == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(flag), "r"(s + 1) : "memory");
         int ok = 1;
-        if (waits) {
-            const unsigned *f = a.flag + (size_t)wait * kFlagStride;
+        if (tid == 0) {  // grid barrier, bounded (seconds)
+            const unsigned target = (unsigned)(s + 1) * T;
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(a.arrived) : "memory");
             long long spins = 0;
             for (;;) {
                 unsigned v;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(f) : "memory");
-                if (v >= (unsigned)(s + 1)) break;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(a.arrived) : "memory");
+                if (v >= target) break;
                 if (++spins > (1ll << 24)) {
                     atomicExch(a.status, (int)DEV_BARRIER_TIMEOUT);
                     ok = 0;
@@ -476,7 +438,7 @@ int exact_build_tables(Handle &h, double Dw, double Dg) {
 
 void exact_alloc_list(Handle &h) {
     const size_t chunks = (h.N + 255) / 256;
-    if (cudaMalloc((void **)&h.exact_list, (h.N + chunks + 1 + (size_t)h.num_sms * kFlagStride) * sizeof(int)) != cudaSuccess ||
+    if (cudaMalloc((void **)&h.exact_list, (h.N + chunks + 2) * sizeof(int)) != cudaSuccess ||
         cudaMalloc((void **)&h.exact_dsum, h.N * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         if (h.exact_list) cudaFree(h.exact_list);
@@ -506,11 +468,11 @@ int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps) {
     a.rho = (Real)rho;
     a.dt = dt;
     a.ih2 = ih2;
-    a.flag = (unsigned *)(h.exact_list + h.N + chunks + 1);
+    a.arrived = (unsigned *)(h.exact_list + h.N + chunks + 1);
     a.status = h.dev_status;
     const void *fn = (const void *)k_exact_resident<Real>;
     GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    GBG_CUDA_TRY(cudaMemsetAsync(a.flag, 0, (size_t)T * kFlagStride * sizeof(unsigned), h.stream));
+    GBG_CUDA_TRY(cudaMemsetAsync(a.arrived, 0, sizeof(unsigned), h.stream));
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel(fn, dim3((unsigned)T), dim3(kResidentThreads), args, smem, h.stream) != cudaSuccess) {
         cudaGetLastError();
@@ -553,7 +515,7 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
     for (long s = 0; s < nsteps; ++s) {
         if (h.exact_full >= 2 && h.exact_list) {
             if (!h.exact_listed) h.prec == GBG_PREC_F64 ? collect(double{}) : collect(float{});
-            if (nsteps - s >= kResidentSteps && nsteps - s < 0x7fffffffL) {
+            if (nsteps - s >= kResidentSteps && nsteps - s < 0x7fffffffL / h.num_sms) {  // arrivals are counted in 32 bits
                 const int rc = h.prec == GBG_PREC_F64 ? resident_steps<double>(h, rho, dt, ih2, nsteps - s)
                                                       : resident_steps<float>(h, rho, dt, ih2, nsteps - s);
                 if (rc == GBG_OK) break;
