@@ -103,19 +103,11 @@ __global__ void k_amr_tables(int nb, RegionTable rt, const Real *__restrict__ pw
         for (int k = 0; k < 7; ++k) {
             const Real a = lab_at(rt, pw, gpw, b, nx[k], ny[k], nz[k]);
             const Real g = lab_at(rt, pg, gpg, b, nx[k], ny[k], nz[k]);
-            const Real brain = a + g;
-            const Real kk = (a * Dw + g * Dg) / brain;
-            inv[k] = 1.0 / (double)kk;
-            if (k == 0) b0[i] = brain;
+            inv[k] = inverse_k(a, g, Dw, Dg);
+            if (k == 0) b0[i] = a + g;
         }
-        for (int f = 0; f < 6; ++f) df[(size_t)i * 6 + f] = 2.0 * (1.0 / (inv[0] + inv[f + 1]));
+        for (int f = 0; f < 6; ++f) df[(size_t)i * 6 + f] = face_k(inv[0], inv[f + 1]);
     }
-}
-
-__device__ __forceinline__ double reaction(double rho, double p) { return rho * p * (1. - p); }
-__device__ __forceinline__ double reaction(float rho, float p) {
-    const float rp = rho * p;
-    return (double)rp * (1. - (double)p);
 }
 
 template <typename Real>
@@ -230,11 +222,11 @@ __global__ void __launch_bounds__(64) k_amr_list(RegionTable rt, const int *__re
             if (d5 == 0 && pF > 0.) d4 *= 2.0;
             sum = d0 + d1 + d2 + d3 + d4 + d5;
         }
-        const double fin = ih2 * (d0 * widen(pW) + d1 * widen(pE) + d2 * widen(pS) + d3 * widen(pN) + d4 * widen(pB) + d5 * widen(pF));
-        const double fout = -(sum * widen(p0) * ih2);
+        const double fin = ih2 * (d0 * (double)pW + d1 * (double)pE + d2 * (double)pS + d3 * (double)pN + d4 * (double)pB + d5 * (double)pF);
+        const double fout = -(sum * (double)p0 * ih2);
         const double react = reaction(rho, p0);
         const Real dphidt = (Real)(fout + fin + react);
-        Real v = (Real)(widen(p0) + dt * (double)dphidt);
+        Real v = (Real)((double)p0 + dt * (double)dphidt);
         v = ((Real)0 < v) ? v : (Real)0;
         v = (v < (Real)1) ? v : (Real)1;
         out[c] = v;
@@ -904,6 +896,10 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
     };
     for (long s = 0; s < nsteps; ++s) {
         void *in = h.amr.phi[h.amr.cur], *out = h.amr.phi[h.amr.cur ^ 1];
+        if (h.amr.full_steps == 1 && h.amr.list) {  // the other buffer's dead cells
+            GBG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)cells * (f64 ? sizeof(double) : sizeof(float)), h.stream));
+            h.amr.full_steps = 2;
+        }
         if (f64)
             step(double{}, in, out);
         else

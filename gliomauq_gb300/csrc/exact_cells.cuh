@@ -1,7 +1,7 @@
 // What the exact steps of the uniform grid (rd_exact.cu) and of the block grid
 // (amr.cu) share: the classes of cells (rd_exact.cu says why), the offsets of
-// their list, and the widening of a float. Both are compiled with
-// -fmad=false.
+// their list, the faces' diffusivities and the reaction. Both are compiled
+// with -fmad=false.
 #pragma once
 
 namespace gbg {
@@ -45,14 +45,26 @@ __global__ void __launch_bounds__(1024) k_exact_offsets(int chunks, int *__restr
     if (threadIdx.x == 0) offset[chunks] = total;
 }
 
-// a float widened with integer operations where it is a normal number (the
-// conversion unit is as narrow as the FP64 pipe); a zero loses its sign
-__device__ __forceinline__ double widen(double p) { return p; }
-__device__ __forceinline__ double widen(float p) {
-    const unsigned u = __float_as_uint(p), m = u & 0x7fffffffu;
-    if (m - 0x00800000u < 0x7f000000u)
-        return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(u << 29));
-    return m ? (double)p : 0.0;
+// The reciprocal conductivity of a cell and the diffusivity of the face between
+// two, without the divisions (a dozen and more FP64 operations each) where the
+// result is NaN: toward and between cells without tissue, two thirds of a grid.
+__device__ __forceinline__ double as_nan() { return __hiloint2double(0x7ff80000, 0); }
+template <typename Real>
+__device__ __forceinline__ double inverse_k(Real a, Real b, Real Dw, Real Dg) {
+    if (a == (Real)0 && b == (Real)0) return as_nan();
+    const Real kk = (a * Dw + b * Dg) / (a + b);
+    return 1.0 / (double)kk;
+}
+__device__ __forceinline__ double face_k(double inv0, double inv1) {
+    const double s = inv0 + inv1;
+    if (((unsigned)__double2hiint(s) & 0x7fffffffu) > 0x7ff00000u) return as_nan();
+    return 2.0 * (1.0 / s);
+}
+
+__device__ __forceinline__ double reaction(double rho, double p) { return rho * p * (1. - p); }
+__device__ __forceinline__ double reaction(float rho, float p) {
+    const float rp = rho * p;
+    return (double)rp * (1. - (double)p);
 }
 
 }  // namespace

@@ -70,8 +70,7 @@ struct AmrState {
     int *bidx = nullptr;       // block index (ix, iy, iz) per block
     int *rkind = nullptr, *rsrc = nullptr;  // remap plan
     // the cells an exact step has to compute (as Handle::exact_list), for the
-    // present grid and tables when listed; steps over every cell since those
-    // or the density were set
+    // present grid and tables when listed; full_steps as Handle::exact_full
     int *list = nullptr;
     double *dsum = nullptr;
     bool listed = false;
@@ -119,8 +118,9 @@ struct Handle {
     // the cells an exact step has to compute (rd_exact.cu): their list, its
     // chunk offsets and its length behind it (null: no memory for it at creation,
     // every step computes every cell); the plain cells' sums of faces; whether
-    // the list is that of the present tables; steps over every cell since the
-    // density or the tables were set
+    // the list is that of the present tables; 0: the density or the tables were
+    // set since the last step, 1: a step over every cell was taken, 2: both
+    // buffers have zeros where no listed cell is
     int *exact_list = nullptr;
     double *exact_dsum = nullptr;
     bool exact_listed = false;

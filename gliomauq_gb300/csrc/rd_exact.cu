@@ -44,25 +44,17 @@ __global__ void k_build_tables(int n, const double *__restrict__ pw, const doubl
         Real bc = 0;
         for (int k = 0; k < 4; ++k) {
             const Real a = (Real)pw[nb[k]], b = (Real)pg[nb[k]];
-            const Real brain = a + b;
-            const Real kk = (a * Dw + b * Dg) / brain;
-            inv[k] = 1.0 / (double)kk;
-            if (k == 0) bc = brain;
+            inv[k] = inverse_k(a, b, Dw, Dg);
+            if (k == 0) bc = a + b;
         }
         b0[c] = bc;
-        dfx[c] = 2.0 * (1.0 / (inv[0] + inv[1]));
-        dfy[c] = 2.0 * (1.0 / (inv[0] + inv[2]));
-        dfz[c] = 2.0 * (1.0 / (inv[0] + inv[3]));
+        dfx[c] = face_k(inv[0], inv[1]);
+        dfy[c] = face_k(inv[0], inv[2]);
+        dfz[c] = face_k(inv[0], inv[3]);
     }
 }
 
 // rho * phi * (1. - phi): (rho*phi) in Real, times (1.0 - phi) in double.
-__device__ __forceinline__ double reaction(double rho, double p) { return rho * p * (1. - p); }
-__device__ __forceinline__ double reaction(float rho, float p) {
-    const float rp = rho * p;
-    return (double)rp * (1. - (double)p);
-}
-
 // One step: RHS of Glioma_ReactionDiffusionOperator<3> (:148-218), the dphidt
 // rounding to Real, and UpdateTumor<3> (:254-261) with std::max / std::min
 // clamping (NaN -> 0).
@@ -117,8 +109,8 @@ __global__ void k_exact_step(int n, const Real *__restrict__ phi, Real *__restri
 //            faces is a constant of the tables
 //   special  anything else: the step as it is written
 // (densities are finite and in [0, 1] from the first step on). k_exact_list
-// runs over the list of plain and special cells; two steps over every cell
-// leave the dead ones' zeros in both buffers. Measured on 64^3 (32 % plain),
+// runs over the list of plain and special cells; a step over every cell leaves
+// the dead ones' zeros in one buffer, and the other is filled with zeros. Measured on 64^3 (32 % plain),
 // 237 steps with upload and download: 7.0 ms on every cell, 2.3 ms on the list
 // with a launch per step, 1.6 in one launch (k_exact_resident).
 struct Cell {
@@ -203,12 +195,12 @@ __device__ __forceinline__ Real listed_step(int e, const double (&t)[6], double 
         }
         sum = d[0] + d[1] + d[2] + d[3] + d[4] + d[5];
     }
-    const double fin = ih2 * (d[0] * widen(p[1]) + d[1] * widen(p[2]) + d[2] * widen(p[3]) + d[3] * widen(p[4]) + d[4] * widen(p[5]) +
-                              d[5] * widen(p[6]));
-    const double fout = -(sum * widen(p[0]) * ih2);
+    const double fin = ih2 * (d[0] * (double)p[1] + d[1] * (double)p[2] + d[2] * (double)p[3] + d[3] * (double)p[4] + d[4] * (double)p[5] +
+                              d[5] * (double)p[6]);
+    const double fout = -(sum * (double)p[0] * ih2);
     const double react = reaction(rho, p[0]);
     const Real dphidt = (Real)(fout + fin + react);
-    return clamp01((Real)(widen(p[0]) + dt * (double)dphidt));
+    return clamp01((Real)((double)p[0] + dt * (double)dphidt));
 }
 
 template <typename Real>
@@ -513,6 +505,10 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
         }
     };
     for (long s = 0; s < nsteps; ++s) {
+        if (h.exact_full == 1 && h.exact_list) {  // the other buffer's dead cells
+            GBG_CUDA_TRY(cudaMemsetAsync(h.phi[h.cur ^ 1], 0, h.N * (h.prec == GBG_PREC_F64 ? sizeof(double) : sizeof(float)), h.stream));
+            h.exact_full = 2;
+        }
         if (h.exact_full >= 2 && h.exact_list) {
             if (!h.exact_listed) h.prec == GBG_PREC_F64 ? collect(double{}) : collect(float{});
             if (nsteps - s >= kResidentSteps && nsteps - s < 0x7fffffffL / h.num_sms) {  // arrivals are counted in 32 bits

@@ -63,7 +63,7 @@ def test_amr_random_fields_match_oracle(gbg, variant):
 @pytest.mark.parametrize("variant", ["f64", "f32"])
 @pytest.mark.parametrize("split", [(1, 1, 3), (2, 1), (5,)])
 def test_amr_listed_steps_match_oracle(gbg, variant, split):
-    """From the third step of a grid on, only the cells that can be nonzero are
+    """From the second step of a grid on, only the cells that can be nonzero are
     stepped and ghosts are evaluated where they are used: the oracle's bits
     over split calls, after a change of the coefficients, and with tables whose
     weights have either sign and any size."""

@@ -158,8 +158,8 @@ def test_exact_steps_over_the_live_cells_equal_oracle(gbg, oracle_lib, prec, kin
 @pytest.mark.parametrize("precision", ["f64", "f32ref"])
 @pytest.mark.parametrize("n,dense", [(5, True), (16, False), (40, True), (64, False), (100, True)])
 def test_exact_steps_in_one_call_equal_single_steps(gbg, precision, n, dense):
-    """Many exact steps in one call run in one launch whose CTAs wait for their
-    neighbours: the bits of the same steps in calls of their own, with fewer
+    """Many exact steps in one call run in one launch whose CTAs meet between
+    steps: the bits of the same steps in calls of their own, with fewer
     cells than CTAs, tissue up to the periodic faces (dense), more cells than
     the CTAs' shared memory holds, and an even and an odd number of steps."""
     rng = np.random.default_rng(n)
