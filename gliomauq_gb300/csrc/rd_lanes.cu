@@ -358,7 +358,11 @@ int lanes_set_anatomy(Handle &h) {
 // fewer: 32.2 ms at 14, the lanes then idle at their barriers). Where samples
 // are few the teams grow until 8 lanes each cover them, down to 4 units per
 // CTA, below which a step is all barrier (6 samples at 32^3: 1.71 ms at 28
-// units, 1.42 ms at 4; 32 at 64^3: 4.9 ms at 28, 4.0 ms at 14).
+// units, 1.42 ms at 4; 32 at 64^3: 4.9 ms at 28, 4.0 ms at 14). A lane has no
+// more warps than its CTA units, and at most 8: a warp that comes to the
+// barrier without work costs the others more than it helps (one sample at
+// 32^3: 0.41 ms with 16 warps, 0.35 with 4; at 64^3 0.47 and 0.43; at 128^3
+// 0.635 with 16, 0.62 with 8 warps, 0.70 with 4).
 static void lane_shape(const Handle &h, int S, LaneArgs &a, int &units) {
     const int nl = std::max(1, h.units[0]), sms = h.num_sms;
     const int wide = sms / ((S + kMaxLanes - 1) / kMaxLanes), least = (nl + 27) / 28, most = (nl + 3) / 4;
@@ -367,8 +371,8 @@ static void lane_shape(const Handle &h, int S, LaneArgs &a, int &units) {
     a.T = sms / a.teams;
     a.teams = std::min(a.teams, S);
     a.lanes = std::min(kMaxLanes, (S + a.teams - 1) / a.teams);
-    a.warps = 4 * kWps / a.lanes;
     units = 2 * ((nl + 2 * a.T - 1) / (2 * a.T));
+    a.warps = std::min({4 * kWps / a.lanes, units, 8});
 }
 
 bool lanes_fit(const Handle &h, int S) {
