@@ -12,9 +12,9 @@
 // live. A thread adds its row's sensitivity products over a block in float, in
 // plane order, and widens them once: the sums of the tile kernel
 // (k_adj_back128), bit for bit. Blocks are dealt to the CTAs one by one, two
-// per CTA on an ellipsoidal brain, one per warp with 8 lanes.
-// 64 samples near the mode at 128^3: the backward kernels 37 ms instead of 56,
-// the whole call 56.1 ms instead of 86.4.
+// per CTA on an ellipsoidal brain, one per warp with 4 lanes.
+// 64 samples near the mode at 128^3: the backward kernels 34 ms instead of
+// 56, the whole call 52.4 ms instead of 86.3.
 #include <algorithm>
 #include <vector>
 
@@ -26,6 +26,13 @@ using namespace lanes;
 
 constexpr int LR = 32, n = 128, plane = n * n, N = n * n * n;
 constexpr int kBlockZ = 16, kBlocks = (n / 2) * (n / kBlockZ);
+// Four lanes of two warps with 255 registers each, and two planes ahead. Eight
+// lanes of two warps leave no registers for the second plane, and their
+// samples' lambda, mu (twice) and states (the step's and the next one's) do not
+// stay in L2 together: 59.6 ms for the call below (on other samples), against
+// 56.5 with four; eight lanes of one warp 64, four lanes with three planes ahead
+// (spilled) 65.
+constexpr int kAdjWarps = 8, kAdjThreads = 32 * kAdjWarps, kAdjLanes = 4;
 constexpr int kMaxBlocks = 4;  // per CTA: 64 units, 224 KB
 
 struct AdjArgs {
@@ -74,80 +81,89 @@ __device__ __forceinline__ void sweep(const float4 *__restrict__ tab, int y, int
                                       const float *g, float *out, const float *__restrict__ cz, float a, float b, long pre, float (&acc)[4]) {
     const int li = threadIdx.x & 31;
     const int o0 = 4 * li + n * y + plane * z, below = z == 0 ? plane * (n - 1) : -plane, dS = south(y), dT = north2(y);
-    const float *pN = f + o0;
+    const float *pN = f + o0;  // the plane last loaded
     out += o0;
     g += o0;
     int zn = z;
-    auto up = [&] { pN += ++zn == n ? -plane * (n - 1) : plane; };
-    V4 P0 = ldp(pN), P1 = ldp(pN + n), B0 = ldp(pN + below), B1 = ldp(pN + below + n);
-    V4 C0 = ldg4(cz + o0 + below), C1 = ldg4(cz + o0 + below + n);
-    V4 S = ldp(pN + dS), T = ldp(pN + dT);
-    up();
-    V4 N0 = ldp(pN), N1 = ldp(pN + n), G0 = ldp(g), G1 = ldp(g + n);
-    B0 = sub(P0, B0);
-    B1 = sub(P1, B1);
-#pragma unroll 1
-    for (int j = 0; j < len; ++j) {
-        auto finish = [&](const V4 &P, const V4 &lap, const V4 &CX, const V4 &G, int r) {
-            float o[4], pa = 0.0f, pb = 0.0f;
+    // Registers in rings, as in the population kernel: the rows of planes j ..
+    // j + 2, the rows beside them and the second operand of planes j and j + 1,
+    // the difference and the face to the plane before.
+    V4 X0[3], X1[3], S[2], T[2], G0[2], G1[2], B0[2], B1[2], C0[2], C1[2];
+    auto load_st = [&](int d) {  // of the plane pN is on; then to the next plane
+        S[d] = ldp(pN + dS);
+        T[d] = ldp(pN + dT);
+        pN += ++zn == n ? -plane * (n - 1) : plane;
+    };
+    X0[0] = ldp(pN);
+    X1[0] = ldp(pN + n);
+    B0[0] = ldp(pN + below);
+    B1[0] = ldp(pN + below + n);
+    C0[0] = ldg4(cz + o0 + below);
+    C1[0] = ldg4(cz + o0 + below + n);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float f0 = P.v[i];
-                if (MU) {
-                    float v = fmaf(a, lap.v[i], f0);
-                    v = fmaf(b * f0, 1.0f - f0, v);
-                    const float gate = (!signbit(CX.v[i]) && v >= 0.0f && v < 1.0f) ? 1.0f : 0.0f;
-                    o[i] = gate * G.v[i];
-                    pa = fmaf(o[i], lap.v[i], pa);
-                    pb = fmaf(o[i] * f0, 1.0f - f0, pb);
-                } else {
-                    o[i] = fmaf(a, lap.v[i], f0 * (1.0f + b * (1.0f - 2.0f * G.v[i])));
-                }
-            }
+    for (int d = 0; d < 2; ++d)
+        if (d < len) {
+            load_st(d);
+            X0[d + 1] = ldp(pN);
+            X1[d + 1] = ldp(pN + n);
+            G0[d] = ldp(g + d * plane);
+            G1[d] = ldp(g + d * plane + n);
+        }
+    B0[0] = sub(X0[0], B0[0]);
+    B1[0] = sub(X1[0], B1[0]);
+    auto finish = [&](const V4 &P, const V4 &lap, const V4 &CX, const V4 &G, int r) {
+        float o[4], pa = 0.0f, pb = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float f0 = P.v[i];
             if (MU) {
-                acc[2 * r] += pa;
-                acc[2 * r + 1] += pb;
+                float v = fmaf(a, lap.v[i], f0);
+                v = fmaf(b * f0, 1.0f - f0, v);
+                const float gate = (!signbit(CX.v[i]) && v >= 0.0f && v < 1.0f) ? 1.0f : 0.0f;
+                o[i] = gate * G.v[i];
+                pa = fmaf(o[i], lap.v[i], pa);
+                pb = fmaf(o[i] * f0, 1.0f - f0, pb);
+            } else {
+                o[i] = fmaf(a, lap.v[i], f0 * (1.0f + b * (1.0f - 2.0f * G.v[i])));
             }
-            *reinterpret_cast<float4 *>(out + r * n) = make_float4(o[0], o[1], o[2], o[3]);
-        };
-        // a row's loads for the next plane go out as soon as this plane's are used
-        const bool more = j + 1 < len;
-        const V4 DY = sub(P1, P0), Y1 = lds(tab + 3 * 32);
-        if (pre) {
-            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(g + pre));
-            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(g + pre + n));
         }
-        const float *pS = pN;  // the plane above this one
-        {
-            const V4 F0 = sub(N0, P0), Z0 = lds(tab + 5 * 32), X0 = lds(tab);
-            finish(P0, lap_row(P0, sub(S, P0), 1.f, DY, B0, F0, X0, lds(tab + 2 * 32), Y1, C0, Z0, li), X0, G0, 0);
-            B0 = F0;
-            C0 = Z0;
-            P0 = N0;
+        if (MU) {
+            acc[2 * r] += pa;
+            acc[2 * r + 1] += pb;
         }
-        if (more) {
-            up();
-            S = ldp(pS + dS);
-            N0 = ldp(pN);
-            G0 = ldp(g + plane);
+        *reinterpret_cast<float4 *>(out + r * n) = make_float4(o[0], o[1], o[2], o[3]);
+    };
+    for (int j = 0; j < len; j += 6) {
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+            if (j + d >= len) break;
+            const V4 &P0 = X0[d % 3], &P1 = X1[d % 3], &N0 = X0[(d + 1) % 3], &N1 = X1[(d + 1) % 3];
+            const int h = d & 1;
+            const V4 DY = sub(P1, P0), Y1 = lds(tab + 3 * 32), CX0 = lds(tab);
+            if (pre) {
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(g + pre));
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(g + pre + n));
+            }
+            B0[h ^ 1] = sub(N0, P0);
+            C0[h ^ 1] = lds(tab + 5 * 32);
+            finish(P0, lap_row(P0, sub(S[h], P0), 1.f, DY, B0[h], B0[h ^ 1], CX0, lds(tab + 2 * 32), Y1, C0[h], C0[h ^ 1], li), CX0, G0[h], 0);
+            __syncwarp();
+            const V4 CX1 = lds(tab + 32);
+            B1[h ^ 1] = sub(N1, P1);
+            C1[h ^ 1] = lds(tab + 6 * 32);
+            finish(P1, lap_row(P1, DY, -1.f, sub(T[h], P1), B1[h], B1[h ^ 1], CX1, Y1, lds(tab + 4 * 32), C1[h], C1[h ^ 1], li), CX1, G1[h], 1);
+            __syncwarp();
+            if (j + d + 2 < len) {
+                load_st(h);
+                X0[d % 3] = ldp(pN);
+                X1[d % 3] = ldp(pN + n);
+                G0[h] = ldp(g + 2 * plane);
+                G1[h] = ldp(g + 2 * plane + n);
+            }
+            g += plane;
+            out += plane;
+            tab += kSlots * 32;
         }
-        __syncwarp();
-        {
-            const V4 F1 = sub(N1, P1), Z1 = lds(tab + 6 * 32), X1 = lds(tab + 32);
-            finish(P1, lap_row(P1, DY, -1.f, sub(T, P1), B1, F1, X1, Y1, lds(tab + 4 * 32), C1, Z1, li), X1, G1, 1);
-            B1 = F1;
-            C1 = Z1;
-            P1 = N1;
-        }
-        if (more) {
-            T = ldp(pS + dT);
-            N1 = ldp(pN + n);
-            G1 = ldp(g + plane + n);
-        }
-        __syncwarp();
-        g += plane;
-        out += plane;
-        tab += kSlots * 32;
     }
 }
 
@@ -156,9 +172,9 @@ struct Job {
     Lane lane;
 };
 
-__global__ void __launch_bounds__(kThreads, 1) k_adj_lanes(AdjArgs p) {
+__global__ void __launch_bounds__(kAdjThreads, 1) k_adj_lanes(AdjArgs p) {
     extern __shared__ __align__(16) float4 tab[];
-    __shared__ Job s_job[kMaxLanes];
+    __shared__ Job s_job[kAdjLanes];
     __shared__ int s_blk[kMaxBlocks], s_at[kMaxBlocks + 1];  // rows | zb << 8 | planes << 16; first unit's table
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = blockIdx.x;
     const int nb = rank < p.nblocks ? (p.nblocks - rank - 1) / p.T + 1 : 0;  // blocks rank, rank + T, ...
@@ -175,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_adj_lanes(AdjArgs p) {
     for (int i = 0; i < nb; ++i) {
         const int blk = s_blk[i], y0 = 2 * (blk & 255), z0 = kBlockZ * (blk >> 8 & 255);
         const unsigned mask = (unsigned)blk >> 16;
-        for (int q = warp; q < kBlockZ * kSlots; q += kThreads / 32) {
+        for (int q = warp; q < kBlockZ * kSlots; q += kAdjThreads / 32) {
             const int j = q / kSlots, c = q % kSlots;
             if (!(mask >> j & 1u)) continue;
             int y = y0 + (c < 2 ? c : (c < 5 ? c - 3 : c - 5));
@@ -284,8 +300,8 @@ int adj_lanes_segment(Handle &h, int S, int k0, int k1, const SampleRec *recs, S
     AdjArgs a;
     a.S = S;
     a.T = std::min(h.num_sms, h.blocks);
-    a.lanes = std::min(kMaxLanes, S);
-    a.warps = 4 * kWps / a.lanes;
+    a.lanes = std::min(kAdjLanes, S);
+    a.warps = kAdjWarps / a.lanes;
     a.k0 = k0;
     a.k1 = k1;
     a.nblocks = h.blocks;
@@ -309,7 +325,7 @@ int adj_lanes_segment(Handle &h, int S, int k0, int k1, const SampleRec *recs, S
     GBG_CUDA_TRY(cudaFuncSetAttribute(k_adj_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     GBG_CUDA_TRY(cudaMemsetAsync(h.lane_sync, 0, (size_t)(a.lanes + 1) * kSyncStride * sizeof(unsigned), h.stream));
     void *args[] = {&a};
-    GBG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_adj_lanes, dim3((unsigned)a.T), dim3(kThreads), args, smem, h.stream));
+    GBG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_adj_lanes, dim3((unsigned)a.T), dim3(kAdjThreads), args, smem, h.stream));
     h.launches++;
     return GBG_OK;
 }
