@@ -25,8 +25,8 @@ namespace gbg {
 namespace {
 
 constexpr int kLikThreads = 256;
-constexpr int kLikPerThread = 8;
-constexpr int kLikChunk = kLikThreads * kLikPerThread;
+constexpr int kLikRuns = 8;  // of kLikThreads entries: a chunk, and the CTAs that share it
+constexpr int kLikChunk = kLikThreads * kLikRuns;
 
 struct LikArgs {
     int n_pet, n_ti, chunks;
@@ -95,41 +95,56 @@ struct CoarseSource {
     __device__ __forceinline__ double ti(const LikArgs &a, int s, int i) const { return at(s, a.ti_idx[i]); }
 };
 
+// The terms are FP64 work (two exponentials and two logarithms an entry of the
+// T1/T2 list, 16 cycles per warp and SM for each operation), and a sample has
+// few entries: with a chunk to a CTA, six SMs of 152 took 112 us for a sample's
+// 10,000 entries. A cluster takes a chunk: a CTA forms the terms of every eighth
+// run of kLikThreads entries, and three of them add a sum each, an entry of
+// every run at a time in the order of the runs, then by warps: 19 us.
+__device__ __forceinline__ void cluster_meet() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 template <class Src>
-__global__ void __launch_bounds__(kLikThreads) k_lik_partial(LikArgs a, Src src) {
-    const int s = blockIdx.y;
-    const int chunk = blockIdx.x;
-    double sp = 0.0, s1 = 0.0, s2 = 0.0;
-    const int base = chunk * kLikChunk;
-    for (int k = 0; k < kLikPerThread; ++k) {
-        const int i = base + k * kLikThreads + threadIdx.x;
-        if (i < a.n_pet) {
-            const double u = src.pet(a, s, i);
-            const double pv = a.pet_val[i];
-            const double r = u - a.pet_scale * pv;
-            sp += r * r;
-        }
-        if (i < a.n_ti) {
-            const double u = src.ti(a, s, i);
-            s1 += log_bernoulli(u, a.t1_val[i], a.t1_uc, a.is2);
-            s2 += log_bernoulli(u, a.t2_val[i], a.t2_uc, a.is2);
+__global__ void __cluster_dims__(kLikRuns, 1, 1) __launch_bounds__(kLikThreads) k_lik_partial(LikArgs a, Src src) {
+    const int s = blockIdx.y, chunk = blockIdx.x / kLikRuns, rank = blockIdx.x % kLikRuns;
+    __shared__ double term[3][kLikThreads];
+    __shared__ double red[kLikThreads / 32];
+    const int i = chunk * kLikChunk + rank * kLikThreads + threadIdx.x;
+    double t[3] = {0.0, 0.0, 0.0};
+    if (i < a.n_pet) {
+        const double u = src.pet(a, s, i);
+        const double pv = a.pet_val[i];
+        const double r = u - a.pet_scale * pv;
+        t[0] = r * r;
+    }
+    if (i < a.n_ti) {
+        const double u = src.ti(a, s, i);
+        t[1] = log_bernoulli(u, a.t1_val[i], a.t1_uc, a.is2);
+        t[2] = log_bernoulli(u, a.t2_val[i], a.t2_uc, a.is2);
+    }
+    for (int k = 0; k < 3; ++k) term[k][threadIdx.x] = t[k];
+    cluster_meet();
+    double sum = 0.0;
+    if (rank < 3) {
+        const unsigned own = (unsigned)__cvta_generic_to_shared(&term[rank][threadIdx.x]);
+#pragma unroll
+        for (int k = 0; k < kLikRuns; ++k) {
+            unsigned at;
+            double v;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own), "r"(k));
+            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
+            sum += v;
         }
     }
-    sp = warp_sum(sp);
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    __shared__ double red[3][kLikThreads / 32];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        red[0][w] = sp;
-        red[1][w] = s1;
-        red[2][w] = s2;
-    }
+    cluster_meet();  // the terms have been read
+    if (rank >= 3) return;
+    sum = warp_sum(sum);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
     __syncthreads();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (int j = 0; j < kLikThreads / 32; ++j) t += red[threadIdx.x][j];
-        a.partials[((size_t)s * a.chunks + chunk) * 3 + threadIdx.x] = t;
+    if (threadIdx.x == 0) {
+        double total = 0.0;
+        for (int j = 0; j < kLikThreads / 32; ++j) total += red[j];
+        a.partials[((size_t)s * a.chunks + chunk) * 3 + rank] = total;
     }
 }
 
@@ -192,7 +207,7 @@ int run_lik(Handle &h, const Src &src, int S, gbg_lik_result *out_device) {
     a.is2 = 1. / h.obs.slope;
     a.stride = h.N;
     a.partials = h.lik_partials;
-    k_lik_partial<<<dim3(chunks, S), kLikThreads, 0, h.stream>>>(a, src);
+    k_lik_partial<<<dim3(chunks * kLikRuns, S), kLikThreads, 0, h.stream>>>(a, src);
     k_lik_final<<<(S + 127) / 128, 128, 0, h.stream>>>(h.lik_partials, chunks, S, h.obs.n_pet,
                                                        h.obs.pet_sigma2, out_device);
     h.launches += 2;
@@ -431,7 +446,7 @@ extern "C" int gbg_loglik_noalloc(const float *phi_device, int n, const int *pet
     a.partials = scratch;
     PhiSource src{phi_device, phi_device, nullptr, nullptr};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    k_lik_partial<<<dim3(chunks, 1), kLikThreads, 0, st>>>(a, src);
+    k_lik_partial<<<dim3(chunks * kLikRuns, 1), kLikThreads, 0, st>>>(a, src);
     k_lik_final<<<1, 128, 0, st>>>(scratch, chunks, 1, (int)n_pet, p->pet_sigma2, out_device);
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;

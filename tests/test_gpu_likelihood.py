@@ -70,3 +70,29 @@ def test_loglik_edge_cases(gbg, oracle_lib):
     assert r["n_pet"] == 0 and r["l_pet"] == 0.0
     for k in ("l_t1", "l_t2", "total"):
         assert abs(r[k] - o[k]) <= REL_TOL * max(1.0, abs(o[k]))
+
+
+@pytest.mark.parametrize("n_pet,n_ti", [(1, 1), (255, 257), (256, 2049), (2047, 256), (2049, 2048), (6000, 1)])
+def test_loglik_at_the_edges_of_the_clusters(gbg, oracle_lib, n_pet, n_ti):
+    """Lists that end inside, at and behind a run of 256 entries and a chunk of
+    eight runs, one longer than the other (the double sums' order differs from
+    the oracle's: REL_TOL)."""
+    n = 32
+    rng = np.random.default_rng(n_pet)
+    model = rng.random((n, n, n))
+    pet = np.zeros(n ** 3)
+    pet[rng.choice(n ** 3, n_pet, replace=False)] = rng.uniform(0.1, 1.0, n_pet)
+    pet = pet.reshape(n, n, n)
+    t1, t2 = ((rng.random((n, n, n)) > 0.5).astype(float) for _ in range(2))
+    c = rng.choice(n ** 3, n_ti, replace=False)
+    pts = np.stack([c % n, c // n % n, c // n ** 2], axis=1).astype(float)
+    params = (0.0025, 1.0, 0.7, 0.25, 0.09)
+    with _lib.Handle(n, "f64") as h:
+        h.set_phi(model)
+        h.set_observations(pet, t1, t2, pts, params, step_pet=1, step_ti=1, selective=True)
+        assert h.observation_counts() == (n_pet, n_ti)
+        r = h.loglik()
+    o = oracle_lib.loglik(model, pet, t1, t2, pts, params, step_pet=1, step_ti=1, selective=True)
+    assert r["n_pet"] == o["n_pet"] == n_pet
+    for k in ("l_pet", "l_t1", "l_t2", "total"):
+        assert abs(r[k] - o[k]) <= REL_TOL * max(1.0, abs(o[k])), (k, r[k], o[k])
