@@ -1342,7 +1342,9 @@ int gbg_autotune(gbg_handle *hh, int probe_samples, const char *cache_path, int 
     int bucket = 1;
     while (bucket < h.max_samples) bucket <<= 1;
     char key[512];
-    std::snprintf(key, sizeof(key), "%s|n=%d|S<=%d|f32", prop.name, h.n, bucket);
+    // "resident": a file written for the list of variants before the resident
+    // kernel headed it has indices of that list, and is measured again
+    std::snprintf(key, sizeof(key), "%s|n=%d|S<=%d|f32|resident", prop.name, h.n, bucket);
     std::map<std::string, int> cache;
     const int nv = gbg::population_variant_count(h.n);
     if (cache_path) {
