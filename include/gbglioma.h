@@ -490,8 +490,8 @@ int gbg_amr_run(gbg_handle *h, const gbg_amr_run_opts *opts, long *steps, int *r
 /* No reference counterpart. Statistics of the handle's latest gbg_amr_run:
  * cell-steps computed (blocks x 4096 summed over the steps), the wall time
  * of the steps and of the regrids (each regrid waits for the steps before
- * it, then FWT on the device, plans and ghost tables on the host, data
- * movement on the device), the number of regrid calls, and the fewest and
+ * it, then FWT, ghost tables and data movement on the device, plans on the
+ * host), the number of regrid calls, and the fewest and
  * most blocks the grid had. */
 typedef struct {
     long long cell_steps;
@@ -540,8 +540,8 @@ int gbg_sync(gbg_handle *h);
  * stream; waits for it to finish. */
 int gbg_last_population_ms(gbg_handle *h, float *ms);
 /* No reference counterpart. Cell-steps the most recent population-kernel
- * launch computed: the tiles it visited times the cells of a tile. The
- * skipping kernel (the batched solver's default) visits only the tiles whose
+ * launch computed: the tiles (in the default kernel units of a few rows) it
+ * visited times their cells. The skipping kernels visit only those whose
  * output can be nonzero, so this is at most the population's step count times
  * n^3; the dense register kernel visits every tile of every active sample.
  * Waits for the launch to finish; GBG_ERR_UNSUPPORTED for the other kernel
