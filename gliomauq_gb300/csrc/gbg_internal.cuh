@@ -185,6 +185,7 @@ struct Handle {
     int units[3] = {0, 0, 0};
     int *block_list = nullptr;
     int blocks = 0;
+    int lane_clusters = -1;  // clusters of the cluster teams' size that run side by side (not asked yet: -1)
     unsigned *lane_sync = nullptr;
 
     // events bracketing the latest population-kernel launch

@@ -91,5 +91,47 @@ __device__ __forceinline__ void lane_barrier(Lane &ln, unsigned *sync, unsigned 
     }
 }
 
+// lane_barrier where the team is a cluster: a CTA arrives at the shared-memory
+// barrier `bar` of every CTA and waits at its own (target counts its phases). A
+// CTA may arrive for phase j + 1 where another's arrival for phase j is still on
+// its way, but no phase ends early: when the first wait for phase j ends anywhere,
+// its barrier has (j + 1) T arrivals, of which none came from a CTA more than j +
+// 1 times, so every CTA has released its step j; the fence before the arrivals
+// carries that on.
+__device__ __forceinline__ void cluster_barrier(Lane &ln, unsigned long long *bar, unsigned *sync, unsigned *queue, int T, int rank,
+                                                int lanes, bool last, int *status) {
+    if (last && rank == 0) *(volatile unsigned *)(sync + 1 + ln.slot) = atomicAdd(queue, 1u) + (unsigned)lanes;
+    const unsigned own = (unsigned)__cvta_generic_to_shared(bar), parity = ln.target & 1u;
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    for (int r = 0; r < T; ++r) {
+        unsigned at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own), "r"(r));
+        asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(at) : "memory");
+    }
+    unsigned done = 0;
+    for (long long spins = 0; !done;) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(own), "r"(parity)
+            : "memory");
+        if (done) break;
+        if (++spins > (1ll << 24)) {
+            atomicExch(status, (int)DEV_BARRIER_TIMEOUT);
+            ln.ok = 0;
+            break;
+        }
+        if ((spins & 1023) == 0 && *(volatile int *)status != DEV_OK) {
+            ln.ok = 0;
+            break;
+        }
+    }
+    ++ln.target;
+    if (last) {
+        ln.next = (int)*(volatile unsigned *)(sync + 1 + ln.slot);
+        ln.slot ^= 1u;
+    }
+}
+
 }  // namespace lanes
 }  // namespace gbg

@@ -1514,7 +1514,7 @@ int fast_steps_single(Handle &h, double Dw, double rho, double dt, long nsteps) 
     float *const buf0 = (float *)h.phi[h.cur], *const buf1 = (float *)h.phi[h.cur ^ 1];
     // The default variant takes any state as a sample of its own that reaches
     // over the whole grid, with zeros in the second buffer where no live unit
-    // writes: 2.1 us a step at 32^3 and 64^3 and 3.5 at 128^3, where the dense
+    // writes: 1.7 us a step at 32^3, 2.1 at 64^3 and 3.5 at 128^3, where the dense
     // kernel takes 5.7, 8.6 and 8.8; the zeros and the unit tables cost 5 us
     // first. Its barrier counts arrivals in 32 bits.
     PopVariant vs[32];

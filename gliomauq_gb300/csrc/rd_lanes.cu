@@ -37,8 +37,15 @@ namespace gbg {
 namespace {
 using namespace lanes;
 
+// At 32^3 a step is little but its barrier. While there are clusters of 16 SMs for
+// all samples, a team is one and its barrier goes through shared memory: 0.33
+// instead of 0.39 ms for 6 samples near the mode. Beyond that (7 on a GB300) waiting
+// for a cluster costs more (16 samples 0.61 against 0.45), and clusters of 8 or 4
+// gain nothing (0.38 and 0.43 for 6).
+constexpr int kClusterTeam = 16;
+
 struct LaneArgs {
-    int S, T, teams, lanes, warps;
+    int S, T, teams, lanes, warps, cluster;
     int nlive, units, grow0;
     size_t stride, slot;  // slot: floats between kept states (kernels with KEEP)
     float *buf0, *buf1;
@@ -161,12 +168,13 @@ __device__ __forceinline__ void march(const float4 *__restrict__ tab, int y, int
 // KEEP: every state is kept (step k reads buf0 + k * slot, writes buf0 + (k + 1)
 // * slot) over arbitrary older contents, so the live units outside the grown
 // support and the units of the fill list are written with zeros.
-template <int LR, int WPS, bool KEEP>
+template <int LR, int WPS, bool KEEP, bool CLUSTER>
 __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
     constexpr int n = 4 * LR, SUB = 32 / LR, ROWS = 2 * SUB;
     extern __shared__ __align__(16) float4 tab[];
     __shared__ int s_unit[kMaxUnits];  // y0 | z << 10 | length of the run of planes from here on << 20
     __shared__ Sample s_smp[kMaxLanes];
+    __shared__ unsigned long long s_bar[kMaxLanes];  // CLUSTER: the lanes' barriers
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, li = lane % LR, sub_r = lane / LR;
     const int team = blockIdx.x / p.T, rank = blockIdx.x % p.T;
     // this CTA's units: two stretches of the list, half the list apart
@@ -188,87 +196,104 @@ __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
         const float *src = c < 2 ? p.cxs : (c < 5 ? p.cy : p.cz);
         tab[q * 32 + lane] = *reinterpret_cast<const float4 *>(src + 4 * li + (size_t)n * (y + (size_t)n * z));
     }
+    if (CLUSTER) {
+        if (threadIdx.x < kMaxLanes)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(s_bar + threadIdx.x)), "r"(p.T)
+                         : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     __syncthreads();
     const int g = warp / p.warps, w = warp % p.warps;
-    if (g >= p.lanes) return;  // named barriers only from here on
-    Sample &sm = s_smp[g];
-    const int tl = g * p.teams + team;
-    if (w == 0 && lane == 0) {
-        sm.lane = Lane{tl, 1, 0u, 0u};
-    }
-    unsigned visited = 0;
-    for (;;) {
-        group_sync(1 + g, 32 * p.warps);
-        const int r = sm.lane.next;
-        if (r >= p.S || !sm.lane.ok) break;
+    // named barriers only from here on, and the cluster's at the end
+    if (g < p.lanes) {
+        Sample &sm = s_smp[g];
+        const int tl = g * p.teams + team;
         if (w == 0 && lane == 0) {
-            sm.rec = p.rec[r];
-            const int4 bx = reinterpret_cast<const int4 *>(p.box)[sm.rec.order];
-            sm.ylo = n - bx.x;
-            sm.yhi = bx.y - 1;
-            sm.zlo = n - bx.z;
-            sm.zhi = bx.w - 1;
-            if (bx.y == 0) sm.rec.a = -1.f;  // no nonzero initial cell: the sample stays 0
+            sm.lane = Lane{tl, 1, 0u, 0u};
         }
-        group_sync(1 + g, 32 * p.warps);
-        const int nsteps = sm.rec.nsteps;
-        if (nsteps <= 0) break;  // sorted: so are all that follow
-        for (int k = 0; k < nsteps; ++k) {
-            {
-                const size_t off = (size_t)sm.rec.order * p.stride;
-                const float *in = (KEEP ? p.buf0 + (size_t)k * p.slot : ((k & 1) ? p.buf1 : p.buf0)) + off;
-                float *out = (KEEP ? p.buf0 + (size_t)(k + 1) * p.slot : ((k & 1) ? p.buf0 : p.buf1)) + off;
-                auto zero = [&](int y0, int z) {  // unit (row group y0, plane z) of the output
-                    float *o = out + 4 * li + (size_t)n * (y0 + 2 * sub_r + (size_t)n * z);
-                    *reinterpret_cast<float4 *>(o) = make_float4(0.f, 0.f, 0.f, 0.f);
-                    *reinterpret_cast<float4 *>(o + n) = make_float4(0.f, 0.f, 0.f, 0.f);
-                };
-                const bool lastk = k == nsteps - 1;
-                const float a = lastk ? sm.rec.a2 : sm.rec.a, b = lastk ? sm.rec.b2 : sm.rec.b;
-                const bool any = sm.rec.a >= 0.f;
-                const int grow = p.grow0 + k + 1, u1 = nu * (w + 1) / p.warps;
-                for (int i = nu * w / p.warps; (KEEP || any) && i < u1;) {
-                    const int un = s_unit[i], y0 = un & 1023, z = un >> 10 & 1023, len = min(un >> 20, u1 - i);
-                    int za = z, zb = z + len;
-                    if (sm.zlo >= grow && sm.zhi + grow < n) {
-                        za = max(za, sm.zlo - grow);
-                        zb = min(zb, sm.zhi + grow + 1);
-                    }
-                    if (!any || !span_hits(sm.ylo, sm.yhi, grow, y0, y0 + ROWS - 1, n)) zb = za;
-                    if (za < zb) {
-                        march<LR>(tab + (i + za - z) * kSlots * 32 + lane, y0 + 2 * sub_r, za, zb - za, in, out, p.cz, a, b);
-                        visited += zb - za;
-                    }
-                    if (KEEP)
-                        for (int q = z; q < z + len; ++q)
-                            if (q < za || q >= zb) zero(y0, q);
-                    i += len;
-                }
-                if (KEEP) {
-                    for (int i = rank + p.T * w; i < p.nfill; i += p.T * p.warps) zero(p.fill[i] / n * ROWS, p.fill[i] % n);
-                } else if (k == 1 && any) {
-                    // units without a live cell that the initial state may have
-                    // left values in: zeros, as their step gives
-                    for (int u = rank + p.T * w; u < p.units; u += p.T * p.warps) {
-                        const int y0 = (u / n) * ROWS, z = u % n;
-                        if (p.live[u] != 1 && span_hits(sm.ylo, sm.yhi, p.grow0, y0, y0 + ROWS - 1, n) &&
-                            span_hits(sm.zlo, sm.zhi, p.grow0, z, z, n))
-                            zero(y0, z);
-                    }
-                }
-            }
-            // barrier of the team's CTAs on this lane
+        unsigned visited = 0;
+        for (;;) {
             group_sync(1 + g, 32 * p.warps);
+            const int r = sm.lane.next;
+            if (r >= p.S || !sm.lane.ok) break;
             if (w == 0 && lane == 0) {
-                lane_barrier(sm.lane, p.sync + (size_t)(tl + 1) * kSyncStride, p.sync, p.T, rank, p.teams * p.lanes, k == nsteps - 1,
-                             p.status);
+                sm.rec = p.rec[r];
+                const int4 bx = reinterpret_cast<const int4 *>(p.box)[sm.rec.order];
+                sm.ylo = n - bx.x;
+                sm.yhi = bx.y - 1;
+                sm.zlo = n - bx.z;
+                sm.zhi = bx.w - 1;
+                if (bx.y == 0) sm.rec.a = -1.f;  // no nonzero initial cell: the sample stays 0
             }
-            if (k == nsteps - 1) break;
             group_sync(1 + g, 32 * p.warps);
-            if (!sm.lane.ok) break;
+            const int nsteps = sm.rec.nsteps;
+            if (nsteps <= 0) break;  // sorted: so are all that follow
+            for (int k = 0; k < nsteps; ++k) {
+                {
+                    const size_t off = (size_t)sm.rec.order * p.stride;
+                    const float *in = (KEEP ? p.buf0 + (size_t)k * p.slot : ((k & 1) ? p.buf1 : p.buf0)) + off;
+                    float *out = (KEEP ? p.buf0 + (size_t)(k + 1) * p.slot : ((k & 1) ? p.buf0 : p.buf1)) + off;
+                    auto zero = [&](int y0, int z) {  // unit (row group y0, plane z) of the output
+                        float *o = out + 4 * li + (size_t)n * (y0 + 2 * sub_r + (size_t)n * z);
+                        *reinterpret_cast<float4 *>(o) = make_float4(0.f, 0.f, 0.f, 0.f);
+                        *reinterpret_cast<float4 *>(o + n) = make_float4(0.f, 0.f, 0.f, 0.f);
+                    };
+                    const bool lastk = k == nsteps - 1;
+                    const float a = lastk ? sm.rec.a2 : sm.rec.a, b = lastk ? sm.rec.b2 : sm.rec.b;
+                    const bool any = sm.rec.a >= 0.f;
+                    const int grow = p.grow0 + k + 1, u1 = nu * (w + 1) / p.warps;
+                    for (int i = nu * w / p.warps; (KEEP || any) && i < u1;) {
+                        const int un = s_unit[i], y0 = un & 1023, z = un >> 10 & 1023, len = min(un >> 20, u1 - i);
+                        int za = z, zb = z + len;
+                        if (sm.zlo >= grow && sm.zhi + grow < n) {
+                            za = max(za, sm.zlo - grow);
+                            zb = min(zb, sm.zhi + grow + 1);
+                        }
+                        if (!any || !span_hits(sm.ylo, sm.yhi, grow, y0, y0 + ROWS - 1, n)) zb = za;
+                        if (za < zb) {
+                            march<LR>(tab + (i + za - z) * kSlots * 32 + lane, y0 + 2 * sub_r, za, zb - za, in, out, p.cz, a, b);
+                            visited += zb - za;
+                        }
+                        if (KEEP)
+                            for (int q = z; q < z + len; ++q)
+                                if (q < za || q >= zb) zero(y0, q);
+                        i += len;
+                    }
+                    if (KEEP) {
+                        for (int i = rank + p.T * w; i < p.nfill; i += p.T * p.warps) zero(p.fill[i] / n * ROWS, p.fill[i] % n);
+                    } else if (k == 1 && any) {
+                        // units without a live cell that the initial state may have
+                        // left values in: zeros, as their step gives
+                        for (int u = rank + p.T * w; u < p.units; u += p.T * p.warps) {
+                            const int y0 = (u / n) * ROWS, z = u % n;
+                            if (p.live[u] != 1 && span_hits(sm.ylo, sm.yhi, p.grow0, y0, y0 + ROWS - 1, n) &&
+                                span_hits(sm.zlo, sm.zhi, p.grow0, z, z, n))
+                                zero(y0, z);
+                        }
+                    }
+                }
+                // barrier of the team's CTAs on this lane
+                group_sync(1 + g, 32 * p.warps);
+                if (w == 0 && lane == 0) {
+                    unsigned *sync = p.sync + (size_t)(tl + 1) * kSyncStride;
+                    if (CLUSTER)
+                        cluster_barrier(sm.lane, s_bar + g, sync, p.sync, p.T, rank, p.teams * p.lanes, k == nsteps - 1, p.status);
+                    else
+                        lane_barrier(sm.lane, sync, p.sync, p.T, rank, p.teams * p.lanes, k == nsteps - 1, p.status);
+                }
+                if (k == nsteps - 1) break;
+                group_sync(1 + g, 32 * p.warps);
+                if (!sm.lane.ok) break;
+            }
         }
+        if (lane == 0 && visited) atomicAdd(p.visited, (unsigned long long)visited);
     }
-    if (lane == 0 && visited) atomicAdd(p.visited, (unsigned long long)visited);
+    if (CLUSTER) {  // no CTA leaves while others may arrive at its barriers
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
 }
 
 // live[u] = unit u (2 rows per lane segment, one plane, full x-rows; u = row
@@ -339,6 +364,27 @@ int lanes_set_anatomy(Handle &h) {
         GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_list, 3 * (nu + 1) * sizeof(int)));
         GBG_CUDA_TRY(cudaMalloc((void **)&h.lane_sync, (size_t)(h.num_sms * kMaxLanes + 1) * kSyncStride * sizeof(unsigned)));
     }
+    if (h.n == 32 && h.lane_clusters < 0) {
+        // how many clusters run side by side, at the most units a CTA of one owns
+        const void *fn = (const void *)k_population10<8, kWps, false, true>;
+        cudaLaunchConfig_t c = {};
+        cudaLaunchAttribute at[1];
+        c.gridDim = dim3(kClusterTeam);
+        c.blockDim = dim3(kThreads);
+        c.dynamicSmemBytes = 2 * ((nu + 2 * kClusterTeam - 1) / (2 * kClusterTeam)) * kUnitBytes;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kClusterTeam;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        c.attrs = at;
+        c.numAttrs = 1;
+        h.lane_clusters = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.dynamicSmemBytes) != cudaSuccess ||
+            cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&h.lane_clusters, fn, &c) != cudaSuccess) {
+            cudaGetLastError();
+            h.lane_clusters = 0;
+        }
+    }
     k_unit_live<<<nu, 128, 0, h.stream>>>(h.n, unit_rows(h.n), h.pw, h.pg, h.unit_live);
     k_unit_rim<<<(nu + 127) / 128, 128, 0, h.stream>>>(h.n, nu, h.unit_live);
     // live units | units without a live cell that a live unit's stencil reads |
@@ -369,6 +415,11 @@ static void lane_shape(const Handle &h, int S, LaneArgs &a, int &units) {
     a.T = std::min(sms, std::max(least, std::min(wide, most)));
     a.teams = sms / a.T;
     a.T = sms / a.teams;
+    a.cluster = h.n == 32 && S <= h.lane_clusters;
+    if (a.cluster) {
+        a.T = kClusterTeam;
+        a.teams = S;
+    }
     a.teams = std::min(a.teams, S);
     a.lanes = std::min(kMaxLanes, (S + a.teams - 1) / a.teams);
     units = 2 * ((nl + 2 * a.T - 1) / (2 * a.T));
@@ -413,9 +464,10 @@ int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, i
     const size_t smem = units * kUnitBytes;
     auto kernel = [&](auto keep) {
         constexpr bool K = decltype(keep)::value;
-        return n == 128  ? (const void *)k_population10<32, kWps, K>
-               : n == 64 ? (const void *)k_population10<16, kWps, K>
-                         : (const void *)k_population10<8, kWps, K>;
+        return n == 128    ? (const void *)k_population10<32, kWps, K, false>
+               : n == 64   ? (const void *)k_population10<16, kWps, K, false>
+               : a.cluster ? (const void *)k_population10<8, kWps, K, true>
+                           : (const void *)k_population10<8, kWps, K, false>;
     };
     const void *fn = slot ? kernel(std::true_type{}) : kernel(std::false_type{});
     GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -428,7 +480,23 @@ int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, i
     GBG_CUDA_TRY(cudaStreamIsCapturing(h.stream, &cap));
     const unsigned evf = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     GBG_CUDA_TRY(cudaEventRecordWithFlags(h.ev_pop[0], h.stream, evf));
-    GBG_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3((unsigned)(a.teams * a.T)), dim3(kThreads), args, smem, h.stream));
+    if (a.cluster) {
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3((unsigned)(a.teams * a.T));
+        c.blockDim = dim3(kThreads);
+        c.dynamicSmemBytes = smem;
+        c.stream = h.stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = a.T;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        c.attrs = at;
+        c.numAttrs = 1;
+        GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        GBG_CUDA_TRY(cudaLaunchKernelExC(&c, fn, args));
+    } else {
+        GBG_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3((unsigned)(a.teams * a.T)), dim3(kThreads), args, smem, h.stream));
+    }
     GBG_CUDA_TRY(cudaEventRecordWithFlags(h.ev_pop[1], h.stream, evf));
     h.ev_pop_recorded = true;
     h.launches++;

@@ -72,3 +72,21 @@ def test_single_solve_equals_the_dense_kernel(gbg, n, steps):
             outs.append(h.get_phi())
     assert np.array_equal(outs[0], outs[1])
     assert outs[0].max() > 0
+
+
+@pytest.mark.parametrize("kind", ["ellipsoid", "full", "scattered"])
+def test_few_samples_at_32_equal_the_same_samples_among_others(gbg, kind):
+    """A few samples at 32^3 run on a cluster of CTAs each; the bits are those of
+    the same samples in a larger call, for one sample up to more than there are
+    clusters for."""
+    rng = np.random.default_rng(8)
+    pw, pg = _tissue(kind, 32, rng)
+    dt = S.reference_dt(32, 0.0013, 3.2)[0]
+    smp = [(0.0013 * rng.uniform(0.3, 1.5), rng.uniform(0.01, 0.2), *rng.uniform(8, 24, 3), dt * rng.uniform(0, 40))
+           for _ in range(24)]
+    with _lib.Handle(32, "f32", max_samples=24) as h:
+        h.set_anatomy(pw, pg)
+        whole = h.batch_solve(smp, 3.2, with_loglik=False, want_phi=True)["phi"]
+        for a, b in ((0, 1), (1, 3), (3, 9), (9, 16), (16, 24)):
+            part = h.batch_solve(smp[a:b], 3.2, with_loglik=False, want_phi=True)["phi"]
+            assert np.array_equal(part, whole[a:b])
