@@ -116,12 +116,12 @@ __device__ __forceinline__ void cluster_barrier(Lane &ln, unsigned long long *ba
             : "r"(own), "r"(parity)
             : "memory");
         if (done) break;
-        if (++spins > (1ll << 24)) {
+        if (++spins > (1ll << 27)) {  // a test is shorter than a load from L2: seconds too
             atomicExch(status, (int)DEV_BARRIER_TIMEOUT);
             ln.ok = 0;
             break;
         }
-        if ((spins & 1023) == 0 && *(volatile int *)status != DEV_OK) {
+        if ((spins & 16383) == 0 && *(volatile int *)status != DEV_OK) {
             ln.ok = 0;
             break;
         }
