@@ -230,7 +230,7 @@ __device__ __forceinline__ float gaussian_ic_value(int x, int y, int z, double x
 // over samples, x over the cells of the box around the seed outside which the
 // screen above gives 0 (the whole grid where it does not apply). Looking at
 // every cell of every field instead took 1.0 ms for 64 samples of 128^3 and 53
-// us for one; beside the fill with zeros, this kernel takes 0.16 ms and 19 us.
+// us for one; beside the fill with zeros, this kernel takes 0.16 ms and 9 us.
 // 32-bit index arithmetic inside a sample (n <= 1024, n^3 < 2^32).
 // box non-null (the skipping population kernels): the y and z extent of the
 // cells given a nonzero value is recorded per sample as four ints
@@ -286,7 +286,9 @@ __global__ void __launch_bounds__(256) k_gaussian_ic(int n, const gbg_sample *__
 
 dim3 ic_grid(const Handle &h, int S) {
     const unsigned per = (unsigned)((h.N + 255) / 256);
-    const unsigned gx = per < 32 ? per : 32;
+    // a box of 35^3 cells on 32 CTAs takes 19 us for one sample, on two per SM
+    // 9 us; 32 do where the samples fill the chip
+    const unsigned gx = std::min(per, std::max(32u, 2u * (unsigned)h.num_sms / (unsigned)S));
     return dim3(gx, (unsigned)(S < 65535 ? S : 65535));
 }
 
