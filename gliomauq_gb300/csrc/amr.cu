@@ -867,12 +867,12 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
         h.amr.tab_Dw = Dw;
         h.amr.tab_Dg = Dg;
         h.amr.tables_valid = true;
-        h.amr.full_steps = 0;
+        h.amr.full_steps = kAnyState;
         h.amr.listed = false;
     }
     auto step = [&](auto real, const void *in, void *out) {
         using Real = decltype(real);
-        if (h.amr.full_steps >= 2 && h.amr.list) {
+        if (h.amr.full_steps == kListed && h.amr.list) {
             const Real *b0 = (const Real *)h.amr.b0;
             if (!h.amr.listed) {
                 k_amr_collect<Real, false><<<chunks, 256, 0, h.stream>>>(cells, b0, h.amr.df, offset, nullptr, nullptr);
@@ -892,13 +892,13 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
         k_amr_step<Real><<<gc, 256, 0, h.stream>>>(h.amr.nb, rt, h.amr.level, (const Real *)in, (const Real *)h.amr.gphi,
                                                    (const Real *)h.amr.b0, h.amr.df, (Real *)out, (Real)rho, dt);
         h.launches += 2;
-        ++h.amr.full_steps;
+        h.amr.full_steps = after_full_step(h.amr.full_steps, rho, dt);
     };
     for (long s = 0; s < nsteps; ++s) {
         void *in = h.amr.phi[h.amr.cur], *out = h.amr.phi[h.amr.cur ^ 1];
-        if (h.amr.full_steps == 1 && h.amr.list) {  // the other buffer's dead cells
+        if (h.amr.full_steps == kDeadZero && h.amr.list) {  // the other buffer's dead cells
             GBG_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)cells * (f64 ? sizeof(double) : sizeof(float)), h.stream));
-            h.amr.full_steps = 2;
+            h.amr.full_steps = kListed;
         }
         if (f64)
             step(double{}, in, out);

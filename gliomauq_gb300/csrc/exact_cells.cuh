@@ -18,6 +18,20 @@ __device__ __forceinline__ int cell_class(double b0, const double (&d)[6]) {
     return nan && b0 >= 0.0 ? kDead : (pos ? kPlain : kSpecial);
 }
 
+// What is known of a density before a step (Handle::exact_full):
+//   kAnyState  nothing: set by the caller, or of other tables
+//   kInRange   a step over every cell gave it: it is in [0, 1]
+//   kDeadZero  and its dead cells are 0
+//   kListed    and the other buffer is 0 where no listed cell is
+enum { kAnyState = 0, kInRange = 1, kDeadZero = 2, kListed = 3 };
+// The state after a step over every cell. From a density in [0, 1] the step
+// leaves dead cells 0. From any finite one it does so too, but for p < 0 where
+// cell and density together are no tissue: the faces count as 0 and p + dt rho p
+// (1 - p) may be positive, if rho and dt are of unlike sign.
+inline int after_full_step(int state, double rho, double dt) {
+    return state == kAnyState && (rho < 0.0) != (dt < 0.0) ? kInRange : kDeadZero;
+}
+
 // counts -> exclusive offsets, the total behind them (one CTA)
 __global__ void __launch_bounds__(1024) k_exact_offsets(int chunks, int *__restrict__ offset) {
     __shared__ int sums[32];

@@ -118,9 +118,8 @@ struct Handle {
     // the cells an exact step has to compute (rd_exact.cu): their list, its
     // chunk offsets and its length behind it (null: no memory for it at creation,
     // every step computes every cell); the plain cells' sums of faces; whether
-    // the list is that of the present tables; 0: the density or the tables were
-    // set since the last step, 1: a step over every cell was taken, 2: both
-    // buffers have zeros where no listed cell is
+    // the list is that of the present tables; exact_full: what is known of the
+    // density (exact_cells.cuh; 0: nothing, as after gbg_set_phi)
     int *exact_list = nullptr;
     double *exact_dsum = nullptr;
     bool exact_listed = false;

@@ -108,9 +108,10 @@ __global__ void k_exact_step(int n, const Real *__restrict__ phi, Real *__restri
 //   plain    b0 > 0 and all six faces positive: no doubling, and the sum of the
 //            faces is a constant of the tables
 //   special  anything else: the step as it is written
-// (densities are finite and in [0, 1] from the first step on). k_exact_list
-// runs over the list of plain and special cells; a step over every cell leaves
-// the dead ones' zeros in one buffer, and the other is filled with zeros. Measured on 64^3 (32 % plain),
+// (densities are finite and in [0, 1] from the first step on; a first step may
+// leave dead cells a positive value, after_full_step). k_exact_list runs over
+// the list of plain and special cells; a step over every cell leaves the dead
+// ones' zeros in one buffer, and the other is filled with zeros. Measured on 64^3 (32 % plain),
 // 237 steps with upload and download: 7.0 ms on every cell, 2.3 ms on the list
 // with a launch per step, 1.6 in one launch (k_exact_resident).
 struct Cell {
@@ -423,7 +424,7 @@ int exact_build_tables(Handle &h, double Dw, double Dg) {
     h.tab_Dw = Dw;
     h.tab_Dg = Dg;
     h.tables_valid = true;
-    h.exact_full = 0;
+    h.exact_full = kAnyState;
     h.exact_listed = false;
     return GBG_OK;
 }
@@ -495,21 +496,21 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
     };
     auto step = [&](auto real, const void *in, void *out) {
         using Real = decltype(real);
-        if (h.exact_full >= 2 && h.exact_list) {
+        if (h.exact_full == kListed && h.exact_list) {
             k_exact_list<Real><<<gl, 64, 0, h.stream>>>(h.n, h.exact_list + h.N + chunks, h.exact_list, h.exact_dsum, (const Real *)in,
                                                         (Real *)out, (const Real *)h.b0, h.dfx, h.dfy, h.dfz, (Real)rho, dt, ih2);
         } else {
             k_exact_step<Real><<<g, 256, 0, h.stream>>>(h.n, (const Real *)in, (Real *)out, (const Real *)h.b0, h.dfx, h.dfy, h.dfz,
                                                         (Real)rho, dt, ih2);
-            ++h.exact_full;
+            h.exact_full = after_full_step(h.exact_full, rho, dt);
         }
     };
     for (long s = 0; s < nsteps; ++s) {
-        if (h.exact_full == 1 && h.exact_list) {  // the other buffer's dead cells
+        if (h.exact_full == kDeadZero && h.exact_list) {  // the other buffer's dead cells
             GBG_CUDA_TRY(cudaMemsetAsync(h.phi[h.cur ^ 1], 0, h.N * (h.prec == GBG_PREC_F64 ? sizeof(double) : sizeof(float)), h.stream));
-            h.exact_full = 2;
+            h.exact_full = kListed;
         }
-        if (h.exact_full >= 2 && h.exact_list) {
+        if (h.exact_full == kListed && h.exact_list) {
             if (!h.exact_listed) h.prec == GBG_PREC_F64 ? collect(double{}) : collect(float{});
             if (nsteps - s >= kResidentSteps && nsteps - s < 0x7fffffffL / h.num_sms) {  // arrivals are counted in 32 bits
                 const int rc = h.prec == GBG_PREC_F64 ? resident_steps<double>(h, rho, dt, ih2, nsteps - s)

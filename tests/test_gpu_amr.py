@@ -257,3 +257,26 @@ def test_fast_f32_fused_step_equals_separate_ghost_pass(gbg, source):
             outs.append(h.get_phi())
     assert np.array_equal(outs[0], outs[1])
     assert np.abs(outs[0]).max() > 0
+
+
+@pytest.mark.parametrize("variant", ["f64", "f32"])
+@pytest.mark.parametrize("rho,dt", [(-1.0, 0.5), (1.0, -0.5), (-1.0, -0.5)])
+def test_amr_steps_from_densities_below_zero_match_oracle(gbg, variant, rho, dt):
+    """As on the uniform grid: a first step whose reaction turns densities below
+    0 positive (rho and dt of unlike sign) in cells without tissue."""
+    d = golden_npz(f"amr64_{variant}.npz")
+    real = REAL[variant]
+    rng = np.random.default_rng(13)
+    phi = rng.uniform(-3.0, 1.0, size=d["phi"].shape).astype(real).astype(np.float64)
+    tabs = (d["ghost_start"], d["ghost_src_block"], d["ghost_src_cell"].astype(np.int32), d["ghost_w"].astype(np.float64))
+    ref = phi.reshape(-1, 4096)
+    Dw, Dg = (float(real(v)) for v in (2e-4, 2e-5))
+    with _lib.AmrHandle(64, PREC[variant]) as h:
+        h.set_grid(d["blocks"], d["p_w"], d["p_g"], phi)
+        h.set_ghosts(*tabs)
+        for n in (1, 1, 2, 3):
+            h.step(Dw, Dg, rho, dt, n)
+            for _ in range(n):
+                ref = A.step(d["blocks"][:, 0], d["p_w"].reshape(-1, 4096), d["p_g"].reshape(-1, 4096), ref,
+                             tabs, Dw, Dg, rho, dt, real).reshape(-1, 4096)
+            assert np.array_equal(h.get_phi().reshape(-1, 4096), ref.astype(np.float64)), n

@@ -181,3 +181,33 @@ def test_exact_steps_in_one_call_equal_single_steps(gbg, precision, n, dense):
     assert outs[0].max() > 0
     for o in outs[1:]:
         assert np.array_equal(o, outs[0])
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32ref"])
+@pytest.mark.parametrize("calls", [(1, 1, 1, 1, 3), (9,), (2, 5)])
+def test_exact_steps_from_densities_below_zero_with_decay(gbg, oracle_lib, prec, calls):
+    """A first step from densities below 0 with a negative rho leaves positive
+    values in cells without tissue, which the second one clears: neither the
+    cells of the list nor those off it may keep them, bit for bit the oracle's
+    steps over every cell, also with a rho of the other sign afterwards."""
+    n, f32 = 14, prec == "f32ref"
+    rng = np.random.default_rng(3)
+    t = (rng.random((n, n, n)) < 0.85).astype(float)
+    w = rng.random((n, n, n))
+    pw, pg = t * w, t * (1.0 - w)
+    phi = rng.uniform(-3.0, 1.0, (n, n, n))
+    dt, dw, dg = S.reference_dt(n, 0.0013, n * 0.1, f32=f32)
+    rho = -0.5 / dt
+    if f32:
+        phi = phi.astype(np.float32).astype(np.float64)
+        rho = float(np.float32(rho))
+    ref = phi
+    with _lib.Handle(n, prec) as h:
+        h.set_anatomy(pw, pg)
+        h.set_phi(phi)
+        for k in calls:
+            h.rd_step(dw, dg, rho, dt, k)
+            ref = oracle_lib.rd_solve(pw, pg, ref, dw, dg, rho, dt, k, prec).astype(np.float64)
+            assert np.array_equal(h.get_phi(), ref), k
+            rho = -rho
+    assert ref.max() > 0
