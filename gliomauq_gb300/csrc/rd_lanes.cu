@@ -63,7 +63,7 @@ struct LaneArgs {
 // what a lane's warps share of the sample they are on
 struct Sample {
     SampleRec rec;
-    int ylo, yhi, zlo, zhi;
+    int ylo, yhi, zlo, zhi, any;  // the initial support, and whether there is one: without, the sample stays 0
     Lane lane;
 };
 
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
                 sm.yhi = bx.y - 1;
                 sm.zlo = n - bx.z;
                 sm.zhi = bx.w - 1;
-                if (bx.y == 0) sm.rec.a = -1.f;  // no nonzero initial cell: the sample stays 0
+                sm.any = bx.y != 0;
             }
             group_sync(1 + g, 32 * p.warps);
             const int nsteps = sm.rec.nsteps;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(128 * WPS, 1) k_population10(LaneArgs p) {
                     };
                     const bool lastk = k == nsteps - 1;
                     const float a = lastk ? sm.rec.a2 : sm.rec.a, b = lastk ? sm.rec.b2 : sm.rec.b;
-                    const bool any = sm.rec.a >= 0.f;
+                    const bool any = sm.any;
                     const int grow = p.grow0 + k + 1, u1 = nu * (w + 1) / p.warps;
                     for (int i = nu * w / p.warps; (KEEP || any) && i < u1;) {
                         const int un = s_unit[i], y0 = un & 1023, z = un >> 10 & 1023, len = min(un >> 20, u1 - i);

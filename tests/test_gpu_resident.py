@@ -90,3 +90,24 @@ def test_few_samples_at_32_equal_the_same_samples_among_others(gbg, kind):
         for a, b in ((0, 1), (1, 3), (3, 9), (9, 16), (16, 24)):
             part = h.batch_solve(smp[a:b], 3.2, with_loglik=False, want_phi=True)["phi"]
             assert np.array_equal(part, whole[a:b])
+
+
+@pytest.mark.parametrize("n", [32, 64, 128])
+def test_negative_step_coefficients_equal_the_dense_kernel(gbg, n):
+    """On the scaled time grid a strongly negative rho makes the step, and so the
+    coefficient of the full steps, negative, with a last (here the only) step of
+    the whole time: a sample like any other."""
+    an = S.make_anatomy(n, seed=2)
+    c = 0.5 * (n - 1)
+    smp = [(0.0013, -3.0, c, c + 0.4, c - 0.3, 0.8), (0.0013, 0.05, c, c, c, 4.0), (0.0009, -2.0, c + 1, c, c, 0.5)]
+    with _lib.Handle(n, "f32", max_samples=len(smp)) as h:
+        h.set_anatomy(an.p_w, an.p_g)
+        names = [h.population_variant_name(i) for i in range(len(h.population_variants()))]
+        out = []
+        for v in ([i for i, nm in enumerate(names) if nm.startswith("k_population8<")][0], 0):
+            h.set_population_variant(v)
+            out.append(h.batch_solve(smp, n * 0.1, with_loglik=False, want_phi=True, dt0=-0.75))
+    assert list(out[0]["nsteps"]) == list(out[1]["nsteps"]) and out[0]["nsteps"][0] == 1
+    for j in range(len(smp)):
+        assert out[0]["phi"][j].max() > 0
+        assert np.array_equal(out[0]["phi"][j], out[1]["phi"][j]), j
