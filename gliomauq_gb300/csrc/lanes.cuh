@@ -3,6 +3,8 @@
 #pragma once
 #include "gbg_internal.cuh"
 
+#include "arrivals.cuh"
+
 namespace gbg {
 namespace lanes {
 
@@ -41,14 +43,6 @@ __device__ __forceinline__ bool span_hits(int lo, int hi, int grow, int a, int b
 __device__ __forceinline__ void group_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void red_release(unsigned *p) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(p) : "memory");
-}
 
 struct V4 {
     float v[4];
@@ -61,34 +55,28 @@ __device__ __forceinline__ V4 sub(const V4 &a, const V4 &b) {
     return V4{{a.v[0] - b.v[0], a.v[1] - b.v[1], a.v[2] - b.v[2], a.v[3] - b.v[3]}};
 }
 
+// The number of the lane's next sample: drawn from `queue` by rank 0 on the way into
+// the barrier of the last step, and read by everyone after it. Two slots in turn,
+// as a CTA may still have to read one when the next is written.
+__device__ __forceinline__ void draw_next(const Lane &ln, unsigned *sync, unsigned *queue, int lanes) {
+    *(volatile unsigned *)(sync + 1 + ln.slot) = atomicAdd(queue, 1u) + (unsigned)lanes;
+}
+__device__ __forceinline__ void read_next(Lane &ln, const unsigned *sync) {
+    ln.next = (int)*(volatile const unsigned *)(sync + 1 + ln.slot);
+    ln.slot ^= 1u;
+}
+
 // Barrier of a team's T CTAs on one lane, by one thread of the lane after its
-// warps have met: sync[0] counts arrivals. With `last` (the sample's last
-// step) rank 0 draws the lane's next sample from `queue` before it arrives, and
-// everyone reads it after: two slots in turn, as a CTA may still have to read
-// one when the next is written. Bounded (seconds); on a timeout the status word
-// is set and every lane leaves at its next barrier.
+// warps have met: sync[0] counts arrivals. last: the sample's last step.
+// Bounded (seconds); on a timeout the status word is set and every lane leaves
+// at its next barrier.
 __device__ __forceinline__ void lane_barrier(Lane &ln, unsigned *sync, unsigned *queue, int T, int rank, int lanes, bool last,
                                              int *status) {
-    const unsigned target = ln.target + T;
-    if (last && rank == 0) *(volatile unsigned *)(sync + 1 + ln.slot) = atomicAdd(queue, 1u) + (unsigned)lanes;
-    red_release(sync);
-    long long spins = 0;
-    while (ld_acquire(sync) < target) {
-        if (++spins > (1ll << 24)) {
-            atomicExch(status, (int)DEV_BARRIER_TIMEOUT);
-            ln.ok = 0;
-            break;
-        }
-        if ((spins & 1023) == 0 && *(volatile int *)status != DEV_OK) {
-            ln.ok = 0;
-            break;
-        }
-    }
-    ln.target = target;
-    if (last) {
-        ln.next = (int)*(volatile unsigned *)(sync + 1 + ln.slot);
-        ln.slot ^= 1u;
-    }
+    if (last && rank == 0) draw_next(ln, sync, queue, lanes);
+    arrive(sync);
+    ln.target += T;
+    if (!wait_for_arrivals(sync, ln.target, status)) ln.ok = 0;
+    if (last) read_next(ln, sync);
 }
 
 // lane_barrier where the team is a cluster: a CTA arrives at the shared-memory
@@ -100,7 +88,7 @@ __device__ __forceinline__ void lane_barrier(Lane &ln, unsigned *sync, unsigned 
 // carries that on.
 __device__ __forceinline__ void cluster_barrier(Lane &ln, unsigned long long *bar, unsigned *sync, unsigned *queue, int T, int rank,
                                                 int lanes, bool last, int *status) {
-    if (last && rank == 0) *(volatile unsigned *)(sync + 1 + ln.slot) = atomicAdd(queue, 1u) + (unsigned)lanes;
+    if (last && rank == 0) draw_next(ln, sync, queue, lanes);
     const unsigned own = (unsigned)__cvta_generic_to_shared(bar), parity = ln.target & 1u;
     asm volatile("fence.acq_rel.cluster;" ::: "memory");
     for (int r = 0; r < T; ++r) {
@@ -127,10 +115,7 @@ __device__ __forceinline__ void cluster_barrier(Lane &ln, unsigned long long *ba
         }
     }
     ++ln.target;
-    if (last) {
-        ln.next = (int)*(volatile unsigned *)(sync + 1 + ln.slot);
-        ln.slot ^= 1u;
-    }
+    if (last) read_next(ln, sync);
 }
 
 }  // namespace lanes

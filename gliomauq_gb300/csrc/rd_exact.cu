@@ -16,6 +16,8 @@
 #include "exact_cells.cuh"
 #include "gbg_internal.cuh"
 
+#include "arrivals.cuh"
+
 namespace gbg {
 namespace {
 
@@ -273,24 +275,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_exact_resident(ExactArg
         if (s == a.nsteps - 1) break;
         __syncthreads();
         int ok = 1;
-        if (tid == 0) {  // grid barrier, bounded (seconds)
-            const unsigned target = (unsigned)(s + 1) * T;
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(a.arrived) : "memory");
-            long long spins = 0;
-            for (;;) {
-                unsigned v;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(a.arrived) : "memory");
-                if (v >= target) break;
-                if (++spins > (1ll << 24)) {
-                    atomicExch(a.status, (int)DEV_BARRIER_TIMEOUT);
-                    ok = 0;
-                    break;
-                }
-                if ((spins & 1023) == 0 && *(volatile int *)a.status != DEV_OK) {
-                    ok = 0;
-                    break;
-                }
-            }
+        if (tid == 0) {
+            arrive(a.arrived);
+            ok = wait_for_arrivals(a.arrived, (unsigned)(s + 1) * T, a.status);
         }
         if (!__syncthreads_and(ok)) break;
         Real *const t = in;
@@ -512,7 +499,7 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
         }
         if (h.exact_full == kListed && h.exact_list) {
             if (!h.exact_listed) h.prec == GBG_PREC_F64 ? collect(double{}) : collect(float{});
-            if (nsteps - s >= kResidentSteps && nsteps - s < 0x7fffffffL / h.num_sms) {  // arrivals are counted in 32 bits
+            if (nsteps - s >= kResidentSteps && nsteps - s <= 0x7fffffffL) {
                 const int rc = h.prec == GBG_PREC_F64 ? resident_steps<double>(h, rho, dt, ih2, nsteps - s)
                                                       : resident_steps<float>(h, rho, dt, ih2, nsteps - s);
                 if (rc == GBG_OK) break;

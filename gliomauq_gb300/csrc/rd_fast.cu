@@ -1518,11 +1518,10 @@ int fast_steps_single(Handle &h, double Dw, double rho, double dt, long nsteps) 
     // over the whole grid, with zeros in the second buffer where no live unit
     // writes: 1.7 us a step at 32^3, 2.1 at 64^3 and 3.5 at 128^3, where the dense
     // kernel takes 5.7, 8.6 and 8.8; the zeros and the unit tables cost 5 us
-    // first. Its barrier counts arrivals in 32 bits.
+    // first.
     PopVariant vs[32];
     const int nv = variants_for(h.n, vs);
-    const bool lanes = nsteps >= 4 && h.pop_variant >= 0 && h.pop_variant < nv && vs[h.pop_variant].resident && lanes_fit(h, 1) &&
-                       nsteps < 0x7fffffffL / h.num_sms;
+    const bool lanes = nsteps >= 4 && h.pop_variant >= 0 && h.pop_variant < nv && vs[h.pop_variant].resident && lanes_fit(h, 1);
     int rc;
     if (lanes) {
         int *box = batch_boxes(h);
