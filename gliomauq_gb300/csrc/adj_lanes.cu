@@ -33,7 +33,7 @@ constexpr int kBlockZ = 16, kBlocks = (n / 2) * (n / kBlockZ);
 // 56.5 with four; eight lanes of one warp 64, four lanes with three planes ahead
 // (spilled) 65.
 constexpr int kAdjWarps = 8, kAdjThreads = 32 * kAdjWarps, kAdjLanes = 4;
-constexpr int kMaxBlocks = 4;  // per CTA: 64 units, 224 KB
+constexpr int kMaxBlocks = kMaxUnits / kBlockZ;  // per CTA
 
 struct AdjArgs {
     int S, T, lanes, warps, k0, k1, nblocks, strideS;
@@ -322,7 +322,7 @@ int adj_lanes_segment(Handle &h, int S, int k0, int k1, const SampleRec *recs, S
     a.gB = gB;
     const size_t smem = (size_t)((h.blocks + a.T - 1) / a.T) * kBlockZ * kUnitBytes;
     GBG_CUDA_TRY(cudaMemcpyAsync(drec, recs, (size_t)S * sizeof(SampleRec), cudaMemcpyHostToDevice, h.stream));
-    GBG_CUDA_TRY(cudaFuncSetAttribute(k_adj_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBG_CUDA_TRY(cudaFuncSetAttribute(k_adj_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes));
     GBG_CUDA_TRY(cudaMemsetAsync(h.lane_sync, 0, (size_t)(a.lanes + 1) * kSyncStride * sizeof(unsigned), h.stream));
     void *args[] = {&a};
     GBG_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_adj_lanes, dim3((unsigned)a.T), dim3(kAdjThreads), args, smem, h.stream));

@@ -19,6 +19,11 @@ constexpr int kMaxLanes = 8;
 constexpr int kSlots = 7;
 constexpr size_t kUnitBytes = (size_t)kSlots * 32 * sizeof(float4);
 constexpr int kMaxUnits = 64;              // units a CTA can own
+// The tables' room in a CTA; the rest of the 227 KB is the kernels' static shared
+// memory. A kernel's limit is the function's, not a handle's: it is always set to
+// this, as a smaller one would fail the launch another thread is about to make.
+constexpr int kTableBytes = 224 * 1024;
+static_assert(kMaxUnits * kUnitBytes <= kTableBytes, "the most units fit");
 // Planes loaded ahead: one plane's arithmetic does not cover an L2 load (170
 // ms), a third plane spills registers (207 ms).
 constexpr int kAhead = 2;

@@ -221,6 +221,9 @@ struct ExactArgs {
 constexpr int kResidentSteps = 4;  // fewer do not repay the fill of shared memory (the faces, once: about a step)
 constexpr int kResidentThreads = 1024;
 constexpr size_t kCellBytes = 7 * sizeof(double) + sizeof(int);
+// shared memory for cells; the limit set for the kernel, whatever a launch takes (it
+// is the function's, shared by handles on other threads)
+constexpr int kCellsBytes = 224 * 1024;
 
 // All steps in one launch: a CTA keeps a stretch of the list, with the faces and
 // their sums, in shared memory (what does not fit it reads again each step). The
@@ -433,7 +436,7 @@ int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps) {
     ExactArgs<Real> a;
     a.n = h.n;
     a.nsteps = (int)nsteps;
-    a.cap = (int)std::min<size_t>((h.N + T - 1) / T, (224 * 1024) / kCellBytes);
+    a.cap = (int)std::min<size_t>((h.N + T - 1) / T, kCellsBytes / kCellBytes);
     a.cap += a.cap & 1;
     const size_t smem = a.cap * kCellBytes;
     a.count = h.exact_list + h.N + chunks;
@@ -451,7 +454,7 @@ int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps) {
     a.arrived = (unsigned *)(h.exact_list + h.N + chunks + 1);
     a.status = h.dev_status;
     const void *fn = (const void *)k_exact_resident<Real>;
-    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kCellsBytes));
     GBG_CUDA_TRY(cudaMemsetAsync(a.arrived, 0, sizeof(unsigned), h.stream));
     void *args[] = {&a};
     if (cudaLaunchCooperativeKernel(fn, dim3((unsigned)T), dim3(kResidentThreads), args, smem, h.stream) != cudaSuccess) {

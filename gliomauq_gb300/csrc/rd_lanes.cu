@@ -378,7 +378,7 @@ int lanes_set_anatomy(Handle &h) {
         c.attrs = at;
         c.numAttrs = 1;
         h.lane_clusters = 0;
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.dynamicSmemBytes) != cudaSuccess ||
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&h.lane_clusters, fn, &c) != cudaSuccess) {
             cudaGetLastError();
@@ -431,8 +431,7 @@ bool lanes_fit(const Handle &h, int S) {
     int units;
     if (!h.unit_list) return false;
     lane_shape(h, S, a, units);
-    // the rest of the 227 KB is the kernel's static shared memory
-    return units <= kMaxUnits && units * kUnitBytes <= 224 * 1024;
+    return units <= kMaxUnits;
 }
 
 int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0, size_t slot,
@@ -470,7 +469,7 @@ int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, i
                            : (const void *)k_population10<8, kWps, K, false>;
     };
     const void *fn = slot ? kernel(std::true_type{}) : kernel(std::false_type{});
-    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes));
     GBG_CUDA_TRY(cudaMemsetAsync(h.barrier, 0, 4 * sizeof(unsigned), h.stream));
     GBG_CUDA_TRY(
         cudaMemsetAsync(h.lane_sync, 0, (size_t)(a.teams * a.lanes + 1) * kSyncStride * sizeof(unsigned), h.stream));
