@@ -870,6 +870,14 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
         h.amr.full_steps = kAnyState;
         h.amr.listed = false;
     }
+    // as in exact_steps (rd_exact.cu)
+    auto forget = [&] {
+        h.amr.full_steps = kAnyState;
+        h.amr.listed = false;
+    };
+    bool capturing;
+    if (int rc = stream_capturing(h, &capturing)) return rc;
+    if (capturing) forget();
     auto step = [&](auto real, const void *in, void *out) {
         using Real = decltype(real);
         if (h.amr.full_steps == kListed && h.amr.list) {
@@ -906,6 +914,7 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
             step(float{}, in, out);
         h.amr.cur ^= 1;
     }
+    if (capturing) forget();
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;
 }

@@ -123,7 +123,8 @@ struct Handle {
     int *exact_list = nullptr;
     double *exact_dsum = nullptr;
     bool exact_listed = false;
-    bool exact_waited = false;  // a launch whose CTAs wait for one another is not yet checked (finish_steps)
+    bool exact_waited = false;    // a launch whose CTAs wait for one another is not yet checked (finish_steps)
+    bool exact_in_graph = false;  // a captured graph has such a launch: it may have run at any time
     int exact_full = 0;
 
     // MALA variant (exact modes): slopes sRho, sD ping-pong in the storage
@@ -308,6 +309,8 @@ int population_variant_name(int n, int vi, char *buf, int len);
 int check_device_status(Handle &h);
 // the stream's work is done; an error if steps among it gave up waiting
 int finish_steps(Handle &h);
+// whether the handle's stream is being captured into a graph
+int stream_capturing(const Handle &h, bool *yes);
 int batch_solve_device(Handle &h, const gbg_sample *samples_device, int S,
                        const gbg_batch_opts &o, gbg_lik_result *loglik_device, long *nsteps_host);
 

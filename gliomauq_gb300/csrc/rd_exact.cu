@@ -431,7 +431,7 @@ void exact_alloc_list(Handle &h) {
 
 // nsteps steps over the list in one launch; GBG_ERR_UNSUPPORTED: not here
 template <typename Real>
-int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps) {
+int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps, bool capturing) {
     const int T = h.num_sms, chunks = (int)((h.N + 255) / 256);
     ExactArgs<Real> a;
     a.n = h.n;
@@ -462,6 +462,7 @@ int resident_steps(Handle &h, double rho, double dt, double ih2, long nsteps) {
         return GBG_ERR_UNSUPPORTED;
     }
     h.exact_waited = true;
+    h.exact_in_graph |= capturing;
     h.launches++;
     if (nsteps & 1) h.cur ^= 1;
     return GBG_OK;
@@ -495,6 +496,15 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
             h.exact_full = after_full_step(h.exact_full, rho, dt);
         }
     };
+    // What is known here does not hold when a captured graph runs: it takes its own
+    // full step and makes its own list, and a call after it does so too.
+    auto forget = [&] {
+        h.exact_full = kAnyState;
+        h.exact_listed = false;
+    };
+    bool capturing;
+    if ((rc = stream_capturing(h, &capturing))) return rc;
+    if (capturing) forget();
     for (long s = 0; s < nsteps; ++s) {
         if (h.exact_full == kDeadZero && h.exact_list) {  // the other buffer's dead cells
             GBG_CUDA_TRY(cudaMemsetAsync(h.phi[h.cur ^ 1], 0, h.N * (h.prec == GBG_PREC_F64 ? sizeof(double) : sizeof(float)), h.stream));
@@ -503,8 +513,8 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
         if (h.exact_full == kListed && h.exact_list) {
             if (!h.exact_listed) h.prec == GBG_PREC_F64 ? collect(double{}) : collect(float{});
             if (nsteps - s >= kResidentSteps && nsteps - s <= 0x7fffffffL) {
-                const int rc = h.prec == GBG_PREC_F64 ? resident_steps<double>(h, rho, dt, ih2, nsteps - s)
-                                                      : resident_steps<float>(h, rho, dt, ih2, nsteps - s);
+                const int rc = h.prec == GBG_PREC_F64 ? resident_steps<double>(h, rho, dt, ih2, nsteps - s, capturing)
+                                                      : resident_steps<float>(h, rho, dt, ih2, nsteps - s, capturing);
                 if (rc == GBG_OK) break;
                 if (rc != GBG_ERR_UNSUPPORTED) return rc;
             }
@@ -516,6 +526,7 @@ int exact_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nst
         h.launches++;
         h.cur ^= 1;
     }
+    if (capturing) forget();
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;
 }

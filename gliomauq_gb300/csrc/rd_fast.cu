@@ -1453,11 +1453,18 @@ int check_device_status(Handle &h) {
 }
 
 int finish_steps(Handle &h) {
-    if (h.exact_waited) {
+    if (h.exact_waited || h.exact_in_graph) {
         h.exact_waited = false;
         return check_device_status(h);
     }
     GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    return GBG_OK;
+}
+
+int stream_capturing(const Handle &h, bool *yes) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    GBG_CUDA_TRY(cudaStreamIsCapturing(h.stream, &s));
+    *yes = s == cudaStreamCaptureStatusActive;
     return GBG_OK;
 }
 
