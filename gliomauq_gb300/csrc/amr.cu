@@ -673,9 +673,10 @@ void amr_free(Handle &h) {
         if (q) cudaFree(q);
 }
 
-// A caller's doubles to the float modes' fields, staged in the face tables,
-// which a new grid makes stale. Converted on the host, a field of 512 blocks
-// took 1.5 ms; this way 1.1, most of it the copy from pageable memory.
+// A caller's doubles to the float modes' fields, staged by halves in the remap's
+// targets (the size of a field in floats each), whose contents nothing keeps; the
+// tables stay, for captured graphs of steps. Converted on the host, a field of
+// 512 blocks took 1.5 ms; this way 1.1, most of it the copy from pageable memory.
 __global__ void k_narrow(long n, const double *__restrict__ in, float *__restrict__ out) {
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) out[i] = (float)in[i];
 }
@@ -692,7 +693,6 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
     }
     GBG_CUDA_TRY(cudaMemcpyAsync(h.amr.level, lv.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h.stream));
     GBG_CUDA_TRY(cudaMemcpyAsync(h.amr.bidx, bi.data(), bi.size() * sizeof(int), cudaMemcpyHostToDevice, h.stream));
-    h.amr.tables_valid = false;
     const double *src[3] = {pw, pg, phi};
     void *dst[3] = {h.amr.pw, h.amr.pg, h.amr.phi[0]};
     if (h.prec == GBG_PREC_F64) {
@@ -701,11 +701,14 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
         GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     } else {
         for (int k = 0; k < 3; ++k) {
-            double *staged = h.amr.df + k * n;
-            GBG_CUDA_TRY(cudaMemcpyAsync(staged, src[k], n * sizeof(double), cudaMemcpyHostToDevice, h.stream));
-            k_narrow<<<grid_blocks(h, (long)n), 256, 0, h.stream>>>((long)n, staged, (float *)dst[k]);
+            for (int half = 0; half < 2; ++half) {
+                double *staged = (double *)(half ? h.amr.pg2 : h.amr.pw2);
+                const size_t m = n / 2;  // blocks have an even number of cells
+                GBG_CUDA_TRY(cudaMemcpyAsync(staged, src[k] + half * m, m * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+                k_narrow<<<grid_blocks(h, (long)m), 256, 0, h.stream>>>((long)m, staged, (float *)dst[k] + half * m);
+            }
         }
-        h.launches += 3;
+        h.launches += 6;
         GBG_CUDA_TRY(cudaGetLastError());
         GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     }

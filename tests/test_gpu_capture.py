@@ -102,7 +102,7 @@ def _block_grid_replays(prec):
     return outs
 
 
-@pytest.mark.parametrize("prec", ["f64"])
+@pytest.mark.parametrize("prec", ["f64", "f32ref", "f32"])
 def test_replays_on_the_block_grid(gbg, prec):
     calls, graph = _block_grid_replays(prec)
     for x, y in zip(calls, graph):
