@@ -282,8 +282,7 @@ __global__ void __launch_bounds__(kBlocks) k_block_list(const unsigned char *__r
 }  // namespace
 
 int adj_lanes_set_anatomy(Handle &h) {
-    if (h.n != n) return GBG_OK;
-    if (!h.block_list) GBG_CUDA_TRY(cudaMalloc((void **)&h.block_list, (kBlocks + 1) * sizeof(int)));
+    if (h.n != n || !reserve_device({{(void **)&h.block_list, (kBlocks + 1) * sizeof(int)}})) return GBG_OK;
     k_block_list<<<1, kBlocks, 0, h.stream>>>(h.unit_live, h.block_list);
     h.launches++;
     GBG_CUDA_TRY(cudaGetLastError());

@@ -654,13 +654,8 @@ int amr_alloc(Handle &h) {
     GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.rkind, (size_t)h.amr.max_blocks * sizeof(int)));
     GBG_CUDA_TRY(cudaMalloc((void **)&h.amr.rsrc, (size_t)h.amr.max_blocks * 8 * sizeof(int)));
     // the exact steps' list; without memory for it every step computes every cell
-    if (h.prec != GBG_PREC_F32 && cells < 0x7fffffff &&
-        (cudaMalloc((void **)&h.amr.list, (cells + cells / 256 + 2) * sizeof(int)) != cudaSuccess ||
-         cudaMalloc((void **)&h.amr.dsum, cells * sizeof(double)) != cudaSuccess)) {
-        cudaGetLastError();
-        if (h.amr.list) cudaFree(h.amr.list);
-        h.amr.list = nullptr;
-    }
+    if (h.prec != GBG_PREC_F32 && cells < 0x7fffffff)
+        reserve_device({{(void **)&h.amr.list, (cells + cells / 256 + 2) * sizeof(int)}, {(void **)&h.amr.dsum, cells * sizeof(double)}});
     return GBG_OK;
 }
 

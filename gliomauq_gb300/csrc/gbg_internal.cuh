@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/gbglioma.h"
+#include "reserve.h"
 
 namespace gbg {
 
@@ -21,6 +22,18 @@ void set_error(const std::string &msg);
             return _e == cudaErrorMemoryAllocation ? GBG_ERR_NOMEM : GBG_ERR_CUDA;    \
         }                                                                             \
     } while (0)
+
+// reserve_all on the current device; its failure is no error of the call
+inline bool reserve_device(std::initializer_list<Want> want) {
+    return reserve_all(
+        want,
+        [](void **p, size_t bytes) {
+            if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+            cudaGetLastError();
+            return false;
+        },
+        [](void *p) { cudaFree(p); });
+}
 
 // Device-side error codes written to the handle's status word.
 // DEV_DRAIN_TIMEOUT: after a copy timeout, waiting for the copies still in

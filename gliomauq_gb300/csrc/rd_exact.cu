@@ -421,12 +421,7 @@ int exact_build_tables(Handle &h, double Dw, double Dg) {
 
 void exact_alloc_list(Handle &h) {
     const size_t chunks = (h.N + 255) / 256;
-    if (cudaMalloc((void **)&h.exact_list, (h.N + chunks + 2) * sizeof(int)) != cudaSuccess ||
-        cudaMalloc((void **)&h.exact_dsum, h.N * sizeof(double)) != cudaSuccess) {
-        cudaGetLastError();
-        if (h.exact_list) cudaFree(h.exact_list);
-        h.exact_list = nullptr;
-    }
+    reserve_device({{(void **)&h.exact_list, (h.N + chunks + 2) * sizeof(int)}, {(void **)&h.exact_dsum, h.N * sizeof(double)}});
 }
 
 // nsteps steps over the list in one launch; GBG_ERR_UNSUPPORTED: not here

@@ -359,11 +359,11 @@ int units_of(int n) { return (n / unit_rows(n)) * n; }
 int lanes_set_anatomy(Handle &h) {
     if (!population_supported(h.n)) return GBG_OK;
     const int nu = units_of(h.n);
-    if (!h.unit_live) {
-        GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_live, nu));
-        GBG_CUDA_TRY(cudaMalloc((void **)&h.unit_list, 3 * (nu + 1) * sizeof(int)));
-        GBG_CUDA_TRY(cudaMalloc((void **)&h.lane_sync, (size_t)(h.num_sms * kMaxLanes + 1) * kSyncStride * sizeof(unsigned)));
-    }
+    // without room for the lists every call takes the tile march (lanes_fit)
+    if (!reserve_device({{(void **)&h.unit_live, (size_t)nu},
+                         {(void **)&h.unit_list, 3 * (nu + 1) * sizeof(int)},
+                         {(void **)&h.lane_sync, (size_t)(h.num_sms * kMaxLanes + 1) * kSyncStride * sizeof(unsigned)}}))
+        return GBG_OK;
     if (h.n == 32 && h.lane_clusters < 0) {
         // how many clusters run side by side, at the most units a CTA of one owns
         const void *fn = (const void *)k_population10<8, kWps, false, true>;
