@@ -176,13 +176,13 @@ int gbg_create(const gbg_config *cfg, gbg_handle **out) {
         TRY_ALLOC(h.dfx, h.N * sizeof(double));
         TRY_ALLOC(h.dfy, h.N * sizeof(double));
         TRY_ALLOC(h.dfz, h.N * sizeof(double));
-        gbg::exact_alloc_list(h);
     }
     h.bwork_bytes = gbg::bwork_total(h);
     TRY_ALLOC(h.bwork, h.bwork_bytes);
     TRY_ALLOC(h.dev_status, sizeof(int));
     TRY_ALLOC(h.barrier, 4 * sizeof(unsigned));
 #undef TRY_ALLOC
+    if (h.prec != GBG_PREC_F32) gbg::exact_alloc_list(h);  // last: the handle does without
     if (cudaMemset(h.dev_status, 0, sizeof(int)) != cudaSuccess ||
         cudaMemset(h.barrier, 0, 4 * sizeof(unsigned)) != cudaSuccess) {
         set_error("memset failed");
