@@ -783,16 +783,25 @@ struct B8 {
     __device__ __forceinline__ float operator[](int e) const { return __bfloat162float(h[e]); }
 };
 
-// The elementwise passes below take a sample per blockIdx.y and (voxel, eight
+// The elementwise passes below take parts of a sample per CTA and (voxel, eight
 // channels) items of it per thread, 32-bit index arithmetic inside a sample.
 // Per-element 64-bit divisions and 2-byte accesses bound their first form: at
 // 64^3 with 8 samples the pooling backward, its addition and the ReLU backward
 // took 184 + 96 + 94 us, the fused pass takes 49 us.
-__device__ __forceinline__ long voxel_of(const Geom &g, int v, int &z, int &y, int &x) {
+struct Part {
+    int sample, first, step;  // this thread's first item of the sample, and from each to the next
+};
+// the grid is B samples of equally many CTAs each, in one dimension (the others end
+// at 65535)
+__device__ __forceinline__ Part part_of(int B) {
+    const unsigned parts = gridDim.x / (unsigned)B;
+    return Part{(int)(blockIdx.x / parts), (int)(blockIdx.x % parts * blockDim.x + threadIdx.x), (int)(parts * blockDim.x)};
+}
+__device__ __forceinline__ long voxel_of(const Geom &g, const Part &t, int v, int &z, int &y, int &x) {
     x = v % g.W;
     y = v / g.W % g.H;
     z = v / (g.W * g.H);
-    return (long)blockIdx.y * g.D * g.H * g.W;
+    return (long)t.sample * g.D * g.H * g.W;
 }
 
 // db[c] += sum_v dy[v][c]
@@ -822,10 +831,11 @@ __global__ void __launch_bounds__(256) k_bias_grad(long nv, int C, Slice dy, flo
 // 2x average pooling: out (D/2, H/2, W/2) <- in
 __global__ void k_pool2(Geom go, int C, Slice in, Slice out) {
     const int G = C / 8, n = go.D * go.H * go.W * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Part t = part_of(go.B);
+    for (int i = t.first; i < n; i += t.step) {
         int z, y, x;
         const int c = i % G * 8;
-        const long base = voxel_of(go, i / G, z, y, x);
+        const long base = voxel_of(go, t, i / G, z, y, x);
         const int Hi = go.H * 2, Wi = go.W * 2;
         float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -846,10 +856,11 @@ __global__ void k_pool2(Geom go, int C, Slice in, Slice out) {
 // ReLU backward of the layer y that was pooled: d = (y > 0) (d + dp / 8)
 __global__ void k_pool2_bwd(Geom gf, int C, Slice dp, Slice y, Slice d) {
     const int G = C / 8, n = gf.D * gf.H * gf.W * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Part t = part_of(gf.B);
+    for (int i = t.first; i < n; i += t.step) {
         int z, yy, x;
         const int c = i % G * 8;
-        const long base = voxel_of(gf, i / G, z, yy, x), v = base + i / G;
+        const long base = voxel_of(gf, t, i / G, z, yy, x), v = base + i / G;
         B8 p, a, r;
         p.load(dp, base / 8 + ((long)(z / 2) * (gf.H / 2) + yy / 2) * (gf.W / 2) + x / 2, c);
         a.load(y, v, c);
@@ -866,10 +877,11 @@ __global__ void k_pool2_bwd(Geom gf, int C, Slice dp, Slice y, Slice d) {
 // 2x nearest upsampling: out (fine) <- in (coarse)
 __global__ void k_up2(Geom gf, int C, Slice in, Slice out) {
     const int G = C / 8, n = gf.D * gf.H * gf.W * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Part t = part_of(gf.B);
+    for (int i = t.first; i < n; i += t.step) {
         int z, y, x;
         const int c = i % G * 8;
-        const long base = voxel_of(gf, i / G, z, y, x);
+        const long base = voxel_of(gf, t, i / G, z, y, x);
         B8 a;
         a.load(in, base / 8 + ((long)(z / 2) * (gf.H / 2) + y / 2) * (gf.W / 2) + x / 2, c);
         a.store(out, base + i / G, c);
@@ -879,10 +891,11 @@ __global__ void k_up2(Geom gf, int C, Slice in, Slice out) {
 // its transpose (sum of 8) and the ReLU backward of the layer y that was upsampled
 __global__ void k_up2_bwd(Geom gc, int C, Slice dout, Slice y, Slice din) {
     const int G = C / 8, n = gc.D * gc.H * gc.W * G;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Part t = part_of(gc.B);
+    for (int i = t.first; i < n; i += t.step) {
         int z, yy, x;
         const int c = i % G * 8;
-        const long base = voxel_of(gc, i / G, z, yy, x);
+        const long base = voxel_of(gc, t, i / G, z, yy, x);
         const int Hf = gc.H * 2, Wf = gc.W * 2;
         float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -957,15 +970,16 @@ struct FeatParams {
     double dw_lo, dw_hi, rho_lo, rho_hi, t_lo, t_hi, L, n_solver, blob_sigma;
 };
 
-// One sample per blockIdx.y. What depends on the sample or on one coordinate
+// Parts of a sample per CTA. What depends on the sample or on one coordinate
 // alone is formed in double once per CTA (per cell it kept the FP64 pipe, 1/64
 // of the FP32 rate here, busy for 2.1 ms on 64 samples of 64^3; now 0.11 ms).
-__global__ void __launch_bounds__(256) k_features(int n, int factor, const gbg_sample *__restrict__ smp,
+__global__ void __launch_bounds__(256) k_features(int B, int n, int factor, const gbg_sample *__restrict__ smp,
                                                   const float *__restrict__ pw, const float *__restrict__ pg, FeatParams fp,
                                                   __nv_bfloat16 *__restrict__ x) {
     extern __shared__ float s_d[];  // distances to the seed per coordinate, x then y then z
     __shared__ float s_front, s_f[3];
-    const gbg_sample q = smp[blockIdx.y];
+    const Part t = part_of(B);
+    const gbg_sample q = smp[t.sample];
     for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) {
         const int a = i / n;
         // cell centre in solver voxel units
@@ -984,8 +998,8 @@ __global__ void __launch_bounds__(256) k_features(int n, int factor, const gbg_s
     const unsigned f34 = pack2(__float2bfloat16(s_f[1]), __float2bfloat16(s_f[2]));
     const __nv_bfloat16 f3 = __float2bfloat16(s_f[0]);
     const int N = n * n * n;
-    uint4 *out = reinterpret_cast<uint4 *>(x) + (size_t)blockIdx.y * N * 2;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+    uint4 *out = reinterpret_cast<uint4 *>(x) + (size_t)t.sample * N * 2;
+    for (int c = t.first; c < N; c += t.step) {
         const float dx = s_d[c % n], dy = s_d[n + c / n % n], dz = s_d[2 * n + c / (n * n)];
         const float d2 = dx * dx + dy * dy + dz * dz;
         uint4 lo;
@@ -1013,11 +1027,12 @@ __global__ void k_down2_f32(int S, int n, const float *__restrict__ in, float *_
 }
 
 // nearest 2x upsampling of float fields m^3 -> (2m)^3, zero outside tissue
-__global__ void k_up2_f32(int m, const float *__restrict__ in, const float *__restrict__ mask, float *__restrict__ out) {
+__global__ void k_up2_f32(int B, int m, const float *__restrict__ in, const float *__restrict__ mask, float *__restrict__ out) {
     const int n = 2 * m, N = n * n * n;
-    in += (size_t)blockIdx.y * m * m * m;
-    out += (size_t)blockIdx.y * N;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+    const Part t = part_of(B);
+    in += (size_t)t.sample * m * m * m;
+    out += (size_t)t.sample * N;
+    for (int c = t.first; c < N; c += t.step) {
         const int x = c % n, y = c / n % n, z = c / (n * n);
         out[c] = mask[c] != 0.f ? in[((z / 2) * m + y / 2) * m + x / 2] : 0.f;
     }
@@ -1224,10 +1239,10 @@ __global__ void k_channel0(long nv, const float *__restrict__ l16, float *__rest
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nv; i += (long)gridDim.x * blockDim.x) l1[i] = l16[i * 16];
 }
 
-// grid of the elementwise passes: sample per y, up to 16 CTAs per SM in all
-dim3 grid_bv(const Surrogate &s, int B, long per_sample) {
+// grid of the elementwise passes (part_of): up to 16 CTAs per SM in all
+unsigned grid_bv(const Surrogate &s, int B, long per_sample) {
     const long want = (per_sample + 255) / 256, cap = std::max<long>(1, (long)s.h->num_sms * 16 / B);
-    return dim3((unsigned)std::min(want, cap), (unsigned)B);
+    return (unsigned)(std::min(want, cap) * B);
 }
 
 // Layer i: out = conv(in) + bias, ReLU except for the last layer, whose
@@ -1339,7 +1354,7 @@ void backward(Surrogate &s, int B) {
 
 void featurise(Surrogate &s, const gbg_sample *dsamples, int B) {
     sg::k_features<<<grid_bv(s, B, (long)s.m * s.m * s.m), 256, 3 * s.m * sizeof(float), s.h->stream>>>(
-        s.m, s.factor, dsamples, s.pw_s, s.pg_s, s.fp, s.x0);
+        B, s.m, s.factor, dsamples, s.pw_s, s.pg_s, s.fp, s.x0);
     s.h->launches++;
 }
 
@@ -1618,7 +1633,7 @@ int surrogate_predict(Surrogate &s, const gbg_sample *samples_device, int B, gbg
     sg::k_loss<<<sg::grid_n(nv, 1024), 256, 0, st>>>(nv, s.pred, nullptr, s.pred, nullptr, nullptr);
     s.h->launches++;
     if (want_field) {
-        sg::k_up2_f32<<<grid_bv(s, B, (long)s.h->N), 256, 0, st>>>(s.m, s.pred, s.mask_solver, s.up_pred);
+        sg::k_up2_f32<<<grid_bv(s, B, (long)s.h->N), 256, 0, st>>>(B, s.m, s.pred, s.mask_solver, s.up_pred);
         s.h->launches++;
     }
     GBG_CUDA_TRY(cudaGetLastError());

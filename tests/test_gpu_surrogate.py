@@ -221,3 +221,34 @@ def test_marching_kernels_vs_oracle(gbg, n, batch):
     assert np.linalg.norm(g - g_o) <= 3e-2 * np.linalg.norm(g_o)
     # fp32 atomics of at most 608 CTAs in any order: 608 roundings of 2^-24
     assert np.linalg.norm(g - g2) <= 608 * 2.0 ** -24 * np.linalg.norm(g)
+
+
+@pytest.mark.parametrize("engine", ["mma.sync", "tcgen05"])
+def test_more_samples_than_a_grids_second_dimension(gbg, engine):
+    """65535 is the most a grid's second and third dimension count: a batch
+    beyond it has the features of its samples and the mean of its parts' losses and
+    gradients (whose order of summation differs: 1e-5, and 1e-3 on the gradient's
+    bf16 roundings)."""
+    n, B = 8, 65536 + 64
+    pw, pg = np.random.default_rng(1).uniform(0.1, 0.9, (2, n, n, n))
+    rng = np.random.default_rng(2)
+    lo, hi = (0.0001, 0.005, 20.0), (0.004, 0.3, 700.0)
+    smp = [tuple(r) for r in np.column_stack([rng.uniform(lo[0], hi[0], B), rng.uniform(lo[1], hi[1], B), rng.uniform(1, 7, (B, 3)),
+                                              rng.uniform(lo[2], hi[2], B)])]
+    targ = rng.uniform(0, 1, (B, 4, 4, 4)).astype(np.float32)
+    with _lib.Handle(n, "f32", max_samples=1) as h:
+        h.set_anatomy(pw, pg)
+        s = _lib.Surrogate(h, 6.4, lo, hi, batch_max=B, seed=3)
+        try:
+            s.set_engine(engine)
+            whole = s.features(smp)
+            assert np.array_equal(whole[-70:], s.features(smp[-70:]))
+            assert np.array_equal(whole[:70], s.features(smp[:70]))
+            loss, grad = s.loss_grad(smp, targ)
+            half = B // 2
+            parts = [s.loss_grad(smp[a:a + half], targ[a:a + half]) for a in (0, half)]
+        finally:
+            s.close()
+    mean = 0.5 * (parts[0][1] + parts[1][1])
+    assert abs(loss - 0.5 * (parts[0][0] + parts[1][0])) <= 1e-5 * loss
+    assert np.linalg.norm(grad - mean) <= 1e-3 * np.linalg.norm(mean)
