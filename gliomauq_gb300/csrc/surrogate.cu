@@ -1213,7 +1213,7 @@ struct Surrogate {
     __nv_bfloat16 *x0 = nullptr, *t0 = nullptr, *c0 = nullptr, *p1 = nullptr, *t1 = nullptr, *c1 = nullptr,
                   *p2 = nullptr, *q2 = nullptr, *u1 = nullptr, *u0 = nullptr;
     __nv_bfloat16 *dt0 = nullptr, *dc0 = nullptr, *dp1 = nullptr, *dt1 = nullptr, *dc1 = nullptr,
-                  *dp2 = nullptr, *dq2 = nullptr, *du1 = nullptr, *du0 = nullptr, *dlog = nullptr, *tmp = nullptr;
+                  *dp2 = nullptr, *dq2 = nullptr, *du1 = nullptr, *du0 = nullptr, *dlog = nullptr;
     float *logits = nullptr, *pred = nullptr, *targ = nullptr, *pw_s = nullptr, *pg_s = nullptr,
           *mask_solver = nullptr, *up_pred = nullptr;
     gbg_sample *dsmp = nullptr;
@@ -1408,7 +1408,7 @@ int surrogate_create(Handle &h, const gbg_surrogate_config &c, Surrogate **out) 
               (s->dc1 = salloc<__nv_bfloat16>(*s, v1 * 64)) && (s->dp2 = salloc<__nv_bfloat16>(*s, v2 * 32)) &&
               (s->dq2 = salloc<__nv_bfloat16>(*s, v2 * 32)) && (s->du1 = salloc<__nv_bfloat16>(*s, v1 * 16)) &&
               (s->du0 = salloc<__nv_bfloat16>(*s, v0 * 16)) && (s->dlog = salloc<__nv_bfloat16>(*s, v0 * 16)) &&
-              (s->tmp = salloc<__nv_bfloat16>(*s, v0 * 32)) && (s->logits = salloc<float>(*s, v0 * 16)) &&
+              (s->logits = salloc<float>(*s, v0 * 16)) &&
               (s->pred = salloc<float>(*s, v0)) && (s->pw_s = salloc<float>(*s, (size_t)s->m * s->m * s->m)) &&
               (s->pg_s = salloc<float>(*s, (size_t)s->m * s->m * s->m)) && (s->mask_solver = salloc<float>(*s, N)) &&
               (s->up_pred = salloc<float>(*s, (size_t)c.batch_max * N)) &&
