@@ -1,6 +1,8 @@
 """GPU: MALA gradients from the discrete adjoint (gbg_adjoint_grad) against
 central finite differences of the same forward model, h = 1e-4 relative to
 each parameter; and independence from the checkpoint interval."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -163,3 +165,53 @@ def test_fused_backward_at_128_matches_fp64_adjoint(gbg):
     assert np.all(np.abs(l32 - l64) <= 1e-4 * np.abs(l64))
     assert np.array_equal(l32, l32b)
     assert np.allclose(g32, g32b, rtol=1e-9, atol=1e-12 * np.abs(g32).max())
+
+
+@pytest.mark.parametrize("kind", ["ellipsoid", "edge", "full", "scattered"])
+def test_backward_at_128_over_many_samples(gbg, kind):
+    """The backward kernel with resident anatomy (four lanes) where its division of
+    work can go wrong: more samples than lanes, of unequal length, so that a lane
+    takes several and ends while others run; seeds at the tissue's edge, whose
+    initial densities reach rows without a live cell; every cell tissue (the most
+    units a CTA owns, stencils across the periodic faces); tissue in short runs of
+    planes. Each gradient is the sample's own (the FP64 atomics' order: 1e-9) and
+    the FP64 states' to 1e-3, as above."""
+    n = 128
+    an = S.make_anatomy(n, seed=4)
+    w = np.random.default_rng(8).random((n, n, n))
+    c, sigma = (63.0, 64.5, 62.0), 1.0
+    if kind == "edge":
+        z, y, x = np.nonzero(an.brain)
+        top = np.argmax(z)
+        c, sigma = (float(x[top]), float(y[top]), float(z[top])), 2.5
+        assert not an.brain[int(c[2]) + 1:].any()
+    elif kind == "full":
+        an = dataclasses.replace(an, p_w=w, p_g=1.0 - w)
+        c = (126.4, 1.3, 0.6)
+    elif kind == "scattered":
+        t = np.ones((n, n, n))
+        t[::6] = 0.0
+        t[:, 3::7] = 0.0
+        t[:, :, 11::13] = 0.0
+        an = dataclasses.replace(an, p_w=t * w, p_g=t * (1.0 - w))
+        c = (63.0, 62.3, 63.1)
+    truth = np.clip(S.gaussian_ic(an, *c, peak=0.9, sigma=4.0), 0, 1)
+    obs = S.make_observations(truth, an, seed=3, centre_xyz=c, radius_vox=12.0)
+    rng = np.random.default_rng(5)
+    samples = [(0.0013 * rng.uniform(0.7, 1.6), rng.uniform(0.03, 0.15), *(np.array(c) + rng.uniform(-0.3, 0.3, 3)), t)
+               for t in (3.0, 26.0, 9.0, 1.0, 14.0, 30.0, 5.0, 18.0, 2.0, 22.0, 11.0)]
+    with _lib.Handle(n, "f32", max_samples=len(samples)) as h:
+        h.set_anatomy(an.p_w, an.p_g)
+        h.set_observations(obs.pet, obs.t1, obs.t2, obs.points, LIK)
+        kw = dict(ic_sigma=sigma, checkpoint_every=6)
+        l32, g32 = h.adjoint_grad(samples, -1.0, an.L, state="f32", **kw)
+        alone = [h.adjoint_grad([s], -1.0, an.L, state="f32", **kw) for s in samples]
+        l64, g64 = h.adjoint_grad(samples, -1.0, an.L, state="f64", **kw)
+    for s in range(len(samples)):
+        assert alone[s][0][0] == l32[s]
+        assert np.allclose(alone[s][1][0], g32[s], rtol=1e-9, atol=1e-12 * np.abs(g32[s]).max()), s
+    err, a, f = _rel_err(g32, g64, samples)
+    print("relative gradient error", err)
+    assert np.all(np.abs(g64).max(axis=1) > 0)
+    assert np.all(err < 1e-3), (err, a, f)
+    assert np.all(np.abs(l32 - l64) <= 1e-4 * np.abs(l64))
