@@ -10,11 +10,11 @@
 // thread that owns the cell.
 // A block is the part of a row pair's 16 planes 16 zb .. 16 zb + 15 that is
 // live. A thread adds its row's sensitivity products over a block in float, in
-// plane order, and widens them once: the sums of the tile kernel
-// (k_adj_back128), bit for bit. Blocks are dealt to the CTAs one by one, two
+// plane order, and widens them once. Blocks are dealt to the CTAs one by one, two
 // per CTA on an ellipsoidal brain, one per warp with 4 lanes.
-// 64 samples near the mode at 128^3: the backward kernels 34 ms instead of
-// 56, the whole call 52.4 ms instead of 86.3.
+// 64 samples near the mode at 128^3: the backward kernels 34 ms, the whole call
+// 52.4 ms, where a kernel that read halo tiles (8 rows x 16 planes, a block
+// barrier per plane) took 56 and 86.3 ms.
 #include <algorithm>
 #include <vector>
 

@@ -244,217 +244,6 @@ __global__ void k_adj_lam(int n, int S, const Real *__restrict__ phi, const Real
     }
 }
 
-// Fused backward step for the float path at n = 128 (k_adj_mu + k_adj_lam in
-// one pass over the state). A CTA of 10 warps owns a tile of 8 rows x TZ
-// planes of one sample. Warp w handles row y0 - 1 + w: marching z from the
-// tile's first plane - 1 to its last + 1 it forms, from phi_k, the pre-clamp
-// update v (the batched solver's operation sequence) and
-//   mu = [m != 0 and 0 <= v < 1] lambda_{k+1},
-// writes mu to a 3-plane shared ring and keeps its own row's last three planes
-// in registers; after one block barrier per plane, warps 1..8 form
-//   lambda_k = mu (1 + b (1 - 2 phi)) + a L(mu)
-// for the plane behind (rows y +- 1 from the ring) and accumulate
-// sum mu L(phi) and sum mu phi (1 - phi) for the tile's own cells.
-// Per sample and step: phi_k and lambda_{k+1} read once, lambda_k written once.
-namespace fb {
-constexpr int LR = 32, NN = 128, RY = 8, NW = RY + 2, TZ = 16;
-}
-
-__device__ __forceinline__ float4 ld4(const float *p, unsigned o) {
-    return __ldcg(reinterpret_cast<const float4 *>(p + o));
-}
-__device__ __forceinline__ float4 lg4(const float *p, unsigned o) {
-    return __ldg(reinterpret_cast<const float4 *>(p + o));
-}
-
-// live[t] = 1 when tile t of k_adj_back128 (rows y0 .. y0 + RY - 1, planes
-// tz0 .. tz0 + TZ - 1, every x) or its one-cell y/z halo holds a cell with
-// mask 1. On a tile without one mu is 0 on the tile and its halo, so
-// lambda_k = mu (1 + b (1 - 2 phi)) + a L(mu) and the tile's sensitivity
-// products are all zero. One block per tile.
-__global__ void k_adj_tile_live(const float *__restrict__ msk, unsigned char *__restrict__ live) {
-    using namespace fb;
-    constexpr int tiles_y = NN / RY;
-    const int t = blockIdx.x, y0 = (t % tiles_y) * RY, tz0 = (t / tiles_y) * TZ;
-    constexpr int cells = (RY + 2) * (TZ + 2) * NN;
-    int any = 0;
-    for (int c = threadIdx.x; c < cells && !any; c += blockDim.x) {
-        const int x = c % NN, r = c / NN, dy = r % (RY + 2), dz = r / (RY + 2);
-        const int y = (y0 - 1 + dy + NN) % NN, z = (tz0 - 1 + dz + NN) % NN;
-        any = msk[(size_t)NN * NN * z + (size_t)NN * y + x] != 0.0f;
-    }
-    any = __syncthreads_or(any);
-    if (threadIdx.x == 0) live[t] = any ? 1 : 0;
-}
-
-// live: k_adj_tile_live's flags. A sample's first two backward steps (k =
-// ns - 1, ns - 2) visit every tile, so that both lambda buffers hold the
-// zeros of the tiles without a live cell (the seed may be nonzero there);
-// later steps skip those tiles, which keeps every value but the sign of a
-// zero.
-__global__ void __launch_bounds__(320, 2)
-    k_adj_back128(int S, int k, const int *__restrict__ ns, const float *__restrict__ phi, float *__restrict__ lam0,
-                  float *__restrict__ lam1,
-                  const float *__restrict__ cxs, const float *__restrict__ cy, const float *__restrict__ cz,
-                  const double *__restrict__ a, const double *__restrict__ b,
-                  double *__restrict__ gA, double *__restrict__ gB, const unsigned char *__restrict__ live) {
-    using namespace fb;
-    constexpr unsigned plane = NN * NN, N = NN * NN * NN;
-    constexpr int tiles_y = NN / RY, tiles = tiles_y * (NN / TZ);
-    __shared__ __align__(16) float ring[3][NW][NN];
-    __shared__ double red[2][NW];
-    const int w = threadIdx.x / LR, li = threadIdx.x % LR, x0 = 4 * li;
-    const int left_l = (li + LR - 1) % LR, right_l = (li + 1) % LR;
-    for (int it = blockIdx.x; it < S * tiles; it += gridDim.x) {
-        const int s = it % S, t = it / S;
-        if (!live[t] && k + 3 <= ns[s]) continue;
-        const int y0 = (t % tiles_y) * RY, tz0 = (t / tiles_y) * TZ;
-        const float *f = phi + (size_t)s * N;
-        const bool odd = ((ns[s] - 1 - k) & 1) != 0;  // lambda of sample s is in lam1
-        const float *li_ = (odd ? lam1 : lam0) + (size_t)s * N;
-        float *lo = (odd ? lam0 : lam1) + (size_t)s * N;
-        const int y = (y0 - 1 + w + NN) % NN;
-        const int ym = y == 0 ? NN - 1 : y - 1, yp = y == NN - 1 ? 0 : y + 1;
-        const bool inner = w >= 1 && w <= RY;
-        const unsigned oy = (unsigned)(x0 + NN * y), oym = (unsigned)(x0 + NN * ym), oyp = (unsigned)(x0 + NN * yp);
-        if (a[s] < 0) {
-            // finished sample: lambda passes through unchanged
-            if (inner)
-                for (int dz = 0; dz < TZ; ++dz) {
-                    const unsigned o = oy + plane * (unsigned)(tz0 + dz);
-                    __stcg(reinterpret_cast<float4 *>(lo + o), ld4(li_, o));
-                }
-            continue;
-        }
-        const float as = (float)a[s], bs = (float)b[s];
-        auto wz = [](int z) { return z < 0 ? z + NN : (z >= NN ? z - NN : z); };
-        const int zstart = tz0 - 1;
-        float4 Pp = ld4(f, oy + plane * (unsigned)wz(zstart - 1));
-        float4 Pc = ld4(f, oy + plane * (unsigned)wz(zstart));
-        float4 CZp = lg4(cz, oy + plane * (unsigned)wz(zstart - 1));
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        float4 U2 = z4, U1 = z4, Pb = z4;  // mu at z-2, z-1; phi at z-1
-        // the previous plane's x/y/z face coefficients: the lambda stage's
-        // (plane z-1) are the mu stage's of one iteration before
-        float4 QX = z4, QY = z4, QZp = z4;
-        float pa_t = 0.0f, pb_t = 0.0f;
-        for (int st = 0; st < TZ + 2; ++st) {
-            const int zu = zstart + st;
-            const unsigned zo = plane * (unsigned)wz(zu), zno = plane * (unsigned)wz(zu + 1);
-            // ---- mu at (y, zu) ----
-            const float4 Pn = ld4(f, oy + zno);
-            const float4 PS = ld4(f, oym + zo), PN = ld4(f, oyp + zo);
-            const float4 CXS = lg4(cxs, oy + zo), CY = lg4(cy, oy + zo), CYm = lg4(cy, oym + zo);
-            const float4 CZ = lg4(cz, oy + zo);
-            const float4 LI = ld4(li_, oy + zo);
-            const float4 CX = make_float4(fabsf(CXS.x), fabsf(CXS.y), fabsf(CXS.z), fabsf(CXS.w));
-            float4 U;
-            {
-                const float left = __shfl_sync(0xffffffffu, Pc.w, left_l);
-                const float right = __shfl_sync(0xffffffffu, Pc.x, right_l);
-                const float cxl = __shfl_sync(0xffffffffu, CX.w, left_l);
-                const float pv[6] = {left, Pc.x, Pc.y, Pc.z, Pc.w, right};
-                const float cxa[5] = {cxl, CX.x, CX.y, CX.z, CX.w};
-                const float ps[4] = {PS.x, PS.y, PS.z, PS.w}, pn[4] = {PN.x, PN.y, PN.z, PN.w};
-                const float pp[4] = {Pp.x, Pp.y, Pp.z, Pp.w}, pq[4] = {Pn.x, Pn.y, Pn.z, Pn.w};
-                const float cy4[4] = {CY.x, CY.y, CY.z, CY.w}, cym4[4] = {CYm.x, CYm.y, CYm.z, CYm.w};
-                const float cz4[4] = {CZ.x, CZ.y, CZ.z, CZ.w}, czp4[4] = {CZp.x, CZp.y, CZp.z, CZp.w};
-                const bool on4[4] = {!signbit(CXS.x), !signbit(CXS.y), !signbit(CXS.z), !signbit(CXS.w)};
-                const float l4[4] = {LI.x, LI.y, LI.z, LI.w};
-                float u[4], pa = 0.0f, pb = 0.0f;
-                const bool own = inner && zu >= tz0 && zu < tz0 + TZ;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float f0 = pv[i + 1];
-                    float lap = cxa[i] * (pv[i] - f0);
-                    lap = fmaf(cxa[i + 1], pv[i + 2] - f0, lap);
-                    lap = fmaf(cym4[i], ps[i] - f0, lap);
-                    lap = fmaf(cy4[i], pn[i] - f0, lap);
-                    lap = fmaf(czp4[i], pp[i] - f0, lap);
-                    lap = fmaf(cz4[i], pq[i] - f0, lap);
-                    float v = fmaf(as, lap, f0);
-                    v = fmaf(bs * f0, 1.0f - f0, v);
-                    const float g = (on4[i] && v >= 0.0f && v < 1.0f) ? 1.0f : 0.0f;
-                    u[i] = g * l4[i];
-                    pa = fmaf(u[i], lap, pa);
-                    pb = fmaf(u[i] * f0, 1.0f - f0, pb);
-                }
-                // a thread's 4 x TZ cells summed in float, widened to double
-                // once per tile: the FP64 pipe on this GPU runs at a small
-                // fraction of the FP32 rate, so a per-plane double add cost
-                // more issue slots than the plane's whole stencil
-                if (own) {
-                    pa_t += pa;
-                    pb_t += pb;
-                }
-                U = make_float4(u[0], u[1], u[2], u[3]);
-            }
-            *reinterpret_cast<float4 *>(&ring[st % 3][w][x0]) = U;
-            __syncthreads();
-            // ---- lambda_k at (y, zu - 1) ----
-            if (st >= 2 && inner) {
-                const unsigned zc = plane * (unsigned)wz(zu - 1);
-                const float4 QYm = lg4(cy, oym + zc);
-                const float4 S1 = *reinterpret_cast<const float4 *>(&ring[(st - 1) % 3][w - 1][x0]);
-                const float4 N1 = *reinterpret_cast<const float4 *>(&ring[(st - 1) % 3][w + 1][x0]);
-                const float left = __shfl_sync(0xffffffffu, U1.w, left_l);
-                const float right = __shfl_sync(0xffffffffu, U1.x, right_l);
-                const float cxl = __shfl_sync(0xffffffffu, QX.w, left_l);
-                const float uv[6] = {left, U1.x, U1.y, U1.z, U1.w, right};
-                const float cxa[5] = {cxl, QX.x, QX.y, QX.z, QX.w};
-                const float us[4] = {S1.x, S1.y, S1.z, S1.w}, un[4] = {N1.x, N1.y, N1.z, N1.w};
-                const float up[4] = {U2.x, U2.y, U2.z, U2.w}, uq[4] = {U.x, U.y, U.z, U.w};
-                const float cy4[4] = {QY.x, QY.y, QY.z, QY.w}, cym4[4] = {QYm.x, QYm.y, QYm.z, QYm.w};
-                const float cz4[4] = {CZp.x, CZp.y, CZp.z, CZp.w}, czp4[4] = {QZp.x, QZp.y, QZp.z, QZp.w};
-                const float p4[4] = {Pb.x, Pb.y, Pb.z, Pb.w};
-                float o[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float u0 = uv[i + 1];
-                    float lu = cxa[i] * (uv[i] - u0);
-                    lu = fmaf(cxa[i + 1], uv[i + 2] - u0, lu);
-                    lu = fmaf(cym4[i], us[i] - u0, lu);
-                    lu = fmaf(cy4[i], un[i] - u0, lu);
-                    lu = fmaf(czp4[i], up[i] - u0, lu);
-                    lu = fmaf(cz4[i], uq[i] - u0, lu);
-                    o[i] = fmaf(as, lu, u0 * (1.0f + bs * (1.0f - 2.0f * p4[i])));
-                }
-                __stcg(reinterpret_cast<float4 *>(lo + oy + zc), make_float4(o[0], o[1], o[2], o[3]));
-            }
-            U2 = U1;
-            U1 = U;
-            Pb = Pc;
-            Pp = Pc;
-            Pc = Pn;
-            QX = CX;
-            QY = CY;
-            QZp = CZp;
-            CZp = CZ;
-        }
-        // per-sample sensitivities of this tile
-        double sa = (double)pa_t, sb = (double)pb_t;
-        for (int o = 16; o > 0; o >>= 1) {
-            sa += __shfl_down_sync(0xffffffffu, sa, o);
-            sb += __shfl_down_sync(0xffffffffu, sb, o);
-        }
-        if (li == 0) {
-            red[0][w] = sa;
-            red[1][w] = sb;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double ta = 0.0, tb = 0.0;
-            for (int j = 0; j < NW; ++j) {
-                ta += red[0][j];
-                tb += red[1][j];
-            }
-            atomicAdd(gA + s, ta);
-            atomicAdd(gB + s, tb);
-        }
-        __syncthreads();
-    }
-}
-
 // dlogL/du at the final state: PET list, then the T list (two launches keep
 // the order of additions fixed where a cell is in both lists)
 template <typename Real>
@@ -519,14 +308,11 @@ __device__ __forceinline__ float rim_lambda(const RimLambda &r, int n, int s, si
 
 // dlogL/dx0 = sum_c lambda0_c * phi0_c * (x_c - x0) / sigma^2 (same for y0, z0)
 template <typename Real>
-// lam1 non-null: lambda_0 of sample s is in lam1 when ns[s] is odd (the fused
-// backward kernel's ping-pong), else in lam
-__global__ void k_adj_ic_grad(int n, const gbg_sample *__restrict__ smp, double sigma, const Real *__restrict__ lam_,
-                              const Real *__restrict__ lam1, const int *__restrict__ ns, const Real *__restrict__ phi0,
+__global__ void k_adj_ic_grad(int n, const gbg_sample *__restrict__ smp, double sigma, const Real *__restrict__ lam,
+                              const Real *__restrict__ phi0,
                               double *__restrict__ gx, RimLambda rim, const int *__restrict__ box) {
     const size_t N = (size_t)n * n * n;
     const int s = blockIdx.y;
-    const Real *lam = (lam1 && (ns[s] & 1)) ? lam1 : lam_;
     double acc[3] = {0, 0, 0};
     // the rows of the initial support's box where one is given
     int y0 = 0, ny = n, z0 = 0, nz = n;
@@ -663,8 +449,7 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
                             (size_t)nmax * S * sizeof(double), (size_t)nmax * S * sizeof(double),
                             (size_t)nmax * S * sizeof(double), (size_t)nmax * S * sizeof(double),
                             3 * S * sizeof(double), S * sizeof(gbg_sample), S * sizeof(gbg_lik_result),
-                            S * sizeof(int), 2 * S * sizeof(SampleRec), S * sizeof(int), 1024,
-                            4 * S * sizeof(int)};
+                            2 * S * sizeof(SampleRec), S * sizeof(int), 4 * S * sizeof(int)};
     size_t total = 0;
     for (size_t b : sizes) total += bwork_align(b);
     if (h.adj_ws_bytes < total) {
@@ -678,10 +463,10 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
         }
         h.adj_ws_bytes = total;
     }
-    void *parts[18];
+    void *parts[16];
     {
         char *q = (char *)h.adj_ws;
-        for (int i = 0; i < 18; ++i) {
+        for (int i = 0; i < 16; ++i) {
             parts[i] = q;
             q += bwork_align(sizes[i]);
         }
@@ -700,11 +485,9 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
     double *gX = (double *)parts[10];
     gbg_sample *dsm = (gbg_sample *)parts[11];
     gbg_lik_result *dlik = (gbg_lik_result *)parts[12];
-    int *dns = (int *)parts[13];
-    SampleRec *drec = (SampleRec *)parts[14], *dsorted = drec + S;
-    int *drank = (int *)parts[15];
-    unsigned char *dlive = (unsigned char *)parts[16];
-    int *dbox = (int *)parts[17];  // initial-support boxes (the skipping population kernel)
+    SampleRec *drec = (SampleRec *)parts[13], *dsorted = drec + S;
+    int *drank = (int *)parts[14];
+    int *dbox = (int *)parts[15];  // initial-support boxes (the skipping population kernel)
     // per-step coefficients; a < 0 marks a finished sample
     std::vector<double> ha((size_t)nmax * S), hb((size_t)nmax * S);
     for (int k = 0; k < nmax; ++k)
@@ -736,7 +519,6 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
     ADJ_TRY(cudaMemcpyAsync(da, ha.data(), ha.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     ADJ_TRY(cudaMemcpyAsync(db, hb.data(), hb.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     ADJ_TRY(cudaMemcpyAsync(dsm, samples, S * sizeof(gbg_sample), cudaMemcpyHostToDevice, st));
-    ADJ_TRY(cudaMemcpyAsync(dns, ns.data(), S * sizeof(int), cudaMemcpyHostToDevice, st));
     ADJ_TRY(cudaMemsetAsync(gA, 0, (size_t)nmax * S * sizeof(double), st));
     ADJ_TRY(cudaMemsetAsync(gB, 0, (size_t)nmax * S * sizeof(double), st));
     ADJ_TRY(cudaMemsetAsync(gX, 0, 3 * S * sizeof(double), st));
@@ -846,29 +628,17 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
             if (loglik) loglik[s] = hl[s].total;
         return GBG_OK;
     }
-    // backward, segment by segment; the float path at n = 128 runs the fused
-    // kernel with lambda ping-ponging between lam and mu
-    // backward, segment by segment, each step over the samples running at it.
-    // The fused float kernel (n = 128) moves lambda between lam and mu, per
-    // sample: before step k sample s has taken ns[s] - 1 - k backward steps, so
-    // its lambda is in mu when that count is odd.
+    // backward, segment by segment, each step over the samples running at it
     const unsigned gcx = (unsigned)std::min<size_t>((N + 255) / 256, (size_t)h.num_sms * 4);
-    // Where the anatomy's units fit the CTAs' shared memory (any on a GB300)
-    // the lanes kernel takes its place: lambda in lam, mu in mu and fin, whose
-    // final states the seed has read.
+    // The float path at n = 128 on resident anatomy, where there are live units and
+    // they fit the CTAs' shared memory (any do on a GB300): lambda in lam, mu in mu
+    // and fin, whose final states the seed has read.
     const bool lanes = f32 && pop_fwd && adj_lanes_fit(h);
-    const bool fused = f32 && n == fb::NN && !lanes;
     if (lanes) {
         ADJ_TRY(cudaMemsetAsync(mu, 0, SN * sizeof(Real), st));
         ADJ_TRY(cudaMemsetAsync(fin, 0, SN * sizeof(Real), st));
     }
     std::vector<SampleRec> rrec(pop_fwd ? S : 0);
-    if (fused) {
-        constexpr int tiles = (fb::NN / fb::RY) * (fb::NN / fb::TZ);
-        static_assert(tiles <= 1024, "live flags");
-        k_adj_tile_live<<<tiles, 256, 0, st>>>((const float *)t.msk, dlive);
-        h.launches++;
-    }
     for (int sgm = (nmax - 1) / K; sgm >= 0; --sgm) {
         const int k0 = sgm * K, k1 = std::min(nmax, k0 + K);
         // recompute states k0+1 .. k1-1 into seg[1..]
@@ -919,28 +689,16 @@ int run_adjoint(Handle &h, const gbg_sample *samples, int S, const gbg_adjoint_o
         }
         for (int k = k1 - 1; k >= k0 && !lanes; --k) {
             const Real *phik = seg + (size_t)(k - k0) * S * N;
-            if (fused) {
-                constexpr int tiles = (fb::NN / fb::RY) * (fb::NN / fb::TZ);
-                const long items = (long)A[k] * tiles;
-                const unsigned grid = (unsigned)std::min<long>(items, (long)h.num_sms * 8);
-                k_adj_back128<<<grid, 320, 0, st>>>(A[k], k, dns, (const float *)phik, (float *)lam, (float *)mu,
-                                                    h.cxs, (const float *)t.cy, (const float *)t.cz,
-                                                    da + (size_t)k * S, db + (size_t)k * S,
-                                                    gA + (size_t)k * S, gB + (size_t)k * S, dlive);
-                h.launches++;
-            } else {
-                const dim3 gC(gcx, (unsigned)A[k]);
-                k_adj_mu<Real><<<gC, 256, 0, st>>>(n, phik, lam, mu, t, da + (size_t)k * S, db + (size_t)k * S,
-                                                   gA + (size_t)k * S, gB + (size_t)k * S);
-                k_adj_lam<Real><<<grid_cells(h, A[k]), 256, 0, st>>>(n, A[k], phik, mu, lam, t,
-                                                                     da + (size_t)k * S, db + (size_t)k * S);
-                h.launches += 2;
-            }
+            const dim3 gC(gcx, (unsigned)A[k]);
+            k_adj_mu<Real><<<gC, 256, 0, st>>>(n, phik, lam, mu, t, da + (size_t)k * S, db + (size_t)k * S,
+                                               gA + (size_t)k * S, gB + (size_t)k * S);
+            k_adj_lam<Real><<<grid_cells(h, A[k]), 256, 0, st>>>(n, A[k], phik, mu, lam, t,
+                                                                 da + (size_t)k * S, db + (size_t)k * S);
+            h.launches += 2;
         }
     }
     const RimLambda rim{lanes ? h.unit_live : nullptr, 2, (const float *)mu, h.cxs, h.cy, h.cz, drec};
-    k_adj_ic_grad<Real><<<dim3(gcx, (unsigned)S), 256, 0, st>>>(n, dsm, o.ic_sigma, lam, fused ? mu : nullptr, dns,
-                                                                ck, gX, rim, f32 ? dbox : nullptr);
+    k_adj_ic_grad<Real><<<dim3(gcx, (unsigned)S), 256, 0, st>>>(n, dsm, o.ic_sigma, lam, ck, gX, rim, f32 ? dbox : nullptr);
     h.launches++;
     ADJ_TRY(cudaGetLastError());
     std::vector<double> hA((size_t)nmax * S), hB((size_t)nmax * S), hX(3 * S);

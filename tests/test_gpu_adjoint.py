@@ -215,3 +215,21 @@ def test_backward_at_128_over_many_samples(gbg, kind):
     assert np.all(np.abs(g64).max(axis=1) > 0)
     assert np.all(err < 1e-3), (err, a, f)
     assert np.all(np.abs(l32 - l64) <= 1e-4 * np.abs(l64))
+
+
+def test_gradient_at_128_without_a_live_cell(gbg):
+    """Tissue of one plane: no cell has six neighbours in it, so the state is 0
+    after a step and the gradient 0, in the float path as with FP64 states."""
+    n = 128
+    an = S.make_anatomy(n, seed=4)
+    t = np.zeros((n, n, n))
+    t[60] = 0.5
+    an = dataclasses.replace(an, p_w=t, p_g=t.copy())
+    c = (63.0, 62.3, 60.0)
+    obs = S.make_observations(np.clip(S.gaussian_ic(an, *c, peak=0.9, sigma=4.0), 0, 1), an, seed=3, centre_xyz=c, radius_vox=9.0)
+    with _lib.Handle(n, "f32", max_samples=2) as h:
+        h.set_anatomy(an.p_w, an.p_g)
+        h.set_observations(obs.pet, obs.t1, obs.t2, obs.points, LIK)
+        out = [h.adjoint_grad([(0.0013, 0.05, *c, 9.0), (0.0017, 0.08, *c, 4.0)], -1.0, an.L, state=p) for p in ("f32", "f64")]
+    assert np.array_equal(out[0][0], out[1][0])
+    assert not out[0][1].any() and not out[1][1].any()
