@@ -369,6 +369,7 @@ int gbg_get_slopes(gbg_handle *hh, double *sRho, double *sD) {
         return GBG_ERR_STATE;
     }
     GBG_CUDA_TRY(cudaSetDevice(h.device));
+    if (int rc = gbg::finish_steps(h)) return rc;
     double *dst[2] = {sRho, sD};
     void *src[2] = {h.sr[h.cur], h.sd[h.cur]};
     for (int k = 0; k < 2; ++k) {
