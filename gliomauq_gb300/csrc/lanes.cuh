@@ -10,9 +10,9 @@ namespace lanes {
 
 constexpr int kWps = 4;                    // warps per scheduler: 16 warps of up to 128 registers
 constexpr int kThreads = 128 * kWps;
-// Samples a team has in flight. More lanes hide more of the barrier (4: 205
-// ms, 8: 164 ms on the 512-sample population); beyond 8 the states of a 128^3
-// population outgrow L2.
+// Samples a team has in flight. More lanes hide more of the barrier (4: 205 ms on
+// the 512-sample population, 8: 164 ms, both with rows moved between planes; in
+// register rings 8 take 150); beyond 8 the states of a 128^3 population outgrow L2.
 constexpr int kMaxLanes = 8;
 // a unit's table, one float4 per lane and slot: cxs (2 rows), cy (rows y-1,
 // y, y+1), cz (2 rows)
@@ -25,7 +25,7 @@ constexpr int kMaxUnits = 64;              // units a CTA can own
 constexpr int kTableBytes = 224 * 1024;
 static_assert(kMaxUnits * kUnitBytes <= kTableBytes, "the most units fit");
 // Planes loaded ahead: one plane's arithmetic does not cover an L2 load (170
-// ms), a third plane spills registers (207 ms).
+// against 164 ms, before the rings), a third plane spills registers (207 ms).
 constexpr int kAhead = 2;
 constexpr int kSyncStride = 32;            // words per lane of the barrier array
 

@@ -20,8 +20,8 @@
 //   * A warp marches its share of units up z, two rows in registers, with the
 //     loads of the next planes in flight.
 // What bounds it: a warp's latencies (16 warps an SM, of which a fifth waits at
-// a barrier; L1's data path is 62 % busy, 28 of the 58 passes a unit takes
-// through it are coefficients, and instructions issue in 44 % of the cycles),
+// a barrier; L1's data path is 67 % busy, 28 of the 58 passes a unit takes
+// through it are coefficients, and instructions issue in 47 % of the cycles),
 // and, for one sample, the barrier.
 // Per-cell operations and their order are those of march_tile_s (a difference
 // taken the other way round is its exact negative), so every population
