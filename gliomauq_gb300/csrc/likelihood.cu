@@ -6,10 +6,10 @@
 //             stepTi (or every voxel): sum of log Bernoulli(alpha(u)) with
 //             alpha = 0.5 + 0.5 sgn(u - uc) (1 - exp(-(u - uc)^2 / slope))
 //             (:136-160)
-// The lists are built once per observation set on the host. Per sample, each
-// CTA reduces a chunk of both lists with warp shuffles into three double
-// partial sums (scratch), and a second pass adds a sample's partials in a
-// fixed order, so results are deterministic. Accumulation is double (the
+// The lists are built once per observation set on the host. Per sample, a CTA or
+// a cluster of them reduces a chunk of both lists into three double partial sums
+// (scratch), and a second pass adds a sample's partials, all in a fixed order, so
+// results are deterministic. Accumulation is double (the
 // reference's is long double).
 //
 // Compiled with -fmad=false: (u - scale*PET)^2 and the exponent round as the
@@ -95,22 +95,10 @@ struct CoarseSource {
     __device__ __forceinline__ double ti(const LikArgs &a, int s, int i) const { return at(s, a.ti_idx[i]); }
 };
 
-// The terms are FP64 work (two exponentials and two logarithms an entry of the
-// T1/T2 list, 16 cycles per warp and SM for each operation), and a sample has
-// few entries: with a chunk to a CTA, six SMs of 152 took 112 us for a sample's
-// 10,000 entries. A cluster takes a chunk: a CTA forms the terms of every eighth
-// run of kLikThreads entries, and three of them add a sum each, an entry of
-// every run at a time in the order of the runs, then by warps: 19 us.
-__device__ __forceinline__ void cluster_meet() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// the three sums' terms of entry i
 template <class Src>
-__global__ void __cluster_dims__(kLikRuns, 1, 1) __launch_bounds__(kLikThreads) k_lik_partial(LikArgs a, Src src) {
-    const int s = blockIdx.y, chunk = blockIdx.x / kLikRuns, rank = blockIdx.x % kLikRuns;
-    __shared__ double term[3][kLikThreads];
-    __shared__ double red[kLikThreads / 32];
-    const int i = chunk * kLikChunk + rank * kLikThreads + threadIdx.x;
-    double t[3] = {0.0, 0.0, 0.0};
+__device__ __forceinline__ void entry_terms(const LikArgs &a, const Src &src, int s, int i, double (&t)[3]) {
+    t[0] = t[1] = t[2] = 0.0;
     if (i < a.n_pet) {
         const double u = src.pet(a, s, i);
         const double pv = a.pet_val[i];
@@ -122,30 +110,86 @@ __global__ void __cluster_dims__(kLikRuns, 1, 1) __launch_bounds__(kLikThreads) 
         t[1] = log_bernoulli(u, a.t1_val[i], a.t1_uc, a.is2);
         t[2] = log_bernoulli(u, a.t2_val[i], a.t2_uc, a.is2);
     }
-    for (int k = 0; k < 3; ++k) term[k][threadIdx.x] = t[k];
-    cluster_meet();
-    double sum = 0.0;
-    if (rank < 3) {
-        const unsigned own = (unsigned)__cvta_generic_to_shared(&term[rank][threadIdx.x]);
-#pragma unroll
-        for (int k = 0; k < kLikRuns; ++k) {
-            unsigned at;
-            double v;
-            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(own), "r"(k));
-            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(at) : "memory");
-            sum += v;
-        }
-    }
-    cluster_meet();  // the terms have been read
-    if (rank >= 3) return;
-    sum = warp_sum(sum);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+}
+
+// A chunk's sums: an entry of every run at a time in the order of the runs, then
+// over 32 neighbouring sums, then over those. The terms are FP64 work (two
+// exponentials and two logarithms an entry of the T1/T2 list, 16 cycles per warp
+// and SM for each operation), and a sample has few entries: with a chunk to a CTA,
+// six SMs of 152 take 112 us for a sample's 10,000 entries. Here a cluster takes
+// a chunk, a CTA of it 32 neighbouring entries of each run: 19 us. (With a run to
+// a CTA, the CTAs whose runs lie behind the T1/T2 list held their places for
+// nothing: 256 models of 1795 and 1292 entries 256 us, this way and with a chunk
+// to a CTA 200.)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+template <class Src>
+__global__ void __cluster_dims__(kLikRuns, 1, 1) __launch_bounds__(kLikThreads) k_lik_partial(LikArgs a, Src src) {
+    const int s = blockIdx.y, chunk = blockIdx.x / kLikRuns, rank = blockIdx.x % kLikRuns;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double term[3][kLikRuns][32];
+    __shared__ double red[3][kLikRuns];  // the first CTA's: every CTA's sums
+    static_assert(kLikThreads == 32 * kLikRuns, "a warp to a run, a CTA to 32 entries of each");
+    cluster_arrive();
+    double t[3];
+    entry_terms(a, src, s, chunk * kLikChunk + warp * kLikThreads + rank * 32 + lane, t);
+    for (int k = 0; k < 3; ++k) term[k][warp][lane] = t[k];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double total = 0.0;
-        for (int j = 0; j < kLikThreads / 32; ++j) total += red[j];
-        a.partials[((size_t)s * a.chunks + chunk) * 3 + rank] = total;
+    double sum = 0.0;
+    if (warp < 3) {
+        for (int k = 0; k < kLikRuns; ++k) sum += term[warp][k][lane];
+        sum = warp_sum(sum);
     }
+    cluster_wait();  // the first CTA runs
+    if (warp < 3 && lane == 0) {
+        unsigned at;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(&red[warp][rank])), "r"(0));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(sum) : "memory");
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (rank == 0 && threadIdx.x < 3) {
+        double total = 0.0;
+        for (int j = 0; j < kLikRuns; ++j) total += red[threadIdx.x][j];
+        a.partials[((size_t)s * a.chunks + chunk) * 3 + threadIdx.x] = total;
+    }
+}
+
+// the same sums with a chunk to a CTA
+template <class Src>
+__global__ void __launch_bounds__(kLikThreads) k_lik_partial_cta(LikArgs a, Src src) {
+    const int s = blockIdx.y, chunk = blockIdx.x, warp = threadIdx.x >> 5;
+    __shared__ double red[3][kLikThreads / 32];
+    double sum[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < kLikRuns; ++k) {
+        double t[3];
+        entry_terms(a, src, s, chunk * kLikChunk + k * kLikThreads + threadIdx.x, t);
+        for (int q = 0; q < 3; ++q) sum[q] += t[q];
+    }
+    for (int q = 0; q < 3; ++q) {
+        sum[q] = warp_sum(sum[q]);
+        if ((threadIdx.x & 31) == 0) red[q][warp] = sum[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double total = 0.0;
+        for (int j = 0; j < kLikThreads / 32; ++j) total += red[threadIdx.x][j];
+        a.partials[((size_t)s * a.chunks + chunk) * 3 + threadIdx.x] = total;
+    }
+}
+
+// Where the chunks alone fill the SMs six times over, a CTA each wastes nothing on
+// meetings: 1024 models of six chunks 3.73 against 3.87 ms, of one chunk 0.65
+// against 0.67. Below, clusters do not leave the last wave's SMs idle: 150 of six
+// 0.61 against 0.68 ms, 384 of one 0.278 against 0.290 (but 300 of one, which fill
+// two waves of CTAs, 0.229 against 0.205).
+template <class Src>
+void lik_partials(const LikArgs &a, const Src &src, int S, int num_sms, cudaStream_t st) {
+    if ((long)a.chunks * S > 6L * num_sms)
+        k_lik_partial_cta<<<dim3(a.chunks, S), kLikThreads, 0, st>>>(a, src);
+    else
+        k_lik_partial<<<dim3(a.chunks * kLikRuns, S), kLikThreads, 0, st>>>(a, src);
 }
 
 __global__ void k_lik_final(const double *__restrict__ partials, int chunks, int S, int n_pet,
@@ -207,7 +251,7 @@ int run_lik(Handle &h, const Src &src, int S, gbg_lik_result *out_device) {
     a.is2 = 1. / h.obs.slope;
     a.stride = h.N;
     a.partials = h.lik_partials;
-    k_lik_partial<<<dim3(chunks * kLikRuns, S), kLikThreads, 0, h.stream>>>(a, src);
+    lik_partials(a, src, S, h.num_sms, h.stream);
     k_lik_final<<<(S + 127) / 128, 128, 0, h.stream>>>(h.lik_partials, chunks, S, h.obs.n_pet,
                                                        h.obs.pet_sigma2, out_device);
     h.launches += 2;
@@ -446,7 +490,10 @@ extern "C" int gbg_loglik_noalloc(const float *phi_device, int n, const int *pet
     a.partials = scratch;
     PhiSource src{phi_device, phi_device, nullptr, nullptr};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    k_lik_partial<<<dim3(chunks * kLikRuns, 1), kLikThreads, 0, st>>>(a, src);
+    int dev = 0, sms = 0;
+    GBG_CUDA_TRY(cudaGetDevice(&dev));
+    GBG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    lik_partials(a, src, 1, sms, st);
     k_lik_final<<<1, 128, 0, st>>>(scratch, chunks, 1, (int)n_pet, p->pet_sigma2, out_device);
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;

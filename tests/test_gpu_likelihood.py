@@ -96,3 +96,27 @@ def test_loglik_at_the_edges_of_the_clusters(gbg, oracle_lib, n_pet, n_ti):
     assert r["n_pet"] == o["n_pet"] == n_pet
     for k in ("l_pet", "l_t1", "l_t2", "total"):
         assert abs(r[k] - o[k]) <= REL_TOL * max(1.0, abs(o[k])), (k, r[k], o[k])
+
+
+@pytest.mark.parametrize("n_pet,n_ti", [(200, 100), (2049, 300), (100, 1900)])
+def test_loglik_of_many_fields_is_each_fields_own(gbg, n_pet, n_ti):
+    """Few chunks of entries are reduced by clusters, many (over six per SM: 912 on
+    a GB300) by a CTA each, in the same order: counts around the change, bit for
+    bit the fields one by one."""
+    n = 32
+    rng = np.random.default_rng(n_ti)
+    pet = np.zeros(n ** 3)
+    pet[rng.choice(n ** 3, n_pet, replace=False)] = rng.uniform(0.1, 1.0, n_pet)
+    t1, t2 = ((rng.random((n, n, n)) > 0.5).astype(float) for _ in range(2))
+    c = rng.choice(n ** 3, n_ti, replace=False)
+    pts = np.stack([c % n, c // n % n, c // n ** 2], axis=1).astype(float)
+    chunks = -(-max(n_pet, n_ti) // 2048)
+    with _lib.Handle(n, "f32") as h:
+        h.set_anatomy(np.full((n, n, n), 0.5), np.full((n, n, n), 0.4))
+        h.set_observations(pet.reshape(n, n, n), t1, t2, pts, (0.0025, 1.0, 0.7, 0.25, 0.09), step_pet=1, step_ti=1, selective=True)
+        h.affine_set(rng.random((n, n, n)), rng.standard_normal((2, n, n, n)))
+        d = rng.uniform(-1, 1, (2000 // chunks, 2))
+        whole = h.affine_loglik(d)
+        for count in (911 // chunks, 912 // chunks, 913 // chunks + 1):
+            assert np.array_equal(h.affine_loglik(d[:count]), whole[:count]), count
+        assert np.array_equal(np.concatenate([h.affine_loglik(x) for x in d[:40]]), whole[:40])
