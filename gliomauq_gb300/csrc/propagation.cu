@@ -130,7 +130,7 @@ int launch_once(cudaStream_t st, int n, int S, const FieldSource &src, int refer
     const size_t N = (size_t)n * n * n, sm = (size_t)C * S * sizeof(float);
     const bool wide = N % 4 == 0 && ((uintptr_t)src.f0 | (uintptr_t)src.f1) % 16 == 0;
     auto *fn = wide ? k_field_stats_once<C, 4> : k_field_stats_once<C, 1>;
-    GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStatBytes));
+    if (sm > 48 * 1024) GBG_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStatBytes));
     fn<<<(unsigned)((N + C - 1) / C), kStatThreads, sm, st>>>(n, S, src, reference_rules, mean, var);
     GBG_CUDA_TRY(cudaGetLastError());
     return GBG_OK;
@@ -139,9 +139,12 @@ int launch_once(cudaStream_t st, int n, int S, const FieldSource &src, int refer
 int launch_stats(int num_sms, cudaStream_t st, int n, int S, const FieldSource &src, int reference_rules,
                  float *mean, float *var) {
     const size_t N = (size_t)n * n * n;
-    // the most cells whose values fit; more samples than fit with 32 cells
-    // (576) read the fields twice
-    const size_t fit = kStatBytes / ((size_t)S * sizeof(float));
+    // Below 16 samples the second read is from L1 and the CTAs of the other form
+    // have little to cover their copies with: 8 of 128^3 23.2 against 32.7 us, 12 31.4
+    // and 34.4, 16 34.8 and 36.5, 24 49.2 and 47.1 (all 2 us more from HBM, where 16
+    // take 43.0 and 38.9). Otherwise the most cells whose values fit; more samples
+    // than fit with 32 cells (576) read the fields twice.
+    const size_t fit = S < 16 ? 0 : kStatBytes / ((size_t)S * sizeof(float));
     if (fit >= 256) return launch_once<256>(st, n, S, src, reference_rules, mean, var);
     if (fit >= 128) return launch_once<128>(st, n, S, src, reference_rules, mean, var);
     if (fit >= 64) return launch_once<64>(st, n, S, src, reference_rules, mean, var);

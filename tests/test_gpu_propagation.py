@@ -102,3 +102,15 @@ def test_field_statistics_at_the_edges_of_the_cell_groups(gbg, oracle_lib, n, co
         om, ov = oracle_lib.propagation_stats(fields, reference_rules=rules)
         assert np.array_equal(mean, om)
         assert np.array_equal(var, ov)
+
+
+@pytest.mark.parametrize("n,count", [(20, 15), (20, 16), (33, 15), (33, 16), (40, 48), (40, 49)])
+def test_field_statistics_around_the_few_sample_form(gbg, oracle_lib, n, count):
+    """Below 16 samples the fields are read twice; up to 48 the values of 256 cells
+    fit the shared memory every launch has."""
+    fields = propagation_fields(n, count, n + count)
+    for rules in (True, False):
+        mean, var = _device_stats(gbg, fields, rules)
+        om, ov = oracle_lib.propagation_stats(fields, reference_rules=rules)
+        assert np.array_equal(mean, om)
+        assert np.array_equal(var, ov)
