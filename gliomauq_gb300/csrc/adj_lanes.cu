@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1) k_adj_lanes(AdjArgs p) {
 }
 
 // blocks with a live unit: rows | zb << 8 | live planes << 16, in order, and their
-// number behind them (one CTA of kBlocks threads)
-__global__ void __launch_bounds__(kBlocks) k_block_list(const unsigned char *__restrict__ live, int *__restrict__ list) {
+// number (one CTA of kBlocks threads)
+__global__ void __launch_bounds__(kBlocks) k_block_list(const unsigned char *__restrict__ live, int *__restrict__ list, int *__restrict__ count) {
     __shared__ int sums[kBlocks / 32];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, yp = t / (n / kBlockZ), zb = t % (n / kBlockZ);
     unsigned mask = 0;
@@ -276,34 +276,32 @@ __global__ void __launch_bounds__(kBlocks) k_block_list(const unsigned char *__r
     int before = 0;
     for (int k = 0; k < warp; ++k) before += sums[k];
     if (mask) list[before + __popc(m & ((1u << lane) - 1u))] = yp | zb << 8 | (int)(mask << 16);
-    if (t == kBlocks - 1) list[kBlocks] = before + __popc(m);
+    if (t == kBlocks - 1) *count = before + __popc(m);
 }
 
 }  // namespace
 
-int adj_lanes_set_anatomy(Handle &h) {
-    if (h.n != n || !reserve_device({{(void **)&h.block_list, (kBlocks + 1) * sizeof(int)}})) return GBG_OK;
-    k_block_list<<<1, kBlocks, 0, h.stream>>>(h.unit_live, h.block_list);
+bool adj_lanes_list(Handle &h, int *count) {
+    if (h.n != n || !reserve_device({{(void **)&h.block_list, kBlocks * sizeof(int)}})) return false;
+    k_block_list<<<1, kBlocks, 0, h.stream>>>(h.unit_live, h.block_list, count);
     h.launches++;
-    GBG_CUDA_TRY(cudaGetLastError());
-    GBG_CUDA_TRY(cudaMemcpyAsync(&h.blocks, h.block_list + kBlocks, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
-    return GBG_OK;
+    return true;
 }
 
 bool adj_lanes_fit(const Handle &h) {
-    return h.n == n && h.block_list && h.blocks > 0 && (h.blocks + h.num_sms - 1) / h.num_sms <= kMaxBlocks;
+    return h.n == n && h.block_list && h.units[3] > 0 && (h.units[3] + h.num_sms - 1) / h.num_sms <= kMaxBlocks;
 }
 
 int adj_lanes_segment(Handle &h, int S, int k0, int k1, const SampleRec *recs, SampleRec *drec, const float *seg, size_t slot,
                       float *lam, float *mu0, float *mu1, int strideS, double *gA, double *gB) {
     AdjArgs a;
     a.S = S;
-    a.T = std::min(h.num_sms, h.blocks);
+    a.T = std::min(h.num_sms, h.units[3]);
     a.lanes = std::min(kAdjLanes, S);
     a.warps = kAdjWarps / a.lanes;
     a.k0 = k0;
     a.k1 = k1;
-    a.nblocks = h.blocks;
+    a.nblocks = h.units[3];
     a.strideS = strideS;
     a.slot = slot;
     a.seg = seg;
@@ -319,7 +317,7 @@ int adj_lanes_segment(Handle &h, int S, int k0, int k1, const SampleRec *recs, S
     a.status = h.dev_status;
     a.gA = gA;
     a.gB = gB;
-    const size_t smem = (size_t)((h.blocks + a.T - 1) / a.T) * kBlockZ * kUnitBytes;
+    const size_t smem = (size_t)((h.units[3] + a.T - 1) / a.T) * kBlockZ * kUnitBytes;
     GBG_CUDA_TRY(cudaMemcpyAsync(drec, recs, (size_t)S * sizeof(SampleRec), cudaMemcpyHostToDevice, h.stream));
     GBG_CUDA_TRY(cudaFuncSetAttribute(k_adj_lanes, cudaFuncAttributeMaxDynamicSharedMemorySize, kTableBytes));
     GBG_CUDA_TRY(cudaMemsetAsync(h.lane_sync, 0, (size_t)(a.lanes + 1) * kSyncStride * sizeof(unsigned), h.stream));

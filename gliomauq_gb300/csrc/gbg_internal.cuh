@@ -190,14 +190,13 @@ struct Handle {
 
     // units of the resident-anatomy kernels (rd_lanes.cu): which hold a live
     // cell (1) or border one that does (2), the lists of the first, the second
-    // and of all but the first with their lengths, and the kernels' barrier
-    // words; for n = 128 the adjoint's blocks of 16 units with a live one
-    // (adj_lanes.cu) and their number
+    // and of all but the first, and the kernels' barrier words; for n = 128 the
+    // adjoint's blocks of 16 units with a live one (adj_lanes.cu); the four
+    // lists' lengths
     unsigned char *unit_live = nullptr;
     int *unit_list = nullptr;
-    int units[3] = {0, 0, 0};
+    int units[4] = {0, 0, 0, 0};
     int *block_list = nullptr;
-    int blocks = 0;
     int lane_clusters = -1;  // clusters of the cluster teams' size that run side by side (not asked yet: -1)
     unsigned *lane_sync = nullptr;
 
@@ -335,7 +334,8 @@ bool lanes_fit(const Handle &h, int S);
 int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, int S, const int *box, int grow0, size_t slot = 0,
                  bool fill_all = true);
 // ---- adj_lanes.cu ----
-int adj_lanes_set_anatomy(Handle &h);
+// lists the blocks with a live unit, their number to *count (device); false: none here
+bool adj_lanes_list(Handle &h, int *count);
 bool adj_lanes_fit(const Handle &h);
 // backward steps of the segment [k0, k1) at n = 128 (float states): lam is
 // lambda at the segment's end and becomes lambda at its start on the live

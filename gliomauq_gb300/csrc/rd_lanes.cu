@@ -326,10 +326,12 @@ __global__ void k_unit_rim(int n, int units, unsigned char *__restrict__ live) {
         live[u] = 2;
 }
 
-// indices of the units with live == want (want < 0: with live != 1) in increasing
-// order, and their count (one CTA)
-__global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned char *__restrict__ live, int want, int *__restrict__ list,
-                                                     int *__restrict__ count) {
+// Three lists of units in increasing order, a CTA each, and their lengths behind
+// them: the live ones, those without a live cell that a live unit's stencil reads,
+// all without a live cell.
+__global__ void __launch_bounds__(1024) k_unit_lists(int units, const unsigned char *__restrict__ live, int *__restrict__ lists) {
+    const int which = blockIdx.x;
+    int *list = lists + which * units;
     __shared__ int sums[32];
     __shared__ int total;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned ch
     __syncthreads();
     for (int base = 0; base < units; base += 1024) {
         const int i = base + threadIdx.x;
-        const int f = i < units && (want < 0 ? live[i] != 1 : live[i] == want);
+        const int f = i < units && (which == 2 ? live[i] != 1 : live[i] == which + 1);
         const unsigned m = __ballot_sync(0xffffffffu, f);
         if (lane == 0) sums[warp] = __popc(m);
         __syncthreads();
@@ -349,7 +351,7 @@ __global__ void __launch_bounds__(1024) k_unit_list(int units, const unsigned ch
             for (int k = 0; k < 32; ++k) total += sums[k];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *count = total;
+    if (threadIdx.x == 0) lists[3 * units + which] = total;
 }
 
 int unit_rows(int n) { return 2 * (32 / (n / 4)); }
@@ -361,7 +363,7 @@ int lanes_set_anatomy(Handle &h) {
     const int nu = units_of(h.n);
     // without room for the lists every call takes the tile march (lanes_fit)
     if (!reserve_device({{(void **)&h.unit_live, (size_t)nu},
-                         {(void **)&h.unit_list, 3 * (nu + 1) * sizeof(int)},
+                         {(void **)&h.unit_list, (3 * nu + 4) * sizeof(int)},
                          {(void **)&h.lane_sync, (size_t)(h.num_sms * kMaxLanes + 1) * kSyncStride * sizeof(unsigned)}}))
         return GBG_OK;
     if (h.n == 32 && h.lane_clusters < 0) {
@@ -387,16 +389,13 @@ int lanes_set_anatomy(Handle &h) {
     }
     k_unit_live<<<nu, 128, 0, h.stream>>>(h.n, unit_rows(h.n), h.pw, h.pg, h.unit_live);
     k_unit_rim<<<(nu + 127) / 128, 128, 0, h.stream>>>(h.n, nu, h.unit_live);
-    // live units | units without a live cell that a live unit's stencil reads |
-    // all units without a live cell, each list with its length behind it
-    for (int l = 0; l < 3; ++l)
-        k_unit_list<<<1, 1024, 0, h.stream>>>(nu, h.unit_live, l == 0 ? 1 : (l == 1 ? 2 : -1), h.unit_list + l * (nu + 1),
-                                              h.unit_list + l * (nu + 1) + nu);
-    h.launches += 5;
+    k_unit_lists<<<3, 1024, 0, h.stream>>>(nu, h.unit_live, h.unit_list);
+    h.launches += 3;
     GBG_CUDA_TRY(cudaGetLastError());
-    for (int l = 0; l < 3; ++l)
-        GBG_CUDA_TRY(cudaMemcpyAsync(&h.units[l], h.unit_list + l * (nu + 1) + nu, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
-    return adj_lanes_set_anatomy(h);
+    const bool blocks = adj_lanes_list(h, h.unit_list + 3 * nu + 3);
+    // one copy of the lengths: each waits for the stream
+    GBG_CUDA_TRY(cudaMemcpyAsync(h.units, h.unit_list + 3 * nu, (blocks ? 4 : 3) * sizeof(int), cudaMemcpyDeviceToHost, h.stream));
+    return GBG_OK;
 }
 
 // Teams and lanes for S samples. A CTA holds at most 28 units where the chip
@@ -452,7 +451,7 @@ int lanes_launch(Handle &h, float *buf0, float *buf1, const SampleRec *sorted, i
     a.cz = h.cz;
     a.rec = sorted;
     a.list = h.unit_list;
-    a.fill = h.unit_list + (fill_all ? 2 : 1) * (a.units + 1);
+    a.fill = h.unit_list + (fill_all ? 2 : 1) * a.units;
     a.nfill = h.units[fill_all ? 2 : 1];
     a.slot = slot;
     a.live = h.unit_live;
