@@ -136,6 +136,7 @@ struct Handle {
     int *exact_list = nullptr;
     double *exact_dsum = nullptr;
     bool exact_listed = false;
+    long exact_fulls = 0;  // steps over every cell with the present tables
     bool exact_waited = false;    // a launch whose CTAs wait for one another is not yet checked (finish_steps)
     bool exact_in_graph = false;  // a captured graph has such a launch: it may have run at any time
     int exact_full = 0;

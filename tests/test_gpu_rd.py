@@ -211,3 +211,26 @@ def test_exact_steps_from_densities_below_zero_with_decay(gbg, oracle_lib, prec,
             assert np.array_equal(h.get_phi(), ref), k
             rho = -rho
     assert ref.max() > 0
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32ref"])
+@pytest.mark.parametrize("n", [13, 48])
+def test_exact_steps_with_other_coefficients_in_each_call(gbg, oracle_lib, prec, n):
+    """Whether a call makes the list depends on the steps ahead of it, on those
+    taken and on the grid (from 200,000 cell-steps, two at 48^3, or five steps on):
+    calls of one to eight steps, some with the coefficients of the one before."""
+    rng = np.random.default_rng(n)
+    t = (rng.random((n, n, n)) < 0.9).astype(float)
+    w = rng.random((n, n, n))
+    pw, pg = t * w, t * (1.0 - w)
+    phi = rng.uniform(0.0, 1.0, (n, n, n)).astype(np.float32).astype(np.float64)
+    with _lib.Handle(n, prec) as h:
+        h.set_anatomy(pw, pg)
+        h.set_phi(phi)
+        ref = phi
+        for k, scale in ((1, 1.0), (2, 0.9), (2, 0.9), (1, 0.9), (1, 0.9), (3, 1.0), (4, 0.8), (1, 0.8), (5, 0.9), (6, 1.0), (8, 0.7)):
+            dt, dw, dg = S.reference_dt(n, 0.0013, n * 0.1, f32=prec == "f32ref")
+            dw = float(np.float32(dw * scale)) if prec == "f32ref" else dw * scale
+            h.rd_step(dw, dg, 0.025, dt, k)
+            ref = oracle_lib.rd_solve(pw, pg, ref, dw, dg, 0.025, dt, k, prec).astype(np.float64)
+            assert np.array_equal(h.get_phi(), ref), (k, scale)
