@@ -668,10 +668,12 @@ void amr_free(Handle &h) {
         if (q) cudaFree(q);
 }
 
-// A caller's doubles to the float modes' fields, staged by halves in the remap's
-// targets (the size of a field in floats each), whose contents nothing keeps; the
-// tables stay, for captured graphs of steps. Converted on the host, a field of
-// 512 blocks took 1.5 ms; this way 1.1, most of it the copy from pageable memory.
+// A caller's doubles to the float modes' fields, staged in the face tables, which
+// a new grid makes stale; but by halves in the remap's targets (the size of a
+// field in floats each), whose contents nothing keeps, where a captured graph of
+// steps may read the tables again (three more copies, 47 us). Converted on the
+// host, a field of 512 blocks took 1.5 ms; this way 1.1, most of it the copy from
+// pageable memory.
 __global__ void k_narrow(long n, const double *__restrict__ in, float *__restrict__ out) {
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) out[i] = (float)in[i];
 }
@@ -688,6 +690,7 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
     }
     GBG_CUDA_TRY(cudaMemcpyAsync(h.amr.level, lv.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h.stream));
     GBG_CUDA_TRY(cudaMemcpyAsync(h.amr.bidx, bi.data(), bi.size() * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+    h.amr.tables_valid = false;
     const double *src[3] = {pw, pg, phi};
     void *dst[3] = {h.amr.pw, h.amr.pg, h.amr.phi[0]};
     if (h.prec == GBG_PREC_F64) {
@@ -696,14 +699,15 @@ int amr_set_grid(Handle &h, int nb, const gbg_block *blocks, const double *pw, c
         GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     } else {
         for (int k = 0; k < 3; ++k) {
-            for (int half = 0; half < 2; ++half) {
-                double *staged = (double *)(half ? h.amr.pg2 : h.amr.pw2);
-                const size_t m = n / 2;  // blocks have an even number of cells
-                GBG_CUDA_TRY(cudaMemcpyAsync(staged, src[k] + half * m, m * sizeof(double), cudaMemcpyHostToDevice, h.stream));
-                k_narrow<<<grid_blocks(h, (long)m), 256, 0, h.stream>>>((long)m, staged, (float *)dst[k] + half * m);
+            const int parts = h.amr.in_graph ? 2 : 1;
+            const size_t m = n / parts;  // blocks have an even number of cells
+            for (int p = 0; p < parts; ++p) {
+                double *staged = !h.amr.in_graph ? h.amr.df + k * n : (double *)(p ? h.amr.pg2 : h.amr.pw2);
+                GBG_CUDA_TRY(cudaMemcpyAsync(staged, src[k] + p * m, m * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+                k_narrow<<<grid_blocks(h, (long)m), 256, 0, h.stream>>>((long)m, staged, (float *)dst[k] + p * m);
+                h.launches++;
             }
         }
-        h.launches += 6;
         GBG_CUDA_TRY(cudaGetLastError());
         GBG_CUDA_TRY(cudaStreamSynchronize(h.stream));
     }
@@ -800,6 +804,9 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
     const long cells = (long)h.amr.nb * BC, ng = (long)h.amr.nb * NG;
     const int gc = grid_blocks(h, cells), gg = grid_blocks(h, ng);
     const bool f64 = h.prec == GBG_PREC_F64;
+    bool capturing;
+    if (int rc = stream_capturing(h, &capturing)) return rc;
+    h.amr.in_graph |= capturing;
     if (h.prec == GBG_PREC_F32) {
         // fast mode: unit coefficients for the ratio Dg/Dw (rounded to float, as
         // the uniform fast path does), the 7-float table in the df storage
@@ -873,8 +880,6 @@ int amr_steps(Handle &h, double Dw, double Dg, double rho, double dt, long nstep
         h.amr.full_steps = kAnyState;
         h.amr.listed = false;
     };
-    bool capturing;
-    if (int rc = stream_capturing(h, &capturing)) return rc;
     if (capturing) forget();
     auto step = [&](auto real, const void *in, void *out) {
         using Real = decltype(real);

@@ -88,6 +88,7 @@ struct AmrState {
     double *dsum = nullptr;
     bool listed = false;
     int full_steps = 0;
+    bool in_graph = false;  // steps were captured into a caller's graph
     bool ghosts_valid = false, tables_valid = false;
     double tab_Dw = -1, tab_Dg = -1;
     std::vector<gbg_block> hblocks;  // host copy of the blocks, in the device order
